@@ -364,16 +364,27 @@ NearTiles near_tiles(const Tree& t, const NearList& nl, int esz) {
   return out;
 }
 
-// Columns one panel item takes before its panel chunk is split over items:
-// far panels above 32 rows are many (one per node and level), near ones are
-// few (leaves above 32 points) and get more, smaller items.
-constexpr int kPanelCols = 256;
-// factor bytes per leaf-panel item, about (HODLR_TUNE_SMALL_ITEM_BYTES overrides it for tuning runs)
+// Factor bytes one warp's item streams before its panel (or block of V) is
+// split over further items, whose partial sums a fix-up adds in order.
+// Large operators have many more items than the GPU has warps, and long items
+// keep the partial sums few: the upper limits below.  In a small operator the
+// longest item is the launch's duration (a warp streams a 128 KB item in
+// 50-190 us, 20x the whole operator's share), so there the phase's bytes are
+// spread over about kSpreadItems items, down to the lower limits, where an
+// item's start-up costs what its bytes do.
+constexpr int64_t kPanelItemBytes = 128 * 1024;  // far panels above 32 rows
+// leaf panels (HODLR_TUNE_SMALL_ITEM_BYTES overrides it for tuning runs)
 #ifndef HODLR_TUNE_SMALL_ITEM_BYTES
 #define HODLR_TUNE_SMALL_ITEM_BYTES (48 * 1024)
 #endif
 constexpr int64_t kSmallItemBytes = HODLR_TUNE_SMALL_ITEM_BYTES;
-constexpr int kNearPanelCols = 48;
+constexpr int64_t kNearItemBytes = 24 * 1024;    // near panels above 32 rows: few, so shorter
+constexpr int64_t kSpreadItems = 152 * 48;  // 48 warps per SM
+constexpr int64_t kMinItemBytes = 8 * 1024;
+
+int64_t item_bytes(int64_t total, int64_t lo, int64_t hi) {
+  return std::min(hi, std::max(lo, (total + kSpreadItems - 1) / kSpreadItems));
+}
 
 // Runs of consecutive segments [begin, end) with about `max_cols` columns each.
 std::vector<std::pair<int32_t, int32_t>> column_groups(const std::vector<Seg>& segs, int64_t begin, int64_t end,
@@ -392,6 +403,31 @@ std::vector<std::pair<int32_t, int32_t>> column_groups(const std::vector<Seg>& s
   return groups;
 }
 
+// Columns of a panel (rows rows per column at most) that make up `bytes`.
+int panel_cols(int64_t bytes, int64_t rows, int esz) {
+  return int(std::max<int64_t>(1, std::min<int64_t>(bytes / (rows * esz), 1 << 28)));
+}
+
+// Items of a panel of at most 32 rows: one warp for the panel, or for each run
+// of about `bytes` of its factors when it has more (partial rows added by the
+// fix-up kernel).
+void add_small_items(const std::vector<Seg>& segs, const Panel& p, int np, int64_t bytes, int esz,
+                     std::vector<Item>& small, std::vector<PanelFix>& pfix, int64_t& nypart) {
+  const std::vector<std::pair<int32_t, int32_t>> groups =
+      column_groups(segs, p.seg_begin, p.seg_end, std::max(64, panel_cols(bytes, p.m, esz)));
+  if (groups.size() == 1) {
+    small.push_back({np, 0, int32_t(p.seg_begin), int32_t(p.seg_end), -1});
+    return;
+  }
+  pfix.push_back({np, 0, int32_t(nypart), int32_t(groups.size())});
+  for (auto& g : groups) small.push_back({np, 0, g.first, g.second, int32_t(nypart++)});
+}
+
+// Whether an operator's items are spread as item_bytes says: all but the
+// members of an FP32-vector batch, whose merged plan has the items of many
+// instances and 32 right-hand sides per partial sum.
+bool spread_items(const hodlr_op* op) { return !(op->keep_host_plans && op->p.precision == HODLR_PREC_MIXED); }
+
 void build_near_plan(hodlr_op* op, const NearTiles& nt, const void* base, Prec a, Plan& plan, cudaStream_t st) {
   const Tree& t = op->tree;
   const int L = t.levels - 1;
@@ -401,6 +437,11 @@ void build_near_plan(hodlr_op* op, const NearTiles& nt, const void* base, Prec a
   std::vector<PanelFix> pfix;
   int64_t nypart = 0;
   const size_t esz = a == Prec::kD ? 8 : 4;
+  const bool spread = spread_items(op);
+  int64_t total = 0;
+  for (const TileDesc& d : nt.tiles) total += int64_t(d.m) * d.n * int64_t(esz);
+  const int64_t small_bytes = spread ? item_bytes(total, kMinItemBytes, int64_t(1) << 40) : int64_t(1) << 40;
+  const int64_t big_bytes = spread ? item_bytes(total, kMinItemBytes, kNearItemBytes) : kNearItemBytes;
   size_t q = 0;
   for (int64_t k = 0; k + 1 < int64_t(op->near.leaf_ptr.size()); k++) {
     const int64_t b = op->near.leaf_ptr[size_t(k)], e = op->near.leaf_ptr[size_t(k + 1)];
@@ -425,12 +466,13 @@ void build_near_plan(hodlr_op* op, const NearTiles& nt, const void* base, Prec a
     const int np = int(panels.size());
     panels.push_back(p);
     if (p.m <= 32) {
-      small.push_back({np, 0, int32_t(p.seg_begin), int32_t(p.seg_end), -1});
+      add_small_items(segs, p, np, small_bytes, int(esz), small, pfix, nypart);
     } else {
-      // as for far panels: runs of about kPanelCols columns per item, partial
-      // row blocks added by the fix-up kernel
-      const std::vector<std::pair<int32_t, int32_t>> groups = column_groups(segs, p.seg_begin, p.seg_end, kNearPanelCols);
+      // as for far panels: runs of columns, partial row blocks added by the
+      // fix-up kernel
       const int rows = rows_per_item(a);
+      const std::vector<std::pair<int32_t, int32_t>> groups =
+          column_groups(segs, p.seg_begin, p.seg_end, panel_cols(big_bytes, rows, int(esz)));
       for (int c = 0; c < int((p.m + rows - 1) / rows); c++) {
         if (groups.size() == 1) {
           big.push_back({np, c, groups[0].first, groups[0].second, -1});
@@ -475,6 +517,17 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
   int64_t zoff = op->n;
   // FP32 / BF16 after the relayout: z = V^T x per chunk of source-node columns
   const bool chunks = a != Prec::kD && !op->vchunks.empty();
+  int64_t utotal = 0, vtotal = 0;  // bytes of the two phases
+  for (size_t q = 0; q < op->far.size(); q++) {
+    const int l = op->far[q].level;
+    const int64_t m = t.count[size_t(t.gid(l, op->far[q].t))], ns = t.count[size_t(t.gid(l, op->far[q].s))];
+    utotal += m * (op->dense[q] ? ns : op->rank[q]) * prec_size(a);
+    if (!op->dense[q]) vtotal += ns * op->rank[q] * prec_size(a);
+  }
+  const bool spread = spread_items(op);
+  const int64_t big_bytes = spread ? item_bytes(utotal, kMinItemBytes, kPanelItemBytes) : kPanelItemBytes;
+  const int64_t small_bytes = spread ? item_bytes(utotal, kMinItemBytes, kSmallItemBytes) : kSmallItemBytes;
+  const int64_t z_bytes = spread ? item_bytes(vtotal, kMinItemBytes, kZItemBytes) : kZItemBytes;
   size_t b = 0;
   while (b < op->far.size()) {
     const int l = op->far[b].level;
@@ -530,21 +583,13 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
       const int np = int(panels.size());
       panels.push_back(p);
       if (p.m <= 32) {
-        // one warp per leaf panel, or per run of about kSmallItemBytes of its
-        // factors when it has more (partial rows added by the fix-up kernel):
         // a few panels with very long interaction lists would otherwise keep
         // single warps busy long after the rest
-        const int max_cols = int(std::max<int64_t>(64, kSmallItemBytes / (int64_t(p.m) * prec_size(a))));
-        const std::vector<std::pair<int32_t, int32_t>> groups = column_groups(segs, p.seg_begin, p.seg_end, max_cols);
-        if (groups.size() == 1) {
-          small.push_back({np, 0, int32_t(p.seg_begin), int32_t(p.seg_end), -1});
-        } else {
-          pfix.push_back({np, 0, int32_t(nypart), int32_t(groups.size())});
-          for (auto& g : groups) small.push_back({np, 0, g.first, g.second, int32_t(nypart++)});
-        }
+        add_small_items(segs, p, np, small_bytes, prec_size(a), small, pfix, nypart);
       } else {
-        const std::vector<std::pair<int32_t, int32_t>> groups = column_groups(segs, p.seg_begin, p.seg_end, kPanelCols);
         const int rows = rows_per_item(a);
+        const std::vector<std::pair<int32_t, int32_t>> groups =
+            column_groups(segs, p.seg_begin, p.seg_end, panel_cols(big_bytes, rows, prec_size(a)));
         const int chunks = int((p.m + rows - 1) / rows);
         for (int c = 0; c < chunks; c++) {
           if (groups.size() == 1) {
@@ -587,7 +632,7 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
   plan.nsmall_far = int(small.size());
   plan.nbig_far = int(big.size());
   // V^T x items: up to 32 sixteen-byte loads of columns by a run of rows of
-  // about kZItemBytes; blocks with more rows split into partial sums
+  // about z_bytes; blocks with more rows split into partial sums
   std::vector<ZItem> zit;
   std::vector<ZFix> zfix;
   int64_t nzpart = 0;
@@ -598,7 +643,7 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
     const int rp = int(vpad(r, esz));
     for (int k0 = 0; k0 < rp; k0 += cmax) {
       const int nk = std::min(cmax, rp - k0);
-      const int rows = std::max(1, kZItemBytes / (nk * esz));
+      const int rows = int(std::max<int64_t>(1, z_bytes / (nk * esz)));
       const int groups = (n + rows - 1) / rows;
       if (groups == 1) {
         zit.push_back({int32_t(q), k0, nk, 0, n, -1, 0, 0});

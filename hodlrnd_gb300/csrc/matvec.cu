@@ -486,6 +486,34 @@ __global__ void __launch_bounds__(kZWarps * 32) zgemv_kernel(const ZBlock* __res
   z_finish<TA, TACC>(acc, P, lane, it, Z, z, zpart);
 }
 
+// Sum of `count` partial sums, `stride` apart, in an order that depends on
+// count alone: one after another up to 8 of them; more (small operators, whose
+// work is cut into many short items) go to 8 running sums, so that 8 loads are
+// in flight instead of one load latency per part.
+template <typename T>
+__device__ __forceinline__ T sum_parts(const T* __restrict__ p, int count, int64_t stride) {
+  T acc = T(0);
+  if (count <= 8) {
+    for (int q = 0; q < count; q++) acc += p[q * stride];
+    return acc;
+  }
+  T a[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) a[k] = p[k * stride];
+  int q = 8;
+  for (; q + 8 <= count; q += 8) {
+    T v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = p[(q + k) * stride];
+#pragma unroll
+    for (int k = 0; k < 8; k++) a[k] += v[k];
+  }
+#pragma unroll
+  for (int k = 0; k < 7; k++)
+    if (q + k < count) a[k] += p[(q + k) * stride];
+  return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+}
+
 template <typename TACC>
 __global__ void zfix_kernel(const ZFix* __restrict__ fix, int nfix, const typename IO<TACC>::TY* __restrict__ zpart,
                             typename IO<TACC>::TI* in, int64_t ld_in) {
@@ -493,8 +521,7 @@ __global__ void zfix_kernel(const ZFix* __restrict__ fix, int nfix, const typena
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nfix) return;
   const ZFix F = fix[f];
-  TY acc = TY(0);
-  for (int q = 0; q < F.count; q++) acc += zpart[F.part + q * kZPart];
+  const TY acc = sum_parts(zpart + F.part, F.count, kZPart);
   in[blockIdx.y * ld_in + F.zpos] = IO<TACC>::from_double(double(acc));
 }
 
@@ -1359,9 +1386,7 @@ __global__ void __launch_bounds__(256) panel_fix_kernel(const Panel* __restrict_
   const Panel P = panels[F.panel];
   const int i = F.chunk * rows + q;
   if (i >= P.m) return;
-  TX acc = TX(0);
-  for (int g = 0; g < F.count; g++) acc += ypart[int64_t(F.part + g) * rows + q];
-  y[int64_t(blockIdx.y) * nslots * ld_y + P.yoff + i] = acc;
+  y[int64_t(blockIdx.y) * nslots * ld_y + P.yoff + i] = sum_parts(ypart + int64_t(F.part) * rows + q, F.count, rows);
 }
 
 template <typename TX, typename TO>
