@@ -173,9 +173,11 @@ struct Plan {
   int nzfix = 0;
   PanelFix* pfix_far = nullptr;
   int npfix_far = 0;
-  PanelFix* pfix_near = nullptr;  // near panels above 32 rows split over items (share ypart with the far ones)
+  PanelFix* pfix_near = nullptr;  // near panels split over items (share ypart with the far ones)
   int npfix_near = 0;
   int64_t nypart_near = 0;
+  // counters of the fixes (zero between launches)
+  unsigned int *zcnt = nullptr, *pcnt_far = nullptr, *pcnt_near = nullptr;
   // small items stream their segments as one byte run (small_items_contiguous)
   bool contig_near = false, contig_far = false;
   int64_t nzpart = 0, nypart = 0;  // partial-sum scratch (elements of the vector type)
@@ -193,7 +195,21 @@ struct Plan {
     std::vector<ZFix> zfix;
   };
   std::shared_ptr<Host> host;
+  PanelItems near_items() const {
+    return {panels_near, segs_near, small_near, big_near, nsmall_near, nbig_near, pfix_near, npfix_near,
+            pcnt_near};
+  }
+  PanelItems far_items() const {
+    return {panels_far, segs_far, small_far, big_far, nsmall_far, nbig_far, pfix_far, npfix_far, pcnt_far};
+  }
 };
+
+// Zeroed counters for k fixes.
+unsigned int* fix_counters(DevMem& mem, size_t k, cudaStream_t st) {
+  unsigned int* c = mem.alloc_n<unsigned int>(std::max<size_t>(k, 1), "fix-up counters");
+  check_cuda(cudaMemsetAsync(c, 0, sizeof(unsigned int) * std::max<size_t>(k, 1), st), "cudaMemset");
+  return c;
+}
 
 }  // namespace
 
@@ -416,11 +432,11 @@ void add_small_items(const std::vector<Seg>& segs, const Panel& p, int np, int64
   const std::vector<std::pair<int32_t, int32_t>> groups =
       column_groups(segs, p.seg_begin, p.seg_end, std::max(64, panel_cols(bytes, p.m, esz)));
   if (groups.size() == 1) {
-    small.push_back({np, 0, int32_t(p.seg_begin), int32_t(p.seg_end), -1});
+    small.push_back({np, 0, int32_t(p.seg_begin), int32_t(p.seg_end), -1, -1});
     return;
   }
   pfix.push_back({np, 0, int32_t(nypart), int32_t(groups.size())});
-  for (auto& g : groups) small.push_back({np, 0, g.first, g.second, int32_t(nypart++)});
+  for (auto& g : groups) small.push_back({np, 0, g.first, g.second, int32_t(nypart++), int32_t(pfix.size() - 1)});
 }
 
 // Whether an operator's items are spread as item_bytes says: all but the
@@ -442,6 +458,14 @@ void build_near_plan(hodlr_op* op, const NearTiles& nt, const void* base, Prec a
   for (const TileDesc& d : nt.tiles) total += int64_t(d.m) * d.n * int64_t(esz);
   const int64_t small_bytes = spread ? item_bytes(total, kMinItemBytes, int64_t(1) << 40) : int64_t(1) << 40;
   const int64_t big_bytes = spread ? item_bytes(total, kMinItemBytes, kNearItemBytes) : kNearItemBytes;
+  // FP64 panels of at most 32 rows: the staged leaf kernel when leaves are tiny
+  // (its one byte run per stage beats a segment per slice: 3D N = 262144, 8
+  // rows, 134 us against 183), else the items of launch_items64 with the larger
+  // panels (4D N = 65536, 16 rows, 198 us against 217; 3D N = 20011, 39 rows, 26 against
+  // 54), which also split; the two meet near 12 rows.
+  int64_t npanels = 0;
+  for (size_t k = 0; k + 1 < op->near.leaf_ptr.size(); k++) npanels += op->near.leaf_ptr[k] < op->near.leaf_ptr[k + 1];
+  const bool leaf = a == Prec::kD && op->n <= 12 * npanels;
   size_t q = 0;
   for (int64_t k = 0; k + 1 < int64_t(op->near.leaf_ptr.size()); k++) {
     const int64_t b = op->near.leaf_ptr[size_t(k)], e = op->near.leaf_ptr[size_t(k + 1)];
@@ -465,8 +489,10 @@ void build_near_plan(hodlr_op* op, const NearTiles& nt, const void* base, Prec a
     p.seg_end = int64_t(segs.size());
     const int np = int(panels.size());
     panels.push_back(p);
-    if (p.m <= 32) {
-      add_small_items(segs, p, np, small_bytes, int(esz), small, pfix, nypart);
+    if (leaf && p.m <= 32) {
+      small.push_back({np, 0, int32_t(p.seg_begin), int32_t(p.seg_end), -1, -1});
+    } else if (p.m <= 32) {
+      add_small_items(segs, p, np, small_bytes, int(esz), a == Prec::kD ? big : small, pfix, nypart);
     } else {
       // as for far panels: runs of columns, partial row blocks added by the
       // fix-up kernel
@@ -475,17 +501,18 @@ void build_near_plan(hodlr_op* op, const NearTiles& nt, const void* base, Prec a
           column_groups(segs, p.seg_begin, p.seg_end, panel_cols(big_bytes, rows, int(esz)));
       for (int c = 0; c < int((p.m + rows - 1) / rows); c++) {
         if (groups.size() == 1) {
-          big.push_back({np, c, groups[0].first, groups[0].second, -1});
+          big.push_back({np, c, groups[0].first, groups[0].second, -1, -1});
           continue;
         }
         pfix.push_back({np, c, int32_t(nypart), int32_t(groups.size())});
-        for (auto& g : groups) big.push_back({np, c, g.first, g.second, int32_t(nypart++)});
+        for (auto& g : groups) big.push_back({np, c, g.first, g.second, int32_t(nypart++), int32_t(pfix.size() - 1)});
       }
     }
   }
   plan.contig_near = small_items_contiguous(panels, segs, small, int(esz));
   plan.pfix_near = upload(op->mem, pfix, st, "near panel fix-ups");
   plan.npfix_near = int(pfix.size());
+  plan.pcnt_near = fix_counters(op->mem, pfix.size(), st);
   plan.nypart_near = nypart * rows_per_item(a);
   plan.a_near = a;
   plan.panels_near = upload(op->mem, panels, st, "near panels");
@@ -593,11 +620,11 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
         const int chunks = int((p.m + rows - 1) / rows);
         for (int c = 0; c < chunks; c++) {
           if (groups.size() == 1) {
-            big.push_back({np, c, groups[0].first, groups[0].second, -1});
+            big.push_back({np, c, groups[0].first, groups[0].second, -1, -1});
             continue;
           }
           pfix.push_back({np, c, int32_t(nypart), int32_t(groups.size())});
-          for (auto& g : groups) big.push_back({np, c, g.first, g.second, int32_t(nypart++)});
+          for (auto& g : groups) big.push_back({np, c, g.first, g.second, int32_t(nypart++), int32_t(pfix.size() - 1)});
         }
       }
     }
@@ -646,13 +673,14 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
       const int rows = int(std::max<int64_t>(1, z_bytes / (nk * esz)));
       const int groups = (n + rows - 1) / rows;
       if (groups == 1) {
-        zit.push_back({int32_t(q), k0, nk, 0, n, -1, 0, 0});
+        zit.push_back({int32_t(q), k0, nk, 0, n, -1, 0, 0, -1});
         z_item_stages(zit.back(), r, esz);
         continue;
       }
-      for (int c = 0; c < nk && k0 + c < r; c++) zfix.push_back({zb[q].z_off + k0 + c, int32_t(nzpart + c), groups});
+      zfix.push_back({zb[q].z_off + k0, int32_t(nzpart), groups, std::min(nk, r - k0), 0});
       for (int g = 0; g < groups; g++) {
-        zit.push_back({int32_t(q), k0, nk, g * rows, std::min(n, (g + 1) * rows), int32_t(nzpart), 0, 0});
+        zit.push_back({int32_t(q), k0, nk, g * rows, std::min(n, (g + 1) * rows), int32_t(nzpart), 0, 0,
+                       int32_t(zfix.size() - 1)});
         z_item_stages(zit.back(), r, esz);
         nzpart += kZPart;
       }
@@ -666,6 +694,8 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
   plan.nzfix = int(zfix.size());
   plan.pfix_far = upload(op->mem, pfix, st, "far panel fix-ups");
   plan.npfix_far = int(pfix.size());
+  plan.zcnt = fix_counters(op->mem, zfix.size(), st);
+  plan.pcnt_far = fix_counters(op->mem, pfix.size(), st);
   plan.nzpart = nzpart;
   plan.nypart = nypart * rows_per_item(a);
   if (op->keep_host_plans) {
@@ -1407,53 +1437,53 @@ struct PrecOf<float> {
   static constexpr Prec v = Prec::kF;
 };
 
-// y = A x, tree order, nrhs = 1; x may alias nothing in the op's buffers.
+// y = A x, one vector; x may alias nothing in the op's buffers.  x and y in
+// tree order, or in the caller's order through `perm`.
 template <typename T>
 cudaError_t apply_tree(hodlr_op* op, const Plan& plan, const T* x, T* y, T* in, T* yslots, cudaStream_t st,
-                       const int64_t* out_perm = nullptr) {
-  const int64_t n = op->n, ldin = n + op->zlen;
-  cudaError_t e = cudaMemcpyAsync(in, x, sizeof(T) * size_t(n), cudaMemcpyDeviceToDevice, st);
-  if (e != cudaSuccess) return e;
-  if (op->nslots > 1) {
-    e = cudaMemsetAsync(yslots + n, 0, sizeof(T) * size_t(n) * size_t(op->nslots - 1), st);
-    if (e != cudaSuccess) return e;
-  }
+                       const int64_t* perm = nullptr) {
+  const int64_t n = op->n;
   const Prec px = PrecOf<T>::v;
-  const int kb = &plan == &op->plan_ref ? HODLR_TRACE_ZGEMV_REF
-                 : px == Prec::kD       ? HODLR_TRACE_ZGEMV_FP64
-                                        : HODLR_TRACE_ZGEMV_FP32;
-  Tracer& tr = op->tr;
-  if (plan.nzb > 0) tr.start(kb + 0, st);
   // FP32 or BF16 factors with FP64 vectors: compensated (or, while the solver
   // allows it, relaxed) FP32 accumulation on split inputs
   const bool df = plan.a_far != Prec::kD && px == Prec::kD;
   const Accum acc = !df                       ? Accum::kByType
                     : op->relaxed || op->p.relax == HODLR_RELAX_ALWAYS ? Accum::kRelaxed
                                                                        : Accum::kCompensated;
-  void* fin = in;
-  if (df) {
-    fin = op->d_in2;
-    if ((e = launch_split(reinterpret_cast<const double*>(in), fin, n, st)) != cudaSuccess) return e;
+  void* fin = df ? op->d_in2 : static_cast<void*>(in);
+  const int kb = &plan == &op->plan_ref ? HODLR_TRACE_ZGEMV_REF
+                 : px == Prec::kD       ? HODLR_TRACE_ZGEMV_FP64
+                                        : HODLR_TRACE_ZGEMV_FP32;
+  Tracer& tr = op->tr;
+  cudaError_t e = launch_prep(px, x, perm, n, in, df ? fin : nullptr, yslots, op->nslots, st);
+  if (e != cudaSuccess) return e;
+  if (!tr.on && px == Prec::kD && plan.a_far == Prec::kD && plan.a_near == Prec::kD) {
+    // all FP64: V^T x and the near field in one launch
+    if ((e = launch_items64(plan.zb, plan.zitems, plan.nzitems, plan.zfix, plan.zcnt, static_cast<double*>(plan.zpart),
+                            plan.near_items(), static_cast<double*>(plan.ypart), reinterpret_cast<double*>(in),
+                            reinterpret_cast<double*>(yslots), st, plan.contig_near)) != cudaSuccess)
+      return e;
+  } else {
+    if (plan.nzb > 0) tr.start(kb + 0, st);
+    if ((e = launch_zgemv(plan.a_far, px, plan.zb, plan.zitems, plan.nzitems, plan.zfix, plan.nzfix, plan.zcnt, plan.zpart,
+                          fin, st,
+                          acc)) != cudaSuccess)
+      return e;
+    if (plan.nzb > 0) tr.stop(st);
+    tr.start(kb + 1, st);
+    if ((e = launch_panels(plan.a_near, px, plan.near_items(), plan.ypart, in, yslots, st, Accum::kByType,
+                           plan.contig_near)) != cudaSuccess)
+      return e;
+    tr.stop(st);
   }
-  if ((e = launch_zgemv(plan.a_far, px, plan.zb, plan.zitems, plan.nzitems, plan.zfix, plan.nzfix, plan.zpart, fin, ldin,
-                        1, st, acc)) != cudaSuccess)
-    return e;
-  if (plan.nzb > 0) tr.stop(st);
-  tr.start(kb + 1, st);
-  if ((e = launch_panels(plan.a_near, px, plan.panels_near, plan.segs_near, plan.small_near, plan.nsmall_near,
-                         plan.big_near, plan.nbig_near, plan.pfix_near, plan.npfix_near, plan.ypart, in, ldin, yslots, n,
-                         op->nslots, 1, st, Accum::kByType, plan.contig_near)) != cudaSuccess)
-    return e;
-  tr.stop(st);
   const bool far = plan.nsmall_far + plan.nbig_far > 0;
   if (far) tr.start(kb + 2, st);
-  if ((e = launch_panels(plan.a_far, px, plan.panels_far, plan.segs_far, plan.small_far, plan.nsmall_far, plan.big_far,
-                         plan.nbig_far, plan.pfix_far, plan.npfix_far, plan.ypart, fin, ldin, yslots, n, op->nslots, 1,
-                         st, acc, plan.contig_far)) != cudaSuccess)
+  if ((e = launch_panels(plan.a_far, px, plan.far_items(), plan.ypart, fin, yslots, st, acc, plan.contig_far)) !=
+      cudaSuccess)
     return e;
   if (far) tr.stop(st);
   tr.start(kb + 3, st);
-  e = launch_combine(px, yslots, n, op->nslots, n, 1, out_perm, y, px, n, st);
+  e = launch_combine(px, yslots, n, op->nslots, n, 1, perm, y, px, n, st);
   tr.stop(st);
   if (tr.used > 8192) tr.harvest();
   return e;
@@ -1927,6 +1957,8 @@ void build_finish(hodlr_op* op, BuildState& bs, cudaStream_t st) {
     op->plan32.nzfix = op->plan64.nzfix;
     op->plan32.pfix_far = op->plan64.pfix_far;
     op->plan32.npfix_far = op->plan64.npfix_far;
+    op->plan32.zcnt = op->plan64.zcnt;
+    op->plan32.pcnt_far = op->plan64.pcnt_far;
     op->plan32.nzpart = op->plan64.nzpart;
     op->plan32.nypart = std::max(op->plan64.nypart, op->plan32.nypart_near);
     op->plan32.zpart = op->mem.alloc(size_t(std::max<int64_t>(op->plan32.nzpart, 1)) * 4, "z partial sums (FP32)");
@@ -1948,6 +1980,7 @@ void build_finish(hodlr_op* op, BuildState& bs, cudaStream_t st) {
     r.nbig_near = op->plan64.nbig_near;
     r.pfix_near = op->plan64.pfix_near;
     r.npfix_near = op->plan64.npfix_near;
+    r.pcnt_near = op->plan64.pcnt_near;
     r.nypart_near = op->plan64.nypart_near;
     r.contig_near = op->plan64.contig_near;
     r.nypart = std::max(r.nypart, r.nypart_near);
@@ -2113,11 +2146,14 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
   h.zb.resize(size_t(tot.zb));
   h.zitems.resize(size_t(tot.zitems));
   h.zfix.resize(size_t(tot.zfix));
-  auto shift_item = [](Item it, int64_t panel_base, int64_t seg_base, int64_t part_base) {
+  auto shift_item = [](Item it, int64_t panel_base, int64_t seg_base, int64_t part_base, int64_t fix_base) {
     it.panel += int32_t(panel_base);
     it.seg_b += int32_t(seg_base);
     it.seg_e += int32_t(seg_base);
-    if (it.part >= 0) it.part += int32_t(part_base);
+    if (it.part >= 0) {
+      it.part += int32_t(part_base);
+      it.fix += int32_t(fix_base);
+    }
     return it;
   };
 #pragma omp parallel for schedule(dynamic, 1) num_threads(std::max(1, std::min<int>(int(nops), 16)))
@@ -2142,9 +2178,9 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
       h.segs_near[size_t(a.segs_near) + k] = sg;
     }
     for (size_t k = 0; k < hn.small_near.size(); k++)
-      h.small_near[size_t(a.small_near) + k] = shift_item(hn.small_near[k], a.panels_near, a.segs_near, a.near_parts);
+      h.small_near[size_t(a.small_near) + k] = shift_item(hn.small_near[k], a.panels_near, a.segs_near, a.near_parts, a.pfix_near);
     for (size_t k = 0; k < hn.big_near.size(); k++)
-      h.big_near[size_t(a.big_near) + k] = shift_item(hn.big_near[k], a.panels_near, a.segs_near, a.near_parts);
+      h.big_near[size_t(a.big_near) + k] = shift_item(hn.big_near[k], a.panels_near, a.segs_near, a.near_parts, a.pfix_near);
     for (size_t k = 0; k < hn.pfix_near.size(); k++) {
       PanelFix f = hn.pfix_near[k];
       f.panel += int32_t(a.panels_near);
@@ -2165,9 +2201,9 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
       h.segs_far[size_t(a.segs_far) + k] = sg;
     }
     for (size_t k = 0; k < hf.small_far.size(); k++)
-      h.small_far[size_t(a.small_far) + k] = shift_item(hf.small_far[k], a.panels_far, a.segs_far, a.far_parts);
+      h.small_far[size_t(a.small_far) + k] = shift_item(hf.small_far[k], a.panels_far, a.segs_far, a.far_parts, a.pfix_far);
     for (size_t k = 0; k < hf.big_far.size(); k++)
-      h.big_far[size_t(a.big_far) + k] = shift_item(hf.big_far[k], a.panels_far, a.segs_far, a.far_parts);
+      h.big_far[size_t(a.big_far) + k] = shift_item(hf.big_far[k], a.panels_far, a.segs_far, a.far_parts, a.pfix_far);
     for (size_t k = 0; k < hf.pfix_far.size(); k++) {
       PanelFix f = hf.pfix_far[k];
       f.panel += int32_t(a.panels_far);
@@ -2184,7 +2220,10 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
     for (size_t k = 0; k < hf.zitems.size(); k++) {
       ZItem it = hf.zitems[k];
       it.zb += int32_t(a.zb);
-      if (it.part >= 0) it.part += int32_t(a.zpart);
+      if (it.part >= 0) {
+        it.part += int32_t(a.zpart);
+        it.fix += int32_t(a.zfix);
+      }
       h.zitems[size_t(a.zitems) + k] = it;
     }
     for (size_t k = 0; k < hf.zfix.size(); k++) {
@@ -2229,6 +2268,9 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
   p.nzitems = int(h.zitems.size());
   p.zfix = upload(b.mem, h.zfix, st, "batch z fix-ups");
   p.nzfix = int(h.zfix.size());
+  p.zcnt = fix_counters(b.mem, h.zfix.size(), st);
+  p.pcnt_near = fix_counters(b.mem, h.pfix_near.size(), st);
+  p.pcnt_far = fix_counters(b.mem, h.pfix_far.size(), st);
   const size_t vsz = f32 ? 4 : 8;
   p.nzpart = zpart;
   p.nypart = std::max(near_parts * rows_per_item(p.a_near), far_parts * rows_per_item(p.a_far));
@@ -2254,12 +2296,14 @@ void batch_apply(hodlr_batch& b, const void* x, void* y, cudaStream_t st) {
     acc = Accum::kCompensated;
     CK(launch_split(static_cast<const double*>(b.d_in), fin, b.ld_in, st));
   }
-  CK(launch_zgemv(p.a_far, b.vec, p.zb, p.zitems, p.nzitems, p.zfix, p.nzfix, p.zpart, fin, b.ld_in, 1, st, acc));
-  CK(launch_panels(p.a_near, b.vec, p.panels_near, p.segs_near, p.small_near, p.nsmall_near, p.big_near, p.nbig_near,
-                   p.pfix_near, p.npfix_near, p.ypart, b.d_in, b.ld_in, b.d_y, b.ycol, 1, 1, st, Accum::kByType,
-                   p.contig_near));
-  CK(launch_panels(p.a_far, b.vec, p.panels_far, p.segs_far, p.small_far, p.nsmall_far, p.big_far, p.nbig_far,
-                   p.pfix_far, p.npfix_far, p.ypart, fin, b.ld_in, b.d_y, b.ycol, 1, 1, st, acc, p.contig_far));
+  if (b.vec == Prec::kD && p.a_far == Prec::kD && p.a_near == Prec::kD) {
+    CK(launch_items64(p.zb, p.zitems, p.nzitems, p.zfix, p.zcnt, static_cast<double*>(p.zpart), p.near_items(),
+                      static_cast<double*>(p.ypart), static_cast<double*>(b.d_in), static_cast<double*>(b.d_y), st, p.contig_near));
+  } else {
+    CK(launch_zgemv(p.a_far, b.vec, p.zb, p.zitems, p.nzitems, p.zfix, p.nzfix, p.zcnt, p.zpart, fin, st, acc));
+    CK(launch_panels(p.a_near, b.vec, p.near_items(), p.ypart, b.d_in, b.d_y, st, Accum::kByType, p.contig_near));
+  }
+  CK(launch_panels(p.a_far, b.vec, p.far_items(), p.ypart, fin, b.d_y, st, acc, p.contig_far));
   CK(launch_batch_combine(b.vec, b.d_inst, int(b.ops.size()), b.max_n, b.d_y, y, st));
 }
 
@@ -2347,7 +2391,7 @@ void tc_panel_items(const std::vector<Panel>& panels, const std::vector<Seg>& se
       while ((16 << bk) < rows) bk++;
       if (nruns > 1) fix.push_back({int32_t(pi), tl, nparts, nruns});
       for (int q = 0; q < nruns; q++) {
-        Item it;
+        Item it{};
         it.panel = int32_t(pi);
         it.chunk = tl;
         it.seg_b = cut[size_t(q)].first;
@@ -2674,9 +2718,8 @@ int hodlr_matvec_device(hodlr_op* op, const double* d_x, double* d_y, int64_t nr
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int64_t n = op->n;
     for (int64_t c = 0; c < nrhs; c++) {
-      // gather into tree order; the combine step scatters back to the caller's order
-      CK(launch_gather(d_x + c * n, Prec::kD, n, op->d_perm, n, 1, op->d_io, Prec::kD, n, st));
-      CK(apply_tree<double>(op, op->plan64, op->d_io, d_y + c * n, op->d_in64, op->d_y64, st, op->d_perm));
+      // gathered into tree order on the way in, scattered back by the combine step
+      CK(apply_tree<double>(op, op->plan64, d_x + c * n, d_y + c * n, op->d_in64, op->d_y64, st, op->d_perm));
     }
     return HODLR_OK;
   });

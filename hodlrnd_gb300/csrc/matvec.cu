@@ -281,7 +281,7 @@ __device__ __forceinline__ float2 to_input<FH>(float a) {
 // consecutive rows, so each 16-byte read of the warp covers G whole rows.
 // Each lane keeps CPL running sums, over rows g, g + G, g + 2G, ... of the
 // item in that order; the groups are added by shuffles once at the end.  A
-// block with more rows than one item takes writes partial sums (zfix_kernel
+// block with more rows than one item takes writes partial sums (the last item
 // adds them in order).
 //
 // An item that covers whole rows (k0 == 0, nk == vpad(r)) reads one
@@ -328,6 +328,35 @@ constexpr int kZStageBytes = HODLR_TUNE_Z_BYTES;  // V bytes per stage
 constexpr int kZXBytes = (kZStageBytes / 16) * 8 + 32;
 constexpr int kZWarpSmem = 64 + kZStages * (kZStageBytes + kZXBytes);
 static_assert(kZWarpSmem % 16 == 0 && kZXBytes % 16 == 0, "bulk copy destinations must stay 16-byte aligned");
+
+// Sum of `count` partial sums, `stride` apart, in an order that depends on
+// count alone: one after another up to 8 of them; more (small operators, whose
+// work is cut into many short items) go to 8 running sums, so that 8 loads are
+// in flight instead of one load latency per part.  Read past L1: other SMs
+// wrote the parts.
+template <typename T>
+__device__ __forceinline__ T sum_parts(const T* p, int count, int64_t stride) {
+  T acc = T(0);
+  if (count <= 8) {
+    for (int q = 0; q < count; q++) acc += __ldcg(p + q * stride);
+    return acc;
+  }
+  T a[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) a[k] = __ldcg(p + k * stride);
+  int q = 8;
+  for (; q + 8 <= count; q += 8) {
+    T v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = __ldcg(p + (q + k) * stride);
+#pragma unroll
+    for (int k = 0; k < 8; k++) a[k] += v[k];
+  }
+#pragma unroll
+  for (int k = 0; k < 7; k++)
+    if (q + k < count) a[k] += __ldcg(p + (q + k) * stride);
+  return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+}
 
 // The end of an item: acc[q] (column p * CPL + q of the item) is summed over
 // the G = 32 / P lanes sharing p by a transposed butterfly -- while a lane
@@ -386,7 +415,7 @@ template <typename TA, typename TACC>
 __global__ void __launch_bounds__(kZWarps * 32) zgemv_kernel(const ZBlock* __restrict__ zb,
                                                            const ZItem* __restrict__ items, int nitems,
                                                            typename IO<TACC>::TY* __restrict__ zpart,
-                                                           typename IO<TACC>::TI* in, int64_t ld_in) {
+                                                           typename IO<TACC>::TI* in) {
   using TX = typename IO<TACC>::TI;
   constexpr int CPL = 16 / int(sizeof(TA));
   using VT = typename Vec16<TA>::type;
@@ -398,8 +427,8 @@ __global__ void __launch_bounds__(kZWarps * 32) zgemv_kernel(const ZBlock* __res
   const ZItem it = items[w];
   const ZBlock Z = zb[it.zb];
   const int64_t rp = vpad(Z.r, int(sizeof(TA)));
-  const TX* x = in + blockIdx.y * ld_in + Z.x_off;
-  TX* z = in + blockIdx.y * ld_in + Z.z_off;
+  const TX* x = in + Z.x_off;
+  TX* z = in + Z.z_off;
   const int lanes = (it.nk + CPL - 1) / CPL;
   const int P = lanes <= 1 ? 1 : 1 << (32 - __clz(lanes - 1));  // next power of two >= lanes
   const int G = 32 / P, g = lane / P, p = lane % P;
@@ -486,43 +515,14 @@ __global__ void __launch_bounds__(kZWarps * 32) zgemv_kernel(const ZBlock* __res
   z_finish<TA, TACC>(acc, P, lane, it, Z, z, zpart);
 }
 
-// Sum of `count` partial sums, `stride` apart, in an order that depends on
-// count alone: one after another up to 8 of them; more (small operators, whose
-// work is cut into many short items) go to 8 running sums, so that 8 loads are
-// in flight instead of one load latency per part.
-template <typename T>
-__device__ __forceinline__ T sum_parts(const T* __restrict__ p, int count, int64_t stride) {
-  T acc = T(0);
-  if (count <= 8) {
-    for (int q = 0; q < count; q++) acc += p[q * stride];
-    return acc;
-  }
-  T a[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) a[k] = p[k * stride];
-  int q = 8;
-  for (; q + 8 <= count; q += 8) {
-    T v[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) v[k] = p[(q + k) * stride];
-#pragma unroll
-    for (int k = 0; k < 8; k++) a[k] += v[k];
-  }
-#pragma unroll
-  for (int k = 0; k < 7; k++)
-    if (q + k < count) a[k] += p[(q + k) * stride];
-  return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
-}
-
+// z of split blocks: each fix's columns summed over its parts.
 template <typename TACC>
-__global__ void zfix_kernel(const ZFix* __restrict__ fix, int nfix, const typename IO<TACC>::TY* __restrict__ zpart,
-                            typename IO<TACC>::TI* in, int64_t ld_in) {
-  using TY = typename IO<TACC>::TY;
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= nfix) return;
-  const ZFix F = fix[f];
-  const TY acc = sum_parts(zpart + F.part, F.count, kZPart);
-  in[blockIdx.y * ld_in + F.zpos] = IO<TACC>::from_double(double(acc));
+__global__ void __launch_bounds__(kZPart) zfix_kernel(const ZFix* __restrict__ fix,
+                                                      const typename IO<TACC>::TY* __restrict__ zpart,
+                                                      typename IO<TACC>::TI* __restrict__ in) {
+  const ZFix F = fix[blockIdx.x];
+  const int c = threadIdx.x;
+  if (c < F.nk) in[F.zpos + c] = IO<TACC>::from_double(double(sum_parts(zpart + F.part + c, F.count, kZPart)));
 }
 
 // Phase 2, panels of at most 32 rows (leaves): lanes form 32 / mpad slices of
@@ -560,9 +560,8 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 template <typename TA, typename TACC>
 __global__ void __launch_bounds__(kSWarps * 32, HODLR_TUNE_S_MINB)
     panel_small_kernel(const Panel* __restrict__ panels, const Seg* __restrict__ segs, const Item* __restrict__ items,
-                       int nitems, const typename IO<TACC>::TI* __restrict__ in, int64_t ld_in,
-                       typename IO<TACC>::TY* __restrict__ y, int64_t ld_y, int nslots,
-                       typename IO<TACC>::TY* __restrict__ ypart) {
+                       int nitems, const typename IO<TACC>::TI* __restrict__ in, typename IO<TACC>::TY* __restrict__ y,
+                       typename IO<TACC>::TY* ypart) {
   using TX = typename IO<TACC>::TI;
   using TY = typename IO<TACC>::TY;
   using AC = Acc<TACC>;
@@ -576,8 +575,8 @@ __global__ void __launch_bounds__(kSWarps * 32, HODLR_TUNE_S_MINB)
   const Item it = items[w];
   const Panel P = panels[it.panel];
   const int m = P.m;
-  const TX* inc = in + blockIdx.y * ld_in;
-  TY* yo = y + int64_t(blockIdx.y) * nslots * ld_y + P.yoff;
+  const TX* inc = in;
+  TY* yo = y + P.yoff;
   int mpad = 1;
   while (mpad < m) mpad <<= 1;
   const int slices = 32 / mpad;
@@ -806,9 +805,8 @@ __device__ __forceinline__ void leaf_products(const TA* __restrict__ su, const T
 template <typename TA, typename TACC>
 __global__ void __launch_bounds__(kLWarps * 32, HODLR_TUNE_L_MINB)
     panel_leaf_kernel(const Panel* __restrict__ panels, const Seg* __restrict__ segs, const Item* __restrict__ items,
-                      int nitems, const typename IO<TACC>::TI* __restrict__ in, int64_t ld_in,
-                      typename IO<TACC>::TY* __restrict__ y, int64_t ld_y, int nslots,
-                      typename IO<TACC>::TY* __restrict__ ypart) {
+                      int nitems, const typename IO<TACC>::TI* __restrict__ in, typename IO<TACC>::TY* __restrict__ y,
+                      typename IO<TACC>::TY* ypart) {
   using TI = typename IO<TACC>::TI;
   using TX = typename LeafX<TACC>::T;
   using TY = typename IO<TACC>::TY;
@@ -825,8 +823,8 @@ __global__ void __launch_bounds__(kLWarps * 32, HODLR_TUNE_L_MINB)
   const Panel P = panels[it.panel];
   const int m = P.m;
   const int colb = m * esz;  // bytes per column
-  const TI* inc = in + blockIdx.y * ld_in;
-  TY* yo = y + int64_t(blockIdx.y) * nslots * ld_y + P.yoff;
+  const TI* inc = in;
+  TY* yo = y + P.yoff;
   int mpad = 1;
   while (mpad < m) mpad <<= 1;
   const int slices = 32 / mpad;
@@ -1065,8 +1063,7 @@ template <typename TA, typename TACC>
 __global__ void __launch_bounds__(kPWarps * 32, HODLR_TUNE_P_MINB)
     panel_tile_kernel(const Panel* __restrict__ panels, const Seg* __restrict__ segs, const Item* __restrict__ items,
                       int nitems, typename IO<TACC>::TY* __restrict__ ypart,
-                      const typename IO<TACC>::TI* __restrict__ in, int64_t ld_in,
-                      typename IO<TACC>::TY* __restrict__ y, int64_t ld_y, int nslots) {
+                      const typename IO<TACC>::TI* __restrict__ in, typename IO<TACC>::TY* __restrict__ y) {
   using TX = typename IO<TACC>::TI;
   using TY = typename IO<TACC>::TY;
   constexpr int RPL = 16 / int(sizeof(TA));
@@ -1080,7 +1077,7 @@ __global__ void __launch_bounds__(kPWarps * 32, HODLR_TUNE_P_MINB)
   const Item it = items[w];
   const Panel P = panels[it.panel];
   const int m = P.m;
-  const TX* inc = in + blockIdx.y * ld_in;
+  const TX* inc = in;
   const int t = it.chunk;
   const int rows = min(T, m - t * T);
   const int64_t h = tile_height(m, t, int(sizeof(TA)));
@@ -1188,188 +1185,10 @@ __global__ void __launch_bounds__(kPWarps * 32, HODLR_TUNE_P_MINB)
   }
   if (act && sl == 0) {
     const int i = t * T + g * RPL;
-    TY* dst = it.part < 0 ? y + int64_t(blockIdx.y) * nslots * ld_y + P.yoff + i
-                          : ypart + int64_t(it.part) * T + g * RPL;
+    TY* dst = it.part < 0 ? y + P.yoff + i : ypart + int64_t(it.part) * T + g * RPL;
 #pragma unroll
     for (int q = 0; q < RPL; q++)
       if (i + q < m) dst[q] = TY(AC::value(a0[q]));
-  }
-}
-
-// ---- direct-load variants, used for FP64 factors ----------------------------
-// FP64 products run on GB300's FP64 pipe, whose rate (not the bytes in
-// flight) bounds these kernels; plain loads with eight warps per CTA keep
-// that pipe busier than the shared-memory staged versions above.  Lane
-// layouts as described above for each phase; the node-panel variant keeps
-// one column per warp step (no column slices), with columns alternating
-// between the two accumulator sets.
-template <typename TA, typename TACC>
-__global__ void __launch_bounds__(256) zgemv_direct_kernel(const ZBlock* __restrict__ zb, const ZItem* __restrict__ items,
-                                                    int nitems, typename IO<TACC>::TY* __restrict__ zpart,
-                                                    typename IO<TACC>::TI* in, int64_t ld_in) {
-  using TX = typename IO<TACC>::TI;
-  constexpr int CPL = 16 / int(sizeof(TA));
-  using VT = typename Vec16<TA>::type;
-  const int w = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (w >= nitems) return;
-  const ZItem it = items[w];
-  const ZBlock Z = zb[it.zb];
-  const int64_t rp = vpad(Z.r, int(sizeof(TA)));
-  const TX* x = in + blockIdx.y * ld_in + Z.x_off;
-  TX* z = in + blockIdx.y * ld_in + Z.z_off;
-  const int lanes = (it.nk + CPL - 1) / CPL;
-  int P = 1;
-  while (P < lanes) P <<= 1;
-  const int G = 32 / P, g = lane / P, p = lane % P;
-  const bool cact = p < lanes;
-  const TA* Vc = static_cast<const TA*>(Z.V) + it.k0 + p * CPL;
-  using AC = Acc<TACC>;
-  typename AC::A acc[CPL];
-#pragma unroll
-  for (int q = 0; q < CPL; q++) acc[q] = AC::zero();
-  int j = it.j0 + g;
-  for (; j + 3 * G < it.j1; j += 4 * G) {
-    VT v[4];
-    typename AC::X xs[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      v[u] = cact ? __ldg(reinterpret_cast<const VT*>(Vc + int64_t(j + u * G) * rp)) : vzero<VT>();
-      xs[u] = AC::in(x[j + u * G]);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; u++) axpy16<TACC>(v[u], xs[u], acc);
-  }
-  for (; j < it.j1; j += G) {
-    const VT v = cact ? __ldg(reinterpret_cast<const VT*>(Vc + int64_t(j) * rp)) : vzero<VT>();
-    axpy16<TACC>(v, AC::in(x[j]), acc);
-  }
-  for (int o = P; o < 32; o <<= 1)
-#pragma unroll
-    for (int q = 0; q < CPL; q++) acc[q] = AC::add(acc[q], AC::shfl_xor(acc[q], o));
-  if (g == 0 && cact) {
-#pragma unroll
-    for (int q = 0; q < CPL; q++) {
-      const int c = p * CPL + q;
-      if (it.part < 0) {
-        if (it.k0 + c < Z.r) z[it.k0 + c] = to_input<TACC>(acc[q]);
-      } else {
-        zpart[it.part + c] = typename IO<TACC>::TY(AC::value(acc[q]));
-      }
-    }
-  }
-}
-
-template <typename TA, typename TACC>
-__global__ void __launch_bounds__(256)
-    panel_small_direct_kernel(const Panel* __restrict__ panels, const Seg* __restrict__ segs, const Item* __restrict__ items,
-                       int nitems, const typename IO<TACC>::TI* __restrict__ in, int64_t ld_in,
-                       typename IO<TACC>::TY* __restrict__ y, int64_t ld_y, int nslots,
-                       typename IO<TACC>::TY* __restrict__ ypart) {
-  using TX = typename IO<TACC>::TI;
-  using TY = typename IO<TACC>::TY;
-  const int w = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (w >= nitems) return;
-  const Item it = items[w];
-  const Panel P = panels[it.panel];
-  const int m = P.m;
-  const TX* inc = in + blockIdx.y * ld_in;
-  TY* yo = y + int64_t(blockIdx.y) * nslots * ld_y + P.yoff;
-  int mpad = 1;
-  while (mpad < m) mpad <<= 1;
-  const int slices = 32 / mpad;
-  const int i = lane & (mpad - 1), sl = lane / mpad;
-  using AC = Acc<TACC>;
-  typename AC::A a0 = AC::zero(), a1 = AC::zero();
-  if (i < m) {
-    for (int64_t s = it.seg_b + sl; s < it.seg_e; s += slices) {
-      const Seg S = segs[s];
-      const TA* A = static_cast<const TA*>(S.A) + i;
-      const TX* x = inc + S.in_off;
-      int j = 0;
-      for (; j + 3 < S.K; j += 4) {
-        const TA v0 = ldg(A + int64_t(j) * m), v1 = ldg(A + int64_t(j + 1) * m);
-        const TA v2 = ldg(A + int64_t(j + 2) * m), v3 = ldg(A + int64_t(j + 3) * m);
-        const TX x0 = x[j], x1 = x[j + 1], x2 = x[j + 2], x3 = x[j + 3];
-        AC::fma(a0, v0, AC::in(x0));
-        AC::fma(a1, v1, AC::in(x1));
-        AC::fma(a0, v2, AC::in(x2));
-        AC::fma(a1, v3, AC::in(x3));
-      }
-      for (; j < S.K; j++) AC::fma(a0, ldg(A + int64_t(j) * m), AC::in(x[j]));
-    }
-  }
-  typename AC::A acc = AC::add(a0, a1);
-  for (int o = mpad; o < 32; o <<= 1) acc = AC::add(acc, AC::shfl_xor(acc, o));
-  // a panel whose columns are split over several items: partial rows at
-  // ypart[part * tile_rows], added in part order by panel_fix_kernel
-  if (sl == 0 && i < m) {
-    if (it.part < 0)
-      yo[i] = TY(AC::value(acc));
-    else
-      ypart[int64_t(it.part) * tile_rows(int(sizeof(TA))) + i] = TY(AC::value(acc));
-  }
-}
-
-template <typename TA, typename TACC>
-__global__ void __launch_bounds__(256)
-    panel_tile_direct_kernel(const Panel* __restrict__ panels, const Seg* __restrict__ segs, const Item* __restrict__ items,
-                      int nitems, typename IO<TACC>::TY* __restrict__ ypart,
-                      const typename IO<TACC>::TI* __restrict__ in, int64_t ld_in,
-                      typename IO<TACC>::TY* __restrict__ y, int64_t ld_y, int nslots) {
-  using TX = typename IO<TACC>::TI;
-  using TY = typename IO<TACC>::TY;
-  constexpr int RPL = 16 / int(sizeof(TA));
-  constexpr int T = 32 * RPL;
-  using VT = typename Vec16<TA>::type;
-  const int w = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (w >= nitems) return;
-  const Item it = items[w];
-  const Panel P = panels[it.panel];
-  const int m = P.m;
-  const TX* inc = in + blockIdx.y * ld_in;
-  const int t = it.chunk;
-  const int rows = min(T, m - t * T);
-  const int64_t h = tile_height(m, t, int(sizeof(TA)));
-  const bool act = lane * RPL < rows;
-  using AC = Acc<TACC>;
-  typename AC::A a0[RPL], a1[RPL];
-#pragma unroll
-  for (int q = 0; q < RPL; q++) a0[q] = a1[q] = AC::zero();
-  for (int64_t s = it.seg_b; s < it.seg_e; s++) {
-    const Seg S = segs[s];
-    const TA* A = static_cast<const TA*>(S.A) + int64_t(t) * T * S.K + lane * RPL;
-    const TX* x = inc + S.in_off;
-    for (int j0 = 0; j0 < S.K; j0 += 32) {
-      const int jn = min(32, S.K - j0);
-      const typename AC::X xl = AC::in(lane < jn ? x[j0 + lane] : TX{});
-      const TA* Aj = A + int64_t(j0) * h;
-      int jj = 0;
-      for (; jj + 3 < jn; jj += 4) {
-        VT v[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-          v[u] = act ? __ldg(reinterpret_cast<const VT*>(Aj + int64_t(jj + u) * h)) : vzero<VT>();
-        axpy16<TACC>(v[0], AC::shfl(xl, jj), a0);
-        axpy16<TACC>(v[1], AC::shfl(xl, jj + 1), a1);
-        axpy16<TACC>(v[2], AC::shfl(xl, jj + 2), a0);
-        axpy16<TACC>(v[3], AC::shfl(xl, jj + 3), a1);
-      }
-      for (; jj < jn; jj++) {
-        const VT v = act ? __ldg(reinterpret_cast<const VT*>(Aj + int64_t(jj) * h)) : vzero<VT>();
-        axpy16<TACC>(v, AC::shfl(xl, jj), a0);
-      }
-    }
-  }
-  if (act) {
-    const int i = t * T + lane * RPL;
-    TY* dst = it.part < 0 ? y + int64_t(blockIdx.y) * nslots * ld_y + P.yoff + i
-                          : ypart + int64_t(it.part) * T + lane * RPL;
-#pragma unroll
-    for (int q = 0; q < RPL; q++)
-      if (i + q < m) dst[q] = TY(AC::value(AC::add(a0[q], a1[q])));
   }
 }
 
@@ -1377,8 +1196,7 @@ __global__ void __launch_bounds__(256)
 template <typename TX>
 __global__ void __launch_bounds__(256) panel_fix_kernel(const Panel* __restrict__ panels,
                                                         const PanelFix* __restrict__ fix, int nfix, int rows,
-                                                        const TX* __restrict__ ypart, TX* __restrict__ y, int64_t ld_y,
-                                                        int nslots) {
+                                                        const TX* __restrict__ ypart, TX* __restrict__ y) {
   const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   const int f = int(t / rows), q = int(t % rows);
   if (f >= nfix) return;
@@ -1386,7 +1204,252 @@ __global__ void __launch_bounds__(256) panel_fix_kernel(const Panel* __restrict_
   const Panel P = panels[F.panel];
   const int i = F.chunk * rows + q;
   if (i >= P.m) return;
-  y[int64_t(blockIdx.y) * nslots * ld_y + P.yoff + i] = sum_parts(ypart + int64_t(F.part) * rows + q, F.count, rows);
+  y[P.yoff + i] = sum_parts(ypart + int64_t(F.part) * rows + q, F.count, rows);
+}
+
+// ---- FP64 factors ------------------------------------------------------------
+// z = V^T x and the panels are the same product: sums over columns j of
+// A(i, j) x(j) for at most 64 rows i that lie together in memory (V is stored
+// row major, so a column j of the product is a point's row of V).  GB300's
+// FP64 pipe -- 2 multiply-adds per clock and SM, 4.9 TB/s of factors -- bounds
+// it, so what matters is that no lane multiplies padding and that the pipe
+// always has a warp ready.  8 lanes take a column, lane g rows g, g + 8, ...
+// (R = ceil(rows / 8) of them: at most 7 idle lanes, where 16-byte loads with
+// the next power of two of lanes idled up to half), and the warp's 4 slices of
+// lanes take 4 consecutive columns; the slices are added by shuffles at the
+// end.  Every kind of item goes into one launch (z items first, then the
+// panels): in a small operator a launch lasts as long as its longest item, and
+// one launch waits for one of them.
+// One product with FP64 factors: 2D N = 2000 130 -> 77 us, 2D N = 10000 165 ->
+// 94 us, 3D N = 30011 764 -> 606 us (0.37 G multiply-adds per ms, 60% of the
+// pipe; the rest is leaf segments of 8 columns and less).
+// Whether this warp, whose lanes have written their partial sums, is the last
+// of `count` to finish on counter *cnt; the last one resets the counter.  (Used
+// by the FP64 items only: in the staged kernels the wait for the partial sums'
+// stores and the registers of the sums cost a large operator more than the two
+// fix-up launches do -- 3D N = 262144 FP32 factors 2.82 -> 3.10 ms.)
+__device__ __forceinline__ bool last_part(unsigned int* cnt, int count, int lane) {
+  __threadfence();
+  __syncwarp();
+  int last = 0;
+  if (lane == 0) {
+    last = atomicAdd(cnt, 1u) == unsigned(count - 1);
+    if (last) *cnt = 0u;
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return false;
+  __threadfence();
+  return true;
+}
+
+// The end of a split z item: the last one adds the parts into z.
+__device__ __forceinline__ void z_fixup(const ZFix* __restrict__ fix, unsigned int* zcnt, int f, const double* zpart,
+                                        double* in, int lane) {
+  const ZFix F = fix[f];
+  if (!last_part(zcnt + f, F.count, lane)) return;
+  for (int c = lane; c < F.nk; c += 32) in[F.zpos + c] = sum_parts(zpart + F.part + c, F.count, kZPart);
+}
+
+// The end of a split panel item (rows rows from row0 of the panel, parts T rows apart).
+__device__ __forceinline__ void panel_fixup(const PanelFix* __restrict__ fix, unsigned int* pcnt, int f,
+                                            const double* ypart, double* y, int rows, int lane) {
+  const PanelFix F = fix[f];
+  if (!last_part(pcnt + f, F.count, lane)) return;
+  for (int i = lane; i < rows; i += 32) y[i] = sum_parts(ypart + int64_t(F.part) * 64 + i, F.count, 64);
+}
+
+struct Items64 {
+  const ZBlock* zb;
+  const ZItem* zitems;
+  int nz;
+  const ZFix* zfix;
+  unsigned int* zcnt;
+  double* zpart;
+  PanelItems L;
+  double* ypart;
+  double* in;
+  double* y;
+};
+
+// acc[q] += sum_j A(g + 8 q, j) x(j), j = sl, sl + 4, ... < K; A points at row
+// g of column 0; okl: row g + 8 (R - 1) exists.
+template <int R>
+__device__ __forceinline__ void cols64(const double* __restrict__ A, int64_t ld, const double* x, int K, bool okl,
+                                       int sl, double (&acc)[R]) {
+  constexpr int U = R <= 2 ? 4 : R <= 4 ? 2 : 1;  // columns in flight per slice
+  for (int b = 0; b < K; b += 4 * U) {
+    double v[U][R], xv[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (b + 4 * u < K) {  // warp-uniform
+        const int j = b + 4 * u + sl;
+        const bool in = j < K;
+        xv[u] = in ? x[j] : 0.0;
+        const double* Aj = A + int64_t(j) * ld;
+#pragma unroll
+        for (int q = 0; q < R; q++) v[u][q] = in && (q < R - 1 || okl) ? __ldg(Aj + 8 * q) : 0.0;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (b + 4 * u < K) {
+#pragma unroll
+        for (int q = 0; q < R; q++) acc[q] += v[u][q] * xv[u];
+      }
+    }
+  }
+}
+
+// acc[q] += sum_j A(g + 8 q, j) x(j) over this slice's own K columns (Km: the
+// most of any slice).
+template <int R>
+__device__ __forceinline__ void segs64(const double* __restrict__ A, int64_t ld, const double* x, int K, int Km,
+                                       bool okl, double (&acc)[R]) {
+  constexpr int U = 4;
+  for (int b = 0; b < Km; b += U) {
+    double v[U][R], xv[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int j = b + u;
+      const bool in = j < K;
+      xv[u] = in ? x[j] : 0.0;
+      const double* Aj = A + int64_t(j) * ld;
+#pragma unroll
+      for (int q = 0; q < R; q++) v[u][q] = in && (q < R - 1 || okl) ? __ldg(Aj + 8 * q) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (b + u < Km) {
+#pragma unroll
+        for (int q = 0; q < R; q++) acc[q] += v[u][q] * xv[u];
+      }
+  }
+}
+
+// One item: its segments' records one per lane (loaded 32 at a time), rows
+// rows with column stride ld, the sums to dst[0 .. rows).  zA / zx / zK: the
+// single segment of a z item (zA non-null).
+template <int R>
+__device__ __forceinline__ void item64(const Seg* __restrict__ segs, int32_t sb, int32_t se, int64_t tile_off,
+                                       const double* zA, int64_t zx, int zK, int rows, int64_t ld, const double* in,
+                                       double* dst, int lane) {
+  const int g = lane & 7, sl = lane >> 3;
+  const bool okl = g + 8 * (R - 1) < rows;
+  double acc[R];
+#pragma unroll
+  for (int q = 0; q < R; q++) acc[q] = 0.0;
+  if (zA) {
+    cols64<R>(zA + g, ld, in + zx, zK, okl, sl, acc);
+  } else {
+    for (int32_t s0 = sb; s0 < se; s0 += 32) {
+      const double* rA = nullptr;
+      int64_t ro = 0;
+      int rK = 0;
+      if (s0 + lane < se) {
+        const Seg S = segs[s0 + lane];
+        rA = static_cast<const double*>(S.A) + tile_off * S.K;
+        ro = S.in_off;
+        rK = S.K;
+      }
+      const int n = min(32, se - s0);
+      if constexpr (R <= 2) {
+        // few rows, and columns of a leaf's few points: a segment for each
+        // slice, so that four of them are in flight
+        for (int k0 = 0; k0 < n; k0 += 4) {
+          const int k = min(k0 + sl, n - 1);
+          const double* A = reinterpret_cast<const double*>(
+              __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(rA), k));
+          const int64_t off = __shfl_sync(0xffffffffu, ro, k);
+          int K = __shfl_sync(0xffffffffu, rK, k);
+          if (k0 + sl >= n) K = 0;
+          int Km = max(K, __shfl_xor_sync(0xffffffffu, K, 8));
+          Km = max(Km, __shfl_xor_sync(0xffffffffu, Km, 16));
+          segs64<R>(A + g, ld, in + off, K, Km, okl, acc);
+        }
+        continue;
+      }
+      for (int k = 0; k < n; k++) {
+        const double* A = reinterpret_cast<const double*>(
+            __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(rA), k));
+        const int64_t off = __shfl_sync(0xffffffffu, ro, k);
+        const int K = __shfl_sync(0xffffffffu, rK, k);
+        cols64<R>(A + g, ld, in + off, K, okl, sl, acc);
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < R; q++) {
+    acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], 8);
+    acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], 16);
+  }
+  if (sl == 0) {
+#pragma unroll
+    for (int q = 0; q < R; q++)
+      if (q < R - 1 || okl) dst[g + 8 * q] = acc[q];
+  }
+}
+
+__global__ void __launch_bounds__(kWarpsPerCta * 32, 4) items64_kernel(const Items64 a) {
+  const int lane = threadIdx.x & 31;
+  int w = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
+  int rows, part, fix;
+  int32_t sb = 0, se = 0;
+  int64_t tile_off = 0, ld, zx = 0;
+  const double* zA = nullptr;
+  int zK = 0;
+  double *dst, *out;
+  const bool isz = w < a.nz;
+  if (isz) {
+    const ZItem it = a.zitems[w];
+    const ZBlock Z = a.zb[it.zb];
+    rows = min(it.nk, Z.r - it.k0);  // without the padding columns of V's rows
+    ld = vpad(Z.r, 8);
+    zA = static_cast<const double*>(Z.V) + int64_t(it.j0) * ld + it.k0;
+    zx = Z.x_off + it.j0;
+    zK = it.j1 - it.j0;
+    part = it.part;
+    fix = it.fix;
+    out = a.in + Z.z_off + it.k0;
+    dst = part < 0 ? out : a.zpart + part;
+  } else {
+    w -= a.nz;
+    if (w >= a.L.nbig + a.L.nsmall) return;
+    const bool big = w < a.L.nbig;
+    const Item it = big ? a.L.big[w] : a.L.small[w - a.L.nbig];
+    const Panel P = a.L.panels[it.panel];
+    constexpr int T = 64;  // tile_rows(8)
+    const int t = big ? it.chunk : 0;
+    rows = min(T, P.m - t * T);
+    ld = P.m > 32 ? tile_height(P.m, t, 8) : P.m;
+    tile_off = int64_t(t) * T;
+    sb = it.seg_b;
+    se = it.seg_e;
+    part = it.part;
+    fix = it.fix;
+    out = a.y + P.yoff + t * T;
+    dst = part < 0 ? out : a.ypart + int64_t(part) * T;
+  }
+#define HODLR_R64(r_)                                                              \
+  case r_:                                                                         \
+    item64<r_>(a.L.segs, sb, se, tile_off, zA, zx, zK, rows, ld, a.in, dst, lane); \
+    break;
+  switch ((rows + 7) / 8) {
+    HODLR_R64(1)
+    HODLR_R64(2)
+    HODLR_R64(3)
+    HODLR_R64(4)
+    HODLR_R64(5)
+    HODLR_R64(6)
+    HODLR_R64(7)
+    HODLR_R64(8)
+    default:
+      break;
+  }
+#undef HODLR_R64
+  if (part < 0) return;
+  if (isz)
+    z_fixup(a.zfix, a.zcnt, fix, a.zpart, a.in, lane);
+  else
+    panel_fixup(a.L.fix, a.L.pcnt, fix, a.ypart, out, rows, lane);
 }
 
 template <typename TX, typename TO>
@@ -1554,41 +1617,54 @@ void z_item_stages(ZItem& it, int r, int esz) {
 
 template <typename TA, typename TACC>
 static void zgemv_t(const ZBlock* zb, const ZItem* items, int nitems, const ZFix* fix, int nfix, void* zpart, void* in,
-                    int64_t ld_in, int nrhs, cudaStream_t st) {
+                    cudaStream_t st) {
   using TI = typename IO<TACC>::TI;
   using TY = typename IO<TACC>::TY;
-  if constexpr (sizeof(TA) == 8) {  // FP64 storage: direct loads
-    dim3 g(warps_grid(nitems), unsigned(nrhs));
-    zgemv_direct_kernel<TA, TACC><<<g, 256, 0, st>>>(zb, items, nitems, static_cast<TY*>(zpart),
-                                                     static_cast<TI*>(in), ld_in);
-  } else {
-    dim3 g(unsigned((nitems + kZWarps - 1) / kZWarps), unsigned(nrhs));
-    cudaFuncSetAttribute(zgemv_kernel<TA, TACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kZWarps * kZWarpSmem);
-    zgemv_kernel<TA, TACC><<<g, kZWarps * 32, kZWarps * kZWarpSmem, st>>>(zb, items, nitems, static_cast<TY*>(zpart),
-                                                                           static_cast<TI*>(in), ld_in);
+  const unsigned g = unsigned((nitems + kZWarps - 1) / kZWarps);
+  cudaFuncSetAttribute(zgemv_kernel<TA, TACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kZWarps * kZWarpSmem);
+  zgemv_kernel<TA, TACC><<<g, kZWarps * 32, kZWarps * kZWarpSmem, st>>>(zb, items, nitems, static_cast<TY*>(zpart),
+                                                                         static_cast<TI*>(in));
+  if (nfix > 0)
+    zfix_kernel<TACC><<<unsigned(nfix), kZPart, 0, st>>>(fix, static_cast<const TY*>(zpart), static_cast<TI*>(in));
+}
+
+cudaError_t launch_items64(const ZBlock* zb, const ZItem* zitems, int nitems, const ZFix* fix, unsigned int* zcnt,
+                           double* zpart, const PanelItems& L, double* ypart, double* in, double* y, cudaStream_t st,
+                           bool contig) {
+  Items64 a{zb, zitems, nitems, fix, zcnt, zpart, L, ypart, in, y};
+  if (contig) a.L.nsmall = 0;
+  const int64_t total = int64_t(nitems) + a.L.nsmall + L.nbig;
+  if (total > 0) {
+    count_launches(1);
+    items64_kernel<<<warps_grid(total), kWarpsPerCta * 32, 0, st>>>(a);
   }
-  if (nfix > 0) {
-    dim3 gf(unsigned((nfix + 255) / 256), unsigned(nrhs));
-    zfix_kernel<TACC><<<gf, 256, 0, st>>>(fix, nfix, static_cast<const TY*>(zpart), static_cast<TI*>(in), ld_in);
+  if (contig && L.nsmall > 0) {
+    count_launches(1);
+    constexpr int bytes = kLWarps * l_warp_smem<double, double>();
+    cudaFuncSetAttribute(panel_leaf_kernel<double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    panel_leaf_kernel<double, double><<<unsigned((L.nsmall + kLWarps - 1) / kLWarps), kLWarps * 32, bytes, st>>>(
+        L.panels, L.segs, L.small, L.nsmall, in, y, ypart);
   }
+  return cudaGetLastError();
 }
 
 cudaError_t launch_zgemv(Prec a, Prec x, const ZBlock* zb, const ZItem* items, int nitems, const ZFix* fix, int nfix,
-                         void* zpart, void* in, int64_t ld_in, int nrhs, cudaStream_t st, Accum acc) {
+                         unsigned int* zcnt, void* zpart, void* in, cudaStream_t st, Accum acc) {
   if (nitems <= 0) return cudaSuccess;
-  count_launches(nfix > 0 ? 2 : 1);
   if (a == Prec::kD && x == Prec::kD)
-    zgemv_t<double, double>(zb, items, nitems, fix, nfix, zpart, in, ld_in, nrhs, st);
-  else if (a == Prec::kF && x == Prec::kD && acc == Accum::kCompensated)
-    zgemv_t<float, DF>(zb, items, nitems, fix, nfix, zpart, in, ld_in, nrhs, st);
+    return launch_items64(zb, items, nitems, fix, zcnt, static_cast<double*>(zpart), PanelItems{}, nullptr,
+                          static_cast<double*>(in), nullptr, st, false);
+  count_launches(nfix > 0 ? 2 : 1);
+  if (a == Prec::kF && x == Prec::kD && acc == Accum::kCompensated)
+    zgemv_t<float, DF>(zb, items, nitems, fix, nfix, zpart, in, st);
   else if (a == Prec::kF && x == Prec::kD && acc == Accum::kRelaxed)
-    zgemv_t<float, FH>(zb, items, nitems, fix, nfix, zpart, in, ld_in, nrhs, st);
+    zgemv_t<float, FH>(zb, items, nitems, fix, nfix, zpart, in, st);
   else if (a == Prec::kB && x == Prec::kD && acc == Accum::kRelaxed)
-    zgemv_t<bf16, FH>(zb, items, nitems, fix, nfix, zpart, in, ld_in, nrhs, st);
+    zgemv_t<bf16, FH>(zb, items, nitems, fix, nfix, zpart, in, st);
   else if (a == Prec::kB && x == Prec::kD)
-    zgemv_t<bf16, DF>(zb, items, nitems, fix, nfix, zpart, in, ld_in, nrhs, st);
+    zgemv_t<bf16, DF>(zb, items, nitems, fix, nfix, zpart, in, st);
   else if (a == Prec::kF && x == Prec::kF)
-    zgemv_t<float, float>(zb, items, nitems, fix, nfix, zpart, in, ld_in, nrhs, st);
+    zgemv_t<float, float>(zb, items, nitems, fix, nfix, zpart, in, st);
   else
     return cudaErrorInvalidValue;
   return cudaGetLastError();
@@ -1596,80 +1672,37 @@ cudaError_t launch_zgemv(Prec a, Prec x, const ZBlock* zb, const ZItem* items, i
 
 // FP32 and BF16 storage: the bulk-copy staged kernels
 template <typename TA, typename TACC>
-static void panels_leaf(const Panel* panels, const Seg* segs, const Item* small, int nsmall, const void* in,
-                        int64_t ld_in, void* ypart, void* y, int64_t ld_y, int nslots, int nrhs, cudaStream_t st) {
+static void panels_t(const PanelItems& L, const void* in, void* ypart, void* y, cudaStream_t st, bool contig) {
   using TI = typename IO<TACC>::TI;
   using TY = typename IO<TACC>::TY;
-  using TX = typename LeafX<TACC>::T;
-  dim3 g(unsigned((nsmall + kLWarps - 1) / kLWarps), unsigned(nrhs));
-  cudaFuncSetAttribute(panel_leaf_kernel<TA, TACC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       kLWarps * l_warp_smem<TA, TX>());
-  panel_leaf_kernel<TA, TACC><<<g, kLWarps * 32, kLWarps * l_warp_smem<TA, TX>(), st>>>(
-      panels, segs, small, nsmall, static_cast<const TI*>(in), ld_in, static_cast<TY*>(y), ld_y, nslots,
-      static_cast<TY*>(ypart));
-}
-
-template <typename TA, typename TACC>
-static void panels_staged(const Panel* panels, const Seg* segs, const Item* small, int nsmall, const Item* big,
-                          int nbig, const void* in, int64_t ld_in, void* ypart, void* y, int64_t ld_y, int nslots,
-                          int nrhs, cudaStream_t st, bool contig) {
-  using TI = typename IO<TACC>::TI;
-  using TY = typename IO<TACC>::TY;
-  if (nbig > 0) {
-    dim3 g(unsigned((nbig + kPWarps - 1) / kPWarps), unsigned(nrhs));
+  const TI* ti = static_cast<const TI*>(in);
+  TY *ty = static_cast<TY*>(y), *tp = static_cast<TY*>(ypart);
+  if (L.nbig > 0) {
     // above the default 48 KB of dynamic shared memory; set on every launch
     // (the attribute is per device and cheap to set)
     cudaFuncSetAttribute(panel_tile_kernel<TA, TACC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          kPWarps * kPWarpSmem);
-    panel_tile_kernel<TA, TACC><<<g, kPWarps * 32, kPWarps * kPWarpSmem, st>>>(
-        panels, segs, big, nbig, static_cast<TY*>(ypart), static_cast<const TI*>(in), ld_in, static_cast<TY*>(y), ld_y,
-        nslots);
+    panel_tile_kernel<TA, TACC><<<unsigned((L.nbig + kPWarps - 1) / kPWarps), kPWarps * 32, kPWarps * kPWarpSmem, st>>>(
+        L.panels, L.segs, L.big, L.nbig, tp, ti, ty);
   }
-  if (nsmall > 0 && contig) {
-    panels_leaf<TA, TACC>(panels, segs, small, nsmall, in, ld_in, ypart, y, ld_y, nslots, nrhs, st);
-  } else if (nsmall > 0) {
-    dim3 g(unsigned((nsmall + kSWarps - 1) / kSWarps), unsigned(nrhs));
-    cudaFuncSetAttribute(panel_small_kernel<TA, TACC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         kSWarps * s_warp_smem<TA>());
-    panel_small_kernel<TA, TACC><<<g, kSWarps * 32, kSWarps * s_warp_smem<TA>(), st>>>(
-        panels, segs, small, nsmall, static_cast<const TI*>(in), ld_in, static_cast<TY*>(y), ld_y, nslots,
-        static_cast<TY*>(ypart));
+  if (L.nsmall > 0 && contig) {
+    using TX = typename LeafX<TACC>::T;
+    constexpr int bytes = kLWarps * l_warp_smem<TA, TX>();
+    cudaFuncSetAttribute(panel_leaf_kernel<TA, TACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    panel_leaf_kernel<TA, TACC><<<unsigned((L.nsmall + kLWarps - 1) / kLWarps), kLWarps * 32, bytes, st>>>(
+        L.panels, L.segs, L.small, L.nsmall, ti, ty, tp);
+  } else if (L.nsmall > 0) {
+    constexpr int bytes = kSWarps * s_warp_smem<TA>();
+    cudaFuncSetAttribute(panel_small_kernel<TA, TACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    panel_small_kernel<TA, TACC><<<unsigned((L.nsmall + kSWarps - 1) / kSWarps), kSWarps * 32, bytes, st>>>(
+        L.panels, L.segs, L.small, L.nsmall, ti, ty, tp);
   }
-}
-
-template <typename TA, typename TACC>
-static void panels_t(const Panel* panels, const Seg* segs, const Item* small, int nsmall, const Item* big, int nbig,
-                     const PanelFix* fix, int nfix, void* ypart, const void* in, int64_t ld_in, void* y, int64_t ld_y,
-                     int nslots, int nrhs, cudaStream_t st, bool contig) {
-  using TI = typename IO<TACC>::TI;
-  using TY = typename IO<TACC>::TY;
-  if constexpr (sizeof(TA) == 8) {  // FP64 storage: direct loads
-    if (nbig > 0) {
-      dim3 g(warps_grid(nbig), unsigned(nrhs));
-      panel_tile_direct_kernel<TA, TACC><<<g, 256, 0, st>>>(panels, segs, big, nbig, static_cast<TY*>(ypart),
-                                                            static_cast<const TI*>(in), ld_in, static_cast<TY*>(y),
-                                                            ld_y, nslots);
-    }
-    if (nsmall > 0 && contig) {
-      panels_leaf<TA, TACC>(panels, segs, small, nsmall, in, ld_in, ypart, y, ld_y, nslots, nrhs, st);
-    } else if (nsmall > 0) {
-      dim3 g(warps_grid(nsmall), unsigned(nrhs));
-      panel_small_direct_kernel<TA, TACC><<<g, 256, 0, st>>>(panels, segs, small, nsmall, static_cast<const TI*>(in),
-                                                             ld_in, static_cast<TY*>(y), ld_y, nslots,
-                                                             static_cast<TY*>(ypart));
-    }
-  } else {
-    panels_staged<TA, TACC>(panels, segs, small, nsmall, big, nbig, in, ld_in, ypart, y, ld_y, nslots, nrhs, st,
-                            contig);
-  }
-  if (nfix > 0) {
+  if (L.nfix > 0) {
     const int rows = int(tile_rows(int(sizeof(TA))));
-    dim3 gf(unsigned((int64_t(nfix) * rows + 255) / 256), unsigned(nrhs));
-    panel_fix_kernel<TY><<<gf, 256, 0, st>>>(panels, fix, nfix, rows, static_cast<const TY*>(ypart),
-                                             static_cast<TY*>(y), ld_y, nslots);
+    panel_fix_kernel<TY><<<unsigned((int64_t(L.nfix) * rows + 255) / 256), 256, 0, st>>>(L.panels, L.fix, L.nfix, rows,
+                                                                                          tp, ty);
   }
 }
-
 
 bool small_items_contiguous(const std::vector<Panel>& panels, const std::vector<Seg>& segs,
                             const std::vector<Item>& small, int esz) {
@@ -1690,30 +1723,23 @@ bool small_items_contiguous(const std::vector<Panel>& panels, const std::vector<
   return true;
 }
 
-cudaError_t launch_panels(Prec a, Prec x, const Panel* panels, const Seg* segs, const Item* small, int nsmall,
-                          const Item* big, int nbig, const PanelFix* fix, int nfix, void* ypart, const void* in,
-                          int64_t ld_in, void* y, int64_t ld_y, int nslots, int nrhs, cudaStream_t st, Accum acc,
-                          bool contig) {
-  if (nsmall + nbig <= 0) return cudaSuccess;
-  count_launches(uint64_t(nbig > 0) + uint64_t(nsmall > 0) + uint64_t(nfix > 0));
+cudaError_t launch_panels(Prec a, Prec x, const PanelItems& L, void* ypart, const void* in, void* y, cudaStream_t st,
+                          Accum acc, bool contig) {
+  if (L.nsmall + L.nbig <= 0) return cudaSuccess;
   if (a == Prec::kD && x == Prec::kD)
-    panels_t<double, double>(panels, segs, small, nsmall, big, nbig, fix, nfix, ypart, in, ld_in, y, ld_y, nslots,
-                             nrhs, st, contig);
-  else if (a == Prec::kF && x == Prec::kD && acc == Accum::kCompensated)
-    panels_t<float, DF>(panels, segs, small, nsmall, big, nbig, fix, nfix, ypart, in, ld_in, y, ld_y, nslots, nrhs,
-                        st, contig);
+    return launch_items64(nullptr, nullptr, 0, nullptr, nullptr, nullptr, L, static_cast<double*>(ypart),
+                          static_cast<double*>(const_cast<void*>(in)), static_cast<double*>(y), st, contig);
+  count_launches(uint64_t(L.nbig > 0) + uint64_t(L.nsmall > 0) + uint64_t(L.nfix > 0));
+  if (a == Prec::kF && x == Prec::kD && acc == Accum::kCompensated)
+    panels_t<float, DF>(L, in, ypart, y, st, contig);
   else if (a == Prec::kF && x == Prec::kD && acc == Accum::kRelaxed)
-    panels_t<float, FH>(panels, segs, small, nsmall, big, nbig, fix, nfix, ypart, in, ld_in, y, ld_y, nslots, nrhs,
-                        st, contig);
+    panels_t<float, FH>(L, in, ypart, y, st, contig);
   else if (a == Prec::kB && x == Prec::kD && acc == Accum::kRelaxed)
-    panels_t<bf16, FH>(panels, segs, small, nsmall, big, nbig, fix, nfix, ypart, in, ld_in, y, ld_y, nslots, nrhs,
-                       st, contig);
+    panels_t<bf16, FH>(L, in, ypart, y, st, contig);
   else if (a == Prec::kB && x == Prec::kD)
-    panels_t<bf16, DF>(panels, segs, small, nsmall, big, nbig, fix, nfix, ypart, in, ld_in, y, ld_y, nslots, nrhs,
-                       st, contig);
+    panels_t<bf16, DF>(L, in, ypart, y, st, contig);
   else if (a == Prec::kF && x == Prec::kF)
-    panels_t<float, float>(panels, segs, small, nsmall, big, nbig, fix, nfix, ypart, in, ld_in, y, ld_y, nslots, nrhs,
-                           st, contig);
+    panels_t<float, float>(L, in, ypart, y, st, contig);
   else
     return cudaErrorInvalidValue;
   return cudaGetLastError();
@@ -1818,6 +1844,36 @@ __global__ void split_kernel(const double* __restrict__ x, float2* __restrict__ 
 cudaError_t launch_split(const double* x, void* out, int64_t n, cudaStream_t st) {
   count_launches(1);
   split_kernel<<<vec_grid(n), 256, 0, st>>>(x, static_cast<float2*>(out), n);
+  return cudaGetLastError();
+}
+
+template <typename T, bool SPLIT>
+__global__ void prep_kernel(const T* __restrict__ x, const int64_t* __restrict__ perm, int64_t n, T* __restrict__ in,
+                            float2* __restrict__ in2, T* __restrict__ y, int nslots) {
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+    const T v = x[perm ? perm[i] : i];
+    in[i] = v;
+    if constexpr (SPLIT) {
+      const float h = __double2float_rn(v);
+      in2[i] = make_float2(h, __double2float_rn(v - double(h)));
+    }
+    for (int s = 1; s < nslots; s++) y[int64_t(s) * n + i] = T(0);
+  }
+}
+
+cudaError_t launch_prep(Prec x, const void* src, const int64_t* perm, int64_t n, void* in, void* in2, void* y,
+                        int nslots, cudaStream_t st) {
+  count_launches(1);
+  const unsigned g = vec_grid(n);
+  if (x == Prec::kF)
+    prep_kernel<float, false><<<g, 256, 0, st>>>(static_cast<const float*>(src), perm, n, static_cast<float*>(in),
+                                                 nullptr, static_cast<float*>(y), nslots);
+  else if (in2)
+    prep_kernel<double, true><<<g, 256, 0, st>>>(static_cast<const double*>(src), perm, n, static_cast<double*>(in),
+                                                 static_cast<float2*>(in2), static_cast<double*>(y), nslots);
+  else
+    prep_kernel<double, false><<<g, 256, 0, st>>>(static_cast<const double*>(src), perm, n, static_cast<double*>(in),
+                                                  nullptr, static_cast<double*>(y), nslots);
   return cudaGetLastError();
 }
 
@@ -2114,13 +2170,15 @@ __global__ void __launch_bounds__(256) zfix_mr_kernel(const ZFix* __restrict__ f
                                                      const float* __restrict__ zpart, int64_t zpart_ld,
                                                      float* __restrict__ in, int64_t ld_in) {
   const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  const int f = int(t / kMR), c = int(t % kMR);
+  const int64_t fc = t / kMR;
+  const int f = int(fc / kZPart), k = int(fc % kZPart), c = int(t % kMR);
   if (f >= nfix) return;
   const ZFix F = fix[f];
+  if (k >= F.nk) return;
   const float* zp = zpart + int64_t(blockIdx.y) * zpart_ld * kMR;
   float acc = 0.f;
-  for (int q = 0; q < F.count; q++) acc += zp[(int64_t(F.part) + int64_t(q) * kZPart) * kMR + c];
-  in[int64_t(blockIdx.y) * ld_in * kMR + F.zpos * kMR + c] = acc;
+  for (int q = 0; q < F.count; q++) acc += zp[(int64_t(F.part) + int64_t(q) * kZPart + k) * kMR + c];
+  in[int64_t(blockIdx.y) * ld_in * kMR + (F.zpos + k) * kMR + c] = acc;
 }
 
 // Leaf panels (m <= 32): one warp per item; lane c keeps m sums.  The item's
@@ -2448,7 +2506,7 @@ cudaError_t launch_zgemv_mr(const ZBlock* zb, const ZItem* items, int nitems, co
   dim3 g(unsigned((nitems + kMWarps - 1) / kMWarps), unsigned(nchunks));
   zgemv_mr_kernel<<<g, kMWarps * 32, kMWarps * kMWarpSmem, st>>>(zb, items, nitems, zpart, zpart_ld, in, ld_in);
   if (nfix > 0) {
-    dim3 gf(unsigned((int64_t(nfix) * kMR + 255) / 256), unsigned(nchunks));
+    dim3 gf(unsigned((int64_t(nfix) * kZPart * kMR + 255) / 256), unsigned(nchunks));
     zfix_mr_kernel<<<gf, 256, 0, st>>>(fix, nfix, zpart, zpart_ld, in, ld_in);
   }
   return cudaGetLastError();

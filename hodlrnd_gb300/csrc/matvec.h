@@ -77,16 +77,19 @@ struct Item {
   int32_t chunk;
   int32_t seg_b, seg_e;
   int32_t part;
+  int32_t fix;  // the PanelFix its partial sums belong to (part >= 0)
 };
 
 // Sum of `count` partial row blocks (parts part .. part+count-1) into the
-// output slot of rows chunk * rows_per_item .. of the panel.
+// output slot of rows chunk * rows_per_item .. of the panel.  The last of the
+// count items to finish adds them (a counter per fix, zero between launches),
+// so the sum needs no launch of its own; its order is the parts' order.
 struct PanelFix {
   int32_t panel;
   int32_t chunk;
   int32_t part;
   int32_t count;
-}; 
+};
 
 
 // V factors are stored row major, n x vpad(r): each row's r values padded to a
@@ -112,6 +115,7 @@ struct ZItem {
   int32_t j0, j1;  // rows j0 .. j1 - 1
   int32_t part;    // < 0: write z; else partial sums at zpart[part + c], c < nk
   int32_t R, nst;  // items of whole rows (staged): V rows per ring stage, stage count; else 0, 0
+  int32_t fix;     // the ZFix its partial sums belong to (part >= 0)
 };
 // Sets R and nst of an item of block rank r stored with esz-byte elements.
 void z_item_stages(ZItem& it, int r, int esz);
@@ -123,11 +127,14 @@ constexpr int kZPart = 128;          // partial-sum stride of one item (>= any n
 #endif
 constexpr int kZItemBytes = HODLR_TUNE_Z_ITEM_BYTES;
 
-// z[zpos] = sum_{q < count} zpart[part + q * kZPart]
+// z[zpos + c] = sum_{q < count} zpart[part + q * kZPart + c], c < nk; added as
+// for PanelFix
 struct ZFix {
   int64_t zpos;
   int32_t part;
   int32_t count;
+  int32_t nk;
+  int32_t pad;
 };
 
 // Element types: A = stored matrix, X = vectors, ACC = accumulation.
@@ -155,9 +162,10 @@ __host__ __device__ inline uint64_t far_v_bytes(int64_t n, int64_t r, bool dense
   return far_v_data_bytes(n, r, dense, p) + ((p == Prec::kB && !dense) ? round16(uint64_t(r) * 4) : 0);
 }
 
-// in:   input buffer [x (ld_in rows of x) | z], nrhs columns with leading dimension ld_in
-// y:    output slots, slot s of column c at y + (c * nslots + s) * ld_y
-// zpart / ypart: scratch of the vector precision (one column of partials).
+// in:   input buffer [x | z]
+// y:    output slots (panel rows at P.yoff)
+// zpart / ypart: scratch of the vector precision.
+// zcnt / pcnt: one counter per fix, zero before and after a launch.
 // acc, for FP32 matrices with FP64 vectors: the input buffer `in` holds each
 // FP64 value split into an (hi, lo) FP32 pair (launch_split), z is written in
 // the same form, outputs and partial sums stay FP64, and products are summed
@@ -166,16 +174,30 @@ __host__ __device__ inline uint64_t far_v_bytes(int64_t n, int64_t r, bool dense
 // Other type pairs ignore it.
 enum class Accum { kByType, kCompensated, kRelaxed };
 cudaError_t launch_zgemv(Prec a, Prec x, const ZBlock* zb, const ZItem* items, int nitems, const ZFix* fix, int nfix,
-                         void* zpart, void* in, int64_t ld_in, int nrhs, cudaStream_t st,
-                         Accum acc = Accum::kByType);
+                         unsigned int* zcnt, void* zpart, void* in, cudaStream_t st, Accum acc = Accum::kByType);
 // `small` items belong to panels of at most 32 rows, `big` ones to larger panels.
 // contig: every small item's segments lie in memory in segment order, each
 // after the end of the previous one (small_items_contiguous), so that the
 // item's factors can be streamed as one byte run.
-cudaError_t launch_panels(Prec a, Prec x, const Panel* panels, const Seg* segs, const Item* small, int nsmall,
-                          const Item* big, int nbig, const PanelFix* fix, int nfix, void* ypart, const void* in,
-                          int64_t ld_in, void* y, int64_t ld_y, int nslots, int nrhs, cudaStream_t st,
+struct PanelItems {
+  const Panel* panels;
+  const Seg* segs;
+  const Item* small;
+  const Item* big;
+  int nsmall, nbig;
+  const PanelFix* fix;
+  int nfix;
+  unsigned int* pcnt;
+};
+cudaError_t launch_panels(Prec a, Prec x, const PanelItems& L, void* ypart, const void* in, void* y, cudaStream_t st,
                           Accum acc = Accum::kByType, bool contig = false);
+// FP64 matrices and vectors: z = V^T x (nitems = 0: none) and the panels of L
+// (no items: none) in one launch; they are independent of each other when L
+// is the near field.  contig: L's small items are unsplit and their segments
+// follow one another in memory; they take the staged leaf kernel.
+cudaError_t launch_items64(const ZBlock* zb, const ZItem* zitems, int nitems, const ZFix* fix, unsigned int* zcnt,
+                           double* zpart, const PanelItems& L, double* ypart, double* in, double* y, cudaStream_t st,
+                           bool contig);
 // Whether the segments of every small item (panels of at most 32 rows) with
 // esz-byte elements follow one another in memory, as launch_panels' contig asks.
 bool small_items_contiguous(const std::vector<Panel>& panels, const std::vector<Seg>& segs,
@@ -232,6 +254,11 @@ cudaError_t launch_batch_combine_mr(const BatchInst* inst, int count, int64_t ma
 
 // out[i] = (hi, lo) FP32 pair of x[i] (hi = x rounded to FP32, lo = the rest)
 cudaError_t launch_split(const double* x, void* out, int64_t n, cudaStream_t st);
+// A product's inputs in one pass: in[i] = x[perm ? perm[i] : i], in2[i] = its
+// (hi, lo) pair (in2 non-null; FP64 vectors), and the output slots 1 ..
+// nslots - 1 (n rows each, which some level's panels may not cover) zeroed.
+cudaError_t launch_prep(Prec x, const void* src, const int64_t* perm, int64_t n, void* in, void* in2, void* y,
+                        int nslots, cudaStream_t st);
 
 // Copies to `host` (pinned) the number of times a streaming kernel on this
 // device gave up waiting for its bulk copies since the library was loaded
