@@ -2,11 +2,18 @@
 #include "device.cuh"
 #include "gmres.h"
 
+#include <algorithm>
 #include <cmath>
 
 namespace hodlr {
 
 namespace {
+
+#define HODLR_TRY(x)                      \
+  do {                                    \
+    cudaError_t e_ = (x);                 \
+    if (e_ != cudaSuccess) return e_;     \
+  } while (0)
 
 constexpr int kThreads = 256;
 
@@ -275,15 +282,510 @@ __global__ void givens_kernel(double* __restrict__ H, int ldh, double* __restric
   scal[0] = fabs(s[i + 1]) / scal[2];
 }
 
+// ---- one Arnoldi step in one launch ------------------------------------------
+// Everything after the product A v_i -- the orthogonalisation, the norm,
+// v_{i+1}, the rotations and the residual estimate -- in one kernel, for
+// vectors short enough that the separate kernels are all start-up (MGS: i + 2
+// launches of 4-8 us; CGS2: nine, 65 us at n = 20011).
+
+// The rotations and the residual estimate (givens_kernel) by one thread, from
+// shared memory: first the earlier rotations cs, sn applied to the Hessenberg
+// column h[0 .. i] (hcol gets its entries 0 .. i - 1; the running entry i is
+// returned), then, once the column's last entry hn is known, the new rotation.
+__device__ __forceinline__ double step_rotate(const double* h, const double* cs, const double* sn, int i, double* hcol) {
+  double hk = h[0];
+  for (int k = 0; k < i; k++) {
+    double hk1 = h[k + 1];
+    apply_rot(hk, hk1, cs[k], sn[k]);
+    hcol[k] = hk;
+    hk = hk1;
+  }
+  return hk;
+}
+__device__ __forceinline__ void step_new_rotation(double hk, double hn, int i, double* hcol, double* rot, int restart,
+                                                  double* scal, double* hres) {
+  double* rcs = rot;
+  double* rsn = rot + (restart + 1);
+  double* rs = rot + 2 * (restart + 1);
+  double hi1 = hn, c, s;
+  gen_rot(hk, hi1, c, s);
+  apply_rot(hk, hi1, c, s);
+  rcs[i] = c;
+  rsn[i] = s;
+  hcol[i] = hk;
+  hcol[i + 1] = hi1;
+  double s0 = rs[i], s1 = rs[i + 1];
+  apply_rot(s0, s1, c, s);
+  rs[i] = s0;
+  rs[i + 1] = s1;
+  const double res = fabs(s1) / scal[2];
+  scal[0] = res;
+  *hres = res;
+}
+
+template <typename T>
+struct StepArgs {
+  const T* w;
+  T* V;
+  int64_t n;
+  int i;        // Arnoldi index: w against v_0 .. v_i, v_{i+1} written
+  double* H;
+  int ldh;
+  double* rot;
+  int restart;  // the allocated one (rot's layout)
+  double* scal;
+  double* hres;  // host-visible: [0] residual estimate, [1] nonzero after a wait gave up
+  // CGS2
+  float2* part;             // kStepMaxBasis x kStepGrid partial pairs, two sets, and the norm's
+  unsigned long long* bar;  // grid barrier arrivals
+  int cached;               // the basis slices fit in shared memory
+};
+
+// MGS: a cluster of CTAs (16, or 8 where 16 do not fit), each with a slice of
+// the vectors; w stays in registers and the next basis vector is loaded before
+// the sum is waited for.  A sum over the cluster is one store per CTA into
+// every other CTA's shared memory and a hardware cluster barrier.  FP64
+// operations (16 cycles a warp on an SM) bound the rest, so a CTA has few
+// threads with up to 8 elements each, and one warp finishes each sum.
+// About 3 us per basis vector (n = 10000, 19 steps: 33 us a step against 100 for
+// the separate kernels); with 640 one-element threads per CTA the FP64 sums of
+// idle-handed warps made it 8 us.
+constexpr int64_t kStepMaxN = 40960;
+constexpr int kStepMaxBasis = 256;  // restart + 1 at most
+constexpr int kStepCtas = 16;
+constexpr int kStepEpt = 8;         // elements per thread at most
+constexpr int kStepThreads = 640;   // 8 CTAs x 640 x 8 = kStepMaxN
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// *p in CTA `cta`'s shared memory = v (p: the address in this CTA's)
+__device__ __forceinline__ void cluster_store(double* p, uint32_t cta, double v) {
+  const uint32_t a = uint32_t(__cvta_generic_to_shared(p));
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(cta));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"(v) : "memory");
+}
+
+__host__ __device__ inline int64_t step_slice(int64_t n, int ctas) { return (n + ctas - 1) / ctas; }
+
+template <typename T>
+__global__ void __launch_bounds__(kStepThreads, 1) mgs_cluster_kernel(const StepArgs<T> a) {
+  __shared__ double slots[2][kStepCtas];  // the CTAs' sums, used in turn
+  __shared__ double red[kStepThreads / 32], total;
+  __shared__ double h[kStepMaxBasis], cs[kStepMaxBasis], sn[kStepMaxBasis];
+  const uint32_t me = cluster_rank(), nc = cluster_size();
+  const int64_t E = step_slice(a.n, int(nc)), e0 = int64_t(me) * E;
+  const int cnt = int(max(int64_t(0), min(E, a.n - e0)));
+  const int t = threadIdx.x, nt = blockDim.x, nv = a.i + 1;
+  const int lane = t & 31, wid = t >> 5, nw = nt >> 5;
+  T* V = a.V + e0;
+  if (me == 0)
+    for (int k = t; k < a.i; k += nt) {
+      cs[k] = a.rot[k];
+      sn[k] = a.rot[a.restart + 1 + k];
+    }
+  T wr[kStepEpt], vr[kStepEpt], vn[kStepEpt];
+#pragma unroll
+  for (int q = 0; q < kStepEpt; q++) {
+    const int e = t + q * nt;
+    wr[q] = e < cnt ? a.w[e0 + e] : T(0);
+    vr[q] = e < cnt ? V[e] : T(0);
+    vn[q] = T(0);
+  }
+  double acc = 0.0;
+#pragma unroll
+  for (int q = 0; q < kStepEpt; q++)
+    if (q * nt < cnt) acc += to_d(wr[q]) * to_d(vr[q]);
+  // no CTA stores into another's shared memory before that one has started
+  cluster_barrier();
+  int set = 0;
+  // the sum of acc over the cluster, the same value in every thread
+  auto cluster_sum = [&](double v) -> double {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) red[wid] = v;
+    __syncthreads();
+    if (wid == 0) {
+      v = lane < nw ? red[lane] : 0.0;
+      for (int o = 16; o > 0; o >>= 1)
+        if (o < nw) v += __shfl_xor_sync(0xffffffffu, v, o);
+      v = __shfl_sync(0xffffffffu, v, 0);
+      if (lane < int(nc)) cluster_store(&slots[set][me], uint32_t(lane), v);
+    }
+    cluster_barrier();
+    if (wid == 0) {
+      v = lane < int(nc) ? slots[set][lane] : 0.0;
+#pragma unroll
+      for (int o = kStepCtas / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) total = v;
+    }
+    set ^= 1;
+    __syncthreads();
+    return total;
+  };
+  for (int k = 0; k < nv; k++) {
+    if (k + 1 < nv) {
+      const T* vk = V + int64_t(k + 1) * a.n;
+#pragma unroll
+      for (int q = 0; q < kStepEpt; q++) {
+        const int e = t + q * nt;
+        if (e < cnt) vn[q] = vk[e];
+      }
+    }
+    const double hk = cluster_sum(acc);
+    if (t == 0) h[k] = hk;
+    acc = 0.0;
+#pragma unroll
+    for (int q = 0; q < kStepEpt; q++) {
+      if (q * nt < cnt) {
+        wr[q] = T(axmy(to_d(wr[q]), hk, to_d(vr[q])));
+        vr[q] = vn[q];
+        acc += to_d(wr[q]) * to_d(k + 1 < nv ? vr[q] : wr[q]);
+      }
+    }
+  }
+  const double hn = sqrt(cluster_sum(acc));
+  const double ih = 1.0 / hn;
+  T* out = V + int64_t(nv) * a.n;
+#pragma unroll
+  for (int q = 0; q < kStepEpt; q++) {
+    const int e = t + q * nt;
+    if (e < cnt) out[e] = T(__dmul_rn(ih, to_d(wr[q])));
+  }
+  if (me == 0 && t == 0) {
+    double* hcol = a.H + int64_t(a.i) * a.ldh;
+    step_new_rotation(step_rotate(h, cs, sn, a.i, hcol), hn, a.i, hcol, a.rot, a.restart, a.scal, a.hres);
+  }
+}
+
+// CGS2: every SM has a slice of the vectors (a cooperative launch, whose CTAs
+// meet at three grid barriers): the projections of a pass are each CTA's
+// partial pairs, summed by every CTA after the barrier.  The products are those
+// of cgs_dots_kernel and cgs_update_kernel (dot2_add, pair_add, one FP64
+// subtraction per element and pass); the basis slices are split once into
+// shared memory where they fit and serve both passes from there.
+// n = 20011, 50 basis vectors: 36 us a step against 75 for the nine kernels; a
+// cluster of 16 CTAs took 105 (its 16 SMs are bound by the splits and products).
+constexpr int kStepGrid = 152;
+constexpr int kCgsThreads = 512;
+constexpr int kCgsWarps = kCgsThreads / 32;
+constexpr int kCgsSliceBytes = 128 * 1024;  // basis slices in shared memory at most
+constexpr unsigned long long kBarrierNs = 2000000000ull;
+
+// a slice: a multiple of 32 elements
+__host__ __device__ inline int cgs_slice(int64_t n) { return int((step_slice(n, kStepGrid - 1) + 31) / 32 * 32); }
+// CTAs: one per slice and one for the rotations, kStepGrid at most
+__host__ inline int cgs_grid(int64_t n) { return int((n + cgs_slice(n) - 1) / cgs_slice(n)) + 1; }
+__host__ inline size_t cgs_smem(int64_t n, int nv, bool cached) {
+  return size_t(cgs_slice(n)) * (sizeof(double) + sizeof(float2)) + (cached ? size_t(nv) * cgs_slice(n) * sizeof(float2) : 0);
+}
+
+// Arrives at the grid barrier and waits for every CTA (at most 2 s); false
+// after a give-up.
+__device__ __forceinline__ bool grid_barrier(unsigned long long* bar) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    const unsigned long long g = gridDim.x, mine = atomicAdd(bar, 1ull), goal = (mine / g + 1) * g;
+    unsigned long long t0, t1;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    int good = 1;
+    for (;;) {
+      unsigned long long v;
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(bar) : "memory");
+      if (v >= goal) break;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+      if (t1 - t0 > kBarrierNs) {
+        good = 0;
+        break;
+      }
+    }
+    __threadfence();
+    ok = good;
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kCgsThreads, 1) cgs2_step_kernel(const StepArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char csm[];
+  __shared__ double h[kStepMaxBasis], cs[kStepMaxBasis], sn[kStepMaxBasis];
+  __shared__ float2 hs[kStepMaxBasis], pairs[kCgsThreads], nrm;
+  const int E = cgs_slice(a.n), G = gridDim.x, cta = blockIdx.x;
+  const int64_t e0 = int64_t(cta) * E;
+  const int cnt = int(max(int64_t(0), min(int64_t(E), a.n - e0)));
+  double* wd = reinterpret_cast<double*>(csm);
+  float2* sw = reinterpret_cast<float2*>(wd + E);
+  float2* sv = sw + E;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nv = a.i + 1;
+  T* V = a.V + e0;
+  // the last CTA has no slice: it applies the earlier rotations to the column
+  // while the others form the second pass's update (one thread, a chain of FP64
+  // operations, 8 us at 50 columns)
+  const bool rotor = cta == G - 1;
+  double hk = 0.0;
+  if (rotor)
+    for (int k = t; k < a.i; k += kCgsThreads) {
+      cs[k] = a.rot[k];
+      sn[k] = a.rot[a.restart + 1 + k];
+    }
+  for (int e = t; e < E; e += kCgsThreads) {
+    const T v = e < cnt ? a.w[e0 + e] : T(0);
+    wd[e] = to_d(v);
+    sw[e] = split_t(v);
+  }
+  if (a.cached && !rotor) {
+    for (int q = wid; q < nv; q += kCgsWarps)
+#pragma unroll 4
+      for (int e = lane; e < E; e += 32) sv[q * E + e] = e < cnt ? split_t(V[int64_t(q) * a.n + e]) : make_float2(0.f, 0.f);
+  }
+  __syncthreads();
+  // the update's warps: EG groups of 32 elements by JG shares of the vectors
+  const int EG = E / 32, JG = max(1, kCgsWarps / EG);
+  const int eg0 = wid % min(EG, kCgsWarps), jg = wid / min(EG, kCgsWarps);
+  float ns = 0.f, nk = 0.f;
+  for (int pass = 0; pass < 2; pass++) {
+    float2* part = a.part + int64_t(pass) * kStepMaxBasis * kStepGrid;
+    for (int j = wid; j < nv; j += kCgsWarps) {
+      float as = 0.f, ac = 0.f;
+      if (rotor) {
+      } else if (a.cached) {
+        const float2* vj = sv + j * E;
+#pragma unroll 4
+        for (int e = lane; e < E; e += 32) dot2_add(as, ac, vj[e], sw[e]);
+      } else {
+        const T* vj = V + int64_t(j) * a.n;
+#pragma unroll 8
+        for (int e = lane; e < cnt; e += 32) dot2_add(as, ac, split_t(vj[e]), sw[e]);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        pair_add(as, ac, __shfl_xor_sync(0xffffffffu, as, o), __shfl_xor_sync(0xffffffffu, ac, o));
+      if (lane == 0) __stcg(part + int64_t(j) * kStepGrid + cta, make_float2(as, ac));
+    }
+    if (!grid_barrier(a.bar)) {
+      if (t == 0) a.hres[1] = 1.0;
+      return;
+    }
+    for (int j = wid; j < nv; j += kCgsWarps) {
+      float as = 0.f, ac = 0.f;
+#pragma unroll
+      for (int q = 0; q < (kStepGrid + 31) / 32; q++) {
+        const int c = lane + 32 * q;
+        const float2 p = c < G ? __ldcg(part + int64_t(j) * kStepGrid + c) : make_float2(0.f, 0.f);
+        pair_add(as, ac, p.x, p.y);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        pair_add(as, ac, __shfl_xor_sync(0xffffffffu, as, o), __shfl_xor_sync(0xffffffffu, ac, o));
+      if (lane == 0) {
+        const double v = __dadd_rn(double(as), double(ac));
+        h[j] = pass ? __dadd_rn(h[j], v) : v;
+        hs[j] = split_d(v);
+      }
+    }
+    __syncthreads();
+    if (rotor) {
+      if (pass && t == 0) hk = step_rotate(h, cs, sn, a.i, a.H + int64_t(a.i) * a.ldh);
+      continue;
+    }
+    for (int b = 0; b < EG; b += kCgsWarps) {
+      const int eg = b + eg0, e = eg * 32 + lane;
+      const bool act = eg < EG && jg < JG;
+      float s = 0.f, c = 0.f;
+      if (act && e < cnt) {
+        if (a.cached) {
+#pragma unroll 4
+          for (int j = jg; j < nv; j += JG) dot2_add(s, c, sv[j * E + e], hs[j]);
+        } else {
+#pragma unroll 8
+          for (int j = jg; j < nv; j += JG) dot2_add(s, c, split_t(V[int64_t(j) * a.n + e]), hs[j]);
+        }
+      }
+      pairs[t] = make_float2(s, c);
+      __syncthreads();
+      if (act && jg == 0 && e < cnt) {
+        for (int g = 1; g < JG; g++) {
+          const float2 q = pairs[(g * min(EG, kCgsWarps) + eg0) * 32 + lane];
+          pair_add(s, c, q.x, q.y);
+        }
+        const T v = T(__dsub_rn(wd[e], __dadd_rn(double(s), double(c))));
+        const float2 vs = split_t(v);
+        wd[e] = to_d(v);
+        sw[e] = vs;
+        if (pass) dot2_add(ns, nk, vs, vs);
+      }
+      __syncthreads();
+    }
+  }
+  // |w|: the CTA's pair, then every CTA's
+  float2* npart = a.part + int64_t(2) * kStepMaxBasis * kStepGrid;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    pair_add(ns, nk, __shfl_xor_sync(0xffffffffu, ns, o), __shfl_xor_sync(0xffffffffu, nk, o));
+  if (lane == 0) pairs[wid] = make_float2(ns, nk);
+  __syncthreads();
+  if (t == 0) {
+    ns = nk = 0.f;
+    for (int q = 0; q < kCgsWarps; q++) pair_add(ns, nk, pairs[q].x, pairs[q].y);
+    __stcg(npart + cta, make_float2(ns, nk));  // the last CTA's is zero, as its projections are
+  }
+  if (!grid_barrier(a.bar)) {
+    if (t == 0) a.hres[1] = 1.0;
+    return;
+  }
+  if (wid == 0) {
+    ns = nk = 0.f;
+#pragma unroll
+    for (int q = 0; q < (kStepGrid + 31) / 32; q++) {
+      const int c = lane + 32 * q;
+      const float2 p = c < G ? __ldcg(npart + c) : make_float2(0.f, 0.f);
+      pair_add(ns, nk, p.x, p.y);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      pair_add(ns, nk, __shfl_xor_sync(0xffffffffu, ns, o), __shfl_xor_sync(0xffffffffu, nk, o));
+    if (lane == 0) nrm = make_float2(ns, nk);
+  }
+  __syncthreads();
+  const double hn = sqrt(__dadd_rn(double(nrm.x), double(nrm.y)));
+  const double ih = 1.0 / hn;
+  T* out = V + int64_t(nv) * a.n;
+  for (int e = t; e < cnt; e += kCgsThreads) out[e] = T(__dmul_rn(ih, wd[e]));
+  if (rotor && t == 0)
+    step_new_rotation(hk, hn, a.i, a.H + int64_t(a.i) * a.ldh, a.rot, a.restart, a.scal, a.hres);
+}
+
+// What the MGS cluster of c CTAs is launched with.
+cudaLaunchConfig_t mgs_config(int64_t n, int c, cudaLaunchAttribute* at, cudaStream_t st) {
+  const int64_t E = step_slice(n, c);
+  cudaLaunchConfig_t cfg{};
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = unsigned(c);
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cfg.gridDim = dim3(unsigned(c));
+  // about 5 elements per thread, 8 at most
+  cfg.blockDim = dim3(unsigned(std::min<int64_t>(kStepThreads, std::max<int64_t>(128, (E / 5 + 31) / 32 * 32))));
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// CTAs of the MGS cluster for vectors of n elements on this device; 0: the
+// separate kernels.
+template <typename T>
+int mgs_ctas(int64_t n, int restart) {
+  if (n > kStepMaxN || restart + 1 > kStepMaxBasis) return 0;
+  for (int c : {kStepCtas, kStepCtas / 2}) {
+    cudaLaunchAttribute at{};
+    const cudaLaunchConfig_t cfg = mgs_config(n, c, &at, nullptr);
+    int clusters = 0;
+    if (cudaFuncSetAttribute(&mgs_cluster_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, &mgs_cluster_kernel<T>, &cfg) == cudaSuccess && clusters > 0)
+      return c;
+    cudaGetLastError();
+  }
+  return 0;
+}
+
+// Whether the CGS2 step kernel takes vectors of n elements on this device.
+template <typename T>
+bool cgs_step_fits(int64_t n, int restart) {
+  if (n > kStepMaxN || restart + 1 > kStepMaxBasis) return false;
+  int dev = 0, sms = 0, coop = 0, per = 0;
+  const bool ok =
+      cudaGetDevice(&dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
+      cudaFuncSetAttribute(&cgs2_step_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           int(kCgsSliceBytes + cgs_smem(kStepMaxN, 0, false))) == cudaSuccess &&
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, &cgs2_step_kernel<T>, kCgsThreads,
+                                                    kCgsSliceBytes + cgs_smem(n, 0, false)) == cudaSuccess &&
+      int64_t(per) * sms >= cgs_grid(n);
+  if (!ok) cudaGetLastError();
+  return ok;
+}
+
+template <typename T>
+cudaError_t launch_mgs_step(const StepArgs<T>& a, int ctas, cudaStream_t st) {
+  cudaLaunchAttribute at{};
+  const cudaLaunchConfig_t cfg = mgs_config(a.n, ctas, &at, st);
+  count_launches(1);
+  return cudaLaunchKernelEx(&cfg, &mgs_cluster_kernel<T>, a);
+}
+
+template <typename T>
+cudaError_t launch_cgs_step(StepArgs<T> a, cudaStream_t st) {
+  const size_t basis = size_t(a.i + 1) * size_t(cgs_slice(a.n)) * sizeof(float2);
+  a.cached = basis <= size_t(kCgsSliceBytes);
+  count_launches(1);
+  void* args[] = {&a};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(&cgs2_step_kernel<T>), dim3(unsigned(cgs_grid(a.n))),
+                                     dim3(kCgsThreads), args, cgs_smem(a.n, a.i + 1, a.cached != 0), st);
+}
+
 // Update (GMRES.hpp:132-146): back substitution into y.
-__global__ void backsolve_kernel(const double* H, int ldh, double* rot, int restart, int k) {
+// One CTA: thread j keeps y_j (Q of them, 1024 apart, for long restarts) and
+// subtracts column i of H times y_i as soon as y_i is known, the operations of
+// the serial loop in its order; the next column is loaded meanwhile.
+// 100 columns: 44 us against 428 for one thread (19: 14 us against 43).
+template <int Q>
+__global__ void __launch_bounds__(1024) backsolve_kernel(const double* __restrict__ H, int ldh, double* rot, int restart,
+                                                         int k) {
+  __shared__ double yi[2];
   const double* s = rot + 2 * (restart + 1);
   double* y = rot + 3 * (restart + 1);
-  for (int i = 0; i <= k; i++) y[i] = s[i];
-  for (int i = k; i >= 0; i--) {
-    y[i] /= H[i + int64_t(i) * ldh];
-    for (int j = i - 1; j >= 0; j--) y[j] = __dsub_rn(y[j], __dmul_rn(H[j + int64_t(i) * ldh], y[i]));
+  const int t = threadIdx.x;
+  double v[Q], hc[Q], hn[Q];
+#pragma unroll
+  for (int q = 0; q < Q; q++) {
+    const int j = t + q * 1024;
+    v[q] = j <= k ? s[j] : 0.0;
+    hc[q] = j <= k ? H[j + int64_t(k) * ldh] : 0.0;
+    hn[q] = 0.0;
   }
+  for (int i = k; i >= 0; i--) {
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      const int j = t + q * 1024;
+      if (j < i) hn[q] = H[j + int64_t(i - 1) * ldh];
+      if (j == i) {
+        v[q] = v[q] / hc[q];
+        yi[i & 1] = v[q];
+        y[i] = v[q];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < Q; q++)
+      if (t + q * 1024 < i) {
+        v[q] = __dsub_rn(v[q], __dmul_rn(hc[q], yi[i & 1]));
+        hc[q] = hn[q];
+      }
+  }
+}
+
+void launch_backsolve(const double* H, int ldh, double* rot, int restart, int k, cudaStream_t st) {
+  count_launches(1);
+  if (k < 1024)
+    backsolve_kernel<1><<<1, unsigned((k + 32) / 32 * 32), 0, st>>>(H, ldh, rot, restart, k);
+  else
+    backsolve_kernel<2><<<1, 1024, 0, st>>>(H, ldh, rot, restart, k);
 }
 
 // x += sum_j V_j y_j, accumulated j by j as the reference does.
@@ -322,12 +824,6 @@ __global__ void fill_zero_kernel(T* x, int64_t n) {
   for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n; i += int64_t(kVecCtas) * kThreads) x[i] = T(0);
 }
 
-#define HODLR_TRY(x)                      \
-  do {                                    \
-    cudaError_t e_ = (x);                 \
-    if (e_ != cudaSuccess) return e_;     \
-  } while (0)
-
 }  // namespace
 
 template <typename T>
@@ -348,6 +844,13 @@ cudaError_t gmres_alloc(GmresWork<T>& W, int64_t n, int restart) {
   HODLR_TRY(cudaMalloc(&W.hc, sizeof(double) * size_t(restart + 1)));
   HODLR_TRY(cudaMalloc(&W.scal, sizeof(double) * 8));
   HODLR_TRY(cudaMallocHost(&W.hscal, sizeof(double) * 8));
+  W.mgs_ctas = mgs_ctas<T>(n, restart);
+  W.cgs_step = cgs_step_fits<T>(n, restart);
+  if (W.cgs_step) {
+    HODLR_TRY(cudaMalloc(&W.step_part, sizeof(float2) * (2 * kStepMaxBasis + 1) * kStepGrid));
+    HODLR_TRY(cudaMalloc(&W.step_bar, sizeof(unsigned long long)));
+    HODLR_TRY(cudaMemset(W.step_bar, 0, sizeof(unsigned long long)));
+  }
   return cudaSuccess;
 }
 
@@ -363,6 +866,8 @@ void gmres_free(GmresWork<T>& W) {
   cudaFree(W.partk);
   cudaFree(W.hc);
   cudaFree(W.scal);
+  cudaFree(W.step_part);
+  cudaFree(W.step_bar);
   if (W.hscal) cudaFreeHost(W.hscal);
   W = GmresWork<T>();
 }
@@ -437,42 +942,55 @@ cudaError_t gmres_solve(GmresWork<T>& W, const TreeMatvec<T>& A, const T* b, T* 
     for (int i = 0; i < m && j <= max_iter; i++, j++) {
       T* vi = W.V + int64_t(i) * n;
       HODLR_TRY(A(vi, W.w));
-      double* plast;
-      if (ortho == Ortho::kMGS) {
-        count_launches(1);
-        dot_partial_kernel<T><<<kVecCtas, kThreads, 0, st>>>(W.w, W.V, n, part0);
-        for (int k = 0; k <= i; k++) {
-          const T* next = k < i ? W.V + int64_t(k + 1) * n : nullptr;
-          double* pin = (k & 1) ? part1 : part0;
-          double* pout = (k & 1) ? part0 : part1;
-          count_launches(1);
-          mgs_step_kernel<T><<<kVecCtas, kThreads, 0, st>>>(W.w, W.V + int64_t(k) * n, next, n, pin, pout,
-                                                             W.H + k + int64_t(i) * ldh);
+      const bool mgs = ortho == Ortho::kMGS;
+      if (mgs ? W.mgs_ctas > 0 : W.cgs_step) {
+        const StepArgs<T> sa{W.w,       W.V,    n,       i,           W.H,
+                             ldh,       W.rot,  W.restart, W.scal,    W.hscal,
+                             static_cast<float2*>(W.step_part), W.step_bar, 0};
+        W.hscal[1] = 0.0;
+        HODLR_TRY(mgs ? launch_mgs_step<T>(sa, W.mgs_ctas, st) : launch_cgs_step<T>(sa, st));
+        HODLR_TRY(cudaStreamSynchronize(st));
+        if (W.hscal[1] != 0.0) {  // a grid barrier gave up
+          HODLR_TRY(cudaMemset(W.step_bar, 0, sizeof(unsigned long long)));
+          return cudaErrorLaunchTimeout;
         }
-        plast = (i & 1) ? part0 : part1;
       } else {
-        // CGS2: two classical passes against v_0 .. v_i, |w|^2 from the second
-        for (int pass = 0; pass < 2; pass++) {
-          count_launches(3);
-          cgs_dots_kernel<T><<<dim3(kDotCtas, unsigned((i + 1 + kDotGroup - 1) / kDotGroup)), kThreads, 0, st>>>(
-              W.w, W.V, n, i + 1, W.partk);
-          cgs_reduce_kernel<<<i + 1, kThreads, 0, st>>>(W.partk, W.hc, W.H + int64_t(i) * ldh, pass);
-          cgs_update_kernel<T><<<kVecCtas, kThreads, 0, st>>>(W.w, W.V, n, i + 1, W.hc, pass == 1 ? part0 : nullptr);
+        double* plast;
+        if (mgs) {
+          count_launches(1);
+          dot_partial_kernel<T><<<kVecCtas, kThreads, 0, st>>>(W.w, W.V, n, part0);
+          for (int k = 0; k <= i; k++) {
+            const T* next = k < i ? W.V + int64_t(k + 1) * n : nullptr;
+            double* pin = (k & 1) ? part1 : part0;
+            double* pout = (k & 1) ? part0 : part1;
+            count_launches(1);
+            mgs_step_kernel<T><<<kVecCtas, kThreads, 0, st>>>(W.w, W.V + int64_t(k) * n, next, n, pin, pout,
+                                                               W.H + k + int64_t(i) * ldh);
+          }
+          plast = (i & 1) ? part0 : part1;
+        } else {
+          // CGS2: two classical passes against v_0 .. v_i, |w|^2 from the second
+          for (int pass = 0; pass < 2; pass++) {
+            count_launches(3);
+            cgs_dots_kernel<T><<<dim3(kDotCtas, unsigned((i + 1 + kDotGroup - 1) / kDotGroup)), kThreads, 0, st>>>(
+                W.w, W.V, n, i + 1, W.partk);
+            cgs_reduce_kernel<<<i + 1, kThreads, 0, st>>>(W.partk, W.hc, W.H + int64_t(i) * ldh, pass);
+            cgs_update_kernel<T><<<kVecCtas, kThreads, 0, st>>>(W.w, W.V, n, i + 1, W.hc, pass == 1 ? part0 : nullptr);
+          }
+          plast = part0;
         }
-        plast = part0;
+        count_launches(2);
+        norm_recip_kernel<<<1, kThreads, 0, st>>>(plast, W.H + (i + 1) + int64_t(i) * ldh, W.scal + 4);
+        normalize_kernel<T><<<kVecCtas, kThreads, 0, st>>>(W.w, W.V + int64_t(i + 1) * n, n, W.scal + 4);
+        count_launches(1);
+        givens_kernel<<<1, 1, 0, st>>>(W.H, ldh, W.rot, W.restart, i, W.scal);
+        HODLR_TRY(cudaGetLastError());
+        HODLR_TRY(host_scal(1));
       }
-      count_launches(2);
-      norm_recip_kernel<<<1, kThreads, 0, st>>>(plast, W.H + (i + 1) + int64_t(i) * ldh, W.scal + 4);
-      normalize_kernel<T><<<kVecCtas, kThreads, 0, st>>>(W.w, W.V + int64_t(i + 1) * n, n, W.scal + 4);
-      count_launches(1);
-      givens_kernel<<<1, 1, 0, st>>>(W.H, ldh, W.rot, W.restart, i, W.scal);
-      HODLR_TRY(cudaGetLastError());
-      HODLR_TRY(host_scal(1));
       resid = W.hscal[0];
       if (progress) progress(resid);
       if (resid < tol) {
-        count_launches(1);
-        backsolve_kernel<<<1, 1, 0, st>>>(W.H, ldh, W.rot, W.restart, i);
+        launch_backsolve(W.H, ldh, W.rot, W.restart, i, st);
         count_launches(1);
         update_x_kernel<T><<<kVecCtas, kThreads, 0, st>>>(x, W.V, n, W.rot, W.restart, i, n);
         HODLR_TRY(cudaGetLastError());
@@ -482,8 +1000,7 @@ cudaError_t gmres_solve(GmresWork<T>& W, const TreeMatvec<T>& A, const T* b, T* 
         return cudaStreamSynchronize(st);
       }
     }
-    count_launches(1);
-    backsolve_kernel<<<1, 1, 0, st>>>(W.H, ldh, W.rot, W.restart, m - 1);
+    launch_backsolve(W.H, ldh, W.rot, W.restart, m - 1, st);
     count_launches(1);
     update_x_kernel<T><<<kVecCtas, kThreads, 0, st>>>(x, W.V, n, W.rot, W.restart, m - 1, n);
     if (progress) progress(1.0);  // the restart's true residual

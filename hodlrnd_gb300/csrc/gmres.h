@@ -17,6 +17,7 @@
 //   launches at any step, and the same orthogonality as MGS or better
 //   (Giraud, Langou, Rozloznik, "The loss of orthogonality in the
 //   Gram-Schmidt processes", Comput. Math. Appl. 50 (2005)).
+// Short vectors take either in one launch per step (mgs_cluster_kernel, cgs2_step_kernel).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -43,6 +44,13 @@ struct GmresWork {
   double* hc = nullptr;    // restart + 1 projection coefficients of one CGS pass
   double* scal = nullptr; // device scalars: [0] resid, [1] beta, [2] normb
   double* hscal = nullptr;  // pinned host mirror of scal
+  // an Arnoldi step in one launch: CTAs of the MGS cluster (0: separate
+  // kernels), whether the CGS2 kernel takes it, and the latter's partial sums
+  // and barrier counter
+  int mgs_ctas = 0;
+  bool cgs_step = false;
+  void* step_part = nullptr;
+  unsigned long long* step_bar = nullptr;
 };
 
 template <typename T>
