@@ -11,6 +11,7 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/hodlrnd.h"
@@ -256,12 +257,12 @@ struct hodlr_op {
   Plan plan_ref;
   // tensor-core products for 64 right-hand sides (BF16 factors; built on first use)
   struct TcPlan {
-    // one launch per (family, small / big, rows bucket): items of at most
+    // one launch per (family, rows bucket): items of at most
     // `rows` output rows, so each launch holds just the tensor memory and
     // shared memory its items need
     struct Run {
       const void* items;  // Item (panels) or TcZGroup (z)
-      int n, rows, big;
+      int n, rows;
     };
     bool built = false;
     std::vector<Run> near, far, z;
@@ -273,6 +274,16 @@ struct hodlr_op {
     int nzfix = 0, zfix_rows = 0;
     uint32_t* in = nullptr;  // [x | z], 64 right-hand sides, packed BF16 pairs
     float *y = nullptr, *part_near = nullptr, *part_far = nullptr, *zpart = nullptr;
+    // panels of at most 32 rows (TcLeafArgs)
+    TcLeafSeg *leaf_near_segs = nullptr, *leaf_far_segs = nullptr;
+    int32_t *leaf_near = nullptr, *leaf_far = nullptr;
+    TcLeafSrc* leaf_srcs = nullptr;
+    TcLeafBatch* leaf_batches = nullptr;
+    TcLeafRun* leaf_runs = nullptr;
+    int nleaf_runs = 0;
+    TcUnit* units = nullptr;
+    uint4* xunits = nullptr;
+    int64_t nunits = 0;
     unsigned int* status = nullptr;
     unsigned int* h_status = nullptr;
   } tc;
@@ -2352,24 +2363,22 @@ int tc_bucket(int rows) {
   return b;
 }
 
-// Items of the tensor-core panel kernels for one family of panels: per panel,
-// its row tiles (one for panels of at most 32 rows) times runs of whole
-// segments of at most kTcColsPerItem columns (a longer segment alone) and at
-// most kTcMaxSegs segments -- a CTA works through an item's columns one
-// 16-column step after another, so long items would leave most SMs idle at
-// the end of a launch.  Runs after the first write partial row blocks that a
-// fix-up adds in order.  Items are listed by launch: small then big panels,
-// each by rows bucket; runs[] gets one entry per non-empty launch (offsets
-// into the items until the array is uploaded).
+// Items of the tcgen05 panel kernels for one family of panels, those above 32
+// rows: per panel, its 64-row chunks times runs of whole segments of at most
+// kTcColsPerItem columns (a longer segment alone) and at most kTcMaxSegs
+// segments -- a CTA works through an item's columns one 32-column step after
+// another, so long items would leave most SMs idle at the end of a launch.
+// Runs after the first write partial row blocks that a fix-up adds in order.
+// Items are listed by launch, one per rows bucket; runs[] gets one entry per
+// non-empty launch (offsets into the items until the array is uploaded).
 constexpr int kTcColsPerItem = 256;
-void tc_panel_items(const std::vector<Panel>& panels, const std::vector<Seg>& segs, std::vector<Item>& items, std::vector<hodlr_op::TcPlan::Run>& runs, std::vector<PanelFix>& fix,
-                    int& nparts) {
-  std::vector<Item> by[2][5];  // [big][bucket]
+void tc_panel_items(const std::vector<Panel>& panels, const std::vector<Seg>& segs, std::vector<Item>& items,
+                    std::vector<hodlr_op::TcPlan::Run>& runs, std::vector<PanelFix>& fix, int& nparts) {
+  std::vector<Item> by[3];  // buckets of 16, 32, 64 rows
   std::vector<std::pair<int32_t, int32_t>> cut;
   for (size_t pi = 0; pi < panels.size(); pi++) {
     const Panel& P = panels[pi];
-    const int64_t ns = P.seg_end - P.seg_begin;
-    if (ns <= 0 || P.m <= 0) continue;
+    if (P.seg_end <= P.seg_begin || P.m <= 32) continue;
     cut.clear();
     int64_t start = P.seg_begin, cols = 0;
     for (int64_t q = P.seg_begin; q < P.seg_end; q++) {
@@ -2383,31 +2392,127 @@ void tc_panel_items(const std::vector<Panel>& panels, const std::vector<Seg>& se
     }
     cut.push_back({int32_t(start), int32_t(P.seg_end)});
     const int nruns = int(cut.size());
-    const bool is_big = P.m > 32;
-    const int tiles = is_big ? int((P.m + kTcRows - 1) / kTcRows) : 1;
-    for (int tl = 0; tl < tiles; tl++) {
-      const int rows = is_big ? std::min<int>(kTcRows, P.m - tl * kTcRows) : P.m;
+    for (int tl = 0; tl < int((P.m + kTcRows - 1) / kTcRows); tl++) {
+      const int rows = std::min<int>(kTcRows, P.m - tl * kTcRows);
       int bk = 0;
       while ((16 << bk) < rows) bk++;
       if (nruns > 1) fix.push_back({int32_t(pi), tl, nparts, nruns});
-      for (int q = 0; q < nruns; q++) {
-        Item it{};
-        it.panel = int32_t(pi);
-        it.chunk = tl;
-        it.seg_b = cut[size_t(q)].first;
-        it.seg_e = cut[size_t(q)].second;
-        it.part = nruns > 1 ? nparts++ : -1;
-        by[is_big][bk].push_back(it);
-      }
+      for (int q = 0; q < nruns; q++)
+        by[bk].push_back({int32_t(pi), tl, cut[size_t(q)].first, cut[size_t(q)].second, nruns > 1 ? nparts++ : -1, -1});
     }
   }
-  for (int big = 0; big < 2; big++)
-    for (int bk = 0; bk < 5; bk++) {
-      const std::vector<Item>& v = by[big][bk];
-      if (v.empty()) continue;
-      runs.push_back({reinterpret_cast<const void*>(items.size()), int(v.size()), 16 << bk, big});
-      items.insert(items.end(), v.begin(), v.end());
+  for (int bk = 0; bk < 3; bk++) {
+    if (by[bk].empty()) continue;
+    runs.push_back({reinterpret_cast<const void*>(items.size()), int(by[bk].size()), 16 << bk});
+    items.insert(items.end(), by[bk].begin(), by[bk].end());
+  }
+}
+
+// Work of the leaf-level kernel (TcLeafArgs) for one family of panels, those of
+// at most 32 rows: groups of kTcLeafGroup consecutive ones, the union of each
+// group's sources in the order of their points, in batches, and runs of at most
+// kTcLeafRunSrcs sources -- enough CTAs for every SM to have several, few
+// partial blocks.  segs[q] of a panel has the source (first point src_off[q],
+// segs[q].n points); a longer source than a batch holds is cut into pieces,
+// whose products add up.  out: the segments in batch order.
+constexpr int kTcLeafRunSrcs = 160;
+struct TcLeafHost {
+  std::vector<TcLeafSrc> srcs;
+  std::vector<TcLeafBatch> batches;
+  std::vector<TcLeafRun> runs;
+  std::vector<TcUnit> units;
+  std::unordered_map<int64_t, std::vector<std::pair<int32_t, int32_t>>> unit_of;  // first point -> (points, first unit)
+  int32_t source_units(int64_t x_off, int32_t n) {
+    auto& v = unit_of[x_off];
+    for (const auto& e : v)
+      if (e.first == n) return e.second;
+    const int32_t u0 = int32_t(units.size());
+    for (int32_t p = 0; p < n; p += 8) units.push_back({x_off + p, std::min(8, n - p), 0});
+    v.push_back({n, u0});
+    return u0;
+  }
+};
+void tc_leaf_work(const std::vector<Panel>& panels, const std::vector<TcLeafSeg>& segs,
+                  const std::vector<int64_t>& src_off, bool near, TcLeafHost& H, std::vector<TcLeafSeg>& out,
+                  std::vector<int32_t>& list, std::vector<PanelFix>& fix, int& nparts) {
+  constexpr int32_t most = 8 * kTcLeafUnits;  // points of a source's piece
+  for (size_t p = 0; p < panels.size(); p++)
+    if (panels[p].m <= 32 && panels[p].seg_end > panels[p].seg_begin) list.push_back(int32_t(p));
+  out.reserve(segs.size());
+  struct Piece {
+    int64_t off;
+    int32_t n, warp;
+    int32_t seg, j;  // segment and first point of the piece
+  };
+  std::vector<Piece> pieces;
+  for (size_t b = 0; b < list.size(); b += kTcLeafGroup) {
+    const int count = int(std::min<size_t>(kTcLeafGroup, list.size() - b));
+    pieces.clear();
+    for (int w = 0; w < count; w++) {
+      const Panel& P = panels[size_t(list[b + size_t(w)])];
+      for (int64_t q = P.seg_begin; q < P.seg_end; q++)
+        for (int32_t j = 0; j < segs[size_t(q)].n; j += most)
+          pieces.push_back({src_off[size_t(q)] + j, std::min(most, segs[size_t(q)].n - j), w, int32_t(q), j});
     }
+    std::sort(pieces.begin(), pieces.end(), [](const Piece& x, const Piece& y) {
+      return x.off != y.off ? x.off < y.off : x.n != y.n ? x.n < y.n : x.warp < y.warp;
+    });
+    const int32_t batch0 = int32_t(H.batches.size()), src0 = int32_t(H.srcs.size());
+    for (size_t k = 0; k < pieces.size();) {
+      // a batch: whole sources while they fit (a panel has one segment per source)
+      TcLeafBatch B{};
+      B.src_b = int32_t(H.srcs.size());
+      B.seg_b = int32_t(out.size());
+      int32_t units = 0;
+      const size_t first = k;
+      std::vector<std::pair<size_t, int32_t>> at;  // end of each source's pieces, its first unit
+      while (k < pieces.size()) {
+        size_t e = k;
+        while (e < pieces.size() && pieces[e].off == pieces[k].off && pieces[e].n == pieces[k].n) e++;
+        const int32_t u = (pieces[k].n + 7) / 8;
+        if (k > first && (units + u > kTcLeafUnits || e - first > size_t(kTcLeafSegs) || at.size() >= 32)) break;
+        H.srcs.push_back({H.source_units(pieces[k].off, pieces[k].n), pieces[k].n});
+        at.push_back({e, units});
+        units += u;
+        k = e;
+      }
+      B.src_e = int32_t(H.srcs.size());
+      for (int w = 0; w < kTcLeafGroup; w++) {
+        B.warp_off[w] = int32_t(out.size()) - B.seg_b;
+        size_t p = first;
+        for (const auto& src : at)
+          for (; p < src.first; p++) {
+            if (pieces[p].warp != w) continue;
+            const Piece& f = pieces[p];
+            TcLeafSeg C = segs[size_t(f.seg)];
+            if (C.n > most) {
+              const int32_t m = panels[size_t(list[b + size_t(w)])].m;
+              if (C.V) {
+                C.V += int64_t(f.j) * C.vstride;
+              } else {
+                C.A = static_cast<const char*>(C.A) + int64_t(f.j) * m * (near ? 8 : 2);
+                if (C.scale) C.scale += f.j;
+                C.K = f.n;
+              }
+              C.n = f.n;
+            }
+            C.unit = src.second;
+            out.push_back(C);
+          }
+      }
+      B.warp_off[kTcLeafGroup] = int32_t(out.size()) - B.seg_b;
+      H.batches.push_back(B);
+    }
+    const int32_t nb = int32_t(H.batches.size()) - batch0, nsrc = int32_t(H.srcs.size()) - src0;
+    if (nb == 0) continue;
+    const int32_t runs = std::min(nb, (nsrc + kTcLeafRunSrcs - 1) / kTcLeafRunSrcs);
+    if (runs > 1)
+      for (int w = 0; w < count; w++) fix.push_back({list[b + size_t(w)], 0, nparts + w * runs, runs});
+    for (int32_t r = 0; r < runs; r++)
+      H.runs.push_back({near ? 1 : 0, int32_t(b), count, batch0 + int32_t(int64_t(nb) * r / runs),
+                        batch0 + int32_t(int64_t(nb) * (r + 1) / runs), runs > 1 ? nparts + r : -1, runs});
+    if (runs > 1) nparts += count * runs;
+  }
 }
 
 void build_tc_plan(hodlr_op* op, cudaStream_t st) {
@@ -2420,23 +2525,56 @@ void build_tc_plan(hodlr_op* op, cudaStream_t st) {
   int pn = 0, pf = 0;
   tc_panel_items(h.panels_near, h.segs_near, ni, T.near, fxn, pn);
   tc_panel_items(h.panels_far, h.segs_far, fi, T.far, fxf, pf);
+  // panels of at most 32 rows: their segments, and the groups' work
+  const Tree& t = op->tree;
+  TcLeafHost H;
+  std::vector<TcLeafSeg> lns(h.segs_near.size()), lfs(h.segs_far.size());
+  std::vector<int64_t> ons(h.segs_near.size()), ofs(h.segs_far.size());
+  for (size_t q = 0; q < h.segs_near.size(); q++) {
+    const Seg& S = h.segs_near[q];
+    lns[q] = {S.A, nullptr, nullptr, S.K, S.K, 0, 0};
+    ons[q] = S.in_off;
+  }
+  // far segments follow the far blocks (dense, or of positive rank) in order
+  std::vector<char> leaf_block(op->far.size(), 0);
+  {
+    size_t seg = 0;
+    for (size_t q = 0; q < op->far.size(); q++) {
+      if (!op->dense[q] && op->rank[q] <= 0) continue;
+      const int64_t gt = t.gid(op->far[q].level, op->far[q].t), gs = t.gid(op->far[q].level, op->far[q].s);
+      const size_t k = seg++;
+      if (t.count[size_t(gt)] > 32) continue;
+      leaf_block[q] = 1;
+      const Seg& S = h.segs_far[k];
+      lfs[k] = {S.A,
+                op->dense[q] ? nullptr : static_cast<const uint16_t*>(op->vptr[q]),
+                op->dense[q] ? S.cscale : op->zsptr[q],
+                int32_t(t.count[size_t(gs)]),
+                S.K,
+                op->dense[q] ? 0 : int32_t(op->vstride[q]),
+                0};
+      ofs[k] = t.begin[size_t(gs)];
+    }
+    if (seg != h.segs_far.size()) throw Failure{HODLR_ERR_STATE, "tensor-core plan: far segments and blocks disagree"};
+  }
+  std::vector<int32_t> lnl, lfl;
+  std::vector<TcLeafSeg> bfs, bns;
+  tc_leaf_work(h.panels_far, lfs, ofs, false, H, bfs, lfl, fxf, pf);
+  tc_leaf_work(h.panels_near, lns, ons, true, H, bns, lnl, fxn, pn);
   // z groups: the rows of z by source node, at most kTcRows rows per group.
-  // Rows are (z block, k0, nk) runs: with source chunks each low-rank block's
-  // own columns of its chunk (its padding columns skipped), else every column
-  // of each z block.  A node is its first point and its size: a node and its
+  // Rows are (z block, k0, nk) runs, each low-rank block's own columns of its
+  // chunk (its padding columns skipped).  A node is its first point and its size: a node and its
   // first child start at the same point.
   struct ZRun {
     int32_t zb, k0, nk;
   };
   std::vector<ZRun> runs;
-  if (!op->vchunk_of.empty()) {
+  {
     for (size_t q = 0; q < op->far.size(); q++) {
       const int32_t c = op->vchunk_of[q];
-      if (c < 0) continue;
+      if (c < 0 || leaf_block[q]) continue;  // leaf panels form their own z
       runs.push_back({c, int32_t(op->zpos[q] - op->vchunks[size_t(c)].zbase), op->rank[q]});
     }
-  } else {
-    for (size_t q = 0; q < h.zb.size(); q++) runs.push_back({int32_t(q), 0, h.zb[q].r});
   }
   auto same_source = [&](const ZBlock& a, const ZBlock& b) { return a.x_off == b.x_off && a.n == b.n; };
   std::stable_sort(runs.begin(), runs.end(), [&](const ZRun& x, const ZRun& y) {
@@ -2508,7 +2646,7 @@ void build_tc_plan(hodlr_op* op, cudaStream_t st) {
     for (const TcZGroup& g : zg)
       if (tc_bucket(g.rows) == (16 << bk)) zgs.push_back(g);
     if (zgs.size() > b0)
-      T.z.push_back({reinterpret_cast<const void*>(b0), int(zgs.size() - b0), 16 << bk, 0});
+      T.z.push_back({reinterpret_cast<const void*>(b0), int(zgs.size() - b0), 16 << bk});
   }
   const Item* d_ni = upload(op->mem, ni, st, "tensor-core near items");
   const Item* d_fi = upload(op->mem, fi, st, "tensor-core far items");
@@ -2516,6 +2654,17 @@ void build_tc_plan(hodlr_op* op, cudaStream_t st) {
   for (auto& r : T.near) r.items = d_ni + reinterpret_cast<size_t>(r.items);
   for (auto& r : T.far) r.items = d_fi + reinterpret_cast<size_t>(r.items);
   for (auto& r : T.z) r.items = d_zg + reinterpret_cast<size_t>(r.items);
+  T.leaf_near = upload(op->mem, lnl, st, "tensor-core leaf panels");
+  T.leaf_far = upload(op->mem, lfl, st, "tensor-core leaf panels");
+  T.leaf_near_segs = upload(op->mem, bns, st, "tensor-core leaf segments");
+  T.leaf_far_segs = upload(op->mem, bfs, st, "tensor-core leaf segments");
+  T.leaf_srcs = upload(op->mem, H.srcs, st, "tensor-core leaf sources");
+  T.leaf_batches = upload(op->mem, H.batches, st, "tensor-core leaf batches");
+  T.leaf_runs = upload(op->mem, H.runs, st, "tensor-core leaf runs");
+  T.nleaf_runs = int(H.runs.size());
+  T.units = upload(op->mem, H.units, st, "tensor-core input units");
+  T.nunits = int64_t(H.units.size());
+  T.xunits = op->mem.alloc_n<uint4>(size_t(std::max<int64_t>(T.nunits, 1)) * 128, "tensor-core input fragments");
   T.fix_near = upload(op->mem, fxn, st, "tensor-core near fix-ups");
   T.fix_far = upload(op->mem, fxf, st, "tensor-core far fix-ups");
   T.nfix_near = int(fxn.size());
@@ -2561,12 +2710,19 @@ void apply_tc(hodlr_op* op, const float* x, int64_t ldx, float* y, int64_t ldy, 
   }
   CK(launch_tc_zfix(T.zfix, T.nzfix, T.zfix_rows, T.zrows, T.zpart, T.in, st));
   a.nz = 0;
-  // near field (FP64 tiles, three BF16 terms), then the far field (BF16)
+  // near field (FP64 tiles, three BF16 terms) and far field (BF16): leaf-level
+  // panels first, then the larger ones
+  CK(launch_tc_units(T.in, T.units, T.nunits, T.xunits, st));
+  const TcLeafArgs la{P.panels_near,   P.panels_far,     T.leaf_near,  T.leaf_far,  T.leaf_near_segs,
+                      T.leaf_far_segs, T.leaf_srcs, T.leaf_batches, T.leaf_runs,
+                      T.nleaf_runs,    T.xunits,         T.y,          T.part_near, T.part_far,
+                      T.status};
+  CK(launch_tc_leaf(la, nrhs, st));
   a.panels = P.panels_near;
   a.segs = P.segs_near;
   a.part = T.part_near;
   for (const auto& r : T.near) {
-    a.items = static_cast<const Item*>(r.items), a.nitems = r.n, a.big = r.big, a.nmax = r.rows;
+    a.items = static_cast<const Item*>(r.items), a.nitems = r.n, a.nmax = r.rows;
     CK(launch_tc(kTcNear, a, st));
   }
   CK(launch_tc_fix(P.panels_near, T.fix_near, T.nfix_near, T.part_near, T.y, st));
@@ -2574,7 +2730,7 @@ void apply_tc(hodlr_op* op, const float* x, int64_t ldx, float* y, int64_t ldy, 
   a.segs = P.segs_far;
   a.part = T.part_far;
   for (const auto& r : T.far) {
-    a.items = static_cast<const Item*>(r.items), a.nitems = r.n, a.big = r.big, a.nmax = r.rows;
+    a.items = static_cast<const Item*>(r.items), a.nitems = r.n, a.nmax = r.rows;
     CK(launch_tc(kTcFar, a, st));
   }
   CK(launch_tc_fix(P.panels_far, T.fix_far, T.nfix_far, T.part_far, T.y, st));

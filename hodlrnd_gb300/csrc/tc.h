@@ -30,8 +30,9 @@ constexpr int kTcMaxSegs = 256;  // segments of one panel item (the host splits 
 // kTcRows rows.
 constexpr int kTcRows = 64;
 
-// kind of product: z = V^T x (one item per low-rank block), near-field panels
-// (FP64 tiles), far-field panels (BF16 dense tiles and U factors)
+// kind of product, for panels above 32 rows: z = V^T x, near-field panels (FP64
+// tiles), far-field panels (BF16 dense tiles and U factors).  Panels of at most
+// 32 rows, their low-rank blocks included, take the kernel of tcleaf.cu.
 enum TcKind { kTcZ = 0, kTcNear = 1, kTcFar = 2 };
 
 // z = V^T x for the low-rank blocks with one source node, grouped: the
@@ -49,9 +50,11 @@ struct TcZGroup {
   int32_t part;    // < 0: the group writes z; else its partial sums go to part block `part` (a fix-up adds them)
   int32_t col0;    // the first column's point within the source node (its row of V): 0 unless a column run
 };
+// (512: with 256, the leaves' parents of 4D N = 65536, 256 points on average,
+// were split half the time, and adding their partial sums took 278 us.)
 // A source node with more points than kTcZCols is split into column runs
 // whose partial sums (blocks of kTcRows rows x 64) a fix-up adds into z.
-constexpr int kTcZCols = 256;
+constexpr int kTcZCols = 512;
 struct TcZRow {        // row i of a split group: where its z goes
   int64_t zpos;
   const float* zscale;  // the row's z scale (BF16), or null
@@ -71,8 +74,7 @@ struct TcLaunch {
   const Panel* panels;
   const Seg* segs;
   const Item* items;
-  int nitems;
-  int big;          // items are 64-row chunks of panels above 32 rows
+  int nitems;       // 64-row chunks of panels above 32 rows
   // z products: blocks, groups by source node, group entries
   const ZBlock* zb;
   const TcZGroup* zgroups;
@@ -81,7 +83,62 @@ struct TcLaunch {
   int nmax;         // largest output row count of the launch's items (N before padding)
 };
 
-// One launch per kind (and small / big items); asynchronous on st.
+// ---- leaf-level products (tcleaf.cu): panels of at most 32 rows ----
+// One segment of such a panel: a near tile (FP64) or a dense far tile (BF16,
+// scale: its column scales), columns = the source's n points; or a low-rank
+// block (V non-null): U m x K, V n x vstride row major, scale: z's K scales.
+struct alignas(16) TcLeafSeg {
+  const void* A;
+  const uint16_t* V;
+  const float* scale;
+  int32_t n;
+  int32_t K;
+  int32_t vstride;
+  int32_t unit;  // its source's first unit within the batch
+};
+// 8 points of a source (n < 8 in its last unit): one operand fragment set
+struct TcUnit {
+  int64_t x_off;
+  int32_t n, pad;
+};
+constexpr int kTcUnitBytes = 2048;  // 64 right-hand sides x 8 points, high and low parts
+constexpr int kTcLeafGroup = 8;     // panels of a group: one per warp of a CTA
+// a batch of sources: at most kTcLeafUnits units, kTcLeafSegs segments and 32
+// sources (two stages of 45 KB, two CTAs per SM)
+constexpr int kTcLeafUnits = 20;
+constexpr int kTcLeafSegs = 96;
+struct TcLeafSrc {
+  int32_t xunit, n;  // first unit; points (at most 8 kTcLeafUnits)
+};
+struct alignas(16) TcLeafBatch {
+  int32_t src_b, src_e;
+  int32_t seg_b;                       // its segments, by panel of the group:
+  int32_t warp_off[kTcLeafGroup + 1];  // panel w's are seg_b + warp_off[w] .. warp_off[w + 1] - 1
+};
+// A group's run of batches: panels panel0 .. panel0 + count - 1 of the near or
+// far list; part < 0: the outputs, else panel w's partial block part + w * part_stride.
+struct TcLeafRun {
+  int32_t near, panel0, count;
+  int32_t batch_b, batch_e;
+  int32_t part, part_stride;
+};
+struct TcLeafArgs {
+  const Panel *near_panels, *far_panels;
+  const int32_t *near_list, *far_list;  // the panels of at most 32 rows
+  const TcLeafSeg *near_segs, *far_segs;  // in batch order
+  const TcLeafSrc* srcs;
+  const TcLeafBatch* batches;
+  const TcLeafRun* runs;
+  int nruns;
+  const uint4* xunits;  // 128 per unit
+  float* y;
+  float *part_near, *part_far;  // part blocks of kTcRows x 64
+  unsigned int* status;
+};
+cudaError_t launch_tc_units(const uint32_t* in, const TcUnit* units, int64_t nunits, uint4* out, cudaStream_t st);
+cudaError_t launch_tc_leaf(const TcLeafArgs& a, int nrhs, cudaStream_t st);
+
+// One launch per kind and rows bucket; asynchronous on st.
 cudaError_t launch_tc(TcKind kind, const TcLaunch& a, cudaStream_t st);
 // in[p * 64 + r] = split(x[perm[p] + r * ld_x]) (x in caller order, column major FP32), p < n,
 // r < nrhs (<= 64); columns r >= nrhs are zero

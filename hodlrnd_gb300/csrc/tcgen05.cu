@@ -233,10 +233,10 @@ __global__ void __launch_bounds__(kTcThreads) tc_kernel(TcLaunch a, int npad_max
       const Item I = a.items[item];
       const Panel P = a.panels[I.panel];
       m = P.m;
-      // big panels: rows row0 .. row0 + 63, inside one storage tile (its rows a multiple of 64)
-      row0 = a.big ? I.chunk * kTcRows : 0;
+      // rows row0 .. row0 + 63, inside one storage tile (its rows a multiple of 64)
+      row0 = I.chunk * kTcRows;
       tile = int(row0 / tile_rows(int(sizeof(TB))));
-      rows = a.big ? min(kTcRows, m - row0) : m;
+      rows = min(kTcRows, m - row0);
       qb = I.seg_b;
       nseg = I.seg_e - I.seg_b;
       if (I.part < 0) {
@@ -310,13 +310,9 @@ __global__ void __launch_bounds__(kTcThreads) tc_kernel(TcLaunch a, int npad_max
             col.pos = S.in_off + j;
             if (S.cscale) col.scale = __ldg(S.cscale + j);
             const TB* A = static_cast<const TB*>(S.A);
-            if (a.big) {
-              const int esz = int(sizeof(TB));
-              const int64_t T = tile_rows(esz), h = tile_height(m, tile, esz);
-              col.ptr = A + int64_t(tile) * T * S.K + int64_t(j) * h + (row0 - int64_t(tile) * T);
-            } else {
-              col.ptr = A + int64_t(j) * m;
-            }
+            const int esz = int(sizeof(TB));
+            const int64_t T = tile_rows(esz), h = tile_height(m, tile, esz);
+            col.ptr = A + int64_t(tile) * T * S.K + int64_t(j) * h + (row0 - int64_t(tile) * T);
           }
         }
         tab[t] = col;
