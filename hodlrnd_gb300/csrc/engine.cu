@@ -406,6 +406,8 @@ constexpr int64_t kPanelItemBytes = 128 * 1024;  // far panels above 32 rows
 #endif
 constexpr int64_t kSmallItemBytes = HODLR_TUNE_SMALL_ITEM_BYTES;
 constexpr int64_t kNearItemBytes = 24 * 1024;    // near panels above 32 rows: few, so shorter
+// members of an FP32-vector batch: a partial sum is 32 right-hand sides wide
+constexpr int64_t kBatchItemBytes = 128 * 1024;
 constexpr int64_t kSpreadItems = 152 * 48;  // 48 warps per SM
 constexpr int64_t kMinItemBytes = 8 * 1024;
 
@@ -563,9 +565,9 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
     if (!op->dense[q]) vtotal += ns * op->rank[q] * prec_size(a);
   }
   const bool spread = spread_items(op);
-  const int64_t big_bytes = spread ? item_bytes(utotal, kMinItemBytes, kPanelItemBytes) : kPanelItemBytes;
+  const int64_t big_bytes = spread ? item_bytes(utotal, kMinItemBytes, kPanelItemBytes) : kBatchItemBytes;
   const int64_t small_bytes = spread ? item_bytes(utotal, kMinItemBytes, kSmallItemBytes) : kSmallItemBytes;
-  const int64_t z_bytes = spread ? item_bytes(vtotal, kMinItemBytes, kZItemBytes) : kZItemBytes;
+  const int64_t z_bytes = spread ? item_bytes(vtotal, kMinItemBytes, kZItemBytes) : kBatchItemBytes;
   size_t b = 0;
   while (b < op->far.size()) {
     const int l = op->far[b].level;
@@ -2113,6 +2115,12 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
     I.in_base = a.in;
     I.y_base = a.y;
     I.perm = op->d_perm;
+    I.iperm = nullptr;
+    if (f32) {
+      int32_t* inv = b.mem.alloc_n<int32_t>(size_t(op->n), "batch inverse permutation");
+      CK(launch_invert_perm(op->d_perm, op->n, inv, st));
+      I.iperm = inv;
+    }
     I.nslots = op->nslots;
     I.pad = 0;
     e.panels_near = a.panels_near + int64_t(hn.panels_near.size());

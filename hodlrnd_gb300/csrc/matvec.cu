@@ -1,6 +1,8 @@
 // HODLR matvec kernels (see matvec.h).
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "bulk.cuh"
 #include "device.cuh"
 #include "matvec.h"
@@ -1999,54 +2001,113 @@ cudaError_t launch_compact(int ndim, const PointsDev& P, const KernelDev& K, con
 // A chunk of kMR right-hand sides is interleaved: entry e of a vector buffer
 // holds its kMR values contiguously (byte offset e * 4 kMR), so one input row
 // or z row is one 128-byte run that the bulk-copy engine stages next to the
-// factor bytes, and every factor entry read from HBM feeds kMR FMAs.  The
-// lane layouts are those of the single-vector kernels, each lane keeping kMR
-// sums per matrix row or column it owns; grid.y runs over chunks.
+// factor bytes, and every factor entry read from HBM feeds kMR FMAs; grid.y runs
+// over chunks.
 // ============================================================================
 namespace {
 
 constexpr int kMWarps = 4;
 constexpr int kMStages = 2;
-constexpr int kMVBytes = 4096;                 // factor bytes per stage
-constexpr int kMXBytes = 4096;                 // input bytes per stage (32 rows of kMR floats)
+constexpr int kMStageBytes = 7424;             // factor and input bytes per stage
 constexpr int kMRowBytes = kMR * 4;            // one interleaved entry
-constexpr int kMWarpSmem = 64 + kMStages * (kMVBytes + kMXBytes);
-static_assert(kMWarpSmem % 16 == 0, "bulk copy destinations must stay 16-byte aligned");
+// a lane's column loads may run up to 496 bytes beyond the last row: 512 bytes at the end
+constexpr int kMWarpSmem = 64 + kMStages * kMStageBytes + 512;
+static_assert(kMWarpSmem % 16 == 0 && kMStageBytes % 16 == 0, "bulk copy destinations must stay 16-byte aligned");
 
-__device__ __forceinline__ void fma4x(float a, const float4& x, float* acc) {
-  acc[0] = __fmaf_rn(a, x.x, acc[0]);
-  acc[1] = __fmaf_rn(a, x.y, acc[1]);
-  acc[2] = __fmaf_rn(a, x.z, acc[2]);
-  acc[3] = __fmaf_rn(a, x.w, acc[3]);
-}
-
-// Lane c of a warp owns right-hand side c of the chunk (kMR = 32 = warp
-// width): it reads its input value of a row with one conflict-free shared
-// load, the row's factor values with broadcast 16-byte loads, and keeps one
-// sum per output row or column it produces -- no cross-lane reductions, and
-// every output row is one coalesced 128-byte store.
-
-// z_b = V_b^T X_s: item = rows [j0, j1) of block zb (all columns); passes of
-// kMCols columns (one pass unless r > kMCols); runs of whole V rows and their
-// input rows staged by bulk copies in a ring of kMStages.
-constexpr int kMCols = 64;
-
-// acc[c] += V[i][c] x[i] over the stage's rows, NC4 groups of 4 columns
-template <int NC4>
-__device__ __forceinline__ void mr_rows(const unsigned char* vs, int rowb, const float* xs, int nr, int lane,
-                                        float (&acc)[kMCols]) {
+// Products of the wide items (V rows of up to 128 columns, U tiles of up to 128
+// rows): out(c, r) += A(k, c) x(k, r), every row k of A and of x staged in
+// shared memory.  A value read from shared memory costs its register write-back
+// (128 bytes per clock and SM: a 16-byte load of a warp 4 clocks, whether or
+// not the lanes read the same address) against a quarter clock per FMA
+// instruction, so with one right-hand side per lane and the factors broadcast
+// the loads took four times as long as the FMAs.  A lane therefore keeps a tile
+// of 4 NQ columns by 8 right-hand sides: lane 4 cg + rg has columns 32 q + 4 cg ..
+// + 3 (q < NQ) and right-hand sides 4 rg .. + 3 and 16 + 4 rg .. + 3, and 2 + NQ
+// loads of 16 bytes feed 32 NQ FMAs.  Columns beyond the item's are computed
+// from whatever follows in the warp's shared memory and never stored.
+// 24 3D operators (420,000 points), 32 right-hand sides: V^T x 4.44 -> 1.52 ms, node
+// panels 2.19 -> 1.24 ms, leaf panels 3.65 -> 1.52 ms (whole product 11.1 -> 4.7 ms;
+// the FMAs alone would take 1.4).
+template <int NQ>
+__device__ __forceinline__ void mr_wide(const unsigned char* as, int rowb, const float* xs, int nr, int lane,
+                                        float (&acc)[4 * NQ][8]) {
+  const int cg = lane >> 2, rg = lane & 3;
+  const unsigned char* ap = as + cg * 16;
+  const float4* x4 = reinterpret_cast<const float4*>(xs) + rg;
+#pragma unroll 2
   for (int i = 0; i < nr; i++) {
-    const float x = xs[i * kMR + lane];
-    const float4* v4 = reinterpret_cast<const float4*>(vs + i * rowb);
+    const float4 xa = x4[i * 8], xb = x4[i * 8 + 4];
+    const float x[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
 #pragma unroll
-    for (int c = 0; c < NC4; c++) {
-      const float4 v = v4[c];
-      acc[4 * c] = __fmaf_rn(v.x, x, acc[4 * c]);
-      acc[4 * c + 1] = __fmaf_rn(v.y, x, acc[4 * c + 1]);
-      acc[4 * c + 2] = __fmaf_rn(v.z, x, acc[4 * c + 2]);
-      acc[4 * c + 3] = __fmaf_rn(v.w, x, acc[4 * c + 3]);
+    for (int q = 0; q < NQ; q++) {
+      const float4 v4 = *reinterpret_cast<const float4*>(ap + i * rowb + q * 128);
+      const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+#pragma unroll
+        for (int r = 0; r < 8; r++) acc[4 * q + e][r] = __fmaf_rn(v[e], x[r], acc[4 * q + e][r]);
     }
   }
+}
+
+// The sums of columns c < n to dst + c * kMR.
+template <int NQ>
+__device__ __forceinline__ void mr_store(float* dst, int n, int lane, const float (&acc)[4 * NQ][8]) {
+  const int cg = lane >> 2, rg = lane & 3;
+#pragma unroll
+  for (int q = 0; q < NQ; q++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const int c = 32 * q + 4 * cg + e;
+      const float* a = acc[4 * q + e];
+      if (c < n) {
+        *reinterpret_cast<float4*>(dst + int64_t(c) * kMR + 4 * rg) = make_float4(a[0], a[1], a[2], a[3]);
+        *reinterpret_cast<float4*>(dst + int64_t(c) * kMR + 16 + 4 * rg) = make_float4(a[4], a[5], a[6], a[7]);
+      }
+    }
+}
+
+// z_b = V_b^T X_s: item = rows [j0, j1) of block zb, columns [k0, k0 + nk) (at
+// most 128); runs of whole V rows and their input rows staged by bulk copies in
+// a ring of kMStages.
+template <int NQ>
+__device__ __forceinline__ void zgemv_mr_item(const ZItem& it, const ZBlock& Z, const float* V, int64_t rp,
+                                              const float* xr, float* dst, unsigned char* base, int lane) {
+  uint64_t* bar = reinterpret_cast<uint64_t*>(base);
+  unsigned char* stage0 = base + 64;
+  const int rowb = int(rp) * 4;  // a multiple of 16
+  const int R = kMStageBytes / (rowb + kMRowBytes);  // rows per stage: their factors, then their inputs
+  const int nrows = it.j1 - it.j0;
+  const int total = (nrows + R - 1) / R;
+  auto issue = [&](int q) {  // lane 0: rows q R ..
+    const int s = q % kMStages, r0 = q * R, nr = min(R, nrows - r0);
+    unsigned char* st = stage0 + s * kMStageBytes;
+    fence_proxy_async();
+    mbar_expect_tx(bar + s, uint32_t(nr) * uint32_t(rowb + kMRowBytes));
+    bulk_g2s(st, V + int64_t(r0) * rp, uint32_t(nr * rowb), bar + s);
+    bulk_g2s(st + R * rowb, xr + int64_t(r0) * kMR, uint32_t(nr * kMRowBytes), bar + s);
+  };
+  if (lane == 0)
+    for (int q = 0; q < min(kMStages, total); q++) issue(q);
+  float acc[4 * NQ][8];
+#pragma unroll
+  for (int c = 0; c < 4 * NQ; c++)
+#pragma unroll
+    for (int r = 0; r < 8; r++) acc[c][r] = 0.f;
+  for (int q = 0; q < total; q++) {
+    const int s = q % kMStages;
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(bar + s, uint32_t(q / kMStages) & 1u));
+    if (!ok) {
+      if (lane == 0) atomicAdd(&g_stream_timeouts, 1u);
+      for (int t = q; t < min(q + kMStages, total); t++) mbar_wait(bar + t % kMStages, uint32_t(t / kMStages) & 1u);
+      return;
+    }
+    const unsigned char* st = stage0 + s * kMStageBytes;
+    mr_wide<NQ>(st + it.k0 * 4, rowb, reinterpret_cast<const float*>(st + R * rowb), min(R, nrows - q * R), lane, acc);
+    __syncwarp();
+    if (lane == 0 && q + kMStages < total) issue(q + kMStages);
+  }
+  mr_store<NQ>(dst, it.part < 0 ? min(it.nk, Z.r - it.k0) : it.nk, lane, acc);
 }
 
 __global__ void __launch_bounds__(kMWarps * 32, 3)
@@ -2061,108 +2122,34 @@ __global__ void __launch_bounds__(kMWarps * 32, 3)
   const int64_t rp = vpad(Z.r, 4);
   float* inc = in + int64_t(blockIdx.y) * ld_in * kMR;
   float* zp = zpart + int64_t(blockIdx.y) * zpart_ld * kMR;
-  unsigned char* base = msm + wid * kMWarpSmem;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(base);
-  unsigned char* stage0 = base + 64;
-  const int rowb = int(rp) * 4;  // 16 .. 512 bytes, a multiple of 16
-  const int R = min(kMVBytes / rowb, kMXBytes / kMRowBytes);  // 0 only for rows above 4096 bytes
-  const int nrows = it.j1 - it.j0;
-  const int nst = (nrows + R - 1) / R;
   const float* V = static_cast<const float*>(Z.V) + int64_t(it.j0) * rp;
   const float* xr = inc + (Z.x_off + it.j0) * kMR;
-  const int npass = (it.nk + kMCols - 1) / kMCols;
-  float acc[kMCols];
-  if (R == 0) {
-    // rows wider than a stage (rank above 1024): direct loads
-    for (int pass = 0; pass < npass; pass++) {
-      const int c0 = it.k0 + pass * kMCols, ncol = min(kMCols, it.k0 + it.nk - c0);
-#pragma unroll
-      for (int c = 0; c < kMCols; c++) acc[c] = 0.f;
-      for (int j = 0; j < nrows; j++) {
-        const float x = xr[int64_t(j) * kMR + lane];
-        const float* vj = V + int64_t(j) * rp + c0;
-#pragma unroll
-        for (int c = 0; c < kMCols; c++)
-          if (c < ncol) acc[c] = __fmaf_rn(__ldg(vj + c), x, acc[c]);
-      }
-#pragma unroll
-      for (int c = 0; c < kMCols; c++)
-        if (c < ncol) {
-          const int col = c0 + c;
-          if (it.part < 0) {
-            if (col < Z.r) inc[(Z.z_off + col) * kMR + lane] = acc[c];
-          } else {
-            zp[(int64_t(it.part) + col - it.k0) * kMR + lane] = acc[c];
-          }
-        }
+  float* dst = it.part < 0 ? inc + (Z.z_off + it.k0) * kMR : zp + int64_t(it.part) * kMR;
+  if (rp * 4 > kMStageBytes / 2) {
+    // rows wider than half a stage (rank above 928): direct loads, a right-hand side per lane
+    for (int c = 0; c < it.nk; c++) {
+      if (it.part < 0 && it.k0 + c >= Z.r) break;
+      float acc = 0.f;
+      for (int j = 0; j < it.j1 - it.j0; j++)
+        acc = __fmaf_rn(__ldg(V + int64_t(j) * rp + it.k0 + c), xr[int64_t(j) * kMR + lane], acc);
+      dst[int64_t(c) * kMR + lane] = acc;
     }
     return;
   }
-  const int total = nst * npass;  // stages over all passes
+  unsigned char* base = msm + wid * kMWarpSmem;
   if (lane == 0) {
+    uint64_t* bar = reinterpret_cast<uint64_t*>(base);
 #pragma unroll
     for (int s = 0; s < kMStages; s++) mbar_init(bar + s, 1);
     fence_mbar_init();
   }
   __syncwarp();
-  // stage q: pass q / nst, rows (q % nst) * R ..
-#define HODLR_MR_ISSUE(q_)                                                                     \
-  do {                                                                                         \
-    const int s_ = (q_) % kMStages;                                                            \
-    const int r0_ = ((q_) % nst) * R, nr_ = min(R, nrows - r0_);                               \
-    unsigned char* st_ = stage0 + s_ * (kMVBytes + kMXBytes);                                  \
-    fence_proxy_async();                                                                       \
-    mbar_expect_tx(bar + s_, uint32_t(nr_) * uint32_t(rowb + kMRowBytes));                     \
-    bulk_g2s(st_, V + int64_t(r0_) * rp, uint32_t(nr_ * rowb), bar + s_);                      \
-    bulk_g2s(st_ + kMVBytes, xr + int64_t(r0_) * kMR, uint32_t(nr_ * kMRowBytes), bar + s_);    \
-  } while (0)
-  if (lane == 0)
-    for (int q = 0; q < min(kMStages, total); q++) HODLR_MR_ISSUE(q);
-  for (int q = 0; q < total; q++) {
-    const int pass = q / nst, c0 = it.k0 + pass * kMCols;
-    const int ncol4 = min(kMCols, it.k0 + it.nk - c0) / 4;
-    if (q % nst == 0) {
-#pragma unroll
-      for (int c = 0; c < kMCols; c++) acc[c] = 0.f;
-    }
-    const int s = q % kMStages;
-    const bool ok = __all_sync(0xffffffffu, mbar_wait(bar + s, uint32_t(q / kMStages) & 1u));
-    if (!ok) {
-      if (lane == 0) atomicAdd(&g_stream_timeouts, 1u);
-      for (int t = q; t < min(q + kMStages, total); t++) mbar_wait(bar + t % kMStages, uint32_t(t / kMStages) & 1u);
-      return;
-    }
-    const int nr = min(R, nrows - (q % nst) * R);
-    const unsigned char* vs = stage0 + s * (kMVBytes + kMXBytes) + c0 * 4;
-    const float* xs = reinterpret_cast<const float*>(stage0 + s * (kMVBytes + kMXBytes) + kMVBytes);
-    switch (ncol4) {  // column count known at compile time: no per-row guards
-#define HODLR_MR_CASE(k_) \
-  case k_:                \
-    mr_rows<k_>(vs, rowb, xs, nr, lane, acc); \
-    break;
-      HODLR_MR_CASE(1) HODLR_MR_CASE(2) HODLR_MR_CASE(3) HODLR_MR_CASE(4) HODLR_MR_CASE(5) HODLR_MR_CASE(6)
-      HODLR_MR_CASE(7) HODLR_MR_CASE(8) HODLR_MR_CASE(9) HODLR_MR_CASE(10) HODLR_MR_CASE(11) HODLR_MR_CASE(12)
-      HODLR_MR_CASE(13) HODLR_MR_CASE(14) HODLR_MR_CASE(15) HODLR_MR_CASE(16)
-#undef HODLR_MR_CASE
-      default:
-        break;
-    }
-    __syncwarp();
-    if (lane == 0 && q + kMStages < total) HODLR_MR_ISSUE(q + kMStages);
-    if (q % nst == nst - 1) {  // end of a pass: columns c0 .. c0 + 4 ncol4
-#pragma unroll
-      for (int c = 0; c < kMCols; c++)
-        if (c < 4 * ncol4) {
-          const int col = c0 + c;
-          if (it.part < 0) {
-            if (col < Z.r) inc[(Z.z_off + col) * kMR + lane] = acc[c];
-          } else {
-            zp[(int64_t(it.part) + col - it.k0) * kMR + lane] = acc[c];
-          }
-        }
-    }
+  switch ((it.nk + 31) / 32) {
+    case 1: zgemv_mr_item<1>(it, Z, V, rp, xr, dst, base, lane); break;
+    case 2: zgemv_mr_item<2>(it, Z, V, rp, xr, dst, base, lane); break;
+    case 3: zgemv_mr_item<3>(it, Z, V, rp, xr, dst, base, lane); break;
+    default: zgemv_mr_item<4>(it, Z, V, rp, xr, dst, base, lane); break;
   }
-#undef HODLR_MR_ISSUE
 }
 
 // z row zpos (all kMR values) = sum of the item partials, in order.
@@ -2181,57 +2168,153 @@ __global__ void __launch_bounds__(256) zfix_mr_kernel(const ZFix* __restrict__ f
   in[int64_t(blockIdx.y) * ld_in * kMR + (F.zpos + k) * kMR + c] = acc;
 }
 
-// Leaf panels (m <= 32): one warp per item; lane c keeps m sums.  The item's
-// segments are cut into pieces that are packed, in order, into stages of at
-// most kMSUBytes of factor bytes (each piece 16-byte aligned, a multiple of 4
-// columns unless it ends its segment) and kMSRows input rows; one lane issues
-// the bulk copies of a stage, every lane replays the same packing to find the
-// pieces.
+// Leaf panels (m <= 32): one warp per item.  The item's segments are cut into
+// pieces that are packed, in order, into stages of at most kMSUBytes of factor
+// bytes (each piece 16-byte aligned, a multiple of 4 columns unless it ends its
+// segment) and kMSRows columns, each lane planning and copying a segment and noting
+// where its columns start.  Lane tiles as in mr_wide, for
+// columns of few rows at any alignment: RR = 1, 2 or 4 groups of lanes take RL =
+// ceil(m / RR) <= 8 (made even) rows each, 4 lanes their 8 right-hand sides each, and the 8 / RR
+// slices left every (8 / RR)-th column of the stage, added by shuffles at the end.
 constexpr int kMSUBytes = 4096;
 constexpr int kMSRows = 32;
 constexpr int kMSXBytes = kMSRows * kMRowBytes;
-constexpr int kMSWarpSmem = 64 + kMStages * (kMSUBytes + kMSXBytes);
-static_assert(kMSWarpSmem % 16 == 0, "bulk copy destinations must stay 16-byte aligned");
+constexpr int kMSStage = kMSUBytes + kMSXBytes + kMSRows * 4;  // factors, inputs, column offsets
+constexpr int kMSWarpSmem = 64 + kMStages * kMSStage;
+static_assert(kMSWarpSmem % 16 == 0 && kMSStage % 16 == 0, "bulk copy destinations must stay 16-byte aligned");
 
-// acc[i] += U[i][j] x[j] over a piece's columns, rows 0 .. MP-1
-template <int MP>
-__device__ __forceinline__ void mr_cols(const float* ua, int m, const float* xr, int nc, float (&acc)[32]) {
-  for (int j = 0; j < nc; j++) {
-    const float x = xr[j * kMR];
+template <int RL>
+__device__ __forceinline__ void small_mr_item(const Seg* __restrict__ segs, const Item& it, int m, int RR,
+                                              const float* inc, float* dst, unsigned char* base, int lane) {
+  uint64_t* bar = reinterpret_cast<uint64_t*>(base);
+  unsigned char* stage0 = base + 64;
+  const int rg = lane & 3, rr = (lane >> 2) & (RR - 1), SL = 8 / RR, sl = (lane >> 2) / RR;
+  // packing cursor (the same in every lane): segment ps, column pc; lane k has the record of segment win + k
+  int32_t ps = it.seg_b, pc = 0, win = it.seg_b - 32;
+  const char* rA = nullptr;
+  int64_t ro = 0;
+  int rK = 0;
+  // Packs and issues the next stage; its column count (0: nothing left).  Lane
+  // k takes segment win + k (from column pc for the cursor's): whole segments
+  // while they fit, or as many columns of the first one as do.  Each lane raises
+  // the stage's transaction count (no arrival) and starts its piece's two copies;
+  // the stage's one arrival comes after them all, so the phase cannot complete
+  // before every copy is accounted for.
+  auto issue = [&](int st) -> int {
+    if (ps >= it.seg_e) return 0;
+    unsigned char* su = stage0 + st * kMSStage;
+    int* co = reinterpret_cast<int*>(su + kMSUBytes + kMSXBytes);
+    if (ps >= win + 24 || ps < win) {  // at least 8 segments in the window (it ends at the item's end)
+      win = ps;
+      rK = 0;
+      if (win + lane < it.seg_e) {
+        const Seg S = segs[win + lane];
+        rA = static_cast<const char*>(S.A);
+        ro = S.in_off;
+        rK = S.K;
+      }
+    }
+    const int k0 = ps - win, c0 = lane == k0 ? pc : 0;
+    int take = lane >= k0 ? rK - c0 : 0;
+    int cols = take, bytes = (take * m * 4 + 15) & ~15;
 #pragma unroll
-    for (int i = 0; i < MP; i++) acc[i] = __fmaf_rn(ua[j * m + i], x, acc[i]);
+    for (int o = 1; o < 32; o <<= 1) {
+      const int vc = __shfl_up_sync(0xffffffffu, cols, o), vb = __shfl_up_sync(0xffffffffu, bytes, o);
+      if (lane >= o) {
+        cols += vc;
+        bytes += vb;
+      }
+    }
+    // the lanes from k0 whose segments fit whole: a run, as both sums grow
+    const bool fits = lane >= k0 && take > 0 && cols <= kMSRows && bytes <= kMSUBytes;
+    const unsigned whole = __ballot_sync(0xffffffffu, fits);
+    int n;
+    if (whole == 0u) {
+      // the cursor's segment is longer than a stage: a multiple of 4 columns, which keeps 16-byte alignment
+      n = min(kMSRows, kMSUBytes / (m * 4)) / 4 * 4;
+      take = lane == k0 ? n : 0;
+      cols = n;
+      bytes = n * m * 4;
+      pc += n;
+    } else {
+      const int last = 31 - __clz(whole);
+      n = __shfl_sync(0xffffffffu, cols, last);
+      if (!fits) take = 0;
+      ps = win + last + 1;
+      pc = 0;
+    }
+    if (take > 0) {
+      const int pb = (take * m * 4 + 15) & ~15, row0 = cols - take, off = bytes - pb;
+      fence_proxy_async();
+      mbar_expect_tx_only(bar + st, uint32_t(pb + take * kMRowBytes));
+      bulk_g2s(su + off, rA + int64_t(c0) * m * 4, uint32_t(pb), bar + st);
+      bulk_g2s(su + kMSUBytes + row0 * kMRowBytes, inc + (ro + c0) * kMR, uint32_t(take * kMRowBytes), bar + st);
+      for (int j = 0; j < take; j++) co[row0 + j] = off + j * m * 4;
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar + st);
+    return n;
+  };
+  static_assert(kMStages == 2, "two column counts");
+  float acc[RL][8];
+#pragma unroll
+  for (int i = 0; i < RL; i++)
+#pragma unroll
+    for (int r = 0; r < 8; r++) acc[i][r] = 0.f;
+  // the last group's rows beyond m read whatever follows in the warp's share and are never stored
+  const int row0 = rr * RL;
+  bool gave_up = false;
+  // q = -2, -1 fill the ring; from then on stage q is consumed and refilled (one
+  // copy of the code: several row counts run on an SM at a time, and unrolled
+  // over the stages they did not fit its instruction cache)
+  int cur = 0, next = 0;
+#pragma unroll 1
+  for (int q = -kMStages; q < 0 || cur > 0; q++) {
+    const int st = q & 1;
+    if (q >= 0) {
+      if (!__all_sync(0xffffffffu, mbar_wait(bar + st, uint32_t(q >> 1) & 1u))) {
+        if (lane == 0) atomicAdd(&g_stream_timeouts, 1u);
+        if (next > 0) mbar_wait(bar + (st ^ 1), uint32_t((q + 1) >> 1) & 1u);
+        gave_up = true;
+        break;
+      }
+      const unsigned char* su = stage0 + st * kMSStage;
+      const float4* x4 = reinterpret_cast<const float4*>(su + kMSUBytes) + rg;
+      const int* co = reinterpret_cast<const int*>(su + kMSUBytes + kMSXBytes);
+#pragma unroll 1
+      for (int c = sl; c < cur; c += SL) {
+        const float* a = reinterpret_cast<const float*>(su + co[c]) + row0;
+        const float4 xa = x4[c * 8], xb = x4[c * 8 + 4];
+        const float x[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+#pragma unroll
+        for (int i = 0; i < RL; i++) {
+          const float v = a[i];
+#pragma unroll
+          for (int r = 0; r < 8; r++) acc[i][r] = __fmaf_rn(v, x[r], acc[i][r]);
+        }
+      }
+      __syncwarp();
+    }
+    cur = next;
+    next = issue(st);  // into the stage just consumed
+  }
+  for (int o = 4 * RR; o < 32; o <<= 1)
+#pragma unroll
+    for (int i = 0; i < RL; i++)
+#pragma unroll
+      for (int r = 0; r < 8; r++) acc[i][r] += __shfl_xor_sync(0xffffffffu, acc[i][r], o);
+  if (sl == 0 && !gave_up) {
+#pragma unroll
+    for (int i = 0; i < RL; i++)
+      if (row0 + i < m) {
+        float* d = dst + int64_t(row0 + i) * kMR + 4 * rg;
+        *reinterpret_cast<float4*>(d) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        *reinterpret_cast<float4*>(d + 16) = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+      }
   }
 }
 
-struct MrCursor {
-  int64_t s;  // segment
-  int c;      // first column of the next piece
-};
-
-// Next piece of a stage holding `used` factor bytes and `rows` input rows;
-// false when the stage is full or the segments are done.
-__device__ __forceinline__ bool mr_next_piece(const Seg* segs, int64_t seg_e, int m, MrCursor& cur, int used, int rows,
-                                              int64_t& s, int& c0, int& nc, int& bytes) {
-  if (cur.s >= seg_e) return false;
-  const int K = segs[cur.s].K;
-  int room_c = min((kMSUBytes - used) / (m * 4), kMSRows - rows);
-  int c = min(K - cur.c, room_c);
-  if (c < K - cur.c) c = c / 4 * 4;  // a piece that does not end its segment keeps 16-byte alignment
-  if (c <= 0) return false;
-  nc = c;
-  bytes = (c * m * 4 + 15) & ~15;
-  if (used + bytes > kMSUBytes) return false;
-  s = cur.s;
-  c0 = cur.c;
-  cur.c += c;
-  if (cur.c >= K) {
-    cur.s++;
-    cur.c = 0;
-  }
-  return true;
-}
-
-__global__ void __launch_bounds__(kMWarps * 32, 3)
+__global__ void __launch_bounds__(kMWarps * 32, 4)
     panel_small_mr_kernel(const Panel* __restrict__ panels, const Seg* __restrict__ segs,
                           const Item* __restrict__ items, int nitems, const float* __restrict__ in, int64_t ld_in,
                           float* __restrict__ y, int64_t ld_y, float* __restrict__ ypart, int64_t ypart_ld) {
@@ -2242,145 +2325,49 @@ __global__ void __launch_bounds__(kMWarps * 32, 3)
   const Item it = items[w];
   const Panel P = panels[it.panel];
   const int m = P.m;
-  int mp = 4;
-  while (mp < m) mp <<= 1;
   const float* inc = in + int64_t(blockIdx.y) * ld_in * kMR;
+  // split panels: partial rows at the part's 128-row block of ypart (panel_fix_mr_kernel)
+  float* dst = it.part < 0 ? y + int64_t(blockIdx.y) * ld_y * kMR + P.yoff * kMR
+                           : ypart + int64_t(blockIdx.y) * ypart_ld * kMR + int64_t(it.part) * 128 * kMR;
   unsigned char* base = msm + wid * kMSWarpSmem;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(base);
-  unsigned char* stage0 = base + 64;
   if (lane == 0) {
+    uint64_t* bar = reinterpret_cast<uint64_t*>(base);
 #pragma unroll
     for (int s = 0; s < kMStages; s++) mbar_init(bar + s, 1);
     fence_mbar_init();
   }
   __syncwarp();
-  MrCursor pc{it.seg_b, 0}, cc{it.seg_b, 0};
-  int issued = 0;
-  // packs and issues the next stage; false when nothing is left
-  // Packs and issues the next stage: per piece, lane 0 raises the stage's
-  // transaction count (no arrival) and starts its two copies; the stage's one
-  // arrival comes after the last piece, so the phase cannot complete before
-  // every copy is accounted for.  ok_ is false when nothing is left.
-#define HODLR_MRS_ISSUE(ok_)                                                                      \
-  do {                                                                                            \
-    const int st_ = issued % kMStages;                                                            \
-    unsigned char* su_ = stage0 + st_ * (kMSUBytes + kMSXBytes);                                  \
-    int used_ = 0, rows_ = 0, nc_, by_, c0_;                                                      \
-    int64_t s_;                                                                                   \
-    if (lane == 0) fence_proxy_async();                                                           \
-    while (mr_next_piece(segs, it.seg_e, m, pc, used_, rows_, s_, c0_, nc_, by_)) {               \
-      if (lane == 0) {                                                                            \
-        const Seg S_ = segs[s_];                                                                  \
-        mbar_expect_tx_only(bar + st_, uint32_t(by_ + nc_ * kMRowBytes));                         \
-        bulk_g2s(su_ + used_, static_cast<const float*>(S_.A) + int64_t(c0_) * m, uint32_t(by_), bar + st_); \
-        bulk_g2s(su_ + kMSUBytes + rows_ * kMRowBytes, inc + (S_.in_off + c0_) * kMR,            \
-                 uint32_t(nc_ * kMRowBytes), bar + st_);                                          \
-      }                                                                                           \
-      used_ += by_;                                                                               \
-      rows_ += nc_;                                                                               \
-    }                                                                                             \
-    ok_ = rows_ > 0;                                                                              \
-    if (ok_) {                                                                                    \
-      if (lane == 0) mbar_arrive(bar + st_);                                                      \
-      issued++;                                                                                   \
-    }                                                                                             \
-  } while (0)
-  bool more = true;
-  for (int q = 0; q < kMStages && more; q++) HODLR_MRS_ISSUE(more);
-  float acc[32];
-#pragma unroll
-  for (int i = 0; i < 32; i++) acc[i] = 0.f;
-  for (int q = 0; q < issued; q++) {
-    const int st = q % kMStages;
-    const bool ok = __all_sync(0xffffffffu, mbar_wait(bar + st, uint32_t(q / kMStages) & 1u));
-    if (!ok) {
-      if (lane == 0) atomicAdd(&g_stream_timeouts, 1u);
-      for (int t = q; t < issued; t++) mbar_wait(bar + t % kMStages, uint32_t(t / kMStages) & 1u);
-      return;
-    }
-    const unsigned char* su = stage0 + st * (kMSUBytes + kMSXBytes);
-    const float* xs = reinterpret_cast<const float*>(su + kMSUBytes);
-    int used = 0, rows = 0, nc, by, c0;
-    int64_t sg;
-    while (mr_next_piece(segs, it.seg_e, m, cc, used, rows, sg, c0, nc, by)) {
-      const float* ua = reinterpret_cast<const float*>(su + used);
-      const float* xr = xs + rows * kMR + lane;
-      // rows 0 .. mp-1 (mp = next power of two >= m, at least 4): sums of rows
-      // m .. mp-1 read neighbouring bytes of the warp's stage and are never stored
-      if (mp <= 4)
-        mr_cols<4>(ua, m, xr, nc, acc);
-      else if (mp <= 8)
-        mr_cols<8>(ua, m, xr, nc, acc);
-      else if (mp <= 16)
-        mr_cols<16>(ua, m, xr, nc, acc);
-      else
-        mr_cols<32>(ua, m, xr, nc, acc);
-      used += by;
-      rows += nc;
-    }
-    __syncwarp();
-    if (more) HODLR_MRS_ISSUE(more);  // into the stage just consumed (the ring is full while more)
+  // rows per lane rounded up to 2, 4, 6 or 8
+  const int RR = m <= 8 ? 1 : m <= 16 ? 2 : 4;
+#define HODLR_SMALL_MR(rl_)                                            \
+  case rl_:                                                            \
+    small_mr_item<2 * rl_>(segs, it, m, RR, inc, dst, base, lane);         \
+    break;
+  switch (((m + RR - 1) / RR + 1) / 2) {
+    HODLR_SMALL_MR(1)
+    HODLR_SMALL_MR(2)
+    HODLR_SMALL_MR(3)
+    HODLR_SMALL_MR(4)
+    default: break;
   }
-#undef HODLR_MRS_ISSUE
-  // split panels: partial rows at the part's 128-row block of ypart (panel_fix_mr_kernel)
-  float* yo = it.part < 0 ? y + int64_t(blockIdx.y) * ld_y * kMR + P.yoff * kMR
-                          : ypart + int64_t(blockIdx.y) * ypart_ld * kMR + int64_t(it.part) * 128 * kMR;
-#pragma unroll
-  for (int i = 0; i < 32; i++)
-    if (i < m) yo[int64_t(i) * kMR + lane] = acc[i];
-}
-
-// acc[i] += U[i][j] x[j] over a stage's columns: H4 groups of 4 rows (a full
-// tile), or h4 of them checked per group (H4 == 0, the last tile)
-template <int H4>
-__device__ __forceinline__ void mr_tile(const unsigned char* us, int colb, const float* xs, int nc, int lane, int h4,
-                                        float (&acc)[128]) {
-  for (int j = 0; j < nc; j++) {
-    const float x = xs[j * kMR + lane];
-    const float4* u4 = reinterpret_cast<const float4*>(us + j * colb);
-#pragma unroll
-    for (int r = 0; r < 32; r++)
-      if (H4 ? r < H4 : r < h4) {
-        const float4 u = u4[r];
-        acc[4 * r] = __fmaf_rn(u.x, x, acc[4 * r]);
-        acc[4 * r + 1] = __fmaf_rn(u.y, x, acc[4 * r + 1]);
-        acc[4 * r + 2] = __fmaf_rn(u.z, x, acc[4 * r + 2]);
-        acc[4 * r + 3] = __fmaf_rn(u.w, x, acc[4 * r + 3]);
-      }
-  }
+#undef HODLR_SMALL_MR
 }
 
 // Panels of more than 32 rows: item = row tile t (up to 128 rows) times a
-// run of segments; lane c keeps the tile's row sums; runs of tile columns and
-// their input rows are staged.
-constexpr int kMTUBytes = 4096;
-constexpr int kMTXBytes = 4096;  // 32 input rows
-constexpr int kMTWarpSmem = 64 + kMStages * (kMTUBytes + kMTXBytes);
-static_assert(kMTWarpSmem % 16 == 0, "bulk copy destinations must stay 16-byte aligned");
-
-__global__ void __launch_bounds__(kMWarps * 32, 2)
-    panel_tile_mr_kernel(const Panel* __restrict__ panels, const Seg* __restrict__ segs,
-                         const Item* __restrict__ items, int nitems, float* __restrict__ ypart, int64_t ypart_ld,
-                         const float* __restrict__ in, int64_t ld_in, float* __restrict__ y, int64_t ld_y) {
+// run of segments; runs of tile columns and their input rows are staged
+// (mr_wide: the tile's columns are the rows of A).
+template <int NQ>
+__device__ __forceinline__ void panel_tile_mr_item(const Seg* __restrict__ segs, const Item& it, int rows, int64_t h,
+                                                   const float* inc, float* dst, unsigned char* base, int lane) {
   constexpr int T = 128;
-  extern __shared__ __align__(16) unsigned char msm[];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int w = blockIdx.x * kMWarps + wid;
-  if (w >= nitems) return;
-  const Item it = items[w];
-  const Panel P = panels[it.panel];
-  const int m = P.m;
-  const float* inc = in + int64_t(blockIdx.y) * ld_in * kMR;
   const int t = it.chunk;
-  const int rows = min(T, m - t * T);
-  const int64_t h = tile_height(m, t, 4);
   const int colb = int(h) * 4;
-  const int h4 = int(h) / 4;
-  const int cps = min(kMTUBytes / colb, kMTXBytes / kMRowBytes);
-  float acc[T];
+  const int cps = kMStageBytes / (colb + kMRowBytes);  // columns per stage, then their inputs
+  float acc[4 * NQ][8];
 #pragma unroll
-  for (int i = 0; i < T; i++) acc[i] = 0.f;
-  unsigned char* base = msm + wid * kMTWarpSmem;
+  for (int c = 0; c < 4 * NQ; c++)
+#pragma unroll
+    for (int r = 0; r < 8; r++) acc[c][r] = 0.f;
   uint64_t* bar = reinterpret_cast<uint64_t*>(base);
   unsigned char* stage0 = base + 64;
   if (lane == 0) {
@@ -2402,12 +2389,12 @@ __global__ void __launch_bounds__(kMWarps * 32, 2)
     const int nc_ = min(cps, S_.K - pc);                                                           \
     if (lane == 0) {                                                                               \
       const int st_ = issued % kMStages;                                                           \
-      unsigned char* dst_ = stage0 + st_ * (kMTUBytes + kMTXBytes);                                \
+      unsigned char* dst_ = stage0 + st_ * kMStageBytes;                                           \
       const float* src_ = static_cast<const float*>(S_.A) + int64_t(t) * T * S_.K + int64_t(pc) * h; \
       fence_proxy_async();                                                                         \
       mbar_expect_tx(bar + st_, uint32_t(nc_) * uint32_t(colb + kMRowBytes));                      \
       bulk_g2s(dst_, src_, uint32_t(nc_ * colb), bar + st_);                                       \
-      bulk_g2s(dst_ + kMTUBytes, inc + (S_.in_off + pc) * kMR, uint32_t(nc_ * kMRowBytes), bar + st_); \
+      bulk_g2s(dst_ + cps * colb, inc + (S_.in_off + pc) * kMR, uint32_t(nc_ * kMRowBytes), bar + st_); \
     }                                                                                              \
     pc += nc_;                                                                                     \
     issued++;                                                                                      \
@@ -2428,72 +2415,122 @@ __global__ void __launch_bounds__(kMWarps * 32, 2)
       for (int u = q; u < issued; u++) mbar_wait(bar + u % kMStages, uint32_t(u / kMStages) & 1u);
       return;
     }
-    const unsigned char* us = stage0 + st * (kMTUBytes + kMTXBytes);
-    const float* xs = reinterpret_cast<const float*>(us + kMTUBytes);
-    if (h4 == T / 4)
-      mr_tile<T / 4>(us, colb, xs, nc, lane, h4, acc);
-    else
-      mr_tile<0>(us, colb, xs, nc, lane, h4, acc);
+    const unsigned char* us = stage0 + st * kMStageBytes;
+    const float* xs = reinterpret_cast<const float*>(us + cps * colb);
+    mr_wide<NQ>(us, colb, xs, nc, lane, acc);
     cc += nc;
     __syncwarp();
     HODLR_MRT_ISSUE();
   }
 #undef HODLR_MRT_ISSUE
-  float* dst = it.part < 0 ? y + int64_t(blockIdx.y) * ld_y * kMR + (P.yoff + int64_t(t) * T) * kMR
-                           : ypart + int64_t(blockIdx.y) * ypart_ld * kMR + int64_t(it.part) * T * kMR;
-#pragma unroll
-  for (int i = 0; i < T; i++)
-    if (i < rows) dst[int64_t(i) * kMR + lane] = acc[i];
+  mr_store<NQ>(dst, rows, lane, acc);
 }
 
+__global__ void __launch_bounds__(kMWarps * 32, 3)
+    panel_tile_mr_kernel(const Panel* __restrict__ panels, const Seg* __restrict__ segs,
+                         const Item* __restrict__ items, int nitems, float* __restrict__ ypart, int64_t ypart_ld,
+                         const float* __restrict__ in, int64_t ld_in, float* __restrict__ y, int64_t ld_y) {
+  constexpr int T = 128;
+  extern __shared__ __align__(16) unsigned char msm[];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int w = blockIdx.x * kMWarps + wid;
+  if (w >= nitems) return;
+  const Item it = items[w];
+  const Panel P = panels[it.panel];
+  const float* inc = in + int64_t(blockIdx.y) * ld_in * kMR;
+  const int rows = min(T, P.m - it.chunk * T);
+  const int64_t h = tile_height(P.m, it.chunk, 4);
+  float* dst = it.part < 0 ? y + int64_t(blockIdx.y) * ld_y * kMR + (P.yoff + int64_t(it.chunk) * T) * kMR
+                           : ypart + int64_t(blockIdx.y) * ypart_ld * kMR + int64_t(it.part) * T * kMR;
+  unsigned char* base = msm + wid * kMWarpSmem;
+  switch (int(h + 31) / 32) {
+    case 1: panel_tile_mr_item<1>(segs, it, rows, h, inc, dst, base, lane); break;
+    case 2: panel_tile_mr_item<2>(segs, it, rows, h, inc, dst, base, lane); break;
+    case 3: panel_tile_mr_item<3>(segs, it, rows, h, inc, dst, base, lane); break;
+    default: panel_tile_mr_item<4>(segs, it, rows, h, inc, dst, base, lane); break;
+  }
+}
+
+// One CTA per split panel chunk, a warp per row (a lane per right-hand side).
 __global__ void __launch_bounds__(256) panel_fix_mr_kernel(const Panel* __restrict__ panels,
-                                                           const PanelFix* __restrict__ fix, int nfix,
+                                                           const PanelFix* __restrict__ fix,
                                                            const float* __restrict__ ypart, int64_t ypart_ld,
                                                            float* __restrict__ y, int64_t ld_y) {
   constexpr int rows = 128;
-  const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  const int64_t fq = t / kMR;
-  const int c = int(t % kMR);
-  const int f = int(fq / rows), q = int(fq % rows);
-  if (f >= nfix) return;
-  const PanelFix F = fix[f];
+  const int lane = threadIdx.x & 31;
+  const PanelFix F = fix[blockIdx.x];
   const Panel P = panels[F.panel];
-  const int i = F.chunk * rows + q;
-  if (i >= P.m) return;
-  const float* yp = ypart + int64_t(blockIdx.y) * ypart_ld * kMR;
-  float acc = 0.f;
-  for (int g = 0; g < F.count; g++) acc += yp[((int64_t(F.part) + g) * rows + q) * kMR + c];
-  y[int64_t(blockIdx.y) * ld_y * kMR + (P.yoff + i) * kMR + c] = acc;
+  const float* yp = ypart + int64_t(blockIdx.y) * ypart_ld * kMR + int64_t(F.part) * rows * kMR + lane;
+  float* yo = y + int64_t(blockIdx.y) * ld_y * kMR + (P.yoff + F.chunk * rows) * kMR + lane;
+  const int n = min(rows, P.m - F.chunk * rows);
+  for (int i = threadIdx.x >> 5; i < n; i += 8)
+    yo[int64_t(i) * kMR] = sum_parts(yp + int64_t(i) * kMR, F.count, int64_t(rows) * kMR);
 }
 
-// in (chunk ch, interleaved) <- x (caller order, column major total_n x k)
+// in (chunk ch, interleaved) <- x (caller order, column major total_n x k): 32
+// points of the caller's order at a time, read column by column, written as
+// whole rows at their tree positions.
 __global__ void __launch_bounds__(256) batch_gather_mr_kernel(const BatchInst* __restrict__ inst,
                                                               const float* __restrict__ x, int64_t total_n, int k,
                                                               float* __restrict__ in, int64_t ld_in, int ch) {
+  __shared__ float tile[32][kMR + 1];
   const BatchInst I = inst[blockIdx.y];
   float* inc = in + int64_t(ch) * ld_in * kMR;
-  for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < I.n * kMR;
-       e += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t r = e / kMR;
-    const int c = int(e % kMR), col = ch * kMR + c;
-    inc[(I.in_base + r) * kMR + c] = col < k ? x[int64_t(col) * total_n + I.x_base + I.perm[r]] : 0.f;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int64_t p0 = int64_t(blockIdx.x) * 32; p0 < I.n; p0 += int64_t(gridDim.x) * 32) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int c = wid * 4 + q, col = ch * kMR + c;
+      tile[lane][c] = col < k && p0 + lane < I.n ? x[int64_t(col) * total_n + I.x_base + p0 + lane] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int64_t p = p0 + wid * 4 + q;
+      if (p < I.n) inc[(I.in_base + I.iperm[p]) * kMR + lane] = tile[wid * 4 + q][lane];
+    }
+    __syncthreads();
   }
 }
 
+// A CTA takes 32 points of one instance in the caller's order: each warp reads
+// whole 128-byte rows of the slots (at the points' tree positions), and the sums
+// are written from shared memory as runs of 32 points of a column (written row
+// by row in tree order, each value was a sector of its own: 313 us for 420,000
+// points against 60).
 __global__ void __launch_bounds__(256) batch_combine_mr_kernel(const BatchInst* __restrict__ inst,
                                                                const float* __restrict__ y, int64_t ld_y,
                                                                float* __restrict__ out, int64_t total_n, int k, int ch) {
+  __shared__ float tile[32][kMR + 1];
   const BatchInst I = inst[blockIdx.y];
   const float* yc = y + int64_t(ch) * ld_y * kMR;
-  for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < I.n * kMR;
-       e += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t r = e / kMR;
-    const int c = int(e % kMR), col = ch * kMR + c;
-    if (col >= k) continue;
-    double acc = double(yc[(I.y_base + r) * kMR + c]);
-    for (int s = 1; s < I.nslots; s++) acc += double(yc[(I.y_base + int64_t(s) * I.n + r) * kMR + c]);
-    out[int64_t(col) * total_n + I.x_base + I.perm[r]] = float(acc);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int64_t p0 = int64_t(blockIdx.x) * 32; p0 < I.n; p0 += int64_t(gridDim.x) * 32) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int64_t p = p0 + wid * 4 + q;
+      if (p < I.n) {
+        const float* yr = yc + (I.y_base + I.iperm[p]) * kMR + lane;
+        // summed as FP32 pairs, rounded once (FP64 sums held the kernel up)
+        float acc = yr[0], err = 0.f;
+        for (int s = 1; s < I.nslots; s++) pair_add(acc, err, yr[int64_t(s) * I.n * kMR], 0.f);
+        tile[wid * 4 + q][lane] = __fadd_rn(acc, err);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int c = wid * 4 + q, col = ch * kMR + c;
+      if (col < k && p0 + lane < I.n) out[int64_t(col) * total_n + I.x_base + p0 + lane] = tile[lane][c];
+    }
+    __syncthreads();
   }
+}
+
+__global__ void __launch_bounds__(256) invert_perm_kernel(const int64_t* __restrict__ perm, int64_t n,
+                                                          int32_t* __restrict__ iperm) {
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+    iperm[perm[i]] = int32_t(i);
 }
 
 }  // namespace
@@ -2518,9 +2555,9 @@ cudaError_t launch_panels_mr(const Panel* panels, const Seg* segs, const Item* s
   if (nsmall + nbig <= 0) return cudaSuccess;
   count_launches(uint64_t(nbig > 0) + uint64_t(nsmall > 0) + uint64_t(nfix > 0));
   if (nbig > 0) {
-    cudaFuncSetAttribute(panel_tile_mr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMWarps * kMTWarpSmem);
+    cudaFuncSetAttribute(panel_tile_mr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMWarps * kMWarpSmem);
     dim3 g(unsigned((nbig + kMWarps - 1) / kMWarps), unsigned(nchunks));
-    panel_tile_mr_kernel<<<g, kMWarps * 32, kMWarps * kMTWarpSmem, st>>>(panels, segs, big, nbig, ypart, ypart_ld, in,
+    panel_tile_mr_kernel<<<g, kMWarps * 32, kMWarps * kMWarpSmem, st>>>(panels, segs, big, nbig, ypart, ypart_ld, in,
                                                                           ld_in, y, ld_y);
   }
   if (nsmall > 0) {
@@ -2530,8 +2567,7 @@ cudaError_t launch_panels_mr(const Panel* panels, const Seg* segs, const Item* s
                                                                            ld_y, ypart, ypart_ld);
   }
   if (nfix > 0) {
-    dim3 gf(unsigned((int64_t(nfix) * 128 * kMR + 255) / 256), unsigned(nchunks));
-    panel_fix_mr_kernel<<<gf, 256, 0, st>>>(panels, fix, nfix, ypart, ypart_ld, y, ld_y);
+    panel_fix_mr_kernel<<<dim3(unsigned(nfix), unsigned(nchunks)), 256, 0, st>>>(panels, fix, ypart, ypart_ld, y, ld_y);
   }
   return cudaGetLastError();
 }
@@ -2541,8 +2577,15 @@ cudaError_t launch_batch_gather_mr(const BatchInst* inst, int count, int64_t max
   if (count <= 0) return cudaSuccess;
   for (int ch = 0; ch < nchunks; ch++) {
     count_launches(1);
-    batch_gather_mr_kernel<<<batch_grid(count, max_n * kMR), 256, 0, st>>>(inst, x, total_n, k, in, ld_in, ch);
+    batch_gather_mr_kernel<<<dim3(unsigned(std::min<int64_t>((max_n + 31) / 32, 2048)), unsigned(count)), 256, 0, st>>>(inst, x, total_n, k, in, ld_in, ch);
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_invert_perm(const int64_t* perm, int64_t n, int32_t* iperm, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  count_launches(1);
+  invert_perm_kernel<<<vec_grid(n), 256, 0, st>>>(perm, n, iperm);
   return cudaGetLastError();
 }
 
@@ -2551,7 +2594,7 @@ cudaError_t launch_batch_combine_mr(const BatchInst* inst, int count, int64_t ma
   if (count <= 0) return cudaSuccess;
   for (int ch = 0; ch < nchunks; ch++) {
     count_launches(1);
-    batch_combine_mr_kernel<<<batch_grid(count, max_n * kMR), 256, 0, st>>>(inst, y, ld_y, out, total_n, k, ch);
+    batch_combine_mr_kernel<<<dim3(unsigned(std::min<int64_t>((max_n + 31) / 32, 2048)), unsigned(count)), 256, 0, st>>>(inst, y, ld_y, out, total_n, k, ch);
   }
   return cudaGetLastError();
 }

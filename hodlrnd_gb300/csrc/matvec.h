@@ -225,8 +225,11 @@ cudaError_t launch_copy_rows(const RowCopy* d, int n, cudaStream_t st);
 struct BatchInst {
   int64_t n, x_base, in_base, y_base;
   const int64_t* perm;  // tree position -> caller index within the instance
+  const int32_t* iperm;  // caller index -> tree position (FP32-vector batches)
   int32_t nslots, pad;
 };
+// iperm[perm[i]] = i
+cudaError_t launch_invert_perm(const int64_t* perm, int64_t n, int32_t* iperm, cudaStream_t st);
 // in[in_base + r] = x[x_base + perm[r]] for every instance (vectors of type x)
 cudaError_t launch_batch_gather(Prec x, const BatchInst* inst, int count, int64_t max_n, const void* src, void* in,
                                 cudaStream_t st);
