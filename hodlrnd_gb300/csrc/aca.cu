@@ -22,10 +22,19 @@
 // block has its own splitmix64 stream seeded from (level, target, source), so
 // blocks can run in any order (the CPU oracle does the same in rng_mode 1).
 //
-// Residual rows/columns are formed with one rounding per operation
-// (__dsub_rn/__dmul_rn) in the same order as the reference, so the factors
-// match the oracle bit for bit; only the norm reductions are summed in a
+// Residual rows/columns are formed with one rounding per operation in the same
+// order as the reference, so the factors match the oracle bit for bit; only the norm reductions are summed in a
 // different order.
+//
+// The FP64 pipe bounds it (20 cycles of an SM per warp instruction; 80-85% busy
+// whenever an SM works), so what need not be FP64 is not: square roots and
+// divisions on the integer pipe (softfp.cuh), pivots compared as integers, eight
+// dot products of the norm estimate reduced together in the warp teams, no lane's
+// FP64 work beyond a warp's share of a row.  3D N = 100003: CTA teams 236 -> 219
+// ms, warp teams 248 -> 184 (a residual row's code at one call site each also
+// keeps the warp teams, which run at different points of it, in the instruction
+// cache).  What is left is the residuals' products and subtractions, which must
+// round one by one.
 //
 // Rows and columns are indexed in the reference's order of the node's points
 // (by caller index; a non-leaf node's tree-order range is grouped by leaf
@@ -65,6 +74,7 @@ __host__ __device__ constexpr int staged_team_bytes(int T, int D) {
 
 template <int D, class Team, bool S = false>
 struct AcaTeam {
+  static constexpr int JU = S ? 1 : Team::kSize == 32 ? 2 : 4;  // entries of a residual row or column a thread forms together
   const AcaArgs& a;
   const AcaBlockDesc& B;
   Team tm;
@@ -260,79 +270,122 @@ struct AcaTeam {
       pi = a.lmap[B.t_map + i0];
       load_point<D>(a.P, pi, xi);
     }
-    double ba = -1.0, bv = 0.0, v0 = 0.0, s = 0.0;
+    unsigned long long bk = 0;
+    double v0 = 0.0, s = 0.0;
     int bi = 0x7fffffff;
-    for (int j = tm.tid(); j < n; j += Team::kSize) {
-      double val;
-      if constexpr (S)
-        val = kernel_entry_xy<D>(K, pi == is[j], xi, xs + j, n);
-      else
-        val = kernel_entry<D>(a.P, K, pi, a.lmap[B.s_map + j], xi);
-      for (int k = 0; k < r; k++) val = __dsub_rn(val, __dmul_rn(U[i0 + int64_t(k) * m], V[j + int64_t(k) * n]));
-      V[j + int64_t(r) * n] = val;
-      s += val * val;
-      if (j == 0) v0 = val;
-      if ((cb[j >> 5] >> (j & 31)) & 1u) {
-        const double av = fabs(val);
-        if (av > ba) {
-          ba = av;
-          bi = j;
-          bv = val;
+    const int w0 = tm.tid() & ~31;  // the warp's first place in the team
+    // JU columns per thread at a time: their chains of subtractions overlap
+    for (int jb = 0; jb + w0 < n; jb += JU * Team::kSize) {
+      double val[JU];
+      int jj[JU];
+#pragma unroll
+      for (int q = 0; q < JU; q++) {
+        if (jb + q * Team::kSize + w0 >= n) break;  // warp-uniform
+        const int j = min(jb + q * Team::kSize + tm.tid(), n - 1);
+        jj[q] = j;
+        if constexpr (S)
+          val[q] = kernel_entry_xy<D>(K, pi == is[j], xi, xs + j, n);
+        else
+          val[q] = kernel_entry<D>(a.P, K, pi, a.lmap[B.s_map + j], xi);
+      }
+      for (int k = 0; k < r; k++) {
+        const double u = U[i0 + int64_t(k) * m];
+        const double* Vk = V + int64_t(k) * n;
+#pragma unroll
+        for (int q = 0; q < JU; q++) {
+          if (jb + q * Team::kSize + w0 >= n) break;
+          val[q] = __dsub_rn(val[q], __dmul_rn(u, Vk[jj[q]]));
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < JU; q++) {
+        const int j = jb + q * Team::kSize + tm.tid();
+        if (j >= n) break;
+        V[j + int64_t(r) * n] = val[q];
+        s += val[q] * val[q];
+        if (j == 0) v0 = val[q];
+        if ((cb[j >> 5] >> (j & 31)) & 1u) {
+          const unsigned long long key = pivot_key(val[q]);
+          if (!pivot_nan(key) && pivot_better(key, j, bk, bi)) {
+            bk = key;
+            bi = j;
+          }
         }
       }
     }
     sq = s;
-    tm.argmax(ba, bi, bv);
+    tm.argmax(bk, bi);
     if (nc == 0) {
       piv = 0;
       mx = tm.bcast(v0);
     } else {
       piv = bi;
-      mx = bv;
+      mx = pivot_value(bk);
     }
     tm.sync();
   }
 
   // Residual column j0 into U[:, r]; argmax over the remaining rows.
   __device__ void gen_col(int j0, int r, int nr, double& mx, int& piv, double& sq) {
-    double ba = -1.0, bv = 0.0, v0 = 0.0, s = 0.0;
+    unsigned long long bk = 0;
+    double v0 = 0.0, s = 0.0;
     int bi = 0x7fffffff;
     const int64_t pj = S ? int64_t(is[j0]) : int64_t(a.lmap[B.s_map + j0]);
-    for (int i = tm.tid(); i < m; i += Team::kSize) {
-      // A(i, j0) with the target point first, as getCol evaluates it
-      // (getMatrixEntry(sources[j], k), kernel_function.hpp:32-40).
-      double xi[D];
-      double val;
-      if constexpr (S) {
+    const int w0 = tm.tid() & ~31;
+    for (int ib = 0; ib + w0 < m; ib += JU * Team::kSize) {
+      double val[JU];
+      int ii[JU];
 #pragma unroll
-        for (int k = 0; k < D; k++) xi[k] = xt[k * m + i];
-        val = kernel_entry_xy<D>(K, it[i] == pj, xi, xs + j0, n);
-      } else {
-        const int64_t pi = a.lmap[B.t_map + i];
-        load_point<D>(a.P, pi, xi);
-        val = kernel_entry<D>(a.P, K, pi, pj, xi);
+      for (int q = 0; q < JU; q++) {
+        if (ib + q * Team::kSize + w0 >= m) break;  // warp-uniform
+        const int i = min(ib + q * Team::kSize + tm.tid(), m - 1);
+        ii[q] = i;
+        // A(i, j0) with the target point first, as getCol evaluates it
+        // (getMatrixEntry(sources[j], k), kernel_function.hpp:32-40).
+        double xi[D];
+        if constexpr (S) {
+#pragma unroll
+          for (int k = 0; k < D; k++) xi[k] = xt[k * m + i];
+          val[q] = kernel_entry_xy<D>(K, it[i] == pj, xi, xs + j0, n);
+        } else {
+          const int64_t pi = a.lmap[B.t_map + i];
+          load_point<D>(a.P, pi, xi);
+          val[q] = kernel_entry<D>(a.P, K, pi, pj, xi);
+        }
       }
-      for (int k = 0; k < r; k++) val = __dsub_rn(val, __dmul_rn(V[j0 + int64_t(k) * n], U[i + int64_t(k) * m]));
-      U[i + int64_t(r) * m] = val;
-      s += val * val;
-      if (i == 0) v0 = val;
-      if ((rb[i >> 5] >> (i & 31)) & 1u) {
-        const double av = fabs(val);
-        if (av > ba) {
-          ba = av;
-          bi = i;
-          bv = val;
+      for (int k = 0; k < r; k++) {
+        const double v = V[j0 + int64_t(k) * n];
+        const double* Uk = U + int64_t(k) * m;
+#pragma unroll
+        for (int q = 0; q < JU; q++) {
+          if (ib + q * Team::kSize + w0 >= m) break;
+          val[q] = __dsub_rn(val[q], __dmul_rn(v, Uk[ii[q]]));
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < JU; q++) {
+        const int i = ib + q * Team::kSize + tm.tid();
+        if (i >= m) break;
+        U[i + int64_t(r) * m] = val[q];
+        s += val[q] * val[q];
+        if (i == 0) v0 = val[q];
+        if ((rb[i >> 5] >> (i & 31)) & 1u) {
+          const unsigned long long key = pivot_key(val[q]);
+          if (!pivot_nan(key) && pivot_better(key, i, bk, bi)) {
+            bk = key;
+            bi = i;
+          }
         }
       }
     }
     sq = s;
-    tm.argmax(ba, bi, bv);
+    tm.argmax(bk, bi);
     if (nr == 0) {
       piv = 0;
       mx = tm.bcast(v0);
     } else {
       piv = bi;
-      mx = bv;
+      mx = pivot_value(bk);
     }
     tm.sync();
   }
@@ -340,8 +393,8 @@ struct AcaTeam {
   // mnorm += 2 |u_k . u_r| |v_k . v_r| for k < r, in order of k (LowRank_matrix.hpp:335-338).
   // A CTA team gives each dot product pair to one warp (a warp reduction, no
   // barrier), writes the terms to shared memory and adds them in order after
-  // one barrier per kNormChunk columns; warp and sub-warp teams reduce each
-  // pair across the team.
+  // one barrier per kNormChunk columns; a warp team reduces eight columns'
+  // products at a time, a sub-warp team each pair across the team.
   __device__ void norm_update(int r, double& mnorm) {
     if constexpr (Team::kSize > 32) {
       constexpr int W = Team::kSize / 32;
@@ -353,13 +406,54 @@ struct AcaTeam {
           double du = 0.0, dv = 0.0;
           for (int i = lane; i < m; i += 32) du += U[i + int64_t(k) * m] * U[i + int64_t(r) * m];
           for (int j = lane; j < n; j += 32) dv += V[j + int64_t(k) * n] * V[j + int64_t(r) * n];
-          du = WarpTeam().sum(du);
-          dv = WarpTeam().sum(dv);
+          WarpTeam().sum2(du, dv);
           if (lane == 0) tm.terms[kk] = __dmul_rn(__dmul_rn(2.0, fabs(du)), fabs(dv));
         }
         __syncthreads();
         for (int kk = 0; kk < kn; kk++) mnorm += tm.terms[kk];
         __syncthreads();
+      }
+    } else if constexpr (Team::kSize == 32) {
+      // eight columns at a time: their 16 dot products are reduced together by a
+      // transposed butterfly (each exchange hands half of the values to the
+      // partner lane) -- 16 FP64 additions instead of 80, which outweighed
+      // the products themselves in blocks of a few points per lane
+      const int lane = threadIdx.x & 31;
+      for (int k0 = 0; k0 < r; k0 += 8) {
+        double d[16];  // u_k . u_r for k0 .. k0 + 7, then v_k . v_r
+#pragma unroll
+        for (int q = 0; q < 16; q++) d[q] = 0.0;
+        const int kn = r - k0;
+        const double *Uk = U + int64_t(k0) * m, *Ur = U + int64_t(r) * m;
+        for (int i = lane; i < m; i += 32) {
+          const double ur = Ur[i];
+#pragma unroll
+          for (int q = 0; q < 8; q++)
+            if (q < kn) d[q] += Uk[i + int64_t(q) * m] * ur;
+        }
+        const double *Vk = V + int64_t(k0) * n, *Vr = V + int64_t(r) * n;
+        for (int j = lane; j < n; j += 32) {
+          const double vr = Vr[j];
+#pragma unroll
+          for (int q = 0; q < 8; q++)
+            if (q < kn) d[8 + q] += Vk[j + int64_t(q) * n] * vr;
+        }
+#pragma unroll
+        for (int w = 8, o = 16; w > 0; w >>= 1, o >>= 1) {
+          const bool up = (lane & o) != 0;
+#pragma unroll
+          for (int q = 0; q < 8; q++)
+            if (q < w) {
+              const double send = up ? d[q] : d[q + w], keep = up ? d[q + w] : d[q];
+              d[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+        // lane 16 h + 2 q (+ 1): the u (h = 0) or v product of column k0 + q
+        const double mine = d[0] + __shfl_xor_sync(0xffffffffu, d[0], 1);
+        const double other = __shfl_xor_sync(0xffffffffu, mine, 16);
+        const bool v = (lane & 16) != 0;
+        const double term = __dmul_rn(__dmul_rn(2.0, fabs(v ? other : mine)), fabs(v ? mine : other));
+        for (int q = 0; q < min(kn, 8); q++) mnorm += __shfl_sync(0xffffffffu, term, 2 * q);
       }
     } else {
       for (int k = 0; k < r; k++) {
@@ -397,10 +491,11 @@ struct AcaTeam {
         break;
       }
       double rsq_p = 0.0, csq_p = 0.0;
-      gen_row(cur_row, r, nc, mx, piv, rsq_p);
       int count = 0;
       bool at_end = false, use_rand = true;
-      while (fabs(mx) < tol && count < kMaxTries && nc > 0 && nr > 0) {
+      for (;;) {  // one call site: the code of a residual row is long
+        gen_row(cur_row, r, nc, mx, piv, rsq_p);
+        if (!(fabs(mx) < tol && count < kMaxTries && nc > 0 && nr > 0)) break;
         int nrw;
         if (r < 3) {
           nrw = at_end ? last(rb, nwr) : first(rb, nwr);
@@ -418,7 +513,6 @@ struct AcaTeam {
         if (tm.tid() == 0) rl[nrow - 1] = nrw;
         if (erase(rb, nrw)) nr--;
         cur_row = nrw;
-        gen_row(cur_row, r, nc, mx, piv, rsq_p);
         count++;
       }
       if (count == kMaxTries || nc == 0 || nr == 0) break;
@@ -426,10 +520,11 @@ struct AcaTeam {
       if (tm.tid() == 0) cl[ncol] = piv;
       ncol++;
       if (erase(cb, piv)) nc--;
-      gamma = __ddiv_rn(1.0, mx);
+      gamma = soft_div(soft_unpack(1.0), 1.0, mx);
       int cur_col = piv;
-      gen_col(cur_col, r, nr, mx, piv, csq_p);
-      while (fabs(mx) < tol && count < kMaxTries && nc > 0 && nr > 0) {
+      for (;;) {
+        gen_col(cur_col, r, nr, mx, piv, csq_p);
+        if (!(fabs(mx) < tol && count < kMaxTries && nc > 0 && nr > 0)) break;
         int ncl;
         if (ncol - 1 < 3) {
           ncl = at_end ? nc : first(cb, nwc);
@@ -447,7 +542,6 @@ struct AcaTeam {
         if (tm.tid() == 0) cl[ncol - 1] = ncl;
         if (erase(cb, ncl)) nc--;
         cur_col = ncl;
-        gen_col(cur_col, r, nr, mx, piv, csq_p);
         count++;
       }
       if (tm.tid() == 0) rl[nrow] = piv;
@@ -458,9 +552,10 @@ struct AcaTeam {
       for (int i = tm.tid(); i < m; i += Team::kSize)
         U[i + int64_t(r) * m] = __dmul_rn(gamma, U[i + int64_t(r) * m]);
       tm.sync();
-      const double rsq = tm.sum(rsq_p), csq = tm.sum(csq_p);
-      row_norm = sqrt(rsq);
-      col_norm = sqrt(csq);
+      double rsq = rsq_p, csq = csq_p;
+      tm.sum2(rsq, csq);
+      row_norm = soft_sqrt(rsq);
+      col_norm = soft_sqrt(csq);
       mnorm += fabs(__dmul_rn(__dmul_rn(__dmul_rn(gamma, gamma), rsq), csq));
       norm_update(r, mnorm);
       r++;
@@ -493,7 +588,7 @@ __device__ __forceinline__ int next_item(const AcaArgs& a, int kind, int first, 
 }
 
 template <int D>
-__global__ void __launch_bounds__(128) aca_warp_kernel(AcaArgs a, const int32_t* __restrict__ list, int count) {
+__global__ void __launch_bounds__(128, 4) aca_warp_kernel(AcaArgs a, const int32_t* __restrict__ list, int count) {
   WarpTeam tm;
   int pass = 0;
   for (;;) {
@@ -507,10 +602,10 @@ __global__ void __launch_bounds__(128) aca_warp_kernel(AcaArgs a, const int32_t*
 
 template <int D>
 __global__ void __launch_bounds__(256) aca_cta_kernel(AcaArgs a, const int32_t* __restrict__ list, int count) {
-  __shared__ double red[256 / 32 + 1];
+  __shared__ double red[256 / 32 + 1], red2[256 / 32 + 1];
   __shared__ double terms[kNormChunk];
   __shared__ int redi[256 / 32 + 1];
-  CtaTeam<256> tm{red, redi, terms};
+  CtaTeam<256> tm{red, red2, redi, terms};
   int pass = 0;
   for (;;) {
     const int q = next_item(a, kAcaTeamCta, int(blockIdx.x), pass, tm);

@@ -6,6 +6,8 @@
 
 #include <atomic>
 
+#include "softfp.cuh"
+
 namespace hodlr {
 
 // Process-wide count of this engine's kernel launches (hodlr_kernel_launches).
@@ -27,6 +29,21 @@ struct PointsDev {
   int64_t ld;
 };
 
+// The kernel of a squared distance, with one rounding per operation; square
+// roots and divisions on the integer pipe (softfp.cuh: 3D assembly of near
+// tiles 1.95 -> 1.05 ms at N = 100003).
+inline __device__ __noinline__ double kernel_log_exp(int kind, double scale, double d2) {
+  const double r = soft_sqrt(d2);
+  return __dmul_rn(scale, kind == kLogR ? log(r) : exp(-r));
+}
+__device__ __forceinline__ double kernel_of(const KernelDev& K, double d2) {
+  switch (K.kind) {
+    case kInvR: return soft_div_sqrt(soft_unpack(K.scale), K.scale, d2);
+    case kInvR2: return soft_div(soft_unpack(K.scale), K.scale, d2);
+    default: return kernel_log_exp(K.kind, K.scale, d2);
+  }
+}
+
 // One matrix entry A(i, j) for tree positions i, j (kernel_function::getRow /
 // getCol / getMatrix + the user getMatrixEntry, include/kernel_function.hpp:20-53).
 // d2 is accumulated in dimension order with one rounding per operation (the
@@ -39,18 +56,14 @@ template <int D>
 __device__ __forceinline__ double kernel_entry(const PointsDev& P, const KernelDev& K, int64_t i, int64_t j,
                                                const double* xi) {
   if (i == j) return K.diag;
-  double d2 = 0.0;
+  double d2;
 #pragma unroll
   for (int k = 0; k < D; k++) {
     const double t = __dsub_rn(xi[k], P.x[k * P.ld + j]);
-    d2 = __dadd_rn(d2, __dmul_rn(t, t));
+    const double tt = __dmul_rn(t, t);
+    d2 = k == 0 ? tt : __dadd_rn(d2, tt);  // 0 + tt is tt
   }
-  switch (K.kind) {
-    case kInvR: return __ddiv_rn(K.scale, __dsqrt_rn(d2));
-    case kInvR2: return __ddiv_rn(K.scale, d2);
-    case kLogR: return __dmul_rn(K.scale, log(__dsqrt_rn(d2)));
-    default: return __dmul_rn(K.scale, exp(-__dsqrt_rn(d2)));
-  }
+  return kernel_of(K, d2);
 }
 
 // The same entry from two staged coordinate vectors (stride ld between
@@ -59,18 +72,14 @@ template <int D>
 __device__ __forceinline__ double kernel_entry_xy(const KernelDev& K, bool same_point, const double* xi,
                                                   const double* xj, int ld) {
   if (same_point) return K.diag;
-  double d2 = 0.0;
+  double d2;
 #pragma unroll
   for (int k = 0; k < D; k++) {
     const double t = __dsub_rn(xi[k], xj[k * ld]);
-    d2 = __dadd_rn(d2, __dmul_rn(t, t));
+    const double tt = __dmul_rn(t, t);
+    d2 = k == 0 ? tt : __dadd_rn(d2, tt);  // 0 + tt is tt
   }
-  switch (K.kind) {
-    case kInvR: return __ddiv_rn(K.scale, __dsqrt_rn(d2));
-    case kInvR2: return __ddiv_rn(K.scale, d2);
-    case kLogR: return __dmul_rn(K.scale, log(__dsqrt_rn(d2)));
-    default: return __dmul_rn(K.scale, exp(-__dsqrt_rn(d2)));
-  }
+  return kernel_of(K, d2);
 }
 
 template <int D>
@@ -120,6 +129,24 @@ __device__ __forceinline__ void pair_add(float& s, float& c, float s2, float c2)
   c = __fadd_rn(__fadd_rn(c, c2), err);
 }
 
+// A pivot candidate's value as an integer that orders like its magnitude: the
+// bits of |v|, with the sign below them (FP64 comparisons take GB300's slow FP64
+// pipe, integer ones do not).  The largest (key >> 1) with the lowest index is the
+// pivot; a NaN is no candidate (it compares false), nor is "none" = (0, INT_MAX),
+// which loses the tie with a zero.
+__device__ __forceinline__ unsigned long long pivot_key(double v) {
+  const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v));
+  return (b << 1) | (b >> 63);
+}
+__device__ __forceinline__ bool pivot_nan(unsigned long long key) { return (key >> 1) > 0x7ff0000000000000ull; }
+__device__ __forceinline__ double pivot_value(unsigned long long key) {
+  return __longlong_as_double(static_cast<long long>((key >> 1) | (key << 63)));
+}
+__device__ __forceinline__ bool pivot_better(unsigned long long k2, int i2, unsigned long long k, int i) {
+  const unsigned long long a2 = k2 >> 1, a = k >> 1;
+  return a2 > a || (a2 == a && i2 < i);
+}
+
 // ---------------------------------------------------------------- teams
 // A "team" is the group of threads that compresses one block: a warp, or a
 // whole CTA.  All members call every team function (uniform control flow).
@@ -133,18 +160,25 @@ struct WarpTeam {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
   }
+  // The sums of a and b (one butterfly: lanes 0-15 end with a's, 16-31 with b's).
+  __device__ __forceinline__ void sum2(double& a, double& b) const {
+    const bool up = (threadIdx.x & 16) != 0;
+    double v = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    a = __shfl_sync(0xffffffffu, v, 0);
+    b = __shfl_sync(0xffffffffu, v, 16);
+  }
   // Largest |v|, lowest index on ties (kernel_function::maxAbsVector keeps the
   // first maximum, include/kernel_function.hpp:55-68).
-  __device__ __forceinline__ void argmax(double& a, int& i, double& v) const {
+  __device__ __forceinline__ void argmax(unsigned long long& k, int& i) const {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      const double a2 = __shfl_xor_sync(0xffffffffu, a, o);
+      const unsigned long long k2 = __shfl_xor_sync(0xffffffffu, k, o);
       const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-      const double v2 = __shfl_xor_sync(0xffffffffu, v, o);
-      if (a2 > a || (a2 == a && i2 < i)) {
-        a = a2;
+      if (pivot_better(k2, i2, k, i)) {
+        k = k2;
         i = i2;
-        v = v2;
       }
     }
   }
@@ -167,16 +201,18 @@ struct SubTeam {
     for (int o = T / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o, T);
     return v;
   }
-  __device__ __forceinline__ void argmax(double& a, int& i, double& v) const {
+  __device__ __forceinline__ void sum2(double& a, double& b) const {
+    a = sum(a);
+    b = sum(b);
+  }
+  __device__ __forceinline__ void argmax(unsigned long long& k, int& i) const {
 #pragma unroll
     for (int o = T / 2; o > 0; o >>= 1) {
-      const double a2 = __shfl_xor_sync(mask, a, o, T);
+      const unsigned long long k2 = __shfl_xor_sync(mask, k, o, T);
       const int i2 = __shfl_xor_sync(mask, i, o, T);
-      const double v2 = __shfl_xor_sync(mask, v, o, T);
-      if (a2 > a || (a2 == a && i2 < i)) {
-        a = a2;
+      if (pivot_better(k2, i2, k, i)) {
+        k = k2;
         i = i2;
-        v = v2;
       }
     }
   }
@@ -189,6 +225,7 @@ struct CtaTeam {
   static constexpr int kSize = NT;
   static constexpr int kWarps = NT / 32;
   double* red;    // shared, kWarps + 1
+  double* red2;   // shared, kWarps + 1
   int* redi;      // shared, kWarps + 1
   double* terms;  // shared, kNormChunk: the norm estimate's terms of one pass (ACA)
   __device__ __forceinline__ int tid() const { return threadIdx.x; }
@@ -210,30 +247,48 @@ struct CtaTeam {
     __syncthreads();
     return v;
   }
-  __device__ __forceinline__ void argmax(double& a, int& i, double& v) const {
+  __device__ __forceinline__ void sum2(double& a, double& b) const {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    WarpTeam().argmax(a, i, v);
-    __shared__ double sa[kWarps + 1], sv[kWarps + 1];
+    WarpTeam().sum2(a, b);
     if (lane == 0) {
-      sa[w] = a;
-      sv[w] = v;
+      red[w] = a;
+      red2[w] = b;
+    }
+    __syncthreads();
+    if (w == 0) {
+      a = lane < kWarps ? red[lane] : 0.0;
+      b = lane < kWarps ? red2[lane] : 0.0;
+      WarpTeam().sum2(a, b);
+      if (lane == 0) {
+        red[kWarps] = a;
+        red2[kWarps] = b;
+      }
+    }
+    __syncthreads();
+    a = red[kWarps];
+    b = red2[kWarps];
+    __syncthreads();
+  }
+  __device__ __forceinline__ void argmax(unsigned long long& k, int& i) const {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    WarpTeam().argmax(k, i);
+    __shared__ unsigned long long sk[kWarps + 1];
+    if (lane == 0) {
+      sk[w] = k;
       redi[w] = i;
     }
     __syncthreads();
     if (w == 0) {
-      a = lane < kWarps ? sa[lane] : -1.0;
+      k = lane < kWarps ? sk[lane] : 0ull;
       i = lane < kWarps ? redi[lane] : 0x7fffffff;
-      v = lane < kWarps ? sv[lane] : 0.0;
-      WarpTeam().argmax(a, i, v);
+      WarpTeam().argmax(k, i);
       if (lane == 0) {
-        sa[kWarps] = a;
-        sv[kWarps] = v;
+        sk[kWarps] = k;
         redi[kWarps] = i;
       }
     }
     __syncthreads();
-    a = sa[kWarps];
-    v = sv[kWarps];
+    k = sk[kWarps];
     i = redi[kWarps];
     __syncthreads();
   }
