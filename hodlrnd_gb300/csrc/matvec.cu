@@ -351,15 +351,18 @@ __device__ __forceinline__ float2 to_input<FH>(float a) {
 // columns) load V directly.
 // Ring shapes (stages x bytes) of the staged kernels; HODLR_TUNE_* override
 // them at compile time for tuning runs.  Two stages per warp measured best on
-// GB300 (the shared memory per warp, not the stage count, limits the warps
-// per SM, and more warps hide more latency than deeper rings); V^T x stages
-// of 4 KB (with V grouped by source node, whole-row runs are long) beat 2 KB
-// by 2% per solve at N = 262144.
+// GB300: the shared memory per warp, not the stage count, limits the warps
+// per SM, and more warps hide more latency than deeper rings.  V^T x stages of
+// 3 KB and at most 64 rows (with V grouped by source node rows are long, and
+// room for the inputs of the narrowest rows took a third of the ring) allow 7
+// CTAs per SM instead of 4: 989 -> 920 us at N = 262144 in 3D (FP32), and 415 ->
+// 309 us for the two stages' worth of most items of 4D N = 65536 (BF16); with
+// 4 KB 922 and 330, with 2 KB 995 and 318.
 #ifndef HODLR_TUNE_Z_STAGES
 #define HODLR_TUNE_Z_STAGES 2
 #endif
 #ifndef HODLR_TUNE_Z_BYTES
-#define HODLR_TUNE_Z_BYTES 4096
+#define HODLR_TUNE_Z_BYTES 3072
 #endif
 #ifndef HODLR_TUNE_P_STAGES
 #define HODLR_TUNE_P_STAGES 2
@@ -382,9 +385,10 @@ __device__ __forceinline__ float2 to_input<FH>(float a) {
 constexpr int kZWarps = 4;                      // warps per CTA of zgemv_kernel
 constexpr int kZStages = HODLR_TUNE_Z_STAGES;   // ring stages per warp
 constexpr int kZStageBytes = HODLR_TUNE_Z_BYTES;  // V bytes per stage
-// input bytes per stage: at most kZStageBytes / 16 rows of 8 bytes, plus 2 x 15
-// bytes of alignment slack, rounded to 16
-constexpr int kZXBytes = (kZStageBytes / 16) * 8 + 32;
+constexpr int kZRows = 64;  // rows per stage at most
+// input bytes per stage: kZRows values of 8 bytes, plus 2 x 15 bytes of alignment
+// slack, rounded to 16
+constexpr int kZXBytes = kZRows * 8 + 32;
 constexpr int kZWarpSmem = 64 + kZStages * (kZStageBytes + kZXBytes);
 static_assert(kZWarpSmem % 16 == 0 && kZXBytes % 16 == 0, "bulk copy destinations must stay 16-byte aligned");
 
@@ -1675,7 +1679,7 @@ void z_item_stages(ZItem& it, int r, int esz) {
   int P = 1;
   while (P < lanes) P <<= 1;
   const int G = 32 / P, rowb = rp * esz;
-  it.R = (kZStageBytes / rowb) / G * G;  // >= G: rowb <= 16 P, kZStageBytes >= 512
+  it.R = std::min(kZStageBytes / rowb, kZRows) / G * G;  // >= G: rowb <= 16 P, kZStageBytes >= 512, kZRows >= 32
   it.nst = (it.j1 - it.j0 + it.R - 1) / it.R;
 }
 
