@@ -2092,7 +2092,7 @@ static_assert(kMWarpSmem % 16 == 0 && kMStageBytes % 16 == 0, "bulk copy destina
 // loads of 16 bytes feed 32 NQ FMAs.  Columns beyond the item's are computed
 // from whatever follows in the warp's shared memory and never stored.
 // 24 3D operators (420,000 points), 32 right-hand sides: V^T x 4.44 -> 1.52 ms, node
-// panels 2.19 -> 1.24 ms, leaf panels 3.65 -> 1.52 ms (whole product 11.1 -> 4.7 ms;
+// panels 2.19 -> 1.24 ms, leaf panels 3.65 -> 1.43 ms (whole product 11.1 -> 4.6 ms;
 // the FMAs alone would take 1.4).
 template <int NQ>
 __device__ __forceinline__ void mr_wide(const unsigned char* as, int rowb, const float* xs, int nr, int lane,
@@ -2322,11 +2322,11 @@ __device__ __forceinline__ void small_mr_item(const Seg* __restrict__ segs, cons
     return n;
   };
   static_assert(kMStages == 2, "two column counts");
-  float acc[RL][8];
+  uint64_t acc2[RL][4];  // pairs of right-hand sides: half the instructions (1.52 -> 1.43 ms for the two launches)
 #pragma unroll
   for (int i = 0; i < RL; i++)
 #pragma unroll
-    for (int r = 0; r < 8; r++) acc[i][r] = 0.f;
+    for (int r = 0; r < 4; r++) acc2[i][r] = 0;
   // the last group's rows beyond m read whatever follows in the warp's share and are never stored
   const int row0 = rr * RL;
   bool gave_up = false;
@@ -2351,12 +2351,12 @@ __device__ __forceinline__ void small_mr_item(const Seg* __restrict__ segs, cons
       for (int c = sl; c < cur; c += SL) {
         const float* a = reinterpret_cast<const float*>(su + co[c]) + row0;
         const float4 xa = x4[c * 8], xb = x4[c * 8 + 4];
-        const float x[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+        const uint64_t x[4] = {pack_f2(xa.x, xa.y), pack_f2(xa.z, xa.w), pack_f2(xb.x, xb.y), pack_f2(xb.z, xb.w)};
 #pragma unroll
         for (int i = 0; i < RL; i++) {
-          const float v = a[i];
+          const uint64_t v = pack_f2(a[i], a[i]);
 #pragma unroll
-          for (int r = 0; r < 8; r++) acc[i][r] = __fmaf_rn(v, x[r], acc[i][r]);
+          for (int r = 0; r < 4; r++) acc2[i][r] = fma_f2(v, x[r], acc2[i][r]);
         }
       }
       __syncwarp();
@@ -2364,6 +2364,11 @@ __device__ __forceinline__ void small_mr_item(const Seg* __restrict__ segs, cons
     cur = next;
     next = issue(st);  // into the stage just consumed
   }
+  float acc[RL][8];
+#pragma unroll
+  for (int i = 0; i < RL; i++)
+#pragma unroll
+    for (int r = 0; r < 4; r++) unpack_f2(acc2[i][r], acc[i][2 * r], acc[i][2 * r + 1]);
   for (int o = 4 * RR; o < 32; o <<= 1)
 #pragma unroll
     for (int i = 0; i < RL; i++)
