@@ -473,9 +473,9 @@ void build_near_plan(hodlr_op* op, const NearTiles& nt, const void* base, Prec a
   const int64_t big_bytes = spread ? item_bytes(total, kMinItemBytes, kNearItemBytes) : kNearItemBytes;
   // FP64 panels of at most 32 rows: the staged leaf kernel when leaves are tiny
   // (its one byte run per stage beats a segment per slice: 3D N = 262144, 8
-  // rows, 134 us against 183), else the items of launch_items64 with the larger
-  // panels (4D N = 65536, 16 rows, 198 us against 217; 3D N = 20011, 39 rows, 26 against
-  // 54), which also split; the two meet near 12 rows.
+  // rows, 127 us against 183), else the items of launch_items64 with the larger
+  // panels (4D N = 65536, 16 rows, 200 us against 199 and one launch less; 3D N =
+  // 20011, 39 rows, 26 against 54), which also split.
   int64_t npanels = 0;
   for (size_t k = 0; k + 1 < op->near.leaf_ptr.size(); k++) npanels += op->near.leaf_ptr[k] < op->near.leaf_ptr[k + 1];
   const bool leaf = a == Prec::kD && op->n <= 12 * npanels;

@@ -34,8 +34,6 @@ __device__ __forceinline__ bf16 ldg<bf16>(const bf16* p) {
   return bf16{__ldg(reinterpret_cast<const unsigned short*>(p))};
 }
 __device__ __forceinline__ float bf2f(unsigned short b) { return __uint_as_float(uint32_t(b) << 16); }
-__device__ __forceinline__ float to_f(float v) { return v; }
-__device__ __forceinline__ float to_f(bf16 v) { return bf2f(v.b); }
 
 template <typename T>
 struct Vec16;
@@ -115,6 +113,7 @@ struct Acc<float> {
   static __device__ __forceinline__ A scale(A a, float s) { return a * s; }
   static __device__ __forceinline__ X xscale(X x, float s) { return x * s; }
   static __device__ __forceinline__ A shfl_xor(A a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+  static __device__ __forceinline__ A shfl_down(A a, int o) { return __shfl_down_sync(0xffffffffu, a, o); }
   static __device__ __forceinline__ X shfl(X x, int src) { return __shfl_sync(0xffffffffu, x, src); }
   static __device__ __forceinline__ double value(A a) { return double(a); }
 };
@@ -132,6 +131,7 @@ struct Acc<double> {
   static __device__ __forceinline__ A scale(A a, float s) { return a * double(s); }
   static __device__ __forceinline__ X xscale(X x, float s) { return x * double(s); }
   static __device__ __forceinline__ A shfl_xor(A a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+  static __device__ __forceinline__ A shfl_down(A a, int o) { return __shfl_down_sync(0xffffffffu, a, o); }
   static __device__ __forceinline__ X shfl(X x, int src) { return __shfl_sync(0xffffffffu, x, src); }
   static __device__ __forceinline__ double value(A a) { return a; }
 };
@@ -191,6 +191,9 @@ struct Acc<DF> {
   static __device__ __forceinline__ A shfl_xor(A a, int o) {
     return DF{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
   }
+  static __device__ __forceinline__ A shfl_down(A a, int o) {
+    return DF{__shfl_down_sync(0xffffffffu, a.hi, o), __shfl_down_sync(0xffffffffu, a.lo, o)};
+  }
   static __device__ __forceinline__ X shfl(X x, int src) {
     return DF{__shfl_sync(0xffffffffu, x.hi, src), __shfl_sync(0xffffffffu, x.lo, src)};
   }
@@ -244,6 +247,7 @@ struct Acc<FH> {
   static __device__ __forceinline__ A scale(A a, float s) { return a * s; }
   static __device__ __forceinline__ X xscale(X x, float s) { return x * s; }
   static __device__ __forceinline__ A shfl_xor(A a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+  static __device__ __forceinline__ A shfl_down(A a, int o) { return __shfl_down_sync(0xffffffffu, a, o); }
   static __device__ __forceinline__ X shfl(X x, int src) { return __shfl_sync(0xffffffffu, x, src); }
   static __device__ __forceinline__ double value(A a) { return double(a); }
 };
@@ -256,8 +260,8 @@ struct IO<FH> {
 };
 
 // a += va * xa, b += vb * xb; compensated sums as packed pairs
-template <typename TACC>
-__device__ __forceinline__ void fma_pair(typename Acc<TACC>::A& a, typename Acc<TACC>::A& b, float va, float vb,
+template <typename TACC, typename V>
+__device__ __forceinline__ void fma_pair(typename Acc<TACC>::A& a, typename Acc<TACC>::A& b, V va, V vb,
                                          typename Acc<TACC>::X xa, typename Acc<TACC>::X xb) {
   if constexpr (std::is_same_v<TACC, DF>) {
     Acc<DF>::fma2(a, b, va, vb, xa, xb);
@@ -352,17 +356,17 @@ __device__ __forceinline__ float2 to_input<FH>(float a) {
 // Ring shapes (stages x bytes) of the staged kernels; HODLR_TUNE_* override
 // them at compile time for tuning runs.  Two stages per warp measured best on
 // GB300: the shared memory per warp, not the stage count, limits the warps
-// per SM, and more warps hide more latency than deeper rings.  V^T x stages of
-// 3 KB and at most 64 rows (with V grouped by source node rows are long, and
-// room for the inputs of the narrowest rows took a third of the ring) allow 7
-// CTAs per SM instead of 4: 989 -> 920 us at N = 262144 in 3D (FP32), and 415 ->
-// 309 us for the two stages' worth of most items of 4D N = 65536 (BF16); with
-// 4 KB 922 and 330, with 2 KB 995 and 318.
+// per SM, and more warps hide more latency than deeper rings.  A stage of V^T x
+// holds its rows of V and after them their inputs, so that rows of any width fill
+// it; 3.4 KB allow 8 CTAs per SM of the kernels that need 64 registers.  (With
+// 4 KB of V and room for the inputs of the narrowest rows apart from it, 4 CTAs
+// fitted.)  N = 262144 in 3D (FP32): 989 -> 919 us; 4D N = 65536 (BF16), where most
+// items are two stages: 415 -> 312.
 #ifndef HODLR_TUNE_Z_STAGES
 #define HODLR_TUNE_Z_STAGES 2
 #endif
 #ifndef HODLR_TUNE_Z_BYTES
-#define HODLR_TUNE_Z_BYTES 3072
+#define HODLR_TUNE_Z_BYTES 3488
 #endif
 #ifndef HODLR_TUNE_P_STAGES
 #define HODLR_TUNE_P_STAGES 2
@@ -384,13 +388,11 @@ __device__ __forceinline__ float2 to_input<FH>(float a) {
 #endif
 constexpr int kZWarps = 4;                      // warps per CTA of zgemv_kernel
 constexpr int kZStages = HODLR_TUNE_Z_STAGES;   // ring stages per warp
-constexpr int kZStageBytes = HODLR_TUNE_Z_BYTES;  // V bytes per stage
-constexpr int kZRows = 64;  // rows per stage at most
-// input bytes per stage: kZRows values of 8 bytes, plus 2 x 15 bytes of alignment
-// slack, rounded to 16
-constexpr int kZXBytes = kZRows * 8 + 32;
-constexpr int kZWarpSmem = 64 + kZStages * (kZStageBytes + kZXBytes);
-static_assert(kZWarpSmem % 16 == 0 && kZXBytes % 16 == 0, "bulk copy destinations must stay 16-byte aligned");
+// V and input bytes per stage: R rows of V and of 8 input bytes, plus 2 x 15
+// bytes of alignment slack, rounded to 16
+constexpr int kZStageBytes = HODLR_TUNE_Z_BYTES;
+constexpr int kZWarpSmem = 64 + kZStages * kZStageBytes;
+static_assert(kZStageBytes % 16 == 0 && kZStageBytes >= 32 + 512 + 32 * 8, "bulk copy destinations must stay 16-byte aligned");
 
 // Sum of `count` partial sums, `stride` apart, in an order that depends on
 // count alone: one after another up to 8 of them; more (small operators, whose
@@ -505,12 +507,10 @@ __global__ void __launch_bounds__(kZWarps * 32) zgemv_kernel(const ZBlock* __res
     // 16-byte boundary), so every stage's source and size are too.  The input
     // run is copied from its 16-byte boundary below to the one above; the
     // input buffers carry 16 bytes of padding at their end for that.  R and
-    // nst come from z_item_stages: R a multiple of G, at most
-    // kZStageBytes / rowb rows.
+    // nst come from z_item_stages: R a multiple of G whose rows fit a stage.
     unsigned char* base = zsm + wid * kZWarpSmem;
     uint64_t* bar = reinterpret_cast<uint64_t*>(base);
     unsigned char* vbuf = base + 64;
-    unsigned char* xbuf = vbuf + kZStages * kZStageBytes;
     const int rowb = int(rp) * int(sizeof(TA));
     const int R = it.R, nst = it.nst;
     const int nrows = it.j1 - it.j0;
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(kZWarps * 32) zgemv_kernel(const ZBlock* __res
       fence_proxy_async();
       mbar_expect_tx(bar + s, vb + xb);
       bulk_g2s(vbuf + s * kZStageBytes, V + int64_t(r0) * rp, vb, bar + s);
-      bulk_g2s(xbuf + s * kZXBytes, xa, xb, bar + s);
+      bulk_g2s(vbuf + s * kZStageBytes + R * rowb, xa, xb, bar + s);
     };
     if (lane == 0)
       for (int q = 0; q < min(kZStages, nst); q++) issue(q);
@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(kZWarps * 32) zgemv_kernel(const ZBlock* __res
       }
       const int r0 = q * R, nr = min(R, nrows - r0);
       const int xo = int((reinterpret_cast<uintptr_t>(xr + r0) & 15u) / sizeof(TX));
-      const TX* xsm = reinterpret_cast<const TX*>(xbuf + s * kZXBytes) + xo;
+      const TX* xsm = reinterpret_cast<const TX*>(vbuf + s * kZStageBytes + R * rowb) + xo;
       const unsigned char* vs = vbuf + s * kZStageBytes + p * 16;
       for (int i = g; i < nr; i += G) {
         const VT v = cact ? *reinterpret_cast<const VT*>(vs + i * rowb) : vzero<VT>();
@@ -763,8 +763,8 @@ __global__ void __launch_bounds__(kSWarps * 32, HODLR_TUNE_S_MINB)
 // rows, so an item's factors form one run of m-row columns (after each
 // segment up to 15 bytes of padding, and for a BF16 dense tile its column
 // scales).  The run is streamed through a per-warp ring of kLStages stages;
-// a stage is the bytes of a run of whole columns -- at most kLStageBytes, at
-// most kLCols columns -- fetched by ONE bulk copy (from the 16-byte boundary
+// a stage is the bytes of a run of whole columns -- at most l_bytes, at
+// most l_cols columns -- fetched by ONE bulk copy (from the 16-byte boundary
 // at or below its first column), and the input values of those columns,
 // gathered into the stage by the lanes with 4- or 8-byte asynchronous copies
 // (cp.async) that complete on the stage's mbarrier.  Relaxed products read
@@ -781,30 +781,31 @@ __global__ void __launch_bounds__(kSWarps * 32, HODLR_TUNE_S_MINB)
 // gathers of columns lane, lane + 32, ... (for BF16 dense tiles also the
 // gathers of their column scales).  After the wait the lanes multiply the
 // staged inputs of BF16 dense tiles by their scales, once per column.  The
-// products then read only shared memory: lanes form slices of mpad lanes
-// (one lane per row), slice sl takes the stage's columns sl, sl + slices,
-// ..., column parity picks the accumulator.
+// products then read only shared memory, whose reads bound this kernel (a
+// factor entry, an input of 8 bytes and a column offset are four clocks of an
+// SM's shared memory against three of FP32 operations when a lane has one row):
+// a lane has two rows, L = ceil(m / 2) lanes make up a slice, and slice sl of S =
+// 32 / L (not a power of two: 17 rows fill 27 lanes, where one row per lane in
+// slices of a power of two left 15 of 32 idle) takes the stage's columns sl,
+// sl + S, ...  4D N = 65536 BF16: 412 -> 316 us, 3D N = 262144 FP32: 407 -> 342,
+// its FP64 near field 138 -> 127.
 #ifndef HODLR_TUNE_L_STAGES
 #define HODLR_TUNE_L_STAGES 2
 #endif
-#ifndef HODLR_TUNE_L_BYTES
-#define HODLR_TUNE_L_BYTES 4096
-#endif
-#ifndef HODLR_TUNE_L_COLS
-#define HODLR_TUNE_L_COLS 128
-#endif
-#ifndef HODLR_TUNE_L_MINB
-#define HODLR_TUNE_L_MINB 5
-#endif
 constexpr int kLWarps = 4;
 constexpr int kLStages = HODLR_TUNE_L_STAGES;
-constexpr int kLStageBytes = HODLR_TUNE_L_BYTES;  // factor bytes per stage at most
-constexpr int kLCols = HODLR_TUNE_L_COLS;         // columns per stage at most
+// factor bytes and columns per stage at most, CTAs per SM to compile for: BF16
+// columns are half as long, and with smaller stages a sixth CTA fits (4D N =
+// 65536: 340 -> 315 us); FP32 and FP64 columns would fill them too early (3D N =
+// 262144 FP32: 344 -> 360 us)
+template <typename TA>
+inline constexpr int l_bytes = sizeof(TA) == 2 ? 3072 : 4096;
+template <typename TA>
+inline constexpr int l_cols = sizeof(TA) == 2 ? 96 : 128;
+template <typename TA>
+inline constexpr int l_minb = sizeof(TA) == 2 ? 6 : 5;
 constexpr int kLHead = 64;                        // barriers and stage descriptors
 static_assert(kLStages >= 2 && kLStages <= 4, "leaf ring: 2 to 4 stages");
-static_assert(kLStageBytes % 16 == 0 && kLStageBytes >= 512 && kLStageBytes <= 65536,
-              "leaf stage: a multiple of 16 bytes in 512 .. 65536 (column offsets are 16-bit)");
-static_assert(kLCols % 32 == 0 && kLCols <= 1024, "leaf stage columns: a multiple of 32");
 static_assert(32 + kLStages * 8 <= kLHead, "leaf ring header too small");
 // The staged input of one column: the input element, or for relaxed products
 // (which read only the high part of a split input) that high part alone.
@@ -820,10 +821,10 @@ struct LeafX<FH> {
 __device__ __forceinline__ void put_staged(float2& d, DF x) { d = make_float2(x.hi, x.lo); }
 __device__ __forceinline__ void put_staged(float& d, float x) { d = x; }
 __device__ __forceinline__ void put_staged(double& d, double x) { d = x; }
-// stage: factor bytes | inputs (kLCols x TX) | column offsets (kLCols x u16) | BF16 scales (kLCols x f32)
+// stage: factor bytes | inputs (kCols x TX) | column offsets (kCols x u16) | BF16 scales (kCols x f32)
 template <typename TA, typename TX>
 __host__ __device__ constexpr int l_stage_smem() {
-  return kLStageBytes + kLCols * int(sizeof(TX)) + kLCols * 2 + (sizeof(TA) == 2 ? kLCols * 4 : 0);
+  return l_bytes<TA> + l_cols<TA> * (int(sizeof(TX)) + 2 + (sizeof(TA) == 2 ? 4 : 0));
 }
 template <typename TA, typename TX>
 __host__ __device__ constexpr int l_warp_smem() { return kLHead + kLStages * l_stage_smem<TA, TX>(); }
@@ -841,37 +842,65 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// The products of one staged stage for one lane (row i of slice sl): columns
-// sl, sl + S, sl + 2S, ... of the stage, alternately into a0 and a1.  S (the
-// slice count) is a compile-time constant so that the column strides are
-// immediate offsets.
-template <int S, typename TA, typename TX, typename TACC>
+// Two elements next to each other in shared memory; EVEN: one load (the first one
+// is aligned for it).
+template <bool EVEN>
+__device__ __forceinline__ void load_two(const float* p, float& a, float& b) {
+  if constexpr (EVEN) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    a = v.x, b = v.y;
+  } else {
+    a = p[0], b = p[1];
+  }
+}
+template <bool EVEN>
+__device__ __forceinline__ void load_two(const double* p, double& a, double& b) {
+  if constexpr (EVEN) {
+    const double2 v = *reinterpret_cast<const double2*>(p);
+    a = v.x, b = v.y;
+  } else {
+    a = p[0], b = p[1];
+  }
+}
+template <bool EVEN>
+__device__ __forceinline__ void load_two(const bf16* p, float& a, float& b) {
+  if constexpr (EVEN) {
+    const uint32_t v = *reinterpret_cast<const uint32_t*>(p);
+    a = __uint_as_float(v << 16), b = __uint_as_float(v & 0xffff0000u);
+  } else {
+    a = bf2f(p[0].b), b = bf2f(p[1].b);
+  }
+}
+
+// The products of one staged stage for one lane (two rows of slice sl, su: the
+// first of them in column 0): columns sl, sl + S, sl + 2 S, ... of the stage.
+template <bool EVEN, typename TA, typename TX, typename TACC>
 __device__ __forceinline__ void leaf_products(const TA* __restrict__ su, const TX* __restrict__ xs,
-                                              const uint16_t* __restrict__ co, int C, int sl, int i,
+                                              const uint16_t* __restrict__ co, int C, int sl, int S,
                                               typename Acc<TACC>::A& a0, typename Acc<TACC>::A& a1) {
   using AC = Acc<TACC>;
-  const TA* sui = su + i;
+  using V = std::conditional_t<sizeof(TA) == 8, double, float>;
   const TX* px = xs + sl;
   const uint16_t* pc = co + sl;
   int c = sl;
-  for (; c + 3 * S < C; c += 4 * S, px += 4 * S, pc += 4 * S) {
-    const typename AC::X x0 = AC::in(px[0]), x1 = AC::in(px[S]), x2 = AC::in(px[2 * S]), x3 = AC::in(px[3 * S]);
-    const TA v0 = sui[pc[0]], v1 = sui[pc[S]], v2 = sui[pc[2 * S]], v3 = sui[pc[3 * S]];
-    if constexpr (std::is_same_v<TACC, DF>) {
-      AC::fma2(a0, a1, to_f(v0), to_f(v1), x0, x1);
-      AC::fma2(a0, a1, to_f(v2), to_f(v3), x2, x3);
-    } else {
-      AC::fma(a0, v0, x0);
-      AC::fma(a1, v1, x1);
-      AC::fma(a0, v2, x2);
-      AC::fma(a1, v3, x3);
-    }
+  for (; c + S < C; c += 2 * S, px += 2 * S, pc += 2 * S) {
+    V v0, v1, w0, w1;
+    load_two<EVEN>(su + pc[0], v0, v1);
+    load_two<EVEN>(su + pc[S], w0, w1);
+    const typename AC::X x = AC::in(px[0]), y = AC::in(px[S]);
+    fma_pair<TACC>(a0, a1, v0, v1, x, x);
+    fma_pair<TACC>(a0, a1, w0, w1, y, y);
   }
-  for (int k = 0; c < C; c += S, px += S, pc += S, k++) AC::fma((k & 1) ? a1 : a0, sui[pc[0]], AC::in(px[0]));
+  if (c < C) {
+    V v0, v1;
+    load_two<EVEN>(su + pc[0], v0, v1);
+    const typename AC::X x = AC::in(px[0]);
+    fma_pair<TACC>(a0, a1, v0, v1, x, x);
+  }
 }
 
 template <typename TA, typename TACC>
-__global__ void __launch_bounds__(kLWarps * 32, HODLR_TUNE_L_MINB)
+__global__ void __launch_bounds__(kLWarps * 32, l_minb<TA>)
     panel_leaf_kernel(const Panel* __restrict__ panels, const Seg* __restrict__ segs, const Item* __restrict__ items,
                       int nitems, const typename IO<TACC>::TI* __restrict__ in, typename IO<TACC>::TY* __restrict__ y,
                       typename IO<TACC>::TY* ypart) {
@@ -882,6 +911,7 @@ __global__ void __launch_bounds__(kLWarps * 32, HODLR_TUNE_L_MINB)
   constexpr int esz = int(sizeof(TA));
   constexpr bool kScaled = esz == 2;
   constexpr int kStage = l_stage_smem<TA, TX>(), kWarpSmem = l_warp_smem<TA, TX>();
+  constexpr int kLStageBytes = l_bytes<TA>, kLCols = l_cols<TA>;
   constexpr int kXOff = kLStageBytes, kOOff = kXOff + kLCols * int(sizeof(TX)), kSOff = kOOff + kLCols * 2;
   extern __shared__ __align__(16) unsigned char lsm[];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -893,10 +923,9 @@ __global__ void __launch_bounds__(kLWarps * 32, HODLR_TUNE_L_MINB)
   const int colb = m * esz;  // bytes per column
   const TI* inc = in;
   TY* yo = y + P.yoff;
-  int mpad = 1;
-  while (mpad < m) mpad <<= 1;
-  const int slices = 32 / mpad;
-  const int i = lane & (mpad - 1), sl = lane / mpad;
+  // L lanes of two rows each per slice; the lanes beyond S L have no work
+  const int L = (m + 1) >> 1, S = 32 / L;
+  const int sl = lane / L, i = 2 * (lane - sl * L);
   unsigned char* base = lsm + wid * kWarpSmem;
   uint64_t* bar = reinterpret_cast<uint64_t*>(base);
   int2* meta = reinterpret_cast<int2*>(base + 32);  // per stage: column count, unused
@@ -1078,15 +1107,13 @@ __global__ void __launch_bounds__(kLWarps * 32, HODLR_TUNE_L_MINB)
       for (int c = lane; c < C; c += 32) put_staged(xw[c], AC::xscale(AC::in(xw[c]), sc[c]));
       __syncwarp();
     }
-    if (i < m) {
-      switch (slices) {
-        case 32: leaf_products<32, TA, TX, TACC>(su, xs, co, C, sl, i, a0acc, a1acc); break;
-        case 16: leaf_products<16, TA, TX, TACC>(su, xs, co, C, sl, i, a0acc, a1acc); break;
-        case 8: leaf_products<8, TA, TX, TACC>(su, xs, co, C, sl, i, a0acc, a1acc); break;
-        case 4: leaf_products<4, TA, TX, TACC>(su, xs, co, C, sl, i, a0acc, a1acc); break;
-        case 2: leaf_products<2, TA, TX, TACC>(su, xs, co, C, sl, i, a0acc, a1acc); break;
-        default: leaf_products<1, TA, TX, TACC>(su, xs, co, C, sl, i, a0acc, a1acc); break;
-      }
+    // an even row count keeps every pair of rows aligned; of an odd one the last
+    // lane's second row is whatever follows the column and is not stored
+    if (sl < S) {
+      if (m & 1)
+        leaf_products<false, TA, TX, TACC>(su + i, xs, co, C, sl, S, a0acc, a1acc);
+      else
+        leaf_products<true, TA, TX, TACC>(su + i, xs, co, C, sl, S, a0acc, a1acc);
     }
     __syncwarp();  // stage k's slot is refilled for stage k + kLStages
     if (issue(st)) {
@@ -1094,13 +1121,20 @@ __global__ void __launch_bounds__(kLWarps * 32, HODLR_TUNE_L_MINB)
       prefetch();
     }
   }
-  typename AC::A acc = AC::add(a0acc, a1acc);
-  for (int o = mpad; o < 32; o <<= 1) acc = AC::add(acc, AC::shfl_xor(acc, o));
-  if (sl == 0 && i < m) {
-    if (it.part < 0)
-      yo[i] = TY(AC::value(acc));
-    else
-      ypart[int64_t(it.part) * tile_rows(int(sizeof(TA))) + i] = TY(AC::value(acc));
+  // slices in pairs, in an order that depends on S alone
+  for (int n = S; n > 1;) {
+    const int half = (n + 1) >> 1;
+    const typename AC::A o0 = AC::shfl_down(a0acc, half * L), o1 = AC::shfl_down(a1acc, half * L);
+    if (sl + half < n) {
+      a0acc = AC::add(a0acc, o0);
+      a1acc = AC::add(a1acc, o1);
+    }
+    n = half;
+  }
+  if (sl == 0) {
+    TY* dst = it.part < 0 ? yo + i : ypart + int64_t(it.part) * tile_rows(int(sizeof(TA))) + i;
+    dst[0] = TY(AC::value(a0acc));
+    if (i + 1 < m) dst[1] = TY(AC::value(a1acc));
   }
 }
 
@@ -1679,7 +1713,7 @@ void z_item_stages(ZItem& it, int r, int esz) {
   int P = 1;
   while (P < lanes) P <<= 1;
   const int G = 32 / P, rowb = rp * esz;
-  it.R = std::min(kZStageBytes / rowb, kZRows) / G * G;  // >= G: rowb <= 16 P, kZStageBytes >= 512, kZRows >= 32
+  it.R = (kZStageBytes - 32) / (rowb + 8) / G * G;  // >= G: rowb <= 16 P
   it.nst = (it.j1 - it.j0 + it.R - 1) / it.R;
 }
 
