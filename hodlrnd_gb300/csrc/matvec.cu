@@ -383,9 +383,6 @@ __device__ __forceinline__ float2 to_input<FH>(float a) {
 #ifndef HODLR_TUNE_S_MINB
 #define HODLR_TUNE_S_MINB 6  // leaf-panel CTAs per SM the register allocation must allow (no spills at 6)
 #endif
-#ifndef HODLR_TUNE_P_MINB
-#define HODLR_TUNE_P_MINB 4
-#endif
 constexpr int kZWarps = 4;                      // warps per CTA of zgemv_kernel
 constexpr int kZStages = HODLR_TUNE_Z_STAGES;   // ring stages per warp
 // V and input bytes per stage: R rows of V and of 8 input bytes, plus 2 x 15
@@ -1161,8 +1158,13 @@ constexpr int kPXBytes = kPCols * 8 + 32;
 constexpr int kPWarpSmem = 64 + kPStages * (kPStageBytes + kPXBytes);
 static_assert(kPWarpSmem % 16 == 0 && kPXBytes % 16 == 0, "bulk copy destinations must stay 16-byte aligned");
 
+// CTAs per SM the register allocation must allow: a sixth (80 registers) helps
+// the four rows of a lane's FP32 load (3D N = 262144: 1020 -> 1001 us), not the
+// eight of a BF16 one, whose sums alone take 32 (4D N = 65536: 135 -> 143 us)
+template <typename TA>
+inline constexpr int p_minb = sizeof(TA) == 2 ? 4 : 6;
 template <typename TA, typename TACC>
-__global__ void __launch_bounds__(kPWarps * 32, HODLR_TUNE_P_MINB)
+__global__ void __launch_bounds__(kPWarps * 32, p_minb<TA>)
     panel_tile_kernel(const Panel* __restrict__ panels, const Seg* __restrict__ segs, const Item* __restrict__ items,
                       int nitems, typename IO<TACC>::TY* __restrict__ ypart,
                       const typename IO<TACC>::TI* __restrict__ in, typename IO<TACC>::TY* __restrict__ y) {
