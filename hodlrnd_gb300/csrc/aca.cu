@@ -46,6 +46,9 @@
 // row and column indices.  A block whose rank would exceed cap reports
 // kAcaOverflow and is rerun by the host with a larger cap.
 #include "aca.h"
+
+#include <type_traits>
+
 #include "device.cuh"
 
 namespace hodlr {
@@ -63,6 +66,84 @@ __device__ __forceinline__ int rng_next(uint64_t& s) {
   z ^= z >> 31;
   return int(z >> 33);
 }
+
+// A cluster of kClusterCtas CTAs on one block: the few blocks of a small build
+// whose work is more than an SM's even share of the whole (2D N = 10000: four
+// blocks of 2500 x 2500 took 11 of 16.6 ms, one SM each, with the other 148
+// idle).  The team's threads are dealt to the CTAs by whole warps in turn, so
+// that a row's 32-entry pieces spread evenly.  Rows, columns and bitmaps lie in global
+// memory; a hardware cluster barrier orders them.  Broadcasts, pivots and the
+// norm estimate's terms are stored into every CTA's shared memory, alternately
+// into two slots, so that one barrier each suffices.  Norms are summed by each
+// CTA for itself in the order of a CTA team, so the factors are those of a
+// CTA team to the last bit.  The four blocks: 11 -> 3.1 ms, the build 16.6 -> 10.9.
+constexpr int kClusterCtas = 8;
+struct ClusterShared {
+  unsigned long long key[2][kClusterCtas];
+  int idx[2][kClusterCtas];
+  double value[2];
+};
+struct ClusterTeam {
+  using Cta = CtaTeam<256>;
+  static constexpr int kSize = 256 * kClusterCtas;
+  Cta cta;
+  ClusterShared* sh;
+  mutable int slot = 0;  // the same in every thread
+  __device__ static uint32_t rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+  }
+  // address of *p in CTA c's shared memory
+  __device__ static uint32_t at(const void* p, int c) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(r)
+                 : "r"(uint32_t(__cvta_generic_to_shared(p))), "r"(uint32_t(c)));
+    return r;
+  }
+  __device__ static void store(uint32_t addr, unsigned long long v) {
+    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
+  }
+  __device__ int tid() const { return int(((threadIdx.x >> 5) * kClusterCtas + rank()) * 32 + (threadIdx.x & 31)); }
+  __device__ void sync() const {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  }
+  // each CTA's own sums (its threads hold the partial sums of a CTA team's)
+  __device__ void sum2(double& a, double& b) const { cta.sum2(a, b); }
+  __device__ void argmax(unsigned long long& k, int& i) const {
+    cta.argmax(k, i);
+    if (threadIdx.x < kClusterCtas) {
+      store(at(&sh->key[slot][rank()], threadIdx.x), k);
+      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at(&sh->idx[slot][rank()], threadIdx.x)), "r"(i) : "memory");
+    }
+    sync();
+    for (int c = 0; c < kClusterCtas; c++)
+      if (pivot_better(sh->key[slot][c], sh->idx[slot][c], k, i)) {
+        k = sh->key[slot][c];
+        i = sh->idx[slot][c];
+      }
+    slot ^= 1;
+  }
+  // of team thread 0: the CTA with rank 0 hands its thread 0's value to all
+  __device__ double bcast(double v) const {
+    if (rank() == 0) {
+      v = __shfl_sync(0xffffffffu, v, 0);
+      if (threadIdx.x < kClusterCtas) store(at(&sh->value[slot], threadIdx.x), (unsigned long long)__double_as_longlong(v));
+    }
+    sync();
+    v = sh->value[slot];
+    slot ^= 1;
+    return v;
+  }
+  __device__ int bcast(int v) const { return int(bcast(double(v))); }
+  __device__ void put_term(int k, double v) const {
+    const int lane = threadIdx.x & 31;
+    if (lane < kClusterCtas) store(at(cta.terms + k, lane), (unsigned long long)__double_as_longlong(v));
+  }
+  __device__ double term(int k) const { return cta.terms[k]; }
+};
 
 // Shared memory of one staged team (blocks of at most T rows and columns):
 // U (T x T), V (T x T), the target and source coordinates (D x T each), then
@@ -398,7 +479,7 @@ struct AcaTeam {
   __device__ void norm_update(int r, double& mnorm) {
     if constexpr (Team::kSize > 32) {
       constexpr int W = Team::kSize / 32;
-      const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+      const int lane = threadIdx.x & 31, w = tm.tid() >> 5;
       for (int k0 = 0; k0 < r; k0 += kNormChunk) {
         const int kn = min(kNormChunk, r - k0);
         for (int kk = w; kk < kn; kk += W) {
@@ -407,11 +488,11 @@ struct AcaTeam {
           for (int i = lane; i < m; i += 32) du += U[i + int64_t(k) * m] * U[i + int64_t(r) * m];
           for (int j = lane; j < n; j += 32) dv += V[j + int64_t(k) * n] * V[j + int64_t(r) * n];
           WarpTeam().sum2(du, dv);
-          if (lane == 0) tm.terms[kk] = __dmul_rn(__dmul_rn(2.0, fabs(du)), fabs(dv));
+          tm.put_term(kk, __dmul_rn(__dmul_rn(2.0, fabs(du)), fabs(dv)));
         }
-        __syncthreads();
-        for (int kk = 0; kk < kn; kk++) mnorm += tm.terms[kk];
-        __syncthreads();
+        tm.sync();
+        for (int kk = 0; kk < kn; kk++) mnorm += tm.term(kk);
+        tm.sync();
       }
     } else if constexpr (Team::kSize == 32) {
       // eight columns at a time: their 16 dot products are reduced together by a
@@ -548,6 +629,13 @@ struct AcaTeam {
       nrow++;
       if (erase(rb, piv)) nr--;
       cur_row = piv;
+      if constexpr (std::is_same_v<Team, ClusterTeam>) {
+        // the partial sums of a CTA team's threads, before the column is scaled
+        rsq_p = csq_p = 0.0;
+        for (int j = threadIdx.x; j < n; j += 256) rsq_p += V[j + int64_t(r) * n] * V[j + int64_t(r) * n];
+        for (int i = threadIdx.x; i < m; i += 256) csq_p += U[i + int64_t(r) * m] * U[i + int64_t(r) * m];
+        tm.sync();
+      }
       // u_r = gamma * col; v_r = row (already in V[:, r])
       for (int i = tm.tid(); i < m; i += Team::kSize)
         U[i + int64_t(r) * m] = __dmul_rn(gamma, U[i + int64_t(r) * m]);
@@ -617,6 +705,20 @@ __global__ void __launch_bounds__(256) aca_cta_kernel(AcaArgs a, const int32_t* 
   }
 }
 
+template <int D>
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(256)
+    aca_cluster_kernel(AcaArgs a, const int32_t* __restrict__ list) {
+  __shared__ double red[256 / 32 + 1], red2[256 / 32 + 1];
+  __shared__ double terms[kNormChunk];
+  __shared__ int redi[256 / 32 + 1];
+  __shared__ ClusterShared sh;
+  ClusterTeam tm{CtaTeam<256>{red, red2, redi, terms}, &sh};
+  const int b = list[blockIdx.x / kClusterCtas];
+  AcaTeam<D, ClusterTeam> t(a, a.blocks[b], tm);
+  t.run(a.out + b);
+  tm.sync();  // no CTA leaves while another may store into its shared memory
+}
+
 // Teams of T = 8 or 16 lanes, 128 / T per CTA, each on one block of at most
 // T rows and columns held in shared memory.
 template <int D, int T>
@@ -657,9 +759,11 @@ template <int D>
 void launch_kind(const AcaArgs& a, const AcaLists& L, int kind, cudaStream_t st) {
   if (L.n[kind] <= 0) return;
   switch (kind) {
-    case kAcaTeamCta:
-      aca_cta_kernel<D><<<aca_grid(a, L.n[kAcaTeamCta], 1), 256, 0, st>>>(a, L.list[kAcaTeamCta], L.n[kAcaTeamCta]);
+    case kAcaTeamCta: {
+      const int n = L.n[kAcaTeamCta] - L.nbig;
+      if (n > 0) aca_cta_kernel<D><<<aca_grid(a, n, 1), 256, 0, st>>>(a, L.list[kAcaTeamCta] + L.nbig, n);
       break;
+    }
     case kAcaTeamWarp:
       aca_warp_kernel<D><<<aca_grid(a, L.n[kAcaTeamWarp], 4), 128, 0, st>>>(a, L.list[kAcaTeamWarp],
                                                                             L.n[kAcaTeamWarp]);
@@ -676,10 +780,16 @@ template <int D>
 cudaError_t preload_d() {
   cudaFuncAttributes fa;
   cudaError_t e = cudaFuncGetAttributes(&fa, aca_cta_kernel<D>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, aca_cluster_kernel<D>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, aca_warp_kernel<D>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, aca_sub_kernel<D, 16>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, aca_sub_kernel<D, 8>);
   return e;
+}
+
+template <int D>
+void launch_big(const AcaArgs& a, const AcaLists& L, cudaStream_t st) {
+  aca_cluster_kernel<D><<<unsigned(L.nbig * kClusterCtas), 256, 0, st>>>(a, L.list[kAcaTeamCta]);
 }
 
 template <int D>
@@ -713,7 +823,7 @@ cudaError_t aca_preload(int ndim) {
 
 cudaError_t launch_aca_kind(int ndim, const AcaArgs& a, const AcaLists& L, int kind, cudaStream_t st) {
   if (kind < 0 || kind >= kAcaTeamKinds) return cudaErrorInvalidValue;
-  if (L.n[kind] <= 0) return cudaSuccess;
+  if (L.n[kind] - (kind == kAcaTeamCta ? L.nbig : 0) <= 0) return cudaSuccess;
   count_launches(1);
   switch (ndim) {
     case 1: launch_kind<1>(a, L, kind, st); break;
@@ -724,6 +834,23 @@ cudaError_t launch_aca_kind(int ndim, const AcaArgs& a, const AcaLists& L, int k
     case 6: launch_kind<6>(a, L, kind, st); break;
     case 7: launch_kind<7>(a, L, kind, st); break;
     case 8: launch_kind<8>(a, L, kind, st); break;
+    default: return cudaErrorInvalidValue;
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_aca_big(int ndim, const AcaArgs& a, const AcaLists& L, cudaStream_t st) {
+  if (L.nbig <= 0) return cudaSuccess;
+  count_launches(1);
+  switch (ndim) {
+    case 1: launch_big<1>(a, L, st); break;
+    case 2: launch_big<2>(a, L, st); break;
+    case 3: launch_big<3>(a, L, st); break;
+    case 4: launch_big<4>(a, L, st); break;
+    case 5: launch_big<5>(a, L, st); break;
+    case 6: launch_big<6>(a, L, st); break;
+    case 7: launch_big<7>(a, L, st); break;
+    case 8: launch_big<8>(a, L, st); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

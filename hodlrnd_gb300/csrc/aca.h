@@ -72,12 +72,17 @@ int aca_team(int m, int n);
 struct AcaLists {
   const int32_t* list[kAcaTeamKinds];
   int n[kAcaTeamKinds];
+  int nbig = 0;  // the first nbig blocks of kind kAcaTeamCta are left to launch_aca_big
 };
 // Asynchronous on st.
 cudaError_t launch_aca(int ndim, const AcaArgs& a, const AcaLists& lists, cudaStream_t st);
 // The team kind `kind` alone (its list in lists), asynchronous on st: the kinds
 // touch disjoint blocks and may run on different streams at once.
 cudaError_t launch_aca_kind(int ndim, const AcaArgs& a, const AcaLists& lists, int kind, cudaStream_t st);
+// The first lists.nbig blocks of kind kAcaTeamCta, a cluster of CTAs each: the
+// factors of launch_aca_kind, in a fraction of the time when a few large blocks
+// would otherwise outlast the rest.  Asynchronous on st.
+cudaError_t launch_aca_big(int ndim, const AcaArgs& a, const AcaLists& lists, cudaStream_t st);
 // Loads the ACA kernels of points in ndim dimensions (before launches that
 // should run concurrently).
 cudaError_t aca_preload(int ndim);

@@ -228,6 +228,11 @@ struct CtaTeam {
   double* red2;   // shared, kWarps + 1
   int* redi;      // shared, kWarps + 1
   double* terms;  // shared, kNormChunk: the norm estimate's terms of one pass (ACA)
+  // terms[k] = v (the same in every lane of a warp)
+  __device__ __forceinline__ void put_term(int k, double v) const {
+    if ((threadIdx.x & 31) == 0) terms[k] = v;
+  }
+  __device__ __forceinline__ double term(int k) const { return terms[k]; }
   __device__ __forceinline__ int tid() const { return threadIdx.x; }
   __device__ __forceinline__ void sync() const { __syncthreads(); }
   __device__ __forceinline__ double sum(double v) const {

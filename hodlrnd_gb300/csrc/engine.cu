@@ -951,10 +951,15 @@ void run_aca(const std::vector<hodlr_op*>& ops, cudaStream_t st) {
   struct Side {
     cudaStream_t s[kAcaTeamKinds] = {};
     cudaEvent_t e[kAcaTeamKinds] = {};
+    cudaStream_t big = nullptr;             // the largest blocks (launch_aca_big)
     cudaStream_t cs = nullptr;              // compaction stream
     cudaEvent_t c0 = nullptr, c1 = nullptr;  // compaction launch timing
     ~Side() {
       if (cs) cudaStreamSynchronize(cs);
+      if (big) {
+        cudaStreamSynchronize(big);
+        cudaStreamDestroy(big);
+      }
       for (int k = 0; k < kAcaTeamKinds; k++) {
         if (s[k]) cudaStreamSynchronize(s[k]);
         if (e[k]) cudaEventDestroy(e[k]);
@@ -969,6 +974,7 @@ void run_aca(const std::vector<hodlr_op*>& ops, cudaStream_t st) {
     check_cuda(cudaStreamCreateWithFlags(&side.s[k], cudaStreamNonBlocking), "cudaStreamCreate");
     check_cuda(cudaEventCreateWithFlags(&side.e[k], cudaEventDisableTiming), "cudaEventCreate");
   }
+  check_cuda(cudaStreamCreateWithFlags(&side.big, cudaStreamNonBlocking), "cudaStreamCreate");
   check_cuda(cudaStreamCreateWithFlags(&side.cs, cudaStreamNonBlocking), "cudaStreamCreate");
   check_cuda(cudaEventCreate(&side.c0), "cudaEventCreate");
   check_cuda(cudaEventCreate(&side.c1), "cudaEventCreate");
@@ -1108,7 +1114,20 @@ void run_aca(const std::vector<hodlr_op*>& ops, cudaStream_t st) {
     } else {
       runs.push_back({0, nq, -1});
     }
-    EventSet rev(2 * kAcaTeamKinds);
+    // The largest blocks, while one of them is more work than an SM's even share
+    // of the batch (by rows plus columns; blocks of the CTA kind only): they are
+    // compressed by clusters of CTAs, or they would outlast everything else.
+    int nbig = 0;
+    if (in_order) {
+      uint64_t work = 0;
+#pragma omp parallel for schedule(static) reduction(+ : work) num_threads(tq)
+      for (int64_t q = 0; q < int64_t(nq); q++) work += uint64_t(om[pos0 + size_t(q)]) + uint64_t(on[pos0 + size_t(q)]);
+      while (size_t(nbig) < nq && qteam[size_t(nbig)] == kAcaTeamCta &&
+             (uint64_t(om[pos0 + size_t(nbig)]) + uint64_t(on[pos0 + size_t(nbig)])) * uint64_t(sms) > work)
+        nbig++;
+    }
+    EventSet rev(2 * kAcaTeamKinds + 1);
+    const cudaEvent_t ev_big = rev.e[2 * kAcaTeamKinds];
     auto ev_copy = [&](size_t r) { return rev.e[r]; };
     auto ev_done = [&](int k) { return rev.e[size_t(kAcaTeamKinds + k)]; };
     std::vector<int32_t> lst(nq);
@@ -1168,10 +1187,17 @@ void run_aca(const std::vector<hodlr_op*>& ops, cudaStream_t st) {
       CK(cudaMemcpyAsync(d_lists_idx + q0, lst.data() + q0, nw * sizeof(int32_t), cudaMemcpyHostToDevice, st));
       if (r == 0) CK(cudaEventRecord(ev_a0, st));  // the launches' span starts here
       CK(cudaEventRecord(ev_copy(r), st));
+      if (al.n[kAcaTeamCta] > 0 && nbig > 0) {  // first, onto idle SMs
+        al.nbig = nbig;
+        CK(cudaStreamWaitEvent(side.big, ev_copy(r), 0));
+        CK(launch_aca_big(ndim, a, al, side.big));
+        CK(cudaEventRecord(ev_big, side.big));
+      }
       for (int k = 0; k < kAcaTeamKinds; k++) {
         if (runs[r].kind >= 0 && k != runs[r].kind) continue;
         CK(cudaStreamWaitEvent(side.s[k], ev_copy(r), 0));
         CK(launch_aca_kind(ndim, a, al, k, side.s[k]));
+        if (k == kAcaTeamCta && al.nbig > 0) CK(cudaStreamWaitEvent(side.s[k], ev_big, 0));
         CK(cudaEventRecord(ev_done(k), side.s[k]));
       }
     }
