@@ -2464,14 +2464,23 @@ struct TcLeafHost {
   std::vector<TcLeafBatch> batches;
   std::vector<TcLeafRun> runs;
   std::vector<TcUnit> units;
-  std::unordered_map<int64_t, std::vector<std::pair<int32_t, int32_t>>> unit_of;  // first point -> (points, first unit)
+  // by first point: the points and first unit of the first source that starts there, further ones
+  std::vector<std::pair<int32_t, int32_t>> unit_at;
+  std::unordered_map<int64_t, std::vector<std::pair<int32_t, int32_t>>> unit_of;
+  explicit TcLeafHost(int64_t n) : unit_at(size_t(n), {0, 0}) {}
   int32_t source_units(int64_t x_off, int32_t n) {
-    auto& v = unit_of[x_off];
-    for (const auto& e : v)
-      if (e.first == n) return e.second;
+    auto& f = unit_at[size_t(x_off)];
+    if (f.first == n) return f.second;
     const int32_t u0 = int32_t(units.size());
+    if (f.first == 0) {
+      f = {n, u0};
+    } else {
+      auto& v = unit_of[x_off];
+      for (const auto& e : v)
+        if (e.first == n) return e.second;
+      v.push_back({n, u0});
+    }
     for (int32_t p = 0; p < n; p += 8) units.push_back({x_off + p, std::min(8, n - p), 0});
-    v.push_back({n, u0});
     return u0;
   }
 };
@@ -2481,80 +2490,129 @@ void tc_leaf_work(const std::vector<Panel>& panels, const std::vector<TcLeafSeg>
   constexpr int32_t most = 8 * kTcLeafUnits;  // points of a source's piece
   for (size_t p = 0; p < panels.size(); p++)
     if (panels[p].m <= 32 && panels[p].seg_end > panels[p].seg_begin) list.push_back(int32_t(p));
-  out.reserve(segs.size());
   struct Piece {
     int64_t off;
     int32_t n, warp;
     int32_t seg, j;  // segment and first point of the piece
   };
-  std::vector<Piece> pieces;
-  for (size_t b = 0; b < list.size(); b += kTcLeafGroup) {
-    const int count = int(std::min<size_t>(kTcLeafGroup, list.size() - b));
-    pieces.clear();
-    for (int w = 0; w < count; w++) {
-      const Panel& P = panels[size_t(list[b + size_t(w)])];
-      for (int64_t q = P.seg_begin; q < P.seg_end; q++)
-        for (int32_t j = 0; j < segs[size_t(q)].n; j += most)
-          pieces.push_back({src_off[size_t(q)] + j, std::min(most, segs[size_t(q)].n - j), w, int32_t(q), j});
-    }
-    std::sort(pieces.begin(), pieces.end(), [](const Piece& x, const Piece& y) {
-      return x.off != y.off ? x.off < y.off : x.n != y.n ? x.n < y.n : x.warp < y.warp;
-    });
-    const int32_t batch0 = int32_t(H.batches.size()), src0 = int32_t(H.srcs.size());
-    for (size_t k = 0; k < pieces.size();) {
-      // a batch: whole sources while they fit (a panel has one segment per source)
-      TcLeafBatch B{};
-      B.src_b = int32_t(H.srcs.size());
-      B.seg_b = int32_t(out.size());
-      int32_t units = 0;
-      const size_t first = k;
-      std::vector<std::pair<size_t, int32_t>> at;  // end of each source's pieces, its first unit
-      while (k < pieces.size()) {
-        size_t e = k;
-        while (e < pieces.size() && pieces[e].off == pieces[k].off && pieces[e].n == pieces[k].n) e++;
-        const int32_t u = (pieces[k].n + 7) / 8;
-        if (k > first && (units + u > kTcLeafUnits || e - first > size_t(kTcLeafSegs) || at.size() >= 32)) break;
-        H.srcs.push_back({H.source_units(pieces[k].off, pieces[k].n), pieces[k].n});
-        at.push_back({e, units});
-        units += u;
-        k = e;
+  // A thread's share of the groups: batches with the sources and segments
+  // counted from the share's first ones, sources as first point and size.
+  struct Src {
+    int64_t off;
+    int32_t n;
+  };
+  struct Group {
+    int32_t b, count, batches, srcs;
+  };
+  struct Share {
+    std::vector<Src> srcs;
+    std::vector<TcLeafBatch> batches;
+    std::vector<TcLeafSeg> segs;
+    std::vector<Group> groups;
+  };
+  const int64_t ngroups = (int64_t(list.size()) + kTcLeafGroup - 1) / kTcLeafGroup;
+  const int T = par_threads(int64_t(segs.size()));
+  std::vector<Share> shares(static_cast<size_t>(T));
+#pragma omp parallel for schedule(static, 1) num_threads(T)
+  for (int th = 0; th < T; th++) {
+    Share& W = shares[size_t(th)];
+    std::vector<Piece> pieces;
+    std::vector<std::pair<size_t, int32_t>> at;  // end of each source's pieces, its first unit
+    for (int64_t gr = ngroups * th / T; gr < ngroups * (th + 1) / T; gr++) {
+      const size_t b = size_t(gr) * kTcLeafGroup;
+      const int count = int(std::min<size_t>(kTcLeafGroup, list.size() - b));
+      pieces.clear();
+      for (int w = 0; w < count; w++) {
+        const Panel& P = panels[size_t(list[b + size_t(w)])];
+        for (int64_t q = P.seg_begin; q < P.seg_end; q++)
+          for (int32_t j = 0; j < segs[size_t(q)].n; j += most)
+            pieces.push_back({src_off[size_t(q)] + j, std::min(most, segs[size_t(q)].n - j), w, int32_t(q), j});
       }
-      B.src_e = int32_t(H.srcs.size());
-      for (int w = 0; w < kTcLeafGroup; w++) {
-        B.warp_off[w] = int32_t(out.size()) - B.seg_b;
-        size_t p = first;
-        for (const auto& src : at)
-          for (; p < src.first; p++) {
-            if (pieces[p].warp != w) continue;
-            const Piece& f = pieces[p];
-            TcLeafSeg C = segs[size_t(f.seg)];
-            if (C.n > most) {
-              const int32_t m = panels[size_t(list[b + size_t(w)])].m;
-              if (C.V) {
-                C.V += int64_t(f.j) * C.vstride;
-              } else {
-                C.A = static_cast<const char*>(C.A) + int64_t(f.j) * m * (near ? 8 : 2);
-                if (C.scale) C.scale += f.j;
-                C.K = f.n;
+      std::sort(pieces.begin(), pieces.end(), [](const Piece& x, const Piece& y) {
+        return x.off != y.off ? x.off < y.off : x.n != y.n ? x.n < y.n : x.warp < y.warp;
+      });
+      const size_t batch0 = W.batches.size(), src0 = W.srcs.size();
+      for (size_t k = 0; k < pieces.size();) {
+        // a batch: whole sources while they fit (a panel has one segment per source)
+        TcLeafBatch B{};
+        B.src_b = int32_t(W.srcs.size());
+        B.seg_b = int32_t(W.segs.size());
+        int32_t units = 0;
+        const size_t first = k;
+        at.clear();
+        while (k < pieces.size()) {
+          size_t e = k;
+          while (e < pieces.size() && pieces[e].off == pieces[k].off && pieces[e].n == pieces[k].n) e++;
+          const int32_t u = (pieces[k].n + 7) / 8;
+          if (k > first && (units + u > kTcLeafUnits || e - first > size_t(kTcLeafSegs) || at.size() >= 32)) break;
+          W.srcs.push_back({pieces[k].off, pieces[k].n});
+          at.push_back({e, units});
+          units += u;
+          k = e;
+        }
+        B.src_e = int32_t(W.srcs.size());
+        for (int w = 0; w < kTcLeafGroup; w++) {
+          B.warp_off[w] = int32_t(W.segs.size()) - B.seg_b;
+          size_t p = first;
+          for (const auto& src : at)
+            for (; p < src.first; p++) {
+              if (pieces[p].warp != w) continue;
+              const Piece& f = pieces[p];
+              TcLeafSeg C = segs[size_t(f.seg)];
+              if (C.n > most) {
+                const int32_t m = panels[size_t(list[b + size_t(w)])].m;
+                if (C.V) {
+                  C.V += int64_t(f.j) * C.vstride;
+                } else {
+                  C.A = static_cast<const char*>(C.A) + int64_t(f.j) * m * (near ? 8 : 2);
+                  if (C.scale) C.scale += f.j;
+                  C.K = f.n;
+                }
+                C.n = f.n;
               }
-              C.n = f.n;
+              C.unit = src.second;
+              W.segs.push_back(C);
             }
-            C.unit = src.second;
-            out.push_back(C);
-          }
+        }
+        B.warp_off[kTcLeafGroup] = int32_t(W.segs.size()) - B.seg_b;
+        W.batches.push_back(B);
       }
-      B.warp_off[kTcLeafGroup] = int32_t(out.size()) - B.seg_b;
+      W.groups.push_back({int32_t(b), count, int32_t(W.batches.size() - batch0), int32_t(W.srcs.size() - src0)});
+    }
+  }
+  // the shares one after another
+  size_t nsegs = 0;
+  std::vector<size_t> seg0;
+  for (const Share& W : shares) {
+    seg0.push_back(nsegs);
+    nsegs += W.segs.size();
+  }
+  out.resize(nsegs);
+#pragma omp parallel for schedule(static, 1) num_threads(T)
+  for (int th = 0; th < T; th++)
+    std::copy(shares[size_t(th)].segs.begin(), shares[size_t(th)].segs.end(), out.begin() + int64_t(seg0[size_t(th)]));
+  for (int th = 0; th < T; th++) {
+    const Share& W = shares[size_t(th)];
+    int32_t batch = int32_t(H.batches.size());
+    const int32_t src0 = int32_t(H.srcs.size());
+    for (TcLeafBatch B : W.batches) {
+      B.src_b += src0;
+      B.src_e += src0;
+      B.seg_b += int32_t(seg0[size_t(th)]);
       H.batches.push_back(B);
     }
-    const int32_t nb = int32_t(H.batches.size()) - batch0, nsrc = int32_t(H.srcs.size()) - src0;
-    if (nb == 0) continue;
-    const int32_t runs = std::min(nb, (nsrc + kTcLeafRunSrcs - 1) / kTcLeafRunSrcs);
-    if (runs > 1)
-      for (int w = 0; w < count; w++) fix.push_back({list[b + size_t(w)], 0, nparts + w * runs, runs});
-    for (int32_t r = 0; r < runs; r++)
-      H.runs.push_back({near ? 1 : 0, int32_t(b), count, batch0 + int32_t(int64_t(nb) * r / runs),
-                        batch0 + int32_t(int64_t(nb) * (r + 1) / runs), runs > 1 ? nparts + r : -1, runs});
-    if (runs > 1) nparts += count * runs;
+    for (const Src& S : W.srcs) H.srcs.push_back({H.source_units(S.off, S.n), S.n});
+    for (const Group& G : W.groups) {
+      if (G.batches == 0) continue;
+      const int32_t runs = std::min(G.batches, (G.srcs + kTcLeafRunSrcs - 1) / kTcLeafRunSrcs);
+      if (runs > 1)
+        for (int w = 0; w < G.count; w++) fix.push_back({list[size_t(G.b + w)], 0, nparts + w * runs, runs});
+      for (int32_t r = 0; r < runs; r++)
+        H.runs.push_back({near ? 1 : 0, G.b, G.count, batch + int32_t(int64_t(G.batches) * r / runs),
+                          batch + int32_t(int64_t(G.batches) * (r + 1) / runs), runs > 1 ? nparts + r : -1, runs});
+      if (runs > 1) nparts += G.count * runs;
+      batch += G.batches;
+    }
   }
 }
 
@@ -2570,7 +2628,7 @@ void build_tc_plan(hodlr_op* op, cudaStream_t st) {
   tc_panel_items(h.panels_far, h.segs_far, fi, T.far, fxf, pf);
   // panels of at most 32 rows: their segments, and the groups' work
   const Tree& t = op->tree;
-  TcLeafHost H;
+  TcLeafHost H(op->n);
   std::vector<TcLeafSeg> lns(h.segs_near.size()), lfs(h.segs_far.size());
   std::vector<int64_t> ons(h.segs_near.size()), ofs(h.segs_far.size());
   for (size_t q = 0; q < h.segs_near.size(); q++) {
