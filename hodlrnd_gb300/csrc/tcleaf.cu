@@ -20,8 +20,8 @@
 // staged in shared memory once for all of them by bulk copies (two stages), and
 // each warp applies its own segments of the batch, asking for the next one's
 // factors before it multiplies.
-// 4D N = 65536, 64 right-hand sides: 1.9-2.0 ms against 5.3 for these blocks through
-// the tcgen05 kernels (the whole product 7.28 -> 3.52 ms).  Of it 0.5 ms waits for
+// 4D N = 65536, 64 right-hand sides: 2.2 ms against 5.3 for these blocks through
+// the tcgen05 kernels (the whole product 7.28 -> 3.6 ms).  Of it 0.5 ms waits for
 // factor loads; the rest is instructions (43% of the issue slots) and the padding
 // of ranks, points and rows to 8.  Measured and not kept: sources read through L1
 // by each warp (3.2 ms), records fetched by each warp (2.8 ms), prefetching the
@@ -47,6 +47,17 @@ __device__ __forceinline__ void mma16(float (&c)[4], const uint4& a, uint32_t b)
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %8}, {%0, %1, %2, %3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b));
+}
+// c += d rounded to nearest: the MMA's own sum is cut off towards zero, which over
+// the hundreds of blocks of a panel adds up (4D N = 65536, against the compensated
+// product: 5.9e-6 with sums in the MMA, 2.4-3.3e-6 so; 2.03 -> 2.18 ms)
+__device__ __forceinline__ void add4(float (&c)[4], const float (&d)[4]) {
+#pragma unroll
+  for (int q = 0; q < 4; q += 2)  // two additions in one instruction
+    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\t"
+        "add.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a;\n\t}"
+        : "+f"(c[q]), "+f"(c[q + 1])
+        : "f"(d[q]), "f"(d[q + 1]));
 }
 // 8 x 8 BF16 matrix transposed across the warp (lane 4 g + t: row g, columns 2 t, 2 t + 1)
 __device__ __forceinline__ uint32_t transpose8(uint32_t v) {
@@ -154,9 +165,12 @@ __device__ __forceinline__ void leaf_step(const TcLeafSeg& S, int c, const LeafR
       {
         const uint4 x = X[(c * 4 + mt) * 32];
 #pragma unroll
-        for (int q = 0; q < 3; q++)
+        for (int nt = 0; nt < NT; nt++) {
+          float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-          for (int nt = 0; nt < NT; nt++) mma16(acc[mt][nt], x, b[nt][q]);
+          for (int q = 2; q >= 0; q--) mma16(d, x, b[nt][q]);
+          add4(acc[mt][nt], d);
+        }
       }
   } else if (S.V) {
     const int units = (S.n + 7) >> 3, k = c + 2 * t;
@@ -195,7 +209,11 @@ __device__ __forceinline__ void leaf_step(const TcLeafSeg& S, int c, const LeafR
         zz.z = pack2(z0 - low_f(zz.x), z1 - high_f(zz.x));
         zz.w = pack2(z2 - low_f(zz.y), z3 - high_f(zz.y));
 #pragma unroll
-        for (int nt = 0; nt < NT; nt++) mma16(acc[mt][nt], zz, ub[nt]);
+        for (int nt = 0; nt < NT; nt++) {
+          float d[4] = {0.f, 0.f, 0.f, 0.f};
+          mma16(d, zz, ub[nt]);
+          add4(acc[mt][nt], d);
+        }
       }
   } else {
     // dense tile: stored entry times its column's scale in two BF16 terms (2^-16)
@@ -211,9 +229,12 @@ __device__ __forceinline__ void leaf_step(const TcLeafSeg& S, int c, const LeafR
       {
         const uint4 x = X[(c * 4 + mt) * 32];
 #pragma unroll
-        for (int q = 0; q < 2; q++)
+        for (int nt = 0; nt < NT; nt++) {
+          float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-          for (int nt = 0; nt < NT; nt++) mma16(acc[mt][nt], x, b[nt][q]);
+          for (int q = 1; q >= 0; q--) mma16(d, x, b[nt][q]);
+          add4(acc[mt][nt], d);
+        }
       }
   }
 }
