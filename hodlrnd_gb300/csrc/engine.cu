@@ -2416,12 +2416,12 @@ int tc_bucket(int rows) {
 // non-empty launch (offsets into the items until the array is uploaded).
 constexpr int kTcColsPerItem = 256;
 void tc_panel_items(const std::vector<Panel>& panels, const std::vector<Seg>& segs, std::vector<Item>& items,
-                    std::vector<hodlr_op::TcPlan::Run>& runs, std::vector<PanelFix>& fix, int& nparts) {
+                    std::vector<hodlr_op::TcPlan::Run>& runs, std::vector<PanelFix>& fix, int& nparts, int above) {
   std::vector<Item> by[3];  // buckets of 16, 32, 64 rows
   std::vector<std::pair<int32_t, int32_t>> cut;
   for (size_t pi = 0; pi < panels.size(); pi++) {
     const Panel& P = panels[pi];
-    if (P.seg_end <= P.seg_begin || P.m <= 32) continue;
+    if (P.seg_end <= P.seg_begin || P.m <= above) continue;
     cut.clear();
     int64_t start = P.seg_begin, cols = 0;
     for (int64_t q = P.seg_begin; q < P.seg_end; q++) {
@@ -2455,10 +2455,12 @@ void tc_panel_items(const std::vector<Panel>& panels, const std::vector<Seg>& se
 // at most 32 rows: groups of kTcLeafGroup consecutive ones, the union of each
 // group's sources in the order of their points, in batches, and runs of at most
 // kTcLeafRunSrcs sources -- enough CTAs for every SM to have several, few
-// partial blocks.  segs[q] of a panel has the source (first point src_off[q],
+// partial blocks; of a small operator shorter runs, about kTcLeafRuns of them
+// 4D N = 12000: 1.62 -> 0.85 ms.  segs[q] of a panel has the source (first point src_off[q],
 // segs[q].n points); a longer source than a batch holds is cut into pieces,
 // whose products add up.  out: the segments in batch order.
-constexpr int kTcLeafRunSrcs = 160;
+constexpr int32_t kTcLeafRunSrcs = 160, kTcLeafRunSrcsMin = 4;
+constexpr size_t kTcLeafRuns = 152 * 4;
 struct TcLeafHost {
   std::vector<TcLeafSrc> srcs;
   std::vector<TcLeafBatch> batches;
@@ -2591,6 +2593,10 @@ void tc_leaf_work(const std::vector<Panel>& panels, const std::vector<TcLeafSeg>
 #pragma omp parallel for schedule(static, 1) num_threads(T)
   for (int th = 0; th < T; th++)
     std::copy(shares[size_t(th)].segs.begin(), shares[size_t(th)].segs.end(), out.begin() + int64_t(seg0[size_t(th)]));
+  size_t nsrcs = 0;
+  for (const Share& W : shares) nsrcs += W.srcs.size();
+  const int32_t run_srcs =
+      std::max(kTcLeafRunSrcsMin, std::min(kTcLeafRunSrcs, int32_t(std::min<size_t>(nsrcs / kTcLeafRuns, 1 << 20))));
   for (int th = 0; th < T; th++) {
     const Share& W = shares[size_t(th)];
     int32_t batch = int32_t(H.batches.size());
@@ -2604,7 +2610,7 @@ void tc_leaf_work(const std::vector<Panel>& panels, const std::vector<TcLeafSeg>
     for (const Src& S : W.srcs) H.srcs.push_back({H.source_units(S.off, S.n), S.n});
     for (const Group& G : W.groups) {
       if (G.batches == 0) continue;
-      const int32_t runs = std::min(G.batches, (G.srcs + kTcLeafRunSrcs - 1) / kTcLeafRunSrcs);
+      const int32_t runs = std::min(G.batches, (G.srcs + run_srcs - 1) / run_srcs);
       if (runs > 1)
         for (int w = 0; w < G.count; w++) fix.push_back({list[size_t(G.b + w)], 0, nparts + w * runs, runs});
       for (int32_t r = 0; r < runs; r++)
@@ -2624,8 +2630,22 @@ void build_tc_plan(hodlr_op* op, cudaStream_t st) {
   std::vector<Item> ni, fi;
   std::vector<PanelFix> fxn, fxf;
   int pn = 0, pf = 0;
-  tc_panel_items(h.panels_near, h.segs_near, ni, T.near, fxn, pn);
-  tc_panel_items(h.panels_far, h.segs_far, fi, T.far, fxf, pf);
+  // The leaf-level kernel pays where a leaf has rows to fill its 8-wide pieces
+  // and sources enough for a run; else the tcgen05 kernels take every panel
+  // (64 right-hand sides, leaf kernel against tcgen05: 2D N = 18000, 25 far blocks a
+  // leaf, 251 us against 186; 3D N = 3000, 5.9 rows, 236 against 224; 3D N = 30000,
+  // 7.3 rows, 809 against 1089; 4D N = 6000, 23 rows, 482 against 570; 4D N = 9000,
+  // 35 rows, so that panels of up to 32 are large and far apart, 722 against 589).
+  int64_t lrows = 0, lsegs = 0, lpanels = 0;
+  for (const Panel& P : h.panels_far)
+    if (P.m <= 32) {
+      lrows += P.m;
+      lsegs += P.seg_end - P.seg_begin;
+      lpanels++;
+    }
+  const bool leaf = lrows > 6 * lpanels && lrows <= 26 * lpanels && lsegs >= 32 * lpanels;
+  tc_panel_items(h.panels_near, h.segs_near, ni, T.near, fxn, pn, leaf ? 32 : 0);
+  tc_panel_items(h.panels_far, h.segs_far, fi, T.far, fxf, pf, leaf ? 32 : 0);
   // panels of at most 32 rows: their segments, and the groups' work
   const Tree& t = op->tree;
   TcLeafHost H(op->n);
@@ -2644,7 +2664,7 @@ void build_tc_plan(hodlr_op* op, cudaStream_t st) {
       if (!op->dense[q] && op->rank[q] <= 0) continue;
       const int64_t gt = t.gid(op->far[q].level, op->far[q].t), gs = t.gid(op->far[q].level, op->far[q].s);
       const size_t k = seg++;
-      if (t.count[size_t(gt)] > 32) continue;
+      if (!leaf || t.count[size_t(gt)] > 32) continue;
       leaf_block[q] = 1;
       const Seg& S = h.segs_far[k];
       lfs[k] = {S.A,
@@ -2660,8 +2680,10 @@ void build_tc_plan(hodlr_op* op, cudaStream_t st) {
   }
   std::vector<int32_t> lnl, lfl;
   std::vector<TcLeafSeg> bfs, bns;
-  tc_leaf_work(h.panels_far, lfs, ofs, false, H, bfs, lfl, fxf, pf);
-  tc_leaf_work(h.panels_near, lns, ons, true, H, bns, lnl, fxn, pn);
+  if (leaf) {
+    tc_leaf_work(h.panels_far, lfs, ofs, false, H, bfs, lfl, fxf, pf);
+    tc_leaf_work(h.panels_near, lns, ons, true, H, bns, lnl, fxn, pn);
+  }
   // z groups: the rows of z by source node, at most kTcRows rows per group.
   // Rows are (z block, k0, nk) runs, each low-rank block's own columns of its
   // chunk (its padding columns skipped).  A node is its first point and its size: a node and its

@@ -310,9 +310,13 @@ __global__ void __launch_bounds__(kTcThreads) tc_kernel(TcLaunch a, int npad_max
             col.pos = S.in_off + j;
             if (S.cscale) col.scale = __ldg(S.cscale + j);
             const TB* A = static_cast<const TB*>(S.A);
-            const int esz = int(sizeof(TB));
-            const int64_t T = tile_rows(esz), h = tile_height(m, tile, esz);
-            col.ptr = A + int64_t(tile) * T * S.K + int64_t(j) * h + (row0 - int64_t(tile) * T);
+            if (m > 32) {
+              const int esz = int(sizeof(TB));
+              const int64_t T = tile_rows(esz), h = tile_height(m, tile, esz);
+              col.ptr = A + int64_t(tile) * T * S.K + int64_t(j) * h + (row0 - int64_t(tile) * T);
+            } else {
+              col.ptr = A + int64_t(j) * m;
+            }
           }
         }
         tab[t] = col;
