@@ -71,16 +71,16 @@ __device__ __forceinline__ uint64_t global_ns() {
   return t;
 }
 
-// Waits for the phase with the given parity; false once kWaitNs nanoseconds
+// Waits for the phase with the given parity; false once `ns` nanoseconds
 // have passed without it completing.
 constexpr uint64_t kWaitNs = 2000000000ull;
 
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64_t ns = kWaitNs) {
   if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = global_ns();
   for (;;) {
     if (mbar_try_wait(bar, parity)) return true;
-    if (global_ns() - t0 > kWaitNs) return false;
+    if (global_ns() - t0 > ns) return false;
   }
 }
 

@@ -286,6 +286,9 @@ struct hodlr_op {
     int64_t nunits = 0;
     unsigned int* status = nullptr;
     unsigned int* h_status = nullptr;
+    // hodlr_test_option
+    uint64_t wait_ns = kTcWaitNs;
+    int32_t drop_copies = -1, drop_release = -1;
   } tc;
   int64_t n = 0, zlen = 0;
   int nslots = 0;
@@ -2839,7 +2842,7 @@ void apply_tc(hodlr_op* op, const float* x, int64_t ldx, float* y, int64_t ldy, 
   const TcLeafArgs la{P.panels_near,   P.panels_far,     T.leaf_near,  T.leaf_far,  T.leaf_near_segs,
                       T.leaf_far_segs, T.leaf_srcs, T.leaf_batches, T.leaf_runs,
                       T.nleaf_runs,    T.xunits,         T.y,          T.part_near, T.part_far,
-                      T.status};
+                      T.status,        T.wait_ns,        T.drop_copies, T.drop_release};
   CK(launch_tc_leaf(la, nrhs, st));
   a.panels = P.panels_near;
   a.segs = P.segs_near;
@@ -3109,6 +3112,23 @@ int hodlr_matvec_tc_device(hodlr_op* op, const float* d_x, float* d_y, int64_t n
     }
     return HODLR_OK;
   });
+}
+
+int hodlr_test_option(hodlr_op* op, int32_t option, int64_t value) {
+  if (!op) return fail(nullptr, HODLR_ERR_INVALID, "hodlr_test_option: null argument");
+  switch (option) {
+    case HODLR_TEST_TC_WAIT_NS:
+      op->tc.wait_ns = value < 0 ? kTcWaitNs : std::min(uint64_t(value), kTcWaitNs);
+      return HODLR_OK;
+    case HODLR_TEST_TC_DROP_COPIES:
+      op->tc.drop_copies = value < 0 ? -1 : int32_t(std::min<int64_t>(value, 1 << 30));
+      return HODLR_OK;
+    case HODLR_TEST_TC_DROP_RELEASE:
+      op->tc.drop_release = value < 0 ? -1 : int32_t(std::min<int64_t>(value, 1 << 30));
+      return HODLR_OK;
+    default:
+      return fail(op->ctx, HODLR_ERR_INVALID, "hodlr_test_option: unknown option");
+  }
 }
 
 int hodlr_set_relax(hodlr_op* op, int32_t relax, double relax_below) {

@@ -102,6 +102,7 @@ struct TcUnit {
   int32_t n, pad;
 };
 constexpr int kTcUnitBytes = 2048;  // 64 right-hand sides x 8 points, high and low parts
+constexpr uint64_t kTcWaitNs = 2000000000ull;  // the longest wait of a leaf-level kernel for a stage
 constexpr int kTcLeafGroup = 8;     // panels of a group: one per warp of a CTA
 // a batch of sources: at most kTcLeafUnits units, kTcLeafSegs segments and 32
 // sources (two stages of 45 KB, two CTAs per SM)
@@ -133,7 +134,11 @@ struct TcLeafArgs {
   const uint4* xunits;  // 128 per unit
   float* y;
   float *part_near, *part_far;  // part blocks of kTcRows x 64
-  unsigned int* status;
+  unsigned int* status;  // counts the warps that gave up a wait (the results are invalid then)
+  uint64_t wait_ns;      // the longest wait for a stage
+  // tests only: the batch of each run whose copies are left out, and the one
+  // after which warp 1 does not hand its stage back (-1: none)
+  int32_t drop_copies, drop_release;
 };
 cudaError_t launch_tc_units(const uint32_t* in, const TcUnit* units, int64_t nunits, uint4* out, cudaStream_t st);
 cudaError_t launch_tc_leaf(const TcLeafArgs& a, int nrhs, cudaStream_t st);

@@ -78,8 +78,10 @@ __device__ __forceinline__ void mbar_arrive_local(uint64_t* bar) {
 }
 
 // A stage: the sources' units, the batch's segment records, its header.  Shared
-// memory of a CTA: the stages' full and empty barriers, then the stages.
+// memory of a CTA: the stages' full and empty barriers, the stop flag, then the
+// stages.
 constexpr int kLeafStages = 2;
+constexpr int kLeafStop = 64;  // byte offset of the stop flag
 constexpr int kStageSegs = kTcLeafUnits * kTcUnitBytes;
 constexpr int kStageHead = kStageSegs + kTcLeafSegs * int(sizeof(TcLeafSeg));
 constexpr int kStageBytes = kStageHead + int(sizeof(TcLeafBatch));
@@ -239,13 +241,24 @@ __device__ __forceinline__ void leaf_step(const TcLeafSeg& S, int c, const LeafR
   }
 }
 
-// One warp's share of a group's run of batches.
+// One warp's share of a group's run of batches.  Every wait is bounded.  A warp
+// that gives one up counts it in *a.status and raises the CTA's stop flag; from
+// then on no warp reads a stage it has not seen complete, nothing more is
+// copied, and warp 0 waits (again with a bound) for the copies in flight before
+// it leaves.
 template <int MT, int NT, bool NEAR>
 __device__ __forceinline__ void leaf_run(const TcLeafArgs& a, const TcLeafRun& R, int m, float* out,
                                          unsigned char* smem, int wid, int lane) {
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
   uint64_t* empty = full + kLeafStages;
+  volatile int* stop = reinterpret_cast<volatile int*>(smem + kLeafStop);
   unsigned char* ring = smem + 128;
+  auto give_up = [&]() {
+    if (lane == 0) {
+      atomicAdd(a.status, 1u);
+      *stop = 1;
+    }
+  };
   float acc[MT][NT > 0 ? NT : 1][4];
 #pragma unroll
   for (int mt = 0; mt < MT; mt++)
@@ -258,6 +271,7 @@ __device__ __forceinline__ void leaf_run(const TcLeafArgs& a, const TcLeafRun& R
   // warp 0 copies a batch: its lanes a source's units each (they lie together),
   // lane 0 the segment records and the header
   auto issue = [&](int b) {
+    if (b == a.drop_copies) return;
     const TcLeafBatch* B = a.batches + R.batch_b + b;
     unsigned char* stage = ring + (b % kLeafStages) * kStageBytes;
     uint64_t* bar = full + b % kLeafStages;
@@ -282,16 +296,20 @@ __device__ __forceinline__ void leaf_run(const TcLeafArgs& a, const TcLeafRun& R
     __syncwarp();
     if (bytes) bulk_g2s(stage + off - bytes, a.xunits + int64_t(S.xunit) * 128, bytes, bar);
   };
+  int issued = min(kLeafStages, nb);  // warp 0's count of batches asked for
   if (wid == 0)
-    for (int b = 0; b < min(kLeafStages, nb); b++) issue(b);
-  for (int b = 0; b < nb; b++) {
+    for (int b = 0; b < issued; b++) issue(b);
+  int b = 0;
+  for (; b < nb; b++) {
     const int st = b % kLeafStages;
     const uint32_t phase = uint32_t(b / kLeafStages) & 1u;
     const unsigned char* stage = ring + st * kStageBytes;
-    if (!__all_sync(0xffffffffu, mbar_wait(full + st, phase))) {
-      if (lane == 0) atomicAdd(a.status, 1u);  // the results are invalid; go on without the data
-      __syncwarp();
-    } else if constexpr (NT > 0) {
+    if (!__all_sync(0xffffffffu, mbar_wait(full + st, phase, a.wait_ns))) {
+      give_up();
+      break;
+    }
+    if (__any_sync(0xffffffffu, *stop != 0)) break;
+    if constexpr (NT > 0) {
       const TcLeafBatch* H = reinterpret_cast<const TcLeafBatch*>(stage + kStageHead);
       const TcLeafSeg* rec = reinterpret_cast<const TcLeafSeg*>(stage + kStageSegs);
       int k = H->warp_off[wid], c = 0;
@@ -322,14 +340,22 @@ __device__ __forceinline__ void leaf_run(const TcLeafArgs& a, const TcLeafRun& R
       }
     }
     __syncwarp();
-    if (lane == 0) mbar_arrive_local(empty + st);
+    if (lane == 0 && !(wid == 1 && b == a.drop_release)) mbar_arrive_local(empty + st);
     if (wid == 0 && b + kLeafStages < nb) {
-      // every warp has left the stage: refill it
-      if (!__all_sync(0xffffffffu, mbar_wait(empty + st, phase))) {
-        if (lane == 0) atomicAdd(a.status, 1u);
+      // refilled once every warp has left the stage
+      if (!__all_sync(0xffffffffu, mbar_wait(empty + st, phase, a.wait_ns))) {
+        give_up();
+        b++;  // this batch's copies are done
+        break;
       }
       issue(b + kLeafStages);
+      issued++;
     }
+  }
+  if (b < nb) {
+    if (wid == 0)
+      for (; b < issued; b++) mbar_wait(full + b % kLeafStages, uint32_t(b / kLeafStages) & 1u, a.wait_ns);
+    return;
   }
   if constexpr (NT > 0) {
     const int g = lane >> 2, t = lane & 3;
@@ -364,6 +390,7 @@ __global__ void __launch_bounds__(kTcLeafGroup * 32, 2) tc_leaf_kernel(const TcL
       mbar_init(full + s, 1u);
       mbar_init(full + kLeafStages + s, kTcLeafGroup);
     }
+    *reinterpret_cast<volatile int*>(lsm + kLeafStop) = 0;
     fence_mbar_init();
   }
   __syncthreads();

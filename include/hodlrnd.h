@@ -336,6 +336,17 @@ int hodlr_aca_block_noalloc(const double* d_points, int64_t ld, int32_t ndim, co
  * (include/HDD_matrix.hpp:42-47). */
 int hodlr_matvec_tc_device(hodlr_op* op, const float* d_x, float* d_y, int64_t nrhs, void* stream);
 
+/* ---- test aids ------------------------------------------------------------
+ * Settings of one operator that no program needs: they make a device wait run
+ * out (every wait in this library is bounded), so that what follows can be
+ * tested.  A negative value restores the default.  No counterpart in the reference. */
+enum {
+  HODLR_TEST_TC_WAIT_NS = 0,     /* longest wait of the leaf-level tensor-core kernel, ns (at most the default) */
+  HODLR_TEST_TC_DROP_COPIES = 1, /* its runs leave out the copies of this batch */
+  HODLR_TEST_TC_DROP_RELEASE = 2 /* one warp of its runs does not hand this batch's stage back */
+};
+int hodlr_test_option(hodlr_op* op, int32_t option, int64_t value);
+
 /* ---- tensor cores ---------------------------------------------------------
  * Self-test of the fifth-generation tensor-core path (tcgen05) the multi-RHS
  * products use: D = A B^T with A (128 x k) and B (n x k) BF16, row major,
