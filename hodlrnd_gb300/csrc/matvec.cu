@@ -6,6 +6,7 @@
 
 #include "bulk.cuh"
 #include "device.cuh"
+#include "fpsum.cuh"
 #include "matvec.h"
 
 namespace hodlr {
@@ -2604,7 +2605,8 @@ __global__ void __launch_bounds__(256) batch_gather_mr_kernel(const BatchInst* _
 // whole 128-byte rows of the slots (at the points' tree positions), and the sums
 // are written from shared memory as runs of 32 points of a column (written row
 // by row in tree order, each value was a sector of its own: 313 us for 420,000
-// points against 60).
+// points against 60).  A row is the FP64 sum of its slots, formed on the FP32 pipe
+// where that gives the same value (fpsum.cuh; 20 us more than a plain FP32 pair).
 __global__ void __launch_bounds__(256) batch_combine_mr_kernel(const BatchInst* __restrict__ inst,
                                                                const float* __restrict__ y, int64_t ld_y,
                                                                float* __restrict__ out, int64_t total_n, int k, int ch) {
@@ -2612,17 +2614,25 @@ __global__ void __launch_bounds__(256) batch_combine_mr_kernel(const BatchInst* 
   const BatchInst I = inst[blockIdx.y];
   const float* yc = y + int64_t(ch) * ld_y * kMR;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t stride = I.n * kMR;
+  const bool live = ch * kMR + lane < k, few = I.nslots <= 8;
   for (int64_t p0 = int64_t(blockIdx.x) * 32; p0 < I.n; p0 += int64_t(gridDim.x) * 32) {
+    // four rows a warp: all their slots' loads first
+    const float* yr[4];
+    float v[4][8];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const int64_t p = p0 + wid * 4 + q;
-      if (p < I.n) {
-        const float* yr = yc + (I.y_base + I.iperm[p]) * kMR + lane;
-        // summed as FP32 pairs, rounded once (FP64 sums held the kernel up)
-        float acc = yr[0], err = 0.f;
-        for (int s = 1; s < I.nslots; s++) pair_add(acc, err, yr[int64_t(s) * I.n * kMR], 0.f);
-        tile[wid * 4 + q][lane] = __fadd_rn(acc, err);
-      }
+      yr[q] = p < I.n && live ? yc + (I.y_base + I.iperm[p]) * kMR + lane : nullptr;
+#pragma unroll
+      for (int s = 0; s < 8; s++) v[q][s] = yr[q] && few && s < I.nslots ? yr[q][s * stride] : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      float r = 0.f;
+      const bool ok = few && sum_few_as_fp64(I.nslots, v[q], r);
+      if (yr[q])
+        tile[wid * 4 + q][lane] = ok ? r : sum_as_fp64(I.nslots, [&](int s) { return yr[q][s * stride]; });
     }
     __syncthreads();
 #pragma unroll
