@@ -1,5 +1,6 @@
 // Restarted GMRES on the device (see gmres.h).
 #include "device.cuh"
+#include "fpsum.cuh"
 #include "gmres.h"
 
 #include <algorithm>
@@ -520,11 +521,42 @@ __device__ __forceinline__ bool grid_barrier(unsigned long long* bar) {
   return ok != 0;
 }
 
+// The sum of the G CTAs' partial pairs at part, by 8 lanes (each gets it; a warp
+// takes four sums at a time, which all its lanes ask for).  Summed as FP32
+// triples: more accurate than FP64 sums, and off the FP64 pipe, which a sum per
+// basis vector on every SM would hold up.  Sums beyond FP32's range are formed in
+// FP64.
+__device__ __forceinline__ double sum_step_parts(const float2* part, int G, int lane) {
+  const int sub = lane & 7;
+  TripleSum a;
+#pragma unroll
+  for (int q = 0; q < kStepGrid / 8; q++) {
+    const int c = sub + 8 * q;
+    const float2 p = c < G ? __ldcg(part + c) : make_float2(0.f, 0.f);
+    a.add(p.x, p.y);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+    a.add(__shfl_xor_sync(0xffffffffu, a.s, o), __shfl_xor_sync(0xffffffffu, a.c, o),
+          __shfl_xor_sync(0xffffffffu, a.t, o));
+  if (!__any_sync(0xffffffffu, !a.finite())) return a.value();
+  double v = 0.0;
+  for (int c = sub; c < G; c += 8) {
+    const float2 p = __ldcg(part + c);
+    v += __dadd_rn(double(p.x), double(p.y));
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+static_assert(kStepGrid % 8 == 0, "shares of 8 lanes");
+
 template <typename T>
 __global__ void __launch_bounds__(kCgsThreads, 1) cgs2_step_kernel(const StepArgs<T> a) {
   extern __shared__ __align__(16) unsigned char csm[];
   __shared__ double h[kStepMaxBasis], cs[kStepMaxBasis], sn[kStepMaxBasis];
-  __shared__ float2 hs[kStepMaxBasis], pairs[kCgsThreads], nrm;
+  __shared__ float2 hs[kStepMaxBasis], pairs[kCgsThreads];
+  __shared__ double nrm;
   const int E = cgs_slice(a.n), G = gridDim.x, cta = blockIdx.x;
   const int64_t e0 = int64_t(cta) * E;
   const int cnt = int(max(int64_t(0), min(int64_t(E), a.n - e0)));
@@ -581,19 +613,10 @@ __global__ void __launch_bounds__(kCgsThreads, 1) cgs2_step_kernel(const StepArg
       if (t == 0) a.hres[1] = 1.0;
       return;
     }
-    for (int j = wid; j < nv; j += kCgsWarps) {
-      float as = 0.f, ac = 0.f;
-#pragma unroll
-      for (int q = 0; q < (kStepGrid + 31) / 32; q++) {
-        const int c = lane + 32 * q;
-        const float2 p = c < G ? __ldcg(part + int64_t(j) * kStepGrid + c) : make_float2(0.f, 0.f);
-        pair_add(as, ac, p.x, p.y);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
-        pair_add(as, ac, __shfl_xor_sync(0xffffffffu, as, o), __shfl_xor_sync(0xffffffffu, ac, o));
-      if (lane == 0) {
-        const double v = __dadd_rn(double(as), double(ac));
+    for (int j0 = wid * 4; j0 < nv; j0 += kCgsWarps * 4) {
+      const int j = min(j0 + (lane >> 3), nv - 1);
+      const double v = sum_step_parts(part + int64_t(j) * kStepGrid, G, lane);
+      if ((lane & 7) == 0 && j == j0 + (lane >> 3)) {
         h[j] = pass ? __dadd_rn(h[j], v) : v;
         hs[j] = split_d(v);
       }
@@ -649,20 +672,11 @@ __global__ void __launch_bounds__(kCgsThreads, 1) cgs2_step_kernel(const StepArg
     return;
   }
   if (wid == 0) {
-    ns = nk = 0.f;
-#pragma unroll
-    for (int q = 0; q < (kStepGrid + 31) / 32; q++) {
-      const int c = lane + 32 * q;
-      const float2 p = c < G ? __ldcg(npart + c) : make_float2(0.f, 0.f);
-      pair_add(ns, nk, p.x, p.y);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      pair_add(ns, nk, __shfl_xor_sync(0xffffffffu, ns, o), __shfl_xor_sync(0xffffffffu, nk, o));
-    if (lane == 0) nrm = make_float2(ns, nk);
+    const double v = sum_step_parts(npart, G, lane);
+    if (lane == 0) nrm = v;
   }
   __syncthreads();
-  const double hn = sqrt(__dadd_rn(double(nrm.x), double(nrm.y)));
+  const double hn = sqrt(nrm);
   const double ih = 1.0 / hn;
   T* out = V + int64_t(nv) * a.n;
   for (int e = t; e < cnt; e += kCgsThreads) out[e] = T(__dmul_rn(ih, wd[e]));

@@ -1,5 +1,7 @@
 // Compares fpsum.cuh's FP32-pair sums with the FP64 sums they stand for, bit for
 // bit, over random and edge operands; prints the number of mismatches.
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -8,6 +10,12 @@
 
 #include "../hodlrnd_gb300/csrc/fpsum.cuh"
 using namespace hodlr;
+
+#ifdef __aarch64__
+using Quad = long double;  // 113 bits
+#else
+using Quad = __float128;
+#endif
 
 static uint64_t rng_state = 88172645463325252ull;
 static uint64_t rnd() {
@@ -69,6 +77,24 @@ int main(int argc, char** argv) {
       bad += !same(sum_few_as_fp64(count, u, r) ? r : sum_in_fp64(count, at));
     }
   }
-  printf("%ld\n", bad);
-  return bad ? 1 : 0;
+  // triples of 152 pairs against sums in 113 bits: no further off than FP64 sums
+  double e3 = 0.0, e64 = 0.0;
+  for (long i = 0; i < n / 152; i++) {
+    TripleSum t;
+    Quad want = 0, mag = 0;
+    volatile double acc = 0.0;
+    for (int q = 0; q < 152; q++) {
+      const float x = make(0), y = x * float(int64_t(rnd() >> 40)) * 0x1p-49f;
+      const float sign = rnd() & 1 ? 1.f : -1.f;
+      t.add(sign * x, sign * y);
+      want += Quad(sign * x) + Quad(sign * y);
+      mag += Quad(x < 0 ? -x : x);
+      acc = acc + (double(sign * x) + double(sign * y));
+    }
+    const double a = double((Quad(t.value()) - want) / mag), b = double((Quad(acc) - want) / mag);
+    e3 = std::max(e3, std::fabs(a));
+    e64 = std::max(e64, std::fabs(b));
+  }
+  printf("%ld %.3e %.3e\n", bad, e3, e64);
+  return bad || e3 > e64 || e3 > 0x1p-53 ? 1 : 0;
 }

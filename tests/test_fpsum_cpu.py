@@ -1,6 +1,8 @@
 """fpsum.cuh: sums of FP32 values on the FP32 pipe equal the FP64 sums rounded to
 FP32, bit for bit (random magnitudes, cancellation, ties, overflow on the way,
-infinities, NaNs, zeros, subnormals; one value to more than the pair takes)."""
+infinities, NaNs, zeros, subnormals; one value to more than the pair takes), and
+sums of 152 FP32 pairs as triples are no further from the sum in 113 bits than
+FP64 sums of the same pairs, and within 2^-53 of the magnitudes added."""
 import os
 import shutil
 import subprocess
