@@ -159,6 +159,8 @@ def lib():
     L.hodlr_matvec_tc_device.restype = ctypes.c_int
     L.hodlr_test_option.argtypes = [P, ctypes.c_int32, ctypes.c_int64]
     L.hodlr_test_option.restype = ctypes.c_int
+    L.hodlr_test_value.argtypes = [P, ctypes.c_int32, I64]
+    L.hodlr_test_value.restype = ctypes.c_int
     L.hodlr_tc_selftest.argtypes = [P, P, ctypes.c_int32, ctypes.c_int32, P]
     L.hodlr_tc_selftest.restype = ctypes.c_int
     for f in ("hodlr_op_save", "hodlr_op_load", "hodlr_set_relax", "hodlr_vec_load", "hodlr_vec_save", "hodlr_ctx_create", "hodlr_ctx_destroy", "hodlr_build", "hodlr_op_destroy", "hodlr_matvec",

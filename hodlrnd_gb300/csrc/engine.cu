@@ -3126,8 +3126,27 @@ int hodlr_test_option(hodlr_op* op, int32_t option, int64_t value) {
     case HODLR_TEST_TC_DROP_RELEASE:
       op->tc.drop_release = value < 0 ? -1 : int32_t(std::min<int64_t>(value, 1 << 30));
       return HODLR_OK;
+    case HODLR_TEST_STEP_WAIT_NS: {
+      const uint64_t ns = value < 0 ? kBarrierNs : std::min(uint64_t(value), kBarrierNs);
+      op->g64.step_wait_ns = op->g32.step_wait_ns = ns;
+      return HODLR_OK;
+    }
     default:
       return fail(op->ctx, HODLR_ERR_INVALID, "hodlr_test_option: unknown option");
+  }
+}
+
+int hodlr_test_value(const hodlr_op* op, int32_t what, int64_t* value) {
+  if (!op || !value) return fail(nullptr, HODLR_ERR_INVALID, "hodlr_test_value: null argument");
+  switch (what) {
+    case HODLR_TEST_STEPS:
+      *value = op->g64.steps + op->g32.steps;
+      return HODLR_OK;
+    case HODLR_TEST_STEP_GIVE_UPS:
+      *value = op->g64.step_give_ups + op->g32.step_give_ups;
+      return HODLR_OK;
+    default:
+      return fail(op->ctx, HODLR_ERR_INVALID, "hodlr_test_value: unknown value");
   }
 }
 

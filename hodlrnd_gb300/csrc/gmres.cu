@@ -326,7 +326,7 @@ __device__ __forceinline__ void step_new_rotation(double hk, double hn, int i, d
 
 template <typename T>
 struct StepArgs {
-  const T* w;
+  T* w;
   T* V;
   int64_t n;
   int i;        // Arnoldi index: w against v_0 .. v_i, v_{i+1} written
@@ -340,6 +340,9 @@ struct StepArgs {
   float2* part;             // kStepMaxBasis x kStepGrid partial pairs, two sets, and the norm's
   unsigned long long* bar;  // grid barrier arrivals
   int cached;               // the basis slices fit in shared memory
+  uint64_t wait_ns;         // longest wait at a barrier
+  int phase;                // one phase per launch: which
+  int redo;                 // a one-launch attempt of this step gave up
 };
 
 // MGS: a cluster of CTAs (16, or 8 where 16 do not fit), each with a slice of
@@ -479,11 +482,13 @@ __global__ void __launch_bounds__(kStepThreads, 1) mgs_cluster_kernel(const Step
 // shared memory where they fit and serve both passes from there.
 // n = 20011, 50 basis vectors: 36 us a step against 75 for the nine kernels; a
 // cluster of 16 CTAs took 105 (its 16 SMs are bound by the splits and products).
+// When other work holds some SMs for longer than kBarrierNs, a barrier gives up,
+// and the step is done again in four launches that need no CTA beside another
+// one: the same operations in the same order, so the results are the same to the last bit.
 constexpr int kStepGrid = 152;
 constexpr int kCgsThreads = 512;
 constexpr int kCgsWarps = kCgsThreads / 32;
 constexpr int kCgsSliceBytes = 128 * 1024;  // basis slices in shared memory at most
-constexpr unsigned long long kBarrierNs = 2000000000ull;
 
 // a slice: a multiple of 32 elements
 __host__ __device__ inline int cgs_slice(int64_t n) { return int((step_slice(n, kStepGrid - 1) + 31) / 32 * 32); }
@@ -493,9 +498,9 @@ __host__ inline size_t cgs_smem(int64_t n, int nv, bool cached) {
   return size_t(cgs_slice(n)) * (sizeof(double) + sizeof(float2)) + (cached ? size_t(nv) * cgs_slice(n) * sizeof(float2) : 0);
 }
 
-// Arrives at the grid barrier and waits for every CTA (at most 2 s); false
+// Arrives at the grid barrier and waits for every CTA (at most wait_ns); false
 // after a give-up.
-__device__ __forceinline__ bool grid_barrier(unsigned long long* bar) {
+__device__ __forceinline__ bool grid_barrier(unsigned long long* bar, uint64_t wait_ns) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -509,7 +514,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned long long* bar) {
       asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(bar) : "memory");
       if (v >= goal) break;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-      if (t1 - t0 > kBarrierNs) {
+      if (t1 - t0 > wait_ns) {
         good = 0;
         break;
       }
@@ -551,7 +556,15 @@ __device__ __forceinline__ double sum_step_parts(const float2* part, int G, int 
 }
 static_assert(kStepGrid % 8 == 0, "shares of 8 lanes");
 
-template <typename T>
+// GRID: the whole step (a cooperative launch); else phase a.phase of it, after
+// which w and the partial sums are in memory:
+//   0: the first pass's projections
+//   1: their sums and update, the second pass's projections
+//   2: their sums and update, the earlier rotations, |w|'s share
+//   3: |w|, v_{i+1}, the new rotation
+// scal[5]: the right-hand side's entry i before the step, scal[6]: the column's
+// running entry after the earlier rotations.
+template <typename T, bool GRID>
 __global__ void __launch_bounds__(kCgsThreads, 1) cgs2_step_kernel(const StepArgs<T> a) {
   extern __shared__ __align__(16) unsigned char csm[];
   __shared__ double h[kStepMaxBasis], cs[kStepMaxBasis], sn[kStepMaxBasis];
@@ -570,6 +583,16 @@ __global__ void __launch_bounds__(kCgsThreads, 1) cgs2_step_kernel(const StepArg
   // operations, 8 us at 50 columns)
   const bool rotor = cta == G - 1;
   double hk = 0.0;
+  auto run = [&](int phase) { return GRID || a.phase == phase; };
+  if (rotor && t == 0) {
+    double* rs = a.rot + 2 * (a.restart + 1);
+    if (GRID) {
+      a.scal[5] = rs[a.i];
+    } else if (a.phase == 0 && a.redo) {  // the attempt's rotation may have been applied
+      rs[a.i] = a.scal[5];
+      rs[a.i + 1] = 0.0;
+    }
+  }
   if (rotor)
     for (int k = t; k < a.i; k += kCgsThreads) {
       cs[k] = a.rot[k];
@@ -580,7 +603,8 @@ __global__ void __launch_bounds__(kCgsThreads, 1) cgs2_step_kernel(const StepArg
     wd[e] = to_d(v);
     sw[e] = split_t(v);
   }
-  if (a.cached && !rotor) {
+  const bool cached = GRID && a.cached;
+  if (cached && !rotor) {
     for (int q = wid; q < nv; q += kCgsWarps)
 #pragma unroll 4
       for (int e = lane; e < E; e += 32) sv[q * E + e] = e < cnt ? split_t(V[int64_t(q) * a.n + e]) : make_float2(0.f, 0.f);
@@ -592,10 +616,10 @@ __global__ void __launch_bounds__(kCgsThreads, 1) cgs2_step_kernel(const StepArg
   float ns = 0.f, nk = 0.f;
   for (int pass = 0; pass < 2; pass++) {
     float2* part = a.part + int64_t(pass) * kStepMaxBasis * kStepGrid;
-    for (int j = wid; j < nv; j += kCgsWarps) {
+    for (int j = run(pass) ? wid : nv; j < nv; j += kCgsWarps) {
       float as = 0.f, ac = 0.f;
       if (rotor) {
-      } else if (a.cached) {
+      } else if (cached) {
         const float2* vj = sv + j * E;
 #pragma unroll 4
         for (int e = lane; e < E; e += 32) dot2_add(as, ac, vj[e], sw[e]);
@@ -609,21 +633,27 @@ __global__ void __launch_bounds__(kCgsThreads, 1) cgs2_step_kernel(const StepArg
         pair_add(as, ac, __shfl_xor_sync(0xffffffffu, as, o), __shfl_xor_sync(0xffffffffu, ac, o));
       if (lane == 0) __stcg(part + int64_t(j) * kStepGrid + cta, make_float2(as, ac));
     }
-    if (!grid_barrier(a.bar)) {
+    if (GRID && !grid_barrier(a.bar, a.wait_ns)) {
       if (t == 0) a.hres[1] = 1.0;
       return;
     }
+    if (!run(pass + 1)) continue;
     for (int j0 = wid * 4; j0 < nv; j0 += kCgsWarps * 4) {
       const int j = min(j0 + (lane >> 3), nv - 1);
       const double v = sum_step_parts(part + int64_t(j) * kStepGrid, G, lane);
+      double first = 0.0;  // the first pass's, for the column
+      if (pass && rotor) first = GRID ? h[j] : sum_step_parts(a.part + int64_t(j) * kStepGrid, G, lane);
       if ((lane & 7) == 0 && j == j0 + (lane >> 3)) {
-        h[j] = pass ? __dadd_rn(h[j], v) : v;
+        h[j] = pass ? __dadd_rn(first, v) : v;
         hs[j] = split_d(v);
       }
     }
     __syncthreads();
     if (rotor) {
-      if (pass && t == 0) hk = step_rotate(h, cs, sn, a.i, a.H + int64_t(a.i) * a.ldh);
+      if (pass && t == 0) {
+        hk = step_rotate(h, cs, sn, a.i, a.H + int64_t(a.i) * a.ldh);
+        if (!GRID) a.scal[6] = hk;
+      }
       continue;
     }
     for (int b = 0; b < EG; b += kCgsWarps) {
@@ -631,7 +661,7 @@ __global__ void __launch_bounds__(kCgsThreads, 1) cgs2_step_kernel(const StepArg
       const bool act = eg < EG && jg < JG;
       float s = 0.f, c = 0.f;
       if (act && e < cnt) {
-        if (a.cached) {
+        if (cached) {
 #pragma unroll 4
           for (int j = jg; j < nv; j += JG) dot2_add(s, c, sv[j * E + e], hs[j]);
         } else {
@@ -650,6 +680,7 @@ __global__ void __launch_bounds__(kCgsThreads, 1) cgs2_step_kernel(const StepArg
         const float2 vs = split_t(v);
         wd[e] = to_d(v);
         sw[e] = vs;
+        if (!GRID) a.w[e0 + e] = v;
         if (pass) dot2_add(ns, nk, vs, vs);
       }
       __syncthreads();
@@ -657,20 +688,23 @@ __global__ void __launch_bounds__(kCgsThreads, 1) cgs2_step_kernel(const StepArg
   }
   // |w|: the CTA's pair, then every CTA's
   float2* npart = a.part + int64_t(2) * kStepMaxBasis * kStepGrid;
+  if (run(2)) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    pair_add(ns, nk, __shfl_xor_sync(0xffffffffu, ns, o), __shfl_xor_sync(0xffffffffu, nk, o));
-  if (lane == 0) pairs[wid] = make_float2(ns, nk);
-  __syncthreads();
-  if (t == 0) {
-    ns = nk = 0.f;
-    for (int q = 0; q < kCgsWarps; q++) pair_add(ns, nk, pairs[q].x, pairs[q].y);
-    __stcg(npart + cta, make_float2(ns, nk));  // the last CTA's is zero, as its projections are
+    for (int o = 16; o > 0; o >>= 1)
+      pair_add(ns, nk, __shfl_xor_sync(0xffffffffu, ns, o), __shfl_xor_sync(0xffffffffu, nk, o));
+    if (lane == 0) pairs[wid] = make_float2(ns, nk);
+    __syncthreads();
+    if (t == 0) {
+      ns = nk = 0.f;
+      for (int q = 0; q < kCgsWarps; q++) pair_add(ns, nk, pairs[q].x, pairs[q].y);
+      __stcg(npart + cta, make_float2(ns, nk));  // the last CTA's is zero, as its projections are
+    }
   }
-  if (!grid_barrier(a.bar)) {
+  if (GRID && !grid_barrier(a.bar, a.wait_ns)) {
     if (t == 0) a.hres[1] = 1.0;
     return;
   }
+  if (!run(3)) return;
   if (wid == 0) {
     const double v = sum_step_parts(npart, G, lane);
     if (lane == 0) nrm = v;
@@ -681,7 +715,7 @@ __global__ void __launch_bounds__(kCgsThreads, 1) cgs2_step_kernel(const StepArg
   T* out = V + int64_t(nv) * a.n;
   for (int e = t; e < cnt; e += kCgsThreads) out[e] = T(__dmul_rn(ih, wd[e]));
   if (rotor && t == 0)
-    step_new_rotation(hk, hn, a.i, a.H + int64_t(a.i) * a.ldh, a.rot, a.restart, a.scal, a.hres);
+    step_new_rotation(GRID ? hk : a.scal[6], hn, a.i, a.H + int64_t(a.i) * a.ldh, a.rot, a.restart, a.scal, a.hres);
 }
 
 // What the MGS cluster of c CTAs is launched with.
@@ -726,9 +760,9 @@ bool cgs_step_fits(int64_t n, int restart) {
       cudaGetDevice(&dev) == cudaSuccess &&
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
-      cudaFuncSetAttribute(&cgs2_step_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaFuncSetAttribute(&cgs2_step_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            int(kCgsSliceBytes + cgs_smem(kStepMaxN, 0, false))) == cudaSuccess &&
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, &cgs2_step_kernel<T>, kCgsThreads,
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, &cgs2_step_kernel<T, true>, kCgsThreads,
                                                     kCgsSliceBytes + cgs_smem(n, 0, false)) == cudaSuccess &&
       int64_t(per) * sms >= cgs_grid(n);
   if (!ok) cudaGetLastError();
@@ -749,8 +783,20 @@ cudaError_t launch_cgs_step(StepArgs<T> a, cudaStream_t st) {
   a.cached = basis <= size_t(kCgsSliceBytes);
   count_launches(1);
   void* args[] = {&a};
-  return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(&cgs2_step_kernel<T>), dim3(unsigned(cgs_grid(a.n))),
+  return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(&cgs2_step_kernel<T, true>), dim3(unsigned(cgs_grid(a.n))),
                                      dim3(kCgsThreads), args, cgs_smem(a.n, a.i + 1, a.cached != 0), st);
+}
+
+// The same step in four launches.
+template <typename T>
+cudaError_t launch_cgs_phases(StepArgs<T> a, bool redo, cudaStream_t st) {
+  a.redo = redo;
+  for (a.phase = 0; a.phase < 4; a.phase++) {
+    count_launches(1);
+    cgs2_step_kernel<T, false>
+        <<<unsigned(cgs_grid(a.n)), kCgsThreads, cgs_smem(a.n, a.i + 1, false), st>>>(a);
+  }
+  return cudaGetLastError();
 }
 
 // Update (GMRES.hpp:132-146): back substitution into y.
@@ -950,6 +996,7 @@ cudaError_t gmres_solve(GmresWork<T>& W, const TreeMatvec<T>& A, const T* b, T* 
     return cudaSuccess;
   }
   int64_t j = 1;
+  bool busy = false;  // the device has no room for every CTA of a step at once
   while (j <= max_iter) {
     count_launches(1);
     start_cycle_kernel<T><<<kVecCtas, kThreads, 0, st>>>(W.r, W.V, n, W.scal, W.rot + 2 * (W.restart + 1), W.restart);
@@ -960,13 +1007,18 @@ cudaError_t gmres_solve(GmresWork<T>& W, const TreeMatvec<T>& A, const T* b, T* 
       if (mgs ? W.mgs_ctas > 0 : W.cgs_step) {
         const StepArgs<T> sa{W.w,       W.V,    n,       i,           W.H,
                              ldh,       W.rot,  W.restart, W.scal,    W.hscal,
-                             static_cast<float2*>(W.step_part), W.step_bar, 0};
+                             static_cast<float2*>(W.step_part), W.step_bar, 0, W.step_wait_ns, 0, 0};
         W.hscal[1] = 0.0;
-        HODLR_TRY(mgs ? launch_mgs_step<T>(sa, W.mgs_ctas, st) : launch_cgs_step<T>(sa, st));
+        W.steps++;
+        HODLR_TRY(mgs ? launch_mgs_step<T>(sa, W.mgs_ctas, st)
+                      : busy ? launch_cgs_phases<T>(sa, false, st) : launch_cgs_step<T>(sa, st));
         HODLR_TRY(cudaStreamSynchronize(st));
-        if (W.hscal[1] != 0.0) {  // a grid barrier gave up
-          HODLR_TRY(cudaMemset(W.step_bar, 0, sizeof(unsigned long long)));
-          return cudaErrorLaunchTimeout;
+        if (W.hscal[1] != 0.0) {  // a barrier gave up: v_0 .. v_i and w are as they were
+          busy = true;            // for the rest of this solve
+          W.step_give_ups++;
+          HODLR_TRY(cudaMemsetAsync(W.step_bar, 0, sizeof(unsigned long long), st));
+          HODLR_TRY(launch_cgs_phases<T>(sa, true, st));
+          HODLR_TRY(cudaStreamSynchronize(st));
         }
       } else {
         double* plast;

@@ -28,6 +28,10 @@
 namespace hodlr {
 
 constexpr int kVecCtas = 152 * 4;  // fixed grid of the vector kernels
+// The longest wait of a one-launch CGS2 step for its CTAs: some 500 steps; beyond
+// that the device is busy with other work, and the step takes a launch for each of
+// its four phases, with the same results.
+constexpr uint64_t kBarrierNs = 20000000ull;
 
 template <typename T>
 struct GmresWork {
@@ -42,7 +46,7 @@ struct GmresWork {
   double* part = nullptr; // 2 x kVecCtas partial sums
   double* partk = nullptr; // (restart + 1) x kVecCtas partial sums (CGS2)
   double* hc = nullptr;    // restart + 1 projection coefficients of one CGS pass
-  double* scal = nullptr; // device scalars: [0] resid, [1] beta, [2] normb
+  double* scal = nullptr; // device scalars: [0] resid, [1] beta, [2] normb, [4] 1 / |w|, [5] and [6] cgs2_step_kernel's
   double* hscal = nullptr;  // pinned host mirror of scal
   // an Arnoldi step in one launch: CTAs of the MGS cluster (0: separate
   // kernels), whether the CGS2 kernel takes it, and the latter's partial sums
@@ -51,6 +55,8 @@ struct GmresWork {
   bool cgs_step = false;
   void* step_part = nullptr;
   unsigned long long* step_bar = nullptr;
+  uint64_t step_wait_ns = kBarrierNs;
+  int64_t steps = 0, step_give_ups = 0;  // one-launch steps so far, and those that had to be done again
 };
 
 template <typename T>
