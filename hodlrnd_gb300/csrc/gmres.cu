@@ -737,8 +737,8 @@ cudaLaunchConfig_t mgs_config(int64_t n, int c, cudaLaunchAttribute* at, cudaStr
 // CTAs of the MGS cluster for vectors of n elements on this device; 0: the
 // separate kernels.
 template <typename T>
-int mgs_ctas(int64_t n, int restart) {
-  if (n > kStepMaxN || restart + 1 > kStepMaxBasis) return 0;
+int mgs_ctas(int64_t n) {
+  if (n > kStepMaxN) return 0;
   for (int c : {kStepCtas, kStepCtas / 2}) {
     cudaLaunchAttribute at{};
     const cudaLaunchConfig_t cfg = mgs_config(n, c, &at, nullptr);
@@ -753,8 +753,8 @@ int mgs_ctas(int64_t n, int restart) {
 
 // Whether the CGS2 step kernel takes vectors of n elements on this device.
 template <typename T>
-bool cgs_step_fits(int64_t n, int restart) {
-  if (n > kStepMaxN || restart + 1 > kStepMaxBasis) return false;
+bool cgs_step_fits(int64_t n) {
+  if (n > kStepMaxN) return false;
   int dev = 0, sms = 0, coop = 0, per = 0;
   const bool ok =
       cudaGetDevice(&dev) == cudaSuccess &&
@@ -904,8 +904,8 @@ cudaError_t gmres_alloc(GmresWork<T>& W, int64_t n, int restart) {
   HODLR_TRY(cudaMalloc(&W.hc, sizeof(double) * size_t(restart + 1)));
   HODLR_TRY(cudaMalloc(&W.scal, sizeof(double) * 8));
   HODLR_TRY(cudaMallocHost(&W.hscal, sizeof(double) * 8));
-  W.mgs_ctas = mgs_ctas<T>(n, restart);
-  W.cgs_step = cgs_step_fits<T>(n, restart);
+  W.mgs_ctas = mgs_ctas<T>(n);
+  W.cgs_step = cgs_step_fits<T>(n);
   if (W.cgs_step) {
     HODLR_TRY(cudaMalloc(&W.step_part, sizeof(float2) * (2 * kStepMaxBasis + 1) * kStepGrid));
     HODLR_TRY(cudaMalloc(&W.step_bar, sizeof(unsigned long long)));
@@ -996,6 +996,10 @@ cudaError_t gmres_solve(GmresWork<T>& W, const TreeMatvec<T>& A, const T* b, T* 
     return cudaSuccess;
   }
   int64_t j = 1;
+  const bool mgs = ortho == Ortho::kMGS;
+  // whether this solve's steps take one launch each (its own cycle counts, not
+  // the longest one the workspace has been allocated for)
+  const bool one_launch = m + 1 <= kStepMaxBasis && (mgs ? W.mgs_ctas > 0 : W.cgs_step);
   bool busy = false;  // the device has no room for every CTA of a step at once
   while (j <= max_iter) {
     count_launches(1);
@@ -1003,8 +1007,7 @@ cudaError_t gmres_solve(GmresWork<T>& W, const TreeMatvec<T>& A, const T* b, T* 
     for (int i = 0; i < m && j <= max_iter; i++, j++) {
       T* vi = W.V + int64_t(i) * n;
       HODLR_TRY(A(vi, W.w));
-      const bool mgs = ortho == Ortho::kMGS;
-      if (mgs ? W.mgs_ctas > 0 : W.cgs_step) {
+      if (one_launch) {
         const StepArgs<T> sa{W.w,       W.V,    n,       i,           W.H,
                              ldh,       W.rot,  W.restart, W.scal,    W.hscal,
                              static_cast<float2*>(W.step_part), W.step_bar, 0, W.step_wait_ns, 0, 0};
