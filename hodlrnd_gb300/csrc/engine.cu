@@ -2070,9 +2070,9 @@ void build_finish(hodlr_op* op, BuildState& bs, cudaStream_t st) {
     op->d_y32 = op->mem.alloc_n<float>(size_t(n) * size_t(op->nslots), "matvec slots (FP32)");
     op->d_r32 = op->mem.alloc_n<float>(size_t(n), "residual (FP32)");
     op->d_d32 = op->mem.alloc_n<float>(size_t(n), "correction (FP32)");
-    CK(gmres_alloc<float>(op->g32, n, restart));
+    CK(gmres_alloc<float>(op->g32, n, restart, st));
   } else {
-    CK(gmres_alloc<double>(op->g64, n, restart));
+    CK(gmres_alloc<double>(op->g64, n, restart, st));
   }
   CK(cudaStreamSynchronize(st));
   op->st.t_build_s = now_s() - bs.t0;
@@ -3172,9 +3172,9 @@ int hodlr_set_solver(hodlr_op* op, int32_t restart, double tol, int64_t max_iter
     op->p.max_outer = max_outer;
     const int r = restart > 0 ? restart : 100;
     if (op->p.precision == HODLR_PREC_MIXED) {
-      if (r > op->g32.restart) CK(gmres_alloc<float>(op->g32, op->n, r));
+      if (r > op->g32.restart) CK(gmres_alloc<float>(op->g32, op->n, r, op->ctx->stream));
     } else if (r > op->g64.restart) {
-      CK(gmres_alloc<double>(op->g64, op->n, r));
+      CK(gmres_alloc<double>(op->g64, op->n, r, op->ctx->stream));
     }
     return HODLR_OK;
   });

@@ -887,7 +887,7 @@ __global__ void fill_zero_kernel(T* x, int64_t n) {
 }  // namespace
 
 template <typename T>
-cudaError_t gmres_alloc(GmresWork<T>& W, int64_t n, int restart) {
+cudaError_t gmres_alloc(GmresWork<T>& W, int64_t n, int restart, cudaStream_t st) {
   gmres_free(W);
   W.n = n;
   W.restart = restart;
@@ -896,9 +896,9 @@ cudaError_t gmres_alloc(GmresWork<T>& W, int64_t n, int restart) {
   HODLR_TRY(cudaMalloc(&W.r, sizeof(T) * size_t(n)));
   HODLR_TRY(cudaMalloc(&W.tmp, sizeof(T) * size_t(n)));
   HODLR_TRY(cudaMalloc(&W.H, sizeof(double) * size_t(restart + 1) * size_t(restart)));
-  HODLR_TRY(cudaMemset(W.H, 0, sizeof(double) * size_t(restart + 1) * size_t(restart)));
+  HODLR_TRY(cudaMemsetAsync(W.H, 0, sizeof(double) * size_t(restart + 1) * size_t(restart), st));
   HODLR_TRY(cudaMalloc(&W.rot, sizeof(double) * 4 * size_t(restart + 1)));
-  HODLR_TRY(cudaMemset(W.rot, 0, sizeof(double) * 4 * size_t(restart + 1)));
+  HODLR_TRY(cudaMemsetAsync(W.rot, 0, sizeof(double) * 4 * size_t(restart + 1), st));
   HODLR_TRY(cudaMalloc(&W.part, sizeof(double) * 2 * kVecCtas));
   HODLR_TRY(cudaMalloc(&W.partk, sizeof(double) * kVecCtas * size_t(restart + 1)));
   HODLR_TRY(cudaMalloc(&W.hc, sizeof(double) * size_t(restart + 1)));
@@ -909,9 +909,9 @@ cudaError_t gmres_alloc(GmresWork<T>& W, int64_t n, int restart) {
   if (W.cgs_step) {
     HODLR_TRY(cudaMalloc(&W.step_part, sizeof(float2) * (2 * kStepMaxBasis + 1) * kStepGrid));
     HODLR_TRY(cudaMalloc(&W.step_bar, sizeof(unsigned long long)));
-    HODLR_TRY(cudaMemset(W.step_bar, 0, sizeof(unsigned long long)));
+    HODLR_TRY(cudaMemsetAsync(W.step_bar, 0, sizeof(unsigned long long), st));
   }
-  return cudaSuccess;
+  return cudaStreamSynchronize(st);  // a solve may follow on any stream
 }
 
 template <typename T>
@@ -1089,8 +1089,8 @@ cudaError_t gmres_solve(GmresWork<T>& W, const TreeMatvec<T>& A, const T* b, T* 
   return cudaSuccess;
 }
 
-template cudaError_t gmres_alloc<double>(GmresWork<double>&, int64_t, int);
-template cudaError_t gmres_alloc<float>(GmresWork<float>&, int64_t, int);
+template cudaError_t gmres_alloc<double>(GmresWork<double>&, int64_t, int, cudaStream_t);
+template cudaError_t gmres_alloc<float>(GmresWork<float>&, int64_t, int, cudaStream_t);
 template void gmres_free<double>(GmresWork<double>&);
 template void gmres_free<float>(GmresWork<float>&);
 template cudaError_t gmres_solve<double>(GmresWork<double>&, const TreeMatvec<double>&, const double*, double*, bool,

@@ -59,8 +59,9 @@ struct GmresWork {
   int64_t steps = 0, step_give_ups = 0;  // one-launch steps so far, and those that had to be done again
 };
 
+// Complete when it returns (its clearing runs on st).
 template <typename T>
-cudaError_t gmres_alloc(GmresWork<T>& W, int64_t n, int restart);
+cudaError_t gmres_alloc(GmresWork<T>& W, int64_t n, int restart, cudaStream_t st);
 template <typename T>
 void gmres_free(GmresWork<T>& W);
 
