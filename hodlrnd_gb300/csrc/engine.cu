@@ -185,8 +185,12 @@ struct Plan {
   void* zpart = nullptr;
   void* ypart = nullptr;
   // host copies of the arrays above, kept for operators of a batch (merged
-  // into the batch's plan)
+  // into the batch's plan) and for the tensor-core plan.  The members of an
+  // FP32-vector batch have items of their own here (merged_items), with the
+  // numbers and sizes that go with them.
   struct Host {
+    bool contig_near = false, contig_far = false;
+    int64_t nypart_near = 0, nzpart = 0;
     std::vector<Panel> panels_near, panels_far;
     std::vector<Seg> segs_near, segs_far;
     std::vector<Item> small_near, big_near, small_far, big_far;
@@ -440,40 +444,54 @@ int panel_cols(int64_t bytes, int64_t rows, int esz) {
   return int(std::max<int64_t>(1, std::min<int64_t>(bytes / (rows * esz), 1 << 28)));
 }
 
-// Items of a panel of at most 32 rows: one warp for the panel, or for each run
-// of about `bytes` of its factors when it has more (partial rows added by the
-// fix-up kernel).
-void add_small_items(const std::vector<Seg>& segs, const Panel& p, int np, int64_t bytes, int esz,
-                     std::vector<Item>& small, std::vector<PanelFix>& pfix, int64_t& nypart) {
-  const std::vector<std::pair<int32_t, int32_t>> groups =
-      column_groups(segs, p.seg_begin, p.seg_end, std::max(64, panel_cols(bytes, p.m, esz)));
+// The items of a family of panels and the fix-ups of the split ones.
+struct PanelList {
+  std::vector<Item> small, big;
+  std::vector<PanelFix> fix;
+  int64_t nypart = 0;  // partial row blocks
+};
+
+// One item for columns of row chunk c of panel np, or one for each run of about
+// `cols` columns when there are more (partial rows added by the fix-up kernel).
+void add_items(const std::vector<Seg>& segs, const Panel& p, int np, int c, int cols, std::vector<Item>& items,
+               PanelList& L) {
+  const std::vector<std::pair<int32_t, int32_t>> groups = column_groups(segs, p.seg_begin, p.seg_end, cols);
   if (groups.size() == 1) {
-    small.push_back({np, 0, int32_t(p.seg_begin), int32_t(p.seg_end), -1, -1});
+    items.push_back({np, c, groups[0].first, groups[0].second, -1, -1});
     return;
   }
-  pfix.push_back({np, 0, int32_t(nypart), int32_t(groups.size())});
-  for (auto& g : groups) small.push_back({np, 0, g.first, g.second, int32_t(nypart++), int32_t(pfix.size() - 1)});
+  L.fix.push_back({np, c, int32_t(L.nypart), int32_t(groups.size())});
+  for (auto& g : groups) items.push_back({np, c, g.first, g.second, int32_t(L.nypart++), int32_t(L.fix.size() - 1)});
+}
+// The items of panel np: of its whole rows when there are at most 32 of them
+// (to `small`, about small_bytes of factors each), else of each chunk of
+// `rows` rows (to L.big, about big_bytes).
+void add_panel_items(const std::vector<Seg>& segs, const Panel& p, int np, int rows, int esz, int64_t small_bytes,
+                     int64_t big_bytes, std::vector<Item>& small, PanelList& L) {
+  if (p.m <= 32) {
+    add_items(segs, p, np, 0, std::max(64, panel_cols(small_bytes, p.m, esz)), small, L);
+    return;
+  }
+  for (int c = 0; c < (p.m + rows - 1) / rows; c++)
+    add_items(segs, p, np, c, panel_cols(big_bytes, rows, esz), L.big, L);
 }
 
-// Whether an operator's items are spread as item_bytes says: all but the
-// members of an FP32-vector batch, whose merged plan has the items of many
-// instances and 32 right-hand sides per partial sum.
-bool spread_items(const hodlr_op* op) { return !(op->keep_host_plans && op->p.precision == HODLR_PREC_MIXED); }
+// Whether the operator's host plan has items of its own: the members of an
+// FP32-vector batch.  Their own products take items spread as item_bytes says,
+// like those of an operator built alone; the merged plan has the items of many
+// instances, and 32 right-hand sides per partial sum, so long items there.
+bool merged_items(const hodlr_op* op) { return op->keep_host_plans && op->p.precision == HODLR_PREC_MIXED; }
 
 void build_near_plan(hodlr_op* op, const NearTiles& nt, const void* base, Prec a, Plan& plan, cudaStream_t st) {
   const Tree& t = op->tree;
   const int L = t.levels - 1;
   std::vector<Panel> panels;
   std::vector<Seg> segs;
-  std::vector<Item> small, big;
-  std::vector<PanelFix> pfix;
-  int64_t nypart = 0;
+  PanelList own, merged;
   const size_t esz = a == Prec::kD ? 8 : 4;
-  const bool spread = spread_items(op);
   int64_t total = 0;
   for (const TileDesc& d : nt.tiles) total += int64_t(d.m) * d.n * int64_t(esz);
-  const int64_t small_bytes = spread ? item_bytes(total, kMinItemBytes, int64_t(1) << 40) : int64_t(1) << 40;
-  const int64_t big_bytes = spread ? item_bytes(total, kMinItemBytes, kNearItemBytes) : kNearItemBytes;
+  const int64_t whole = int64_t(1) << 40;
   // FP64 panels of at most 32 rows: the staged leaf kernel when leaves are tiny
   // (its one byte run per stage beats a segment per slice: 3D N = 262144, 8
   // rows, 127 us against 183), else the items of launch_items64 with the larger
@@ -505,45 +523,36 @@ void build_near_plan(hodlr_op* op, const NearTiles& nt, const void* base, Prec a
     p.seg_end = int64_t(segs.size());
     const int np = int(panels.size());
     panels.push_back(p);
-    if (leaf && p.m <= 32) {
-      small.push_back({np, 0, int32_t(p.seg_begin), int32_t(p.seg_end), -1, -1});
-    } else if (p.m <= 32) {
-      add_small_items(segs, p, np, small_bytes, int(esz), a == Prec::kD ? big : small, pfix, nypart);
-    } else {
-      // as for far panels: runs of columns, partial row blocks added by the
-      // fix-up kernel
-      const int rows = rows_per_item(a);
-      const std::vector<std::pair<int32_t, int32_t>> groups =
-          column_groups(segs, p.seg_begin, p.seg_end, panel_cols(big_bytes, rows, int(esz)));
-      for (int c = 0; c < int((p.m + rows - 1) / rows); c++) {
-        if (groups.size() == 1) {
-          big.push_back({np, c, groups[0].first, groups[0].second, -1, -1});
-          continue;
-        }
-        pfix.push_back({np, c, int32_t(nypart), int32_t(groups.size())});
-        for (auto& g : groups) big.push_back({np, c, g.first, g.second, int32_t(nypart++), int32_t(pfix.size() - 1)});
-      }
-    }
+    auto add = [&](PanelList& L, int64_t small_bytes, int64_t big_bytes) {
+      add_panel_items(segs, p, np, int(rows_per_item(a)), int(esz), leaf ? whole : small_bytes, big_bytes,
+                      leaf || a != Prec::kD ? L.small : L.big, L);
+    };
+    add(own, item_bytes(total, kMinItemBytes, whole), item_bytes(total, kMinItemBytes, kNearItemBytes));
+    if (merged_items(op)) add(merged, whole, kNearItemBytes);
   }
-  plan.contig_near = small_items_contiguous(panels, segs, small, int(esz));
-  plan.pfix_near = upload(op->mem, pfix, st, "near panel fix-ups");
-  plan.npfix_near = int(pfix.size());
-  plan.pcnt_near = fix_counters(op->mem, pfix.size(), st);
-  plan.nypart_near = nypart * rows_per_item(a);
+  plan.contig_near = small_items_contiguous(panels, segs, own.small, int(esz));
+  plan.pfix_near = upload(op->mem, own.fix, st, "near panel fix-ups");
+  plan.npfix_near = int(own.fix.size());
+  plan.pcnt_near = fix_counters(op->mem, own.fix.size(), st);
+  plan.nypart_near = own.nypart * rows_per_item(a);
   plan.a_near = a;
   plan.panels_near = upload(op->mem, panels, st, "near panels");
   plan.segs_near = upload(op->mem, segs, st, "near segments");
-  plan.small_near = upload(op->mem, small, st, "near items");
-  plan.big_near = upload(op->mem, big, st, "near items");
-  plan.nsmall_near = int(small.size());
-  plan.nbig_near = int(big.size());
+  plan.small_near = upload(op->mem, own.small, st, "near items");
+  plan.big_near = upload(op->mem, own.big, st, "near items");
+  plan.nsmall_near = int(own.small.size());
+  plan.nbig_near = int(own.big.size());
   if (op->keep_host_plans) {
     if (!plan.host) plan.host = std::make_shared<Plan::Host>();
-    plan.host->panels_near = panels;
-    plan.host->segs_near = segs;
-    plan.host->small_near = small;
-    plan.host->big_near = big;
-    plan.host->pfix_near = pfix;
+    Plan::Host& h = *plan.host;
+    const PanelList& L = merged_items(op) ? merged : own;
+    h.panels_near = panels;
+    h.segs_near = segs;
+    h.small_near = L.small;
+    h.big_near = L.big;
+    h.pfix_near = L.fix;
+    h.nypart_near = L.nypart * rows_per_item(a);
+    h.contig_near = small_items_contiguous(panels, segs, L.small, int(esz));
   }
 }
 
@@ -553,10 +562,8 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
   const Tree& t = op->tree;
   std::vector<Panel> panels;
   std::vector<Seg> segs;
-  std::vector<Item> small, big;
+  PanelList own, merged;
   std::vector<ZBlock> zb;
-  std::vector<PanelFix> pfix;
-  int64_t nypart = 0;
   int64_t zoff = op->n;
   // FP32 / BF16 after the relayout: z = V^T x per chunk of source-node columns
   const bool chunks = a != Prec::kD && !op->vchunks.empty();
@@ -567,10 +574,6 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
     utotal += m * (op->dense[q] ? ns : op->rank[q]) * prec_size(a);
     if (!op->dense[q]) vtotal += ns * op->rank[q] * prec_size(a);
   }
-  const bool spread = spread_items(op);
-  const int64_t big_bytes = spread ? item_bytes(utotal, kMinItemBytes, kPanelItemBytes) : kBatchItemBytes;
-  const int64_t small_bytes = spread ? item_bytes(utotal, kMinItemBytes, kSmallItemBytes) : kSmallItemBytes;
-  const int64_t z_bytes = spread ? item_bytes(vtotal, kMinItemBytes, kZItemBytes) : kBatchItemBytes;
   size_t b = 0;
   while (b < op->far.size()) {
     const int l = op->far[b].level;
@@ -625,24 +628,13 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
     if (p.seg_end > p.seg_begin) {
       const int np = int(panels.size());
       panels.push_back(p);
-      if (p.m <= 32) {
-        // a few panels with very long interaction lists would otherwise keep
-        // single warps busy long after the rest
-        add_small_items(segs, p, np, small_bytes, prec_size(a), small, pfix, nypart);
-      } else {
-        const int rows = rows_per_item(a);
-        const std::vector<std::pair<int32_t, int32_t>> groups =
-            column_groups(segs, p.seg_begin, p.seg_end, panel_cols(big_bytes, rows, prec_size(a)));
-        const int chunks = int((p.m + rows - 1) / rows);
-        for (int c = 0; c < chunks; c++) {
-          if (groups.size() == 1) {
-            big.push_back({np, c, groups[0].first, groups[0].second, -1, -1});
-            continue;
-          }
-          pfix.push_back({np, c, int32_t(nypart), int32_t(groups.size())});
-          for (auto& g : groups) big.push_back({np, c, g.first, g.second, int32_t(nypart++), int32_t(pfix.size() - 1)});
-        }
-      }
+      // (a few leaf panels with very long interaction lists would otherwise keep
+      // single warps busy long after the rest)
+      auto add = [&](PanelList& L, int64_t small_bytes, int64_t big_bytes) {
+        add_panel_items(segs, p, np, int(rows_per_item(a)), prec_size(a), small_bytes, big_bytes, L.small, L);
+      };
+      add(own, item_bytes(utotal, kMinItemBytes, kSmallItemBytes), item_bytes(utotal, kMinItemBytes, kPanelItemBytes));
+      if (merged_items(op)) add(merged, kSmallItemBytes, kBatchItemBytes);
     }
     b = e;
   }
@@ -667,63 +659,77 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
   // operator read from a file): their panels always take the direct-load
   // kernel, whose results do not depend on the layout.  FP32 and BF16 factors
   // are laid out in panel order (relayout_far).
-  plan.contig_far = a != Prec::kD && small_items_contiguous(panels, segs, small, prec_size(a));
+  auto contig = [&](const PanelList& L) { return a != Prec::kD && small_items_contiguous(panels, segs, L.small, prec_size(a)); };
+  plan.contig_far = contig(own);
   plan.panels_far = upload(op->mem, panels, st, "far panels");
   plan.segs_far = upload(op->mem, segs, st, "far segments");
-  plan.small_far = upload(op->mem, small, st, "far items");
-  plan.big_far = upload(op->mem, big, st, "far items");
-  plan.nsmall_far = int(small.size());
-  plan.nbig_far = int(big.size());
+  plan.small_far = upload(op->mem, own.small, st, "far items");
+  plan.big_far = upload(op->mem, own.big, st, "far items");
+  plan.nsmall_far = int(own.small.size());
+  plan.nbig_far = int(own.big.size());
   // V^T x items: up to 32 sixteen-byte loads of columns by a run of rows of
   // about z_bytes; blocks with more rows split into partial sums
-  std::vector<ZItem> zit;
-  std::vector<ZFix> zfix;
-  int64_t nzpart = 0;
+  struct ZList {
+    std::vector<ZItem> items;
+    std::vector<ZFix> fix;
+    int64_t nzpart = 0;
+  };
   const int esz = prec_size(a);
   const int cmax = std::min(32 * (16 / esz), kZPart);  // BF16: 128 of the 256 a warp could load
-  for (size_t q = 0; q < zb.size(); q++) {
-    const int n = zb[q].n, r = zb[q].r;
-    const int rp = int(vpad(r, esz));
-    for (int k0 = 0; k0 < rp; k0 += cmax) {
-      const int nk = std::min(cmax, rp - k0);
-      const int rows = int(std::max<int64_t>(1, z_bytes / (nk * esz)));
-      const int groups = (n + rows - 1) / rows;
-      if (groups == 1) {
-        zit.push_back({int32_t(q), k0, nk, 0, n, -1, 0, 0, -1});
-        z_item_stages(zit.back(), r, esz);
-        continue;
-      }
-      zfix.push_back({zb[q].z_off + k0, int32_t(nzpart), groups, std::min(nk, r - k0), 0});
-      for (int g = 0; g < groups; g++) {
-        zit.push_back({int32_t(q), k0, nk, g * rows, std::min(n, (g + 1) * rows), int32_t(nzpart), 0, 0,
-                       int32_t(zfix.size() - 1)});
-        z_item_stages(zit.back(), r, esz);
-        nzpart += kZPart;
+  auto z_list = [&](int64_t z_bytes) {
+    ZList Z;
+    for (size_t q = 0; q < zb.size(); q++) {
+      const int n = zb[q].n, r = zb[q].r;
+      const int rp = int(vpad(r, esz));
+      for (int k0 = 0; k0 < rp; k0 += cmax) {
+        const int nk = std::min(cmax, rp - k0);
+        const int rows = int(std::max<int64_t>(1, z_bytes / (nk * esz)));
+        const int groups = (n + rows - 1) / rows;
+        if (groups == 1) {
+          Z.items.push_back({int32_t(q), k0, nk, 0, n, -1, 0, 0, -1});
+          z_item_stages(Z.items.back(), r, esz);
+          continue;
+        }
+        Z.fix.push_back({zb[q].z_off + k0, int32_t(Z.nzpart), groups, std::min(nk, r - k0), 0});
+        for (int g = 0; g < groups; g++) {
+          Z.items.push_back({int32_t(q), k0, nk, g * rows, std::min(n, (g + 1) * rows), int32_t(Z.nzpart), 0, 0,
+                             int32_t(Z.fix.size() - 1)});
+          z_item_stages(Z.items.back(), r, esz);
+          Z.nzpart += kZPart;
+        }
       }
     }
-  }
+    return Z;
+  };
+  const ZList Z = z_list(item_bytes(vtotal, kMinItemBytes, kZItemBytes));
   plan.zb = upload(op->mem, zb, st, "far z blocks");
   plan.nzb = int(zb.size());
-  plan.zitems = upload(op->mem, zit, st, "far z items");
-  plan.nzitems = int(zit.size());
-  plan.zfix = upload(op->mem, zfix, st, "far z fix-ups");
-  plan.nzfix = int(zfix.size());
-  plan.pfix_far = upload(op->mem, pfix, st, "far panel fix-ups");
-  plan.npfix_far = int(pfix.size());
-  plan.zcnt = fix_counters(op->mem, zfix.size(), st);
-  plan.pcnt_far = fix_counters(op->mem, pfix.size(), st);
-  plan.nzpart = nzpart;
-  plan.nypart = nypart * rows_per_item(a);
+  plan.zitems = upload(op->mem, Z.items, st, "far z items");
+  plan.nzitems = int(Z.items.size());
+  plan.zfix = upload(op->mem, Z.fix, st, "far z fix-ups");
+  plan.nzfix = int(Z.fix.size());
+  plan.pfix_far = upload(op->mem, own.fix, st, "far panel fix-ups");
+  plan.npfix_far = int(own.fix.size());
+  plan.zcnt = fix_counters(op->mem, Z.fix.size(), st);
+  plan.pcnt_far = fix_counters(op->mem, own.fix.size(), st);
+  plan.nzpart = Z.nzpart;
+  plan.nypart = own.nypart * rows_per_item(a);
   if (op->keep_host_plans) {
     if (!plan.host) plan.host = std::make_shared<Plan::Host>();
-    plan.host->panels_far = panels;
-    plan.host->segs_far = segs;
-    plan.host->small_far = small;
-    plan.host->big_far = big;
-    plan.host->pfix_far = pfix;
-    plan.host->zb = zb;
-    plan.host->zitems = zit;
-    plan.host->zfix = zfix;
+    Plan::Host& h = *plan.host;
+    const bool m = merged_items(op);
+    const PanelList& L = m ? merged : own;
+    h.panels_far = panels;
+    h.segs_far = segs;
+    h.small_far = L.small;
+    h.big_far = L.big;
+    h.pfix_far = L.fix;
+    h.contig_far = contig(L);
+    h.zb = zb;
+    const ZList& HZ = m ? z_list(kBatchItemBytes) : Z;
+    h.zitems = HZ.items;
+    h.zfix = HZ.fix;
+    h.nzpart = HZ.nzpart;
   }
 }
 
@@ -2166,7 +2172,7 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
     e.small_near = a.small_near + int64_t(hn.small_near.size());
     e.big_near = a.big_near + int64_t(hn.big_near.size());
     e.pfix_near = a.pfix_near + int64_t(hn.pfix_near.size());
-    e.near_parts = a.near_parts + pn.nypart_near / rows_per_item(pn.a_near);
+    e.near_parts = a.near_parts + hn.nypart_near / rows_per_item(pn.a_near);
     e.panels_far = a.panels_far + int64_t(hf.panels_far.size());
     e.segs_far = a.segs_far + int64_t(hf.segs_far.size());
     e.small_far = a.small_far + int64_t(hf.small_far.size());
@@ -2178,7 +2184,7 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
     e.zb = a.zb + int64_t(hf.zb.size());
     e.zitems = a.zitems + int64_t(hf.zitems.size());
     e.zfix = a.zfix + int64_t(hf.zfix.size());
-    e.zpart = a.zpart + op->plan64.nzpart;
+    e.zpart = a.zpart + hf.nzpart;
     e.in = a.in + op->n + op->zlen;
     e.y = a.y + int64_t(op->nslots) * op->n;
     e.x = a.x + op->n;
@@ -2186,8 +2192,8 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
     b.max_n = std::max(b.max_n, op->n);
     // the merged items reference the same factor bytes, so their layout
     // test is each instance's own
-    contig_near = contig_near && pn.contig_near;
-    contig_far = contig_far && op->plan64.contig_far;
+    contig_near = contig_near && hn.contig_near;
+    contig_far = contig_far && hf.contig_far;
   }
   const Base& tot = base[nops];
   h.panels_near.resize(size_t(tot.panels_near));
