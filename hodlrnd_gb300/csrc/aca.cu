@@ -29,10 +29,10 @@
 // The FP64 pipe bounds it (20 cycles of an SM per warp instruction; 80-85% busy
 // whenever an SM works), so what need not be FP64 is not: square roots and
 // divisions on the integer pipe (softfp.cuh), pivots compared as integers, eight
-// dot products of the norm estimate reduced together in the warp teams, no lane's
-// FP64 work beyond a warp's share of a row.  3D N = 100003: CTA teams 236 -> 219
-// ms, warp teams 248 -> 184 (a residual row's code at one call site each also
-// keeps the warp teams, which run at different points of it, in the instruction
+// dot products of the norm estimate reduced together in the warp teams.  3D N =
+// 100003 (FP64, 1e-8): CTA teams 93 -> 72 ms, warp teams 142 -> 102 (a residual
+// row's code at one call site each also keeps the warp teams, which run at
+// different points of it, in the instruction
 // cache).  What is left is the residuals' products and subtractions, which must
 // round one by one.
 //
@@ -155,7 +155,7 @@ __host__ __device__ constexpr int staged_team_bytes(int T, int D) {
 
 template <int D, class Team, bool S = false>
 struct AcaTeam {
-  static constexpr int JU = S ? 1 : Team::kSize == 32 ? 2 : 4;  // entries of a residual row or column a thread forms together
+  
   const AcaArgs& a;
   const AcaBlockDesc& B;
   Team tm;
@@ -339,6 +339,30 @@ struct AcaTeam {
     return tm.bcast(r);
   }
 
+  // val - A[0] B[0] - A[lda] B[ldb] - ... over r columns, in order, with one rounding
+  // per operation.  Four columns' loads are in flight together: at high ranks
+  // the factors lie beyond L1.  (Several entries of a thread side by side, a
+  // load each per column, measured slower at every rank: CTA teams with four,
+  // 4D N = 20000 with ranks up to 618 1085 ms against 840, 3D N = 100003 229 against 224.)
+  __device__ __forceinline__ static double subtract(double val, const double* A, int64_t lda, const double* B,
+                                                    int64_t ldb, int r) {
+    int k = 0;
+    if constexpr (!S) {
+      for (; k + 4 <= r; k += 4) {
+        double x[4], y[4];
+#pragma unroll
+        for (int z = 0; z < 4; z++) {
+          x[z] = A[int64_t(k + z) * lda];
+          y[z] = B[int64_t(k + z) * ldb];
+        }
+#pragma unroll
+        for (int z = 0; z < 4; z++) val = __dsub_rn(val, __dmul_rn(x[z], y[z]));
+      }
+    }
+    for (; k < r; k++) val = __dsub_rn(val, __dmul_rn(A[int64_t(k) * lda], B[int64_t(k) * ldb]));
+    return val;
+  }
+
   // Residual row i0 into V[:, r]; argmax over the remaining columns.
   __device__ void gen_row(int i0, int r, int nc, double& mx, int& piv, double& sq) {
     double xi[D];
@@ -354,43 +378,21 @@ struct AcaTeam {
     unsigned long long bk = 0;
     double v0 = 0.0, s = 0.0;
     int bi = 0x7fffffff;
-    const int w0 = tm.tid() & ~31;  // the warp's first place in the team
-    // JU columns per thread at a time: their chains of subtractions overlap
-    for (int jb = 0; jb + w0 < n; jb += JU * Team::kSize) {
-      double val[JU];
-      int jj[JU];
-#pragma unroll
-      for (int q = 0; q < JU; q++) {
-        if (jb + q * Team::kSize + w0 >= n) break;  // warp-uniform
-        const int j = min(jb + q * Team::kSize + tm.tid(), n - 1);
-        jj[q] = j;
-        if constexpr (S)
-          val[q] = kernel_entry_xy<D>(K, pi == is[j], xi, xs + j, n);
-        else
-          val[q] = kernel_entry<D>(a.P, K, pi, a.lmap[B.s_map + j], xi);
-      }
-      for (int k = 0; k < r; k++) {
-        const double u = U[i0 + int64_t(k) * m];
-        const double* Vk = V + int64_t(k) * n;
-#pragma unroll
-        for (int q = 0; q < JU; q++) {
-          if (jb + q * Team::kSize + w0 >= n) break;
-          val[q] = __dsub_rn(val[q], __dmul_rn(u, Vk[jj[q]]));
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < JU; q++) {
-        const int j = jb + q * Team::kSize + tm.tid();
-        if (j >= n) break;
-        V[j + int64_t(r) * n] = val[q];
-        s += val[q] * val[q];
-        if (j == 0) v0 = val[q];
-        if ((cb[j >> 5] >> (j & 31)) & 1u) {
-          const unsigned long long key = pivot_key(val[q]);
-          if (!pivot_nan(key) && pivot_better(key, j, bk, bi)) {
-            bk = key;
-            bi = j;
-          }
+    for (int j = tm.tid(); j < n; j += Team::kSize) {
+      double val;
+      if constexpr (S)
+        val = kernel_entry_xy<D>(K, pi == is[j], xi, xs + j, n);
+      else
+        val = kernel_entry<D>(a.P, K, pi, a.lmap[B.s_map + j], xi);
+      val = subtract(val, U + i0, m, V + j, n, r);
+      V[j + int64_t(r) * n] = val;
+      s += val * val;
+      if (j == 0) v0 = val;
+      if ((cb[j >> 5] >> (j & 31)) & 1u) {
+        const unsigned long long key = pivot_key(val);
+        if (!pivot_nan(key) && pivot_better(key, j, bk, bi)) {
+          bk = key;
+          bi = j;
         }
       }
     }
@@ -412,50 +414,29 @@ struct AcaTeam {
     double v0 = 0.0, s = 0.0;
     int bi = 0x7fffffff;
     const int64_t pj = S ? int64_t(is[j0]) : int64_t(a.lmap[B.s_map + j0]);
-    const int w0 = tm.tid() & ~31;
-    for (int ib = 0; ib + w0 < m; ib += JU * Team::kSize) {
-      double val[JU];
-      int ii[JU];
+    for (int i = tm.tid(); i < m; i += Team::kSize) {
+      // A(i, j0) with the target point first, as getCol evaluates it
+      // (getMatrixEntry(sources[j], k), kernel_function.hpp:32-40).
+      double xi[D];
+      double val;
+      if constexpr (S) {
 #pragma unroll
-      for (int q = 0; q < JU; q++) {
-        if (ib + q * Team::kSize + w0 >= m) break;  // warp-uniform
-        const int i = min(ib + q * Team::kSize + tm.tid(), m - 1);
-        ii[q] = i;
-        // A(i, j0) with the target point first, as getCol evaluates it
-        // (getMatrixEntry(sources[j], k), kernel_function.hpp:32-40).
-        double xi[D];
-        if constexpr (S) {
-#pragma unroll
-          for (int k = 0; k < D; k++) xi[k] = xt[k * m + i];
-          val[q] = kernel_entry_xy<D>(K, it[i] == pj, xi, xs + j0, n);
-        } else {
-          const int64_t pi = a.lmap[B.t_map + i];
-          load_point<D>(a.P, pi, xi);
-          val[q] = kernel_entry<D>(a.P, K, pi, pj, xi);
-        }
+        for (int k = 0; k < D; k++) xi[k] = xt[k * m + i];
+        val = kernel_entry_xy<D>(K, it[i] == pj, xi, xs + j0, n);
+      } else {
+        const int64_t pi = a.lmap[B.t_map + i];
+        load_point<D>(a.P, pi, xi);
+        val = kernel_entry<D>(a.P, K, pi, pj, xi);
       }
-      for (int k = 0; k < r; k++) {
-        const double v = V[j0 + int64_t(k) * n];
-        const double* Uk = U + int64_t(k) * m;
-#pragma unroll
-        for (int q = 0; q < JU; q++) {
-          if (ib + q * Team::kSize + w0 >= m) break;
-          val[q] = __dsub_rn(val[q], __dmul_rn(v, Uk[ii[q]]));
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < JU; q++) {
-        const int i = ib + q * Team::kSize + tm.tid();
-        if (i >= m) break;
-        U[i + int64_t(r) * m] = val[q];
-        s += val[q] * val[q];
-        if (i == 0) v0 = val[q];
-        if ((rb[i >> 5] >> (i & 31)) & 1u) {
-          const unsigned long long key = pivot_key(val[q]);
-          if (!pivot_nan(key) && pivot_better(key, i, bk, bi)) {
-            bk = key;
-            bi = i;
-          }
+      val = subtract(val, V + j0, n, U + i, m, r);
+      U[i + int64_t(r) * m] = val;
+      s += val * val;
+      if (i == 0) v0 = val;
+      if ((rb[i >> 5] >> (i & 31)) & 1u) {
+        const unsigned long long key = pivot_key(val);
+        if (!pivot_nan(key) && pivot_better(key, i, bk, bi)) {
+          bk = key;
+          bi = i;
         }
       }
     }
