@@ -2171,26 +2171,35 @@ __device__ __forceinline__ void mr_store(float* dst, int n, int lane, const floa
 }
 
 // z_b = V_b^T X_s: item = rows [j0, j1) of block zb, columns [k0, k0 + nk) (at
-// most 128); runs of whole V rows and their input rows staged by bulk copies in
-// a ring of kMStages.
-template <int NQ>
+// most 128); runs of V rows and their input rows staged by bulk copies in a ring
+// of kMStages: one copy for a run of whole rows, one for each row when the item
+// has only some of a wider block's columns.
+template <int NQ, bool WHOLE>
 __device__ __forceinline__ void zgemv_mr_item(const ZItem& it, const ZBlock& Z, const float* V, int64_t rp,
                                               const float* xr, float* dst, unsigned char* base, int lane) {
   uint64_t* bar = reinterpret_cast<uint64_t*>(base);
   unsigned char* stage0 = base + 64;
-  const int rowb = int(rp) * 4;  // a multiple of 16
+  const int rowb = it.nk * 4;  // a multiple of 16, as k0 and rp
   const int R = kMStageBytes / (rowb + kMRowBytes);  // rows per stage: their factors, then their inputs
   const int nrows = it.j1 - it.j0;
   const int total = (nrows + R - 1) / R;
-  auto issue = [&](int q) {  // lane 0: rows q R ..
+  auto issue = [&](int q) {  // rows q R ..
     const int s = q % kMStages, r0 = q * R, nr = min(R, nrows - r0);
     unsigned char* st = stage0 + s * kMStageBytes;
     fence_proxy_async();
-    mbar_expect_tx(bar + s, uint32_t(nr) * uint32_t(rowb + kMRowBytes));
-    bulk_g2s(st, V + int64_t(r0) * rp, uint32_t(nr * rowb), bar + s);
-    bulk_g2s(st + R * rowb, xr + int64_t(r0) * kMR, uint32_t(nr * kMRowBytes), bar + s);
+    if (lane == 0) {
+      mbar_expect_tx(bar + s, uint32_t(nr) * uint32_t(rowb + kMRowBytes));
+      if (WHOLE) bulk_g2s(st, V + int64_t(r0) * rp, uint32_t(nr * rowb), bar + s);
+      bulk_g2s(st + R * rowb, xr + int64_t(r0) * kMR, uint32_t(nr * kMRowBytes), bar + s);
+    }
+    if (!WHOLE) {
+      __syncwarp();
+      for (int r = lane; r < nr; r += 32)
+        bulk_g2s(st + r * rowb, V + int64_t(r0 + r) * rp + it.k0, uint32_t(rowb), bar + s);
+    }
   };
-  if (lane == 0)
+  const bool copies = !WHOLE || lane == 0;
+  if (copies)
     for (int q = 0; q < min(kMStages, total); q++) issue(q);
   float acc[4 * NQ][8];
 #pragma unroll
@@ -2206,9 +2215,9 @@ __device__ __forceinline__ void zgemv_mr_item(const ZItem& it, const ZBlock& Z, 
       return;
     }
     const unsigned char* st = stage0 + s * kMStageBytes;
-    mr_wide<NQ>(st + it.k0 * 4, rowb, reinterpret_cast<const float*>(st + R * rowb), min(R, nrows - q * R), lane, acc);
+    mr_wide<NQ>(st, rowb, reinterpret_cast<const float*>(st + R * rowb), min(R, nrows - q * R), lane, acc);
     __syncwarp();
-    if (lane == 0 && q + kMStages < total) issue(q + kMStages);
+    if (copies && q + kMStages < total) issue(q + kMStages);
   }
   mr_store<NQ>(dst, it.part < 0 ? min(it.nk, Z.r - it.k0) : it.nk, lane, acc);
 }
@@ -2228,17 +2237,6 @@ __global__ void __launch_bounds__(kMWarps * 32, 3)
   const float* V = static_cast<const float*>(Z.V) + int64_t(it.j0) * rp;
   const float* xr = inc + (Z.x_off + it.j0) * kMR;
   float* dst = it.part < 0 ? inc + (Z.z_off + it.k0) * kMR : zp + int64_t(it.part) * kMR;
-  if (rp * 4 > kMStageBytes / 2) {
-    // rows wider than half a stage (rank above 928): direct loads, a right-hand side per lane
-    for (int c = 0; c < it.nk; c++) {
-      if (it.part < 0 && it.k0 + c >= Z.r) break;
-      float acc = 0.f;
-      for (int j = 0; j < it.j1 - it.j0; j++)
-        acc = __fmaf_rn(__ldg(V + int64_t(j) * rp + it.k0 + c), xr[int64_t(j) * kMR + lane], acc);
-      dst[int64_t(c) * kMR + lane] = acc;
-    }
-    return;
-  }
   unsigned char* base = msm + wid * kMWarpSmem;
   if (lane == 0) {
     uint64_t* bar = reinterpret_cast<uint64_t*>(base);
@@ -2247,11 +2245,15 @@ __global__ void __launch_bounds__(kMWarps * 32, 3)
     fence_mbar_init();
   }
   __syncwarp();
+  if (it.nk < rp) {
+    zgemv_mr_item<4, false>(it, Z, V, rp, xr, dst, base, lane);
+    return;
+  }
   switch ((it.nk + 31) / 32) {
-    case 1: zgemv_mr_item<1>(it, Z, V, rp, xr, dst, base, lane); break;
-    case 2: zgemv_mr_item<2>(it, Z, V, rp, xr, dst, base, lane); break;
-    case 3: zgemv_mr_item<3>(it, Z, V, rp, xr, dst, base, lane); break;
-    default: zgemv_mr_item<4>(it, Z, V, rp, xr, dst, base, lane); break;
+    case 1: zgemv_mr_item<1, true>(it, Z, V, rp, xr, dst, base, lane); break;
+    case 2: zgemv_mr_item<2, true>(it, Z, V, rp, xr, dst, base, lane); break;
+    case 3: zgemv_mr_item<3, true>(it, Z, V, rp, xr, dst, base, lane); break;
+    default: zgemv_mr_item<4, true>(it, Z, V, rp, xr, dst, base, lane); break;
   }
 }
 
