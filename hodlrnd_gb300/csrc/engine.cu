@@ -291,6 +291,7 @@ struct hodlr_op {
     unsigned int* status = nullptr;
     unsigned int* h_status = nullptr;
     // hodlr_test_option
+    int force_leaf = 0;  // 1: always the leaf-level kernel, 2: never (before the first product)
     uint64_t wait_ns = kTcWaitNs;
     int32_t drop_copies = -1, drop_release = -1;
   } tc;
@@ -2648,24 +2649,39 @@ void build_tc_plan(hodlr_op* op, cudaStream_t st) {
   std::vector<Item> ni, fi;
   std::vector<PanelFix> fxn, fxf;
   int pn = 0, pf = 0;
-  // The leaf-level kernel pays where a leaf has rows to fill its 8-wide pieces
-  // and sources enough for a run; else the tcgen05 kernels take every panel
-  // (64 right-hand sides, leaf kernel against tcgen05: 2D N = 18000, 25 far blocks a
-  // leaf, 251 us against 186; 3D N = 3000, 5.9 rows, 236 against 224; 3D N = 30000,
-  // 7.3 rows, 809 against 1089; 4D N = 6000, 23 rows, 482 against 570; 4D N = 9000,
-  // 35 rows, so that panels of up to 32 are large and far apart, 722 against 589).
-  int64_t lrows = 0, lsegs = 0, lpanels = 0;
+  const Tree& t = op->tree;
+  // The leaf-level kernel pays where a leaf has rows to fill its 8-wide pieces,
+  // sources enough for a run, and z rows that it keeps out of memory to outweigh
+  // the near field, whose tiles of more than 16 rows the tcgen05 kernels take in
+  // fewer steps; else those take every panel.  Leaf kernel against tcgen05, us at 64
+  // right-hand sides (rows a panel, far blocks a panel, z rows per 8 x 8 near piece):
+  //   2D N = 18000 (18, 14, 0.4)  224 : 171     3D N = 30000 (7.3, 106, 8) 723 : 1019
+  //   3D N = 20000 (30, 82, 1.1)  736 : 619     3D N = 60000 (15, 106, 4.6) 1030 : 1443
+  //   3D N = 27538 (6.7, 106, 3.8) 633 : 572    3D N = 9000 (18, 83, 3.5)  373 : 385
+  //   3D N = 100000 (24, 39, 0.2) 997 : 772     4D N = 6000 (23, 206, 5.1) 480 : 567
+  //   3D N = 9000 (18, 38, 1.7)   242 : 191     4D N = 5000 (20, 217, 0.7) 177 : 229
+  //   5D N = 20000 (20, 199, 0.3) 789 : 675     4D N = 40000 (9.8, 128, 1.0) 713 : 736
+  int64_t lrows = 0, lsegs = 0, lpanels = 0, lz = 0, lnear = 0;
   for (const Panel& P : h.panels_far)
     if (P.m <= 32) {
       lrows += P.m;
       lsegs += P.seg_end - P.seg_begin;
       lpanels++;
     }
-  const bool leaf = lrows > 6 * lpanels && lrows <= 26 * lpanels && lsegs >= 32 * lpanels;
+#pragma omp parallel for schedule(static) reduction(+ : lz) num_threads(par_threads(int64_t(op->far.size())))
+  for (int64_t q = 0; q < int64_t(op->far.size()); q++)
+    if (!op->dense[size_t(q)] && t.count[size_t(t.gid(op->far[size_t(q)].level, op->far[size_t(q)].t))] <= 32)
+      lz += op->rank[size_t(q)];
+  for (const Panel& P : h.panels_near)
+    for (int64_t q = P.seg_begin; P.m <= 32 && q < P.seg_end; q++)
+      lnear += int64_t((P.m + 7) / 8) * ((h.segs_near[size_t(q)].K + 7) / 8);
+  const bool many = lsegs >= 150 * lpanels;
+  const bool pays = lsegs >= 32 * lpanels && lrows > (many ? 6 : 7) * lpanels && lrows <= 26 * lpanels &&
+                    (2 * lrows <= 33 * lpanels || 10 * lz >= (many ? 6 : 21) * lnear);
+  const bool leaf = T.force_leaf ? T.force_leaf == 1 && lpanels > 0 : lpanels > 0 && pays;
   tc_panel_items(h.panels_near, h.segs_near, ni, T.near, fxn, pn, leaf ? 32 : 0);
   tc_panel_items(h.panels_far, h.segs_far, fi, T.far, fxf, pf, leaf ? 32 : 0);
   // panels of at most 32 rows: their segments, and the groups' work
-  const Tree& t = op->tree;
   TcLeafHost H(op->n);
   std::vector<TcLeafSeg> lns(h.segs_near.size()), lfs(h.segs_far.size());
   std::vector<int64_t> ons(h.segs_near.size()), ofs(h.segs_far.size());
@@ -2749,19 +2765,21 @@ void build_tc_plan(hodlr_op* op, cudaStream_t st) {
       zg.push_back(g);
     }
   }
-  // groups over more than kTcZCols points: column runs writing partial sums,
-  // added into z (and scaled) by a fix-up
+  // groups over more than about kTcZCols points: column runs of about that many
+  // each (whole 32-column steps) writing partial sums, added into z (and scaled)
+  // by a fix-up
   std::vector<TcZFix> zfix;
   std::vector<TcZRow> zrows;
   int zparts = 0;
   {
     std::vector<TcZGroup> split;
     for (const TcZGroup& g : zg) {
-      if (g.n <= kTcZCols) {
+      const int parts = (g.n + kTcZCols / 2) / kTcZCols;  // rounded
+      if (parts <= 1) {
         split.push_back(g);
         continue;
       }
-      const int runs = (g.n + kTcZCols - 1) / kTcZCols;
+      const int cols = ((g.n + parts - 1) / parts + 31) / 32 * 32, runs = (g.n + cols - 1) / cols;
       zfix.push_back({zparts, runs, g.rows, int32_t(zrows.size())});
       T.zfix_rows = std::max(T.zfix_rows, g.rows);
       for (int32_t e = g.e_begin; e < g.e_end; e++) {
@@ -2771,9 +2789,9 @@ void build_tc_plan(hodlr_op* op, cudaStream_t st) {
       }
       for (int c = 0; c < runs; c++) {
         TcZGroup r = g;
-        r.x_off = g.x_off + int64_t(c) * kTcZCols;
-        r.col0 = c * kTcZCols;
-        r.n = std::min(kTcZCols, g.n - c * kTcZCols);
+        r.x_off = g.x_off + int64_t(c) * cols;
+        r.col0 = c * cols;
+        r.n = std::min(cols, g.n - c * cols);
         r.part = zparts++;
         split.push_back(r);
       }
@@ -3141,6 +3159,10 @@ int hodlr_test_option(hodlr_op* op, int32_t option, int64_t value) {
     case HODLR_TEST_TC_DROP_RELEASE:
       op->tc.drop_release = value < 0 ? -1 : int32_t(std::min<int64_t>(value, 1 << 30));
       return HODLR_OK;
+    case HODLR_TEST_TC_LEAF:
+      if (op->tc.built) return fail(op->ctx, HODLR_ERR_STATE, "hodlr_test_option: the tensor-core plan is built");
+      op->tc.force_leaf = value < 0 ? 0 : value != 0 ? 1 : 2;
+      return HODLR_OK;
     case HODLR_TEST_STEP_WAIT_NS: {
       const uint64_t ns = value < 0 ? kBarrierNs : std::min(uint64_t(value), kBarrierNs);
       op->g64.step_wait_ns = op->g32.step_wait_ns = ns;
@@ -3154,6 +3176,9 @@ int hodlr_test_option(hodlr_op* op, int32_t option, int64_t value) {
 int hodlr_test_value(const hodlr_op* op, int32_t what, int64_t* value) {
   if (!op || !value) return fail(nullptr, HODLR_ERR_INVALID, "hodlr_test_value: null argument");
   switch (what) {
+    case HODLR_TEST_TC_LEAF_RUNS:
+      *value = op->tc.nleaf_runs;
+      return HODLR_OK;
     case HODLR_TEST_STEPS:
       *value = op->g64.steps + op->g32.steps;
       return HODLR_OK;

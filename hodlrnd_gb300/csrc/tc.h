@@ -44,17 +44,19 @@ struct TcZEntry {
 };
 struct TcZGroup {
   int64_t x_off;   // first point of the group's columns (of the source node)
-  int32_t n;       // columns: all points of the source node, or a run of at most kTcZCols of them
+  int32_t n;       // columns: all points of the source node, or a run of about kTcZCols of them
   int32_t e_begin, e_end;  // entries
   int32_t rows;    // sum of nk
   int32_t part;    // < 0: the group writes z; else its partial sums go to part block `part` (a fix-up adds them)
   int32_t col0;    // the first column's point within the source node (its row of V): 0 unless a column run
 };
-// (512: with 256, the leaves' parents of 4D N = 65536, 256 points on average,
-// were split half the time, and adding their partial sums took 278 us.)
-// A source node with more points than kTcZCols is split into column runs
-// whose partial sums (blocks of kTcRows rows x 64) a fix-up adds into z.
-constexpr int kTcZCols = 512;
+// A source node with more points than about kTcZCols is split into column runs
+// whose partial sums (blocks of kTcRows rows x 64) a fix-up adds into z.  A CTA
+// works through its run step by step, so long runs leave SMs idle (runs of 512
+// instead of 256: 3D N = 30000 725 -> 874 us, 2D N = 18000 159 -> 176); but a node just
+// above the limit is not worth two (4D N = 65536, whose leaves' parents have 256
+// points on average: half of them split took 3.94 ms, none 3.55).
+constexpr int kTcZCols = 256;
 struct TcZRow {        // row i of a split group: where its z goes
   int64_t zpos;
   const float* zscale;  // the row's z scale (BF16), or null

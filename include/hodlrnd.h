@@ -344,13 +344,15 @@ enum {
   HODLR_TEST_TC_WAIT_NS = 0,     /* longest wait of the leaf-level tensor-core kernel, ns (at most the default) */
   HODLR_TEST_TC_DROP_COPIES = 1, /* its runs leave out the copies of this batch */
   HODLR_TEST_TC_DROP_RELEASE = 2, /* one warp of its runs does not hand this batch's stage back */
-  HODLR_TEST_STEP_WAIT_NS = 3     /* longest wait of a one-launch CGS2 step for its CTAs, ns (at most the default) */
+  HODLR_TEST_STEP_WAIT_NS = 3,    /* longest wait of a one-launch CGS2 step for its CTAs, ns (at most the default) */
+  HODLR_TEST_TC_LEAF = 4          /* leaf-level tensor-core kernel always (1) or never (0); before the first product */
 };
 int hodlr_test_option(hodlr_op* op, int32_t option, int64_t value);
 /* Which path an operator's calls have taken so far. */
 enum {
-  HODLR_TEST_STEPS = 0,        /* Arnoldi steps by the step kernels */
-  HODLR_TEST_STEP_GIVE_UPS = 1 /* of them: steps whose wait ran out, done again phase by phase */
+  HODLR_TEST_STEPS = 0,         /* Arnoldi steps by the step kernels */
+  HODLR_TEST_STEP_GIVE_UPS = 1, /* of them: steps whose wait ran out, done again phase by phase */
+  HODLR_TEST_TC_LEAF_RUNS = 2   /* runs of the leaf-level tensor-core kernel in a product (0: not taken) */
 };
 int hodlr_test_value(const hodlr_op* op, int32_t what, int64_t* value);
 
