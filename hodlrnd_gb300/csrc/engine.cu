@@ -181,6 +181,8 @@ struct Plan {
   unsigned int *zcnt = nullptr, *pcnt_far = nullptr, *pcnt_near = nullptr;
   // small items stream their segments as one byte run (small_items_contiguous)
   bool contig_near = false, contig_far = false;
+  Item* plain_far = nullptr;  // PanelItems::plain
+  int nplain_far = 0;
   int64_t nzpart = 0, nypart = 0;  // partial-sum scratch (elements of the vector type)
   void* zpart = nullptr;
   void* ypart = nullptr;
@@ -193,7 +195,7 @@ struct Plan {
     int64_t nypart_near = 0, nzpart = 0;
     std::vector<Panel> panels_near, panels_far;
     std::vector<Seg> segs_near, segs_far;
-    std::vector<Item> small_near, big_near, small_far, big_far;
+    std::vector<Item> small_near, big_near, small_far, big_far, plain_far;
     std::vector<PanelFix> pfix_near, pfix_far;
     std::vector<ZBlock> zb;
     std::vector<ZItem> zitems;
@@ -202,10 +204,11 @@ struct Plan {
   std::shared_ptr<Host> host;
   PanelItems near_items() const {
     return {panels_near, segs_near, small_near, big_near, nsmall_near, nbig_near, pfix_near, npfix_near,
-            pcnt_near};
+            pcnt_near, nullptr, 0};
   }
   PanelItems far_items() const {
-    return {panels_far, segs_far, small_far, big_far, nsmall_far, nbig_far, pfix_far, npfix_far, pcnt_far};
+    return {panels_far, segs_far, small_far, big_far, nsmall_far, nbig_far, pfix_far, npfix_far, pcnt_far,
+            plain_far, nplain_far};
   }
 };
 
@@ -661,11 +664,32 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
   // kernel, whose results do not depend on the layout.  FP32 and BF16 factors
   // are laid out in panel order (relayout_far).
   auto contig = [&](const PanelList& L) { return a != Prec::kD && small_items_contiguous(panels, segs, L.small, prec_size(a)); };
+  // FP64 leaf panels: plain loads with few registers (twice the warps of
+  // launch_items64's kernel on an SM) where it is the segments that take time, many
+  // of them and tiny; elsewhere their items go with the larger panels'.  us a
+  // product, plain against not (rows a panel, segments a panel, segments in all):
+  //   3D N = 60000 (1, 18, 4.7M)  937 : 1045    5D N = 6526 (6.4, 897, 0.9M) 469 : 575
+  //   4D N = 20000 (4.9, 504, 2M) 830 : 885     5D N = 10000 (9.8, 902, 0.9M) 841 : 880
+  //   3D N = 20000 (4.9, 116, 0.5M) 326 : 274   4D N = 40000 (9.8, 509, 2M) 1953 : 1912
+  //   3D N = 5000 (1.2, 65, 0.3M) 116 : 102     3D N = 200000 (6.1, 133, 4.4M) 3266 : 3157
+  //   3D N = 100000 (5.4, 123, 4M) 1386 : 1430
+  int64_t lrows = 0, lsegs = 0, lpanels = 0;
+  for (const Panel& p : panels)
+    if (p.m <= 32) {
+      lrows += p.m;
+      lsegs += p.seg_end - p.seg_begin;
+      lpanels++;
+    }
+  std::vector<Item> plain;
+  if (a == Prec::kD && lsegs >= (int64_t(1) << 19) && (2 * lrows <= 11 * lpanels || lsegs >= 600 * lpanels))
+    plain.swap(own.small);
   plan.contig_far = contig(own);
   plan.panels_far = upload(op->mem, panels, st, "far panels");
   plan.segs_far = upload(op->mem, segs, st, "far segments");
   plan.small_far = upload(op->mem, own.small, st, "far items");
   plan.big_far = upload(op->mem, own.big, st, "far items");
+  plan.plain_far = upload(op->mem, plain, st, "far items");
+  plan.nplain_far = int(plain.size());
   plan.nsmall_far = int(own.small.size());
   plan.nbig_far = int(own.big.size());
   // V^T x items: up to 32 sixteen-byte loads of columns by a run of rows of
@@ -726,6 +750,7 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
     h.big_far = L.big;
     h.pfix_far = L.fix;
     h.contig_far = contig(L);
+    h.plain_far = plain;
     h.zb = zb;
     const ZList& HZ = m ? z_list(kBatchItemBytes) : Z;
     h.zitems = HZ.items;
@@ -1540,7 +1565,7 @@ cudaError_t apply_tree(hodlr_op* op, const Plan& plan, const T* x, T* y, T* in, 
       return e;
     tr.stop(st);
   }
-  const bool far = plan.nsmall_far + plan.nbig_far > 0;
+  const bool far = plan.nsmall_far + plan.nbig_far + plan.nplain_far > 0;
   if (far) tr.start(kb + 2, st);
   if ((e = launch_panels(plan.a_far, px, plan.far_items(), plan.ypart, fin, yslots, st, acc, plan.contig_far)) !=
       cudaSuccess)
@@ -2149,7 +2174,7 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
   // the instances), then the records themselves, instances in parallel
   struct Base {
     int64_t panels_near = 0, segs_near = 0, small_near = 0, big_near = 0, pfix_near = 0, near_parts = 0;
-    int64_t panels_far = 0, segs_far = 0, small_far = 0, big_far = 0, pfix_far = 0, far_parts = 0;
+    int64_t panels_far = 0, segs_far = 0, small_far = 0, big_far = 0, plain_far = 0, pfix_far = 0, far_parts = 0;
     int64_t zb = 0, zitems = 0, zfix = 0, zpart = 0, in = 0, y = 0, x = 0;
   };
   std::vector<Base> base(nops + 1);
@@ -2187,6 +2212,7 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
     e.segs_far = a.segs_far + int64_t(hf.segs_far.size());
     e.small_far = a.small_far + int64_t(hf.small_far.size());
     e.big_far = a.big_far + int64_t(hf.big_far.size());
+    e.plain_far = a.plain_far + int64_t(hf.plain_far.size());
     e.pfix_far = a.pfix_far + int64_t(hf.pfix_far.size());
     int64_t op_far_parts = 0;
     for (const PanelFix& f : hf.pfix_far) op_far_parts += f.count;
@@ -2215,6 +2241,7 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
   h.segs_far.resize(size_t(tot.segs_far));
   h.small_far.resize(size_t(tot.small_far));
   h.big_far.resize(size_t(tot.big_far));
+  h.plain_far.resize(size_t(tot.plain_far));
   h.pfix_far.resize(size_t(tot.pfix_far));
   h.zb.resize(size_t(tot.zb));
   h.zitems.resize(size_t(tot.zitems));
@@ -2277,6 +2304,8 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
       h.small_far[size_t(a.small_far) + k] = shift_item(hf.small_far[k], a.panels_far, a.segs_far, a.far_parts, a.pfix_far);
     for (size_t k = 0; k < hf.big_far.size(); k++)
       h.big_far[size_t(a.big_far) + k] = shift_item(hf.big_far[k], a.panels_far, a.segs_far, a.far_parts, a.pfix_far);
+    for (size_t k = 0; k < hf.plain_far.size(); k++)
+      h.plain_far[size_t(a.plain_far) + k] = shift_item(hf.plain_far[k], a.panels_far, a.segs_far, a.far_parts, a.pfix_far);
     for (size_t k = 0; k < hf.pfix_far.size(); k++) {
       PanelFix f = hf.pfix_far[k];
       f.panel += int32_t(a.panels_far);
@@ -2333,6 +2362,8 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
   p.big_far = upload(b.mem, h.big_far, st, "batch far items");
   p.nsmall_far = int(h.small_far.size());
   p.nbig_far = int(h.big_far.size());
+  p.plain_far = upload(b.mem, h.plain_far, st, "batch far items");
+  p.nplain_far = int(h.plain_far.size());
   p.pfix_far = upload(b.mem, h.pfix_far, st, "batch far fix-ups");
   p.npfix_far = int(h.pfix_far.size());
   p.zb = upload(b.mem, h.zb, st, "batch z blocks");

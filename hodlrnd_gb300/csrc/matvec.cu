@@ -1557,6 +1557,49 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) items64_kernel(const Ite
     panel_fixup(a.L.fix, a.L.pcnt, fix, a.ypart, out, rows, lane);
 }
 
+// Leaf panels of many tiny segments (PanelItems::plain), which latency bounds:
+// slices of mpad lanes (the next power of two of the rows), a segment for each
+// slice and a row for each lane, in so few registers that an SM holds twice the
+// warps of items64_kernel.
+__global__ void __launch_bounds__(kWarpsPerCta * 32)
+    panel_small64_kernel(const PanelItems L, const double* __restrict__ in, double* __restrict__ ypart,
+                         double* __restrict__ y) {
+  const int w = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (w >= L.nplain) return;
+  const Item it = L.plain[w];
+  const Panel P = L.panels[it.panel];
+  const int m = P.m;
+  int mpad = 1;
+  while (mpad < m) mpad <<= 1;
+  const int slices = 32 / mpad;
+  const int i = lane & (mpad - 1), sl = lane / mpad;
+  double a0 = 0.0, a1 = 0.0;
+  if (i < m) {
+    for (int64_t s = it.seg_b + sl; s < it.seg_e; s += slices) {
+      const Seg S = L.segs[s];
+      const double* A = static_cast<const double*>(S.A) + i;
+      const double* x = in + S.in_off;
+      int j = 0;
+      for (; j + 3 < S.K; j += 4) {
+        const double v0 = __ldg(A + int64_t(j) * m), v1 = __ldg(A + int64_t(j + 1) * m);
+        const double v2 = __ldg(A + int64_t(j + 2) * m), v3 = __ldg(A + int64_t(j + 3) * m);
+        const double x0 = x[j], x1 = x[j + 1], x2 = x[j + 2], x3 = x[j + 3];
+        a0 += v0 * x0;
+        a1 += v1 * x1;
+        a0 += v2 * x2;
+        a1 += v3 * x3;
+      }
+      for (; j < S.K; j++) a0 += __ldg(A + int64_t(j) * m) * x[j];
+    }
+  }
+  double acc = a0 + a1;
+  for (int o = mpad; o < 32; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  double* out = y + P.yoff;
+  if (sl == 0 && i < m) (it.part < 0 ? out : ypart + int64_t(it.part) * 64)[i] = acc;
+  if (it.part >= 0) panel_fixup(L.fix, L.pcnt, it.fix, ypart, out, m, lane);
+}
+
 template <typename TX, typename TO>
 __global__ void combine_kernel(const TX* __restrict__ y, int64_t ld_y, int nslots, int64_t n,
                                const int64_t* __restrict__ perm, TO* __restrict__ out, int64_t ld_out) {
@@ -1743,6 +1786,10 @@ cudaError_t launch_items64(const ZBlock* zb, const ZItem* zitems, int nitems, co
     count_launches(1);
     items64_kernel<<<warps_grid(total), kWarpsPerCta * 32, 0, st>>>(a);
   }
+  if (L.nplain > 0) {
+    count_launches(1);
+    panel_small64_kernel<<<warps_grid(L.nplain), kWarpsPerCta * 32, 0, st>>>(L, in, ypart, y);
+  }
   if (contig && L.nsmall > 0) {
     count_launches(1);
     constexpr int bytes = kLWarps * l_warp_smem<double, double>();
@@ -1830,7 +1877,7 @@ bool small_items_contiguous(const std::vector<Panel>& panels, const std::vector<
 
 cudaError_t launch_panels(Prec a, Prec x, const PanelItems& L, void* ypart, const void* in, void* y, cudaStream_t st,
                           Accum acc, bool contig) {
-  if (L.nsmall + L.nbig <= 0) return cudaSuccess;
+  if (L.nsmall + L.nbig + L.nplain <= 0) return cudaSuccess;
   if (a == Prec::kD && x == Prec::kD)
     return launch_items64(nullptr, nullptr, 0, nullptr, nullptr, nullptr, L, static_cast<double*>(ypart),
                           static_cast<double*>(const_cast<void*>(in)), static_cast<double*>(y), st, contig);

@@ -188,6 +188,9 @@ struct PanelItems {
   const PanelFix* fix;
   int nfix;
   unsigned int* pcnt;
+  // FP64: small items of many tiny segments, which take a kernel of their own
+  const Item* plain;
+  int nplain;
 };
 cudaError_t launch_panels(Prec a, Prec x, const PanelItems& L, void* ypart, const void* in, void* y, cudaStream_t st,
                           Accum acc = Accum::kByType, bool contig = false);
