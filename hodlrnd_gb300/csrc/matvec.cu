@@ -1495,7 +1495,7 @@ __device__ __forceinline__ void item64(const Seg* __restrict__ segs, int32_t sb,
 
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) items64_kernel(const Items64 a) {
   const int lane = threadIdx.x & 31;
-  int w = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
+  int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   int rows, part, fix;
   int32_t sb = 0, se = 0;
   int64_t tile_off = 0, ld, zx = 0;
@@ -1784,7 +1784,10 @@ cudaError_t launch_items64(const ZBlock* zb, const ZItem* zitems, int nitems, co
   const int64_t total = int64_t(nitems) + a.L.nsmall + L.nbig;
   if (total > 0) {
     count_launches(1);
-    items64_kernel<<<warps_grid(total), kWarpsPerCta * 32, 0, st>>>(a);
+    // as few warps a CTA as fill the SMs: items on one SM share its FP64 pipe
+    int warps = 1;
+    while (warps < kWarpsPerCta && total > 152 * warps) warps *= 2;
+    items64_kernel<<<unsigned((total + warps - 1) / warps), unsigned(warps * 32), 0, st>>>(a);
   }
   if (L.nplain > 0) {
     count_launches(1);
