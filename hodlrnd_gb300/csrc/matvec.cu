@@ -796,12 +796,21 @@ constexpr int kLStages = HODLR_TUNE_L_STAGES;
 // columns are half as long, and with smaller stages a sixth CTA fits (4D N =
 // 65536: 340 -> 315 us); FP32 and FP64 columns would fill them too early (3D N =
 // 262144 FP32: 344 -> 360 us)
+#ifndef HODLR_TUNE_L_BYTES  // 0: by type, as below
+#define HODLR_TUNE_L_BYTES 0
+#endif
+#ifndef HODLR_TUNE_L_COLS
+#define HODLR_TUNE_L_COLS 0
+#endif
+#ifndef HODLR_TUNE_L_MINB
+#define HODLR_TUNE_L_MINB 0
+#endif
 template <typename TA>
-inline constexpr int l_bytes = sizeof(TA) == 2 ? 3072 : 4096;
+inline constexpr int l_bytes = HODLR_TUNE_L_BYTES ? HODLR_TUNE_L_BYTES : sizeof(TA) == 2 ? 3072 : 4096;
 template <typename TA>
-inline constexpr int l_cols = sizeof(TA) == 2 ? 96 : 128;
+inline constexpr int l_cols = HODLR_TUNE_L_COLS ? HODLR_TUNE_L_COLS : sizeof(TA) == 2 ? 96 : 128;
 template <typename TA>
-inline constexpr int l_minb = sizeof(TA) == 2 ? 6 : 5;
+inline constexpr int l_minb = HODLR_TUNE_L_MINB ? HODLR_TUNE_L_MINB : sizeof(TA) == 2 ? 6 : 5;
 constexpr int kLHead = 64;                        // barriers and stage descriptors
 static_assert(kLStages >= 2 && kLStages <= 4, "leaf ring: 2 to 4 stages");
 static_assert(32 + kLStages * 8 <= kLHead, "leaf ring header too small");
@@ -1162,8 +1171,11 @@ static_assert(kPWarpSmem % 16 == 0 && kPXBytes % 16 == 0, "bulk copy destination
 // CTAs per SM the register allocation must allow: a sixth (80 registers) helps
 // the four rows of a lane's FP32 load (3D N = 262144: 1020 -> 1001 us), not the
 // eight of a BF16 one, whose sums alone take 32 (4D N = 65536: 135 -> 143 us)
+#ifndef HODLR_TUNE_P_MINB  // 0: by type
+#define HODLR_TUNE_P_MINB 0
+#endif
 template <typename TA>
-inline constexpr int p_minb = sizeof(TA) == 2 ? 4 : 6;
+inline constexpr int p_minb = HODLR_TUNE_P_MINB ? HODLR_TUNE_P_MINB : sizeof(TA) == 2 ? 4 : 6;
 template <typename TA, typename TACC>
 __global__ void __launch_bounds__(kPWarps * 32, p_minb<TA>)
     panel_tile_kernel(const Panel* __restrict__ panels, const Seg* __restrict__ segs, const Item* __restrict__ items,

@@ -25,6 +25,7 @@ matvec.cu (a one-row leaf would get no columns per piece).
 import argparse
 import json
 import os
+import re
 import subprocess
 import sys
 
@@ -43,7 +44,19 @@ DEFAULT_VARIANTS = {
 TUNED_SOURCES = ("matvec.cu", "engine.cu")
 
 
+def macros():
+    """The names a variant can override: those the sources read."""
+    names = set()
+    for f in TUNED_SOURCES + ("matvec.h",):
+        with open(os.path.join(B.CSRC, f)) as h:
+            names |= set(re.findall(r"#ifndef HODLR_TUNE_(\w+)", h.read()))
+    return names
+
+
 def _variant_lib(name, overrides):
+    unknown = sorted(set(overrides) - macros())
+    if unknown:
+        raise ValueError(f"variant {name}: unknown macros {', '.join(unknown)}")
     tdir = os.path.join(B.HERE, "_tune")
     os.makedirs(tdir, exist_ok=True)
     tag = "".join(c if c.isalnum() else "_" for c in name)
