@@ -49,6 +49,7 @@
 
 #include <type_traits>
 
+#include "cluster.cuh"
 #include "device.cuh"
 
 namespace hodlr {
@@ -89,34 +90,16 @@ struct ClusterTeam {
   Cta cta;
   ClusterShared* sh;
   mutable int slot = 0;  // the same in every thread
-  __device__ static uint32_t rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-  }
-  // address of *p in CTA c's shared memory
-  __device__ static uint32_t at(const void* p, int c) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-                 : "=r"(r)
-                 : "r"(uint32_t(__cvta_generic_to_shared(p))), "r"(uint32_t(c)));
-    return r;
-  }
-  __device__ static void store(uint32_t addr, unsigned long long v) {
-    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
-  }
+  __device__ static uint32_t rank() { return cluster_rank(); }
   __device__ int tid() const { return int(((threadIdx.x >> 5) * kClusterCtas + rank()) * 32 + (threadIdx.x & 31)); }
-  __device__ void sync() const {
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-  }
+  __device__ void sync() const { cluster_barrier(); }
   // each CTA's own sums (its threads hold the partial sums of a CTA team's)
   __device__ void sum2(double& a, double& b) const { cta.sum2(a, b); }
   __device__ void argmax(unsigned long long& k, int& i) const {
     cta.argmax(k, i);
     if (threadIdx.x < kClusterCtas) {
-      store(at(&sh->key[slot][rank()], threadIdx.x), k);
-      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at(&sh->idx[slot][rank()], threadIdx.x)), "r"(i) : "memory");
+      cluster_store(cluster_addr(&sh->key[slot][rank()], threadIdx.x), k);
+      cluster_store(cluster_addr(&sh->idx[slot][rank()], threadIdx.x), i);
     }
     sync();
     for (int c = 0; c < kClusterCtas; c++)
@@ -130,7 +113,7 @@ struct ClusterTeam {
   __device__ double bcast(double v) const {
     if (rank() == 0) {
       v = __shfl_sync(0xffffffffu, v, 0);
-      if (threadIdx.x < kClusterCtas) store(at(&sh->value[slot], threadIdx.x), (unsigned long long)__double_as_longlong(v));
+      if (threadIdx.x < kClusterCtas) cluster_store(cluster_addr(&sh->value[slot], threadIdx.x), v);
     }
     sync();
     v = sh->value[slot];
@@ -140,7 +123,7 @@ struct ClusterTeam {
   __device__ int bcast(int v) const { return int(bcast(double(v))); }
   __device__ void put_term(int k, double v) const {
     const int lane = threadIdx.x & 31;
-    if (lane < kClusterCtas) store(at(cta.terms + k, lane), (unsigned long long)__double_as_longlong(v));
+    if (lane < kClusterCtas) cluster_store(cluster_addr(cta.terms + k, lane), v);
   }
   __device__ double term(int k) const { return cta.terms[k]; }
 };

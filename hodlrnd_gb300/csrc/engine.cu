@@ -177,7 +177,7 @@ struct Plan {
   PanelFix* pfix_near = nullptr;  // near panels split over items (share ypart with the far ones)
   int npfix_near = 0;
   int64_t nypart_near = 0;
-  // counters of the fixes (zero between launches)
+  // counters of the FP64 items' fixes (zero between launches)
   unsigned int *zcnt = nullptr, *pcnt_far = nullptr, *pcnt_near = nullptr;
   // small items stream their segments as one byte run (small_items_contiguous)
   bool contig_near = false, contig_far = false;
@@ -537,7 +537,7 @@ void build_near_plan(hodlr_op* op, const NearTiles& nt, const void* base, Prec a
   plan.contig_near = small_items_contiguous(panels, segs, own.small, int(esz));
   plan.pfix_near = upload(op->mem, own.fix, st, "near panel fix-ups");
   plan.npfix_near = int(own.fix.size());
-  plan.pcnt_near = fix_counters(op->mem, own.fix.size(), st);
+  if (a == Prec::kD) plan.pcnt_near = fix_counters(op->mem, own.fix.size(), st);
   plan.nypart_near = own.nypart * rows_per_item(a);
   plan.a_near = a;
   plan.panels_near = upload(op->mem, panels, st, "near panels");
@@ -735,8 +735,10 @@ void build_far_plan(hodlr_op* op, const std::vector<const void*>& uptr, const st
   plan.nzfix = int(Z.fix.size());
   plan.pfix_far = upload(op->mem, own.fix, st, "far panel fix-ups");
   plan.npfix_far = int(own.fix.size());
-  plan.zcnt = fix_counters(op->mem, Z.fix.size(), st);
-  plan.pcnt_far = fix_counters(op->mem, own.fix.size(), st);
+  if (a == Prec::kD) {
+    plan.zcnt = fix_counters(op->mem, Z.fix.size(), st);
+    plan.pcnt_far = fix_counters(op->mem, own.fix.size(), st);
+  }
   plan.nzpart = Z.nzpart;
   plan.nypart = own.nypart * rows_per_item(a);
   if (op->keep_host_plans) {
@@ -2049,8 +2051,6 @@ void build_finish(hodlr_op* op, BuildState& bs, cudaStream_t st) {
     op->plan32.nzfix = op->plan64.nzfix;
     op->plan32.pfix_far = op->plan64.pfix_far;
     op->plan32.npfix_far = op->plan64.npfix_far;
-    op->plan32.zcnt = op->plan64.zcnt;
-    op->plan32.pcnt_far = op->plan64.pcnt_far;
     op->plan32.nzpart = op->plan64.nzpart;
     op->plan32.nypart = std::max(op->plan64.nypart, op->plan32.nypart_near);
     op->plan32.zpart = op->mem.alloc(size_t(std::max<int64_t>(op->plan32.nzpart, 1)) * 4, "z partial sums (FP32)");
@@ -2372,9 +2372,11 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
   p.nzitems = int(h.zitems.size());
   p.zfix = upload(b.mem, h.zfix, st, "batch z fix-ups");
   p.nzfix = int(h.zfix.size());
-  p.zcnt = fix_counters(b.mem, h.zfix.size(), st);
-  p.pcnt_near = fix_counters(b.mem, h.pfix_near.size(), st);
-  p.pcnt_far = fix_counters(b.mem, h.pfix_far.size(), st);
+  if (p.a_near == Prec::kD) p.pcnt_near = fix_counters(b.mem, h.pfix_near.size(), st);
+  if (p.a_far == Prec::kD) {
+    p.zcnt = fix_counters(b.mem, h.zfix.size(), st);
+    p.pcnt_far = fix_counters(b.mem, h.pfix_far.size(), st);
+  }
   const size_t vsz = f32 ? 4 : 8;
   p.nzpart = zpart;
   p.nypart = std::max(near_parts * rows_per_item(p.a_near), far_parts * rows_per_item(p.a_far));
@@ -2456,8 +2458,9 @@ int tc_bucket(int rows) {
   return b;
 }
 
-// Items of the tcgen05 panel kernels for one family of panels, those above 32
-// rows: per panel, its 64-row chunks times runs of whole segments of at most
+// Items of the tcgen05 panel kernels for one family of panels, those of more than
+// `above` rows (32 where the leaf-level kernel takes the others, else 0): per
+// panel, its 64-row chunks times runs of whole segments of at most
 // kTcColsPerItem columns (a longer segment alone) and at most kTcMaxSegs
 // segments -- a CTA works through an item's columns one 32-column step after
 // another, so long items would leave most SMs idle at the end of a launch.
@@ -2506,7 +2509,7 @@ void tc_panel_items(const std::vector<Panel>& panels, const std::vector<Seg>& se
 // group's sources in the order of their points, in batches, and runs of at most
 // kTcLeafRunSrcs sources -- enough CTAs for every SM to have several, few
 // partial blocks; of a small operator shorter runs, about kTcLeafRuns of them
-// 4D N = 12000: 1.62 -> 0.85 ms.  segs[q] of a panel has the source (first point src_off[q],
+// (4D N = 12000: 1.62 -> 0.85 ms).  segs[q] of a panel has the source (first point src_off[q],
 // segs[q].n points); a longer source than a batch holds is cut into pieces,
 // whose products add up.  out: the segments in batch order.
 constexpr int32_t kTcLeafRunSrcs = 160, kTcLeafRunSrcsMin = 4;

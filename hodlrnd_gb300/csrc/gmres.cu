@@ -1,4 +1,5 @@
 // Restarted GMRES on the device (see gmres.h).
+#include "cluster.cuh"
 #include "device.cuh"
 #include "fpsum.cuh"
 #include "gmres.h"
@@ -360,28 +361,6 @@ constexpr int kStepCtas = 16;
 constexpr int kStepEpt = 8;         // elements per thread at most
 constexpr int kStepThreads = 640;   // 8 CTAs x 640 x 8 = kStepMaxN
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// *p in CTA `cta`'s shared memory = v (p: the address in this CTA's)
-__device__ __forceinline__ void cluster_store(double* p, uint32_t cta, double v) {
-  const uint32_t a = uint32_t(__cvta_generic_to_shared(p));
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(cta));
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"(v) : "memory");
-}
-
 __host__ __device__ inline int64_t step_slice(int64_t n, int ctas) { return (n + ctas - 1) / ctas; }
 
 template <typename T>
@@ -426,7 +405,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) mgs_cluster_kernel(const Step
       for (int o = 16; o > 0; o >>= 1)
         if (o < nw) v += __shfl_xor_sync(0xffffffffu, v, o);
       v = __shfl_sync(0xffffffffu, v, 0);
-      if (lane < int(nc)) cluster_store(&slots[set][me], uint32_t(lane), v);
+      if (lane < int(nc)) cluster_store(cluster_addr(&slots[set][me], uint32_t(lane)), v);
     }
     cluster_barrier();
     if (wid == 0) {
@@ -800,52 +779,37 @@ cudaError_t launch_cgs_phases(StepArgs<T> a, bool redo, cudaStream_t st) {
 }
 
 // Update (GMRES.hpp:132-146): back substitution into y.
-// One CTA: thread j keeps y_j (Q of them, 1024 apart, for long restarts) and
-// subtracts column i of H times y_i as soon as y_i is known, the operations of
-// the serial loop in its order; the next column is loaded meanwhile.
+// One CTA: thread j keeps y_j and subtracts column i of H times y_i as soon as y_i
+// is known, the operations of the serial loop in its order; the next column is
+// loaded meanwhile.  k < kMaxBasis <= 1024.
 // 100 columns: 44 us against 428 for one thread (19: 14 us against 43).
-template <int Q>
+static_assert(kMaxBasis <= 1024, "a thread per column");
 __global__ void __launch_bounds__(1024) backsolve_kernel(const double* __restrict__ H, int ldh, double* rot, int restart,
                                                          int k) {
   __shared__ double yi[2];
   const double* s = rot + 2 * (restart + 1);
   double* y = rot + 3 * (restart + 1);
-  const int t = threadIdx.x;
-  double v[Q], hc[Q], hn[Q];
-#pragma unroll
-  for (int q = 0; q < Q; q++) {
-    const int j = t + q * 1024;
-    v[q] = j <= k ? s[j] : 0.0;
-    hc[q] = j <= k ? H[j + int64_t(k) * ldh] : 0.0;
-    hn[q] = 0.0;
-  }
+  const int j = threadIdx.x;
+  double v = j <= k ? s[j] : 0.0;
+  double hc = j <= k ? H[j + int64_t(k) * ldh] : 0.0, hn = 0.0;
   for (int i = k; i >= 0; i--) {
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-      const int j = t + q * 1024;
-      if (j < i) hn[q] = H[j + int64_t(i - 1) * ldh];
-      if (j == i) {
-        v[q] = v[q] / hc[q];
-        yi[i & 1] = v[q];
-        y[i] = v[q];
-      }
+    if (j < i) hn = H[j + int64_t(i - 1) * ldh];
+    if (j == i) {
+      v = v / hc;
+      yi[i & 1] = v;
+      y[i] = v;
     }
     __syncthreads();
-#pragma unroll
-    for (int q = 0; q < Q; q++)
-      if (t + q * 1024 < i) {
-        v[q] = __dsub_rn(v[q], __dmul_rn(hc[q], yi[i & 1]));
-        hc[q] = hn[q];
-      }
+    if (j < i) {
+      v = __dsub_rn(v, __dmul_rn(hc, yi[i & 1]));
+      hc = hn;
+    }
   }
 }
 
 void launch_backsolve(const double* H, int ldh, double* rot, int restart, int k, cudaStream_t st) {
   count_launches(1);
-  if (k < 1024)
-    backsolve_kernel<1><<<1, unsigned((k + 32) / 32 * 32), 0, st>>>(H, ldh, rot, restart, k);
-  else
-    backsolve_kernel<2><<<1, 1024, 0, st>>>(H, ldh, rot, restart, k);
+  backsolve_kernel<<<1, unsigned((k + 32) / 32 * 32), 0, st>>>(H, ldh, rot, restart, k);
 }
 
 // x += sum_j V_j y_j, accumulated j by j as the reference does.

@@ -21,19 +21,10 @@ namespace {
 
 constexpr int kWarpsPerCta = 8;
 
-template <typename T>
-__device__ __forceinline__ T ldg(const T* p) {
-  return __ldg(p);
-}
-
 // BF16 storage element (bits only; arithmetic converts to FP32)
 struct bf16 {
   unsigned short b;
 };
-template <>
-__device__ __forceinline__ bf16 ldg<bf16>(const bf16* p) {
-  return bf16{__ldg(reinterpret_cast<const unsigned short*>(p))};
-}
 __device__ __forceinline__ float bf2f(unsigned short b) { return __uint_as_float(uint32_t(b) << 16); }
 
 template <typename T>
@@ -45,10 +36,6 @@ struct Vec16<bf16> {
 template <>
 struct Vec16<float> {
   using type = float4;
-};
-template <>
-struct Vec16<double> {
-  using type = double2;
 };
 
 // Two FP32 operations in one instruction (packed pairs), each rounded to nearest
@@ -279,12 +266,6 @@ __device__ __forceinline__ void axpy16(const float4& a, X x, typename Acc<TACC>:
   fma_pair<TACC>(acc[2], acc[3], a.z, a.w, x, x);
 }
 template <typename TACC, typename X>
-__device__ __forceinline__ void axpy16(const double2& a, X x, typename Acc<TACC>::A* acc) {
-  Acc<TACC>::fma(acc[0], a.x, x);
-  Acc<TACC>::fma(acc[1], a.y, x);
-}
-
-template <typename TACC, typename X>
 __device__ __forceinline__ void axpy16(const uint4& a, X x, typename Acc<TACC>::A* acc) {
   fma_pair<TACC>(acc[0], acc[1], __uint_as_float(a.x << 16), __uint_as_float(a.x & 0xffff0000u), x, x);
   fma_pair<TACC>(acc[2], acc[3], __uint_as_float(a.y << 16), __uint_as_float(a.y & 0xffff0000u), x, x);
@@ -302,11 +283,6 @@ template <>
 __device__ __forceinline__ float4 vzero<float4>() {
   return make_float4(0.f, 0.f, 0.f, 0.f);
 }
-template <>
-__device__ __forceinline__ double2 vzero<double2>() {
-  return make_double2(0.0, 0.0);
-}
-
 // Input value of column j of a segment: x_j, times the column scale of a BF16
 // dense tile (cs non-null).
 template <typename TACC, typename TX>
@@ -614,10 +590,6 @@ static_assert(kSUBytes >= 2048 && kSUBytes % 16 == 0, "leaf-panel stage too smal
 static_assert(s_warp_smem<float>() % 16 == 0 && s_warp_smem<bf16>() % 16 == 0,
               "bulk copy destinations must stay 16-byte aligned");
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
 template <typename TA, typename TACC>
 __global__ void __launch_bounds__(kSWarps * 32, HODLR_TUNE_S_MINB)
     panel_small_kernel(const Panel* __restrict__ panels, const Seg* __restrict__ segs, const Item* __restrict__ items,
@@ -827,7 +799,6 @@ struct LeafX<FH> {
 // An input after scaling, in its staged form.
 __device__ __forceinline__ void put_staged(float2& d, DF x) { d = make_float2(x.hi, x.lo); }
 __device__ __forceinline__ void put_staged(float& d, float x) { d = x; }
-__device__ __forceinline__ void put_staged(double& d, double x) { d = x; }
 // stage: factor bytes | inputs (kCols x TX) | column offsets (kCols x u16) | BF16 scales (kCols x f32)
 template <typename TA, typename TX>
 __host__ __device__ constexpr int l_stage_smem() {

@@ -81,9 +81,9 @@ struct Item {
 };
 
 // Sum of `count` partial row blocks (parts part .. part+count-1) into the
-// output slot of rows chunk * rows_per_item .. of the panel.  The last of the
-// count items to finish adds them (a counter per fix, zero between launches),
-// so the sum needs no launch of its own; its order is the parts' order.
+// output slot of rows chunk * rows_per_item .. of the panel, in the parts' order:
+// by the last of the count FP64 items to finish (a counter per fix, zero between
+// launches), by a launch of its own in the other types.
 struct PanelFix {
   int32_t panel;
   int32_t chunk;
@@ -165,7 +165,7 @@ __host__ __device__ inline uint64_t far_v_bytes(int64_t n, int64_t r, bool dense
 // in:   input buffer [x | z]
 // y:    output slots (panel rows at P.yoff)
 // zpart / ypart: scratch of the vector precision.
-// zcnt / pcnt: one counter per fix, zero before and after a launch.
+// zcnt / pcnt: FP64 matrices and vectors: one counter per fix, zero before and after a launch.
 // acc, for FP32 matrices with FP64 vectors: the input buffer `in` holds each
 // FP64 value split into an (hi, lo) FP32 pair (launch_split), z is written in
 // the same form, outputs and partial sums stay FP64, and products are summed

@@ -72,7 +72,8 @@ HODLR_HD uint64_t mulhi64(uint64_t a, uint64_t b) {
 HODLR_HD uint32_t mulhi32(uint32_t a, uint32_t b) { return uint32_t((uint64_t(a) * b) >> 32); }
 
 // Single-precision seeds 1 / sqrt(f), f in [1, 4), and 1 / f, f in [1, 2), as
-// r 2^32 in (2^31, 2^32); anything within 2^-20 relative will do.
+// r 2^32 in (2^31, 2^32); anything within 2^-21 relative will do (CUDA's own are
+// within 2^-22).
 #ifndef HODLR_SOFT_SEED_NOISE
 #define HODLR_SOFT_SEED_NOISE(r) (r)
 #endif
@@ -157,7 +158,7 @@ HODLR_HD SoftRoot soft_root(uint64_t b) {
   const int64_t h = int64_t(0x4000000000000000ull - mulhi64(X, uint64_t(y0) * y0));  // 1 - X y^2
   const int64_t hq = h >> 20;
   const uint64_t h2 = uint64_t(hq * hq) >> 22;  // h^2 in units of 2^-62
-  // y (1 + h / 2 + 3 h^2 / 8); the next term, 5 h^3 / 16, is below 2^-61
+  // y (1 + h / 2 + 3 h^2 / 8); the next term, 5 h^3 / 16, is below 2^-61 (h below 2^-20)
   const uint64_t y = (uint64_t(y0) << 31) + uint64_t(soft_y_h(y0, h)) + ((uint64_t(y0) * (3u * uint32_t(h2))) >> 34);
   uint64_t S = mulhi64(X, y) >> 8;  // floor(sqrt(M 2^54)), at most one off
   const int64_t r = int64_t((M << 54) - S * S);

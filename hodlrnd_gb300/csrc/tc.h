@@ -30,14 +30,15 @@ constexpr int kTcMaxSegs = 256;  // segments of one panel item (the host splits 
 // kTcRows rows.
 constexpr int kTcRows = 64;
 
-// kind of product, for panels above 32 rows: z = V^T x, near-field panels (FP64
-// tiles), far-field panels (BF16 dense tiles and U factors).  Panels of at most
-// 32 rows, their low-rank blocks included, take the kernel of tcleaf.cu.
+// kind of product: z = V^T x, near-field panels (FP64 tiles), far-field panels
+// (BF16 dense tiles and U factors).  Panels of at most 32 rows, their low-rank
+// blocks included, take the kernel of tcleaf.cu instead where the plan's rule says
+// that it pays (build_tc_plan).
 enum TcKind { kTcZ = 0, kTcNear = 1, kTcFar = 2 };
 
 // z = V^T x for the low-rank blocks with one source node, grouped: the
 // group's rows are rows k0 .. k0 + nk - 1 of z_b for each of its entries
-// (at most 256 rows in all), and its columns the source node's points.
+// (at most kTcRows rows in all), and its columns the source node's points.
 struct TcZEntry {
   int32_t zb;      // index into the z blocks
   int32_t k0, nk;  // rows (columns of V) of z_b in this group

@@ -73,10 +73,6 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {  // BF16, rounde
 __device__ __forceinline__ float low_f(uint32_t p) { return __uint_as_float(p << 16); }
 __device__ __forceinline__ float high_f(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
 __device__ __forceinline__ uint32_t ldu16(const uint16_t* p) { return __ldg(p); }
-__device__ __forceinline__ void mbar_arrive_local(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
 // A stage: the sources' units, the batch's segment records, its header.  Shared
 // memory of a CTA: the stages' full and empty barriers, the stop flag, then the
 // stages.
@@ -340,7 +336,7 @@ __device__ __forceinline__ void leaf_run(const TcLeafArgs& a, const TcLeafRun& R
       }
     }
     __syncwarp();
-    if (lane == 0 && !(wid == 1 && b == a.drop_release)) mbar_arrive_local(empty + st);
+    if (lane == 0 && !(wid == 1 && b == a.drop_release)) mbar_arrive(empty + st);
     if (wid == 0 && b + kLeafStages < nb) {
       // refilled once every warp has left the stage
       if (!__all_sync(0xffffffffu, mbar_wait(empty + st, phase, a.wait_ns))) {
