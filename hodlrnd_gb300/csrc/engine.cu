@@ -2702,7 +2702,8 @@ void build_tc_plan(hodlr_op* op, cudaStream_t st) {
       lsegs += P.seg_end - P.seg_begin;
       lpanels++;
     }
-#pragma omp parallel for schedule(static) reduction(+ : lz) num_threads(par_threads(int64_t(op->far.size())))
+  // (a team of another size than the loops around it have costs 1 ms: few blocks alone)
+#pragma omp parallel for schedule(static) reduction(+ : lz) if (op->far.size() > size_t(1) << 19)
   for (int64_t q = 0; q < int64_t(op->far.size()); q++)
     if (!op->dense[size_t(q)] && t.count[size_t(t.gid(op->far[size_t(q)].level, op->far[size_t(q)].t))] <= 32)
       lz += op->rank[size_t(q)];

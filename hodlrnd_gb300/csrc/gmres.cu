@@ -512,12 +512,15 @@ __device__ __forceinline__ bool grid_barrier(unsigned long long* bar, uint64_t w
 // FP64.
 __device__ __forceinline__ double sum_step_parts(const float2* part, int G, int lane) {
   const int sub = lane & 7;
+  constexpr int Q = kStepGrid / 8;
+  float2 p[Q];
+#pragma unroll
+  for (int q = 0; q < Q; q++) p[q] = sub + 8 * q < G ? __ldcg(part + sub + 8 * q) : make_float2(0.f, 0.f);
   TripleSum a;
 #pragma unroll
-  for (int q = 0; q < kStepGrid / 8; q++) {
-    const int c = sub + 8 * q;
-    const float2 p = c < G ? __ldcg(part + c) : make_float2(0.f, 0.f);
-    a.add(p.x, p.y);
+  for (int q = 0; q < Q; q++) {
+    if (8 * q >= G) break;
+    a.add(p[q].x, p[q].y);
   }
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1)
