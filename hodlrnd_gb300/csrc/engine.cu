@@ -2134,6 +2134,7 @@ struct hodlr_batch {
   DevMem mem;
   Plan plan;
   int64_t ld_in = 0, ycol = 0, total_n = 0, max_n = 0;
+  int max_slots = 0;
   std::vector<int64_t> offsets;  // instance i: rows offsets[i] .. offsets[i+1] of the caller's vectors
   BatchInst* d_inst = nullptr;
   void* d_in = nullptr;   // [x | z] of every instance, vector type
@@ -2226,6 +2227,7 @@ void build_batch_plan(hodlr_batch& b, cudaStream_t st) {
     e.x = a.x + op->n;
     b.offsets.push_back(e.x);
     b.max_n = std::max(b.max_n, op->n);
+    b.max_slots = std::max(b.max_slots, int(op->nslots));
     // the merged items reference the same factor bytes, so their layout
     // test is each instance's own
     contig_near = contig_near && hn.contig_near;
@@ -2446,7 +2448,7 @@ void batch_apply_mr(hodlr_batch& b, const float* x, float* y, int64_t nrhs, cuda
                       p.npfix_near, b.d_ypart_mr, yld, b.d_in_mr, b.ld_in, b.d_y_mr, b.ycol, nch, st));
   CK(launch_panels_mr(p.panels_far, p.segs_far, p.small_far, p.nsmall_far, p.big_far, p.nbig_far, p.pfix_far,
                       p.npfix_far, b.d_ypart_mr, yld, b.d_in_mr, b.ld_in, b.d_y_mr, b.ycol, nch, st));
-  CK(launch_batch_combine_mr(b.d_inst, count, b.max_n, b.d_y_mr, b.ycol, y, b.total_n, int(nrhs), nch, st));
+  CK(launch_batch_combine_mr(b.d_inst, count, b.max_n, b.max_slots, b.d_y_mr, b.ycol, y, b.total_n, int(nrhs), nch, st));
 }
 
 // ---- tensor-core products for 64 right-hand sides ---------------------------

@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) mgs_cluster_kernel(const Step
 // of cgs_dots_kernel and cgs_update_kernel (dot2_add, pair_add, one FP64
 // subtraction per element and pass); the basis slices are split once into
 // shared memory where they fit and serve both passes from there.
-// n = 20011, 50 basis vectors: 36 us a step against 75 for the nine kernels; a
+// n = 20011, 50 basis vectors: 37 us a step against 75 for the nine kernels; a
 // cluster of 16 CTAs took 105 (its 16 SMs are bound by the splits and products).
 // When other work holds some SMs for longer than kBarrierNs, a barrier gives up,
 // and the step is done again in four launches that need no CTA beside another

@@ -2205,14 +2205,14 @@ __device__ __forceinline__ void mr_store(float* dst, int n, int lane, const floa
 
 // z_b = V_b^T X_s: item = rows [j0, j1) of block zb, columns [k0, k0 + nk) (at
 // most 128); runs of V rows and their input rows staged by bulk copies in a ring
-// of kMStages: one copy for a run of whole rows, one for each row when the item
-// has only some of a wider block's columns.
+// of kMStages: one copy for a run of whole rows (WHOLE), or one for each row of just
+// the item's columns.
 template <int NQ, bool WHOLE>
 __device__ __forceinline__ void zgemv_mr_item(const ZItem& it, const ZBlock& Z, const float* V, int64_t rp,
                                               const float* xr, float* dst, unsigned char* base, int lane) {
   uint64_t* bar = reinterpret_cast<uint64_t*>(base);
   unsigned char* stage0 = base + 64;
-  const int rowb = it.nk * 4;  // a multiple of 16, as k0 and rp
+  const int rowb = WHOLE ? int(rp) * 4 : it.nk * 4;  // a multiple of 16, as k0
   const int R = kMStageBytes / (rowb + kMRowBytes);  // rows per stage: their factors, then their inputs
   const int nrows = it.j1 - it.j0;
   const int total = (nrows + R - 1) / R;
@@ -2248,7 +2248,8 @@ __device__ __forceinline__ void zgemv_mr_item(const ZItem& it, const ZBlock& Z, 
       return;
     }
     const unsigned char* st = stage0 + s * kMStageBytes;
-    mr_wide<NQ>(st, rowb, reinterpret_cast<const float*>(st + R * rowb), min(R, nrows - q * R), lane, acc);
+    mr_wide<NQ>(st + (WHOLE ? it.k0 * 4 : 0), rowb, reinterpret_cast<const float*>(st + R * rowb),
+                min(R, nrows - q * R), lane, acc);
     __syncwarp();
     if (copies && q + kMStages < total) issue(q + kMStages);
   }
@@ -2278,7 +2279,12 @@ __global__ void __launch_bounds__(kMWarps * 32, 3)
     fence_mbar_init();
   }
   __syncwarp();
-  if (it.nk < rp) {
+  // just the item's columns where a stage does not hold two whole rows (rank above
+  // 928: 4D N = 40000, ranks up to 1227, 2.3 ms; whole rows read by plain loads
+  // instead took 7.0); below, the short copies of an item of few columns cost more
+  // than the rows' other columns (2D N = 6934, d' = 1, ranks about 130: 353 us
+  // against 191)
+  if (it.nk < rp && rp * 4 > kMStageBytes / 2) {
     zgemv_mr_item<4, false>(it, Z, V, rp, xr, dst, base, lane);
     return;
   }
@@ -2642,6 +2648,8 @@ __global__ void __launch_bounds__(256) batch_gather_mr_kernel(const BatchInst* _
 // by row in tree order, each value was a sector of its own: 313 us for 420,000
 // points against 60).  A row is the FP64 sum of its slots, formed on the FP32 pipe
 // where that gives the same value (fpsum.cuh; 20 us more than a plain FP32 pair).
+// Q rows of up to U slots are read before their sums (others one by one).
+template <int U, int Q>
 __global__ void __launch_bounds__(256) batch_combine_mr_kernel(const BatchInst* __restrict__ inst,
                                                                const float* __restrict__ y, int64_t ld_y,
                                                                float* __restrict__ out, int64_t total_n, int k, int ch) {
@@ -2650,24 +2658,26 @@ __global__ void __launch_bounds__(256) batch_combine_mr_kernel(const BatchInst* 
   const float* yc = y + int64_t(ch) * ld_y * kMR;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t stride = I.n * kMR;
-  const bool live = ch * kMR + lane < k, few = I.nslots <= 8;
+  const bool live = ch * kMR + lane < k, few = I.nslots <= U;
   for (int64_t p0 = int64_t(blockIdx.x) * 32; p0 < I.n; p0 += int64_t(gridDim.x) * 32) {
-    // four rows a warp: all their slots' loads first
-    const float* yr[4];
-    float v[4][8];
+#pragma unroll 1
+    for (int q0 = 0; q0 < 4; q0 += Q) {  // four rows a warp
+      const float* yr[Q];
+      float v[Q][U];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int64_t p = p0 + wid * 4 + q;
-      yr[q] = p < I.n && live ? yc + (I.y_base + I.iperm[p]) * kMR + lane : nullptr;
+      for (int q = 0; q < Q; q++) {
+        const int64_t p = p0 + wid * 4 + q0 + q;
+        yr[q] = p < I.n && live ? yc + (I.y_base + I.iperm[p]) * kMR + lane : nullptr;
 #pragma unroll
-      for (int s = 0; s < 8; s++) v[q][s] = yr[q] && few && s < I.nslots ? yr[q][s * stride] : 0.f;
-    }
+        for (int s = 0; s < U; s++) v[q][s] = yr[q] && few && s < I.nslots ? yr[q][s * stride] : 0.f;
+      }
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      float r = 0.f;
-      const bool ok = few && sum_few_as_fp64(I.nslots, v[q], r);
-      if (yr[q])
-        tile[wid * 4 + q][lane] = ok ? r : sum_as_fp64(I.nslots, [&](int s) { return yr[q][s * stride]; });
+      for (int q = 0; q < Q; q++) {
+        float r = 0.f;
+        const bool ok = few && sum_few_as_fp64(I.nslots, v[q], r);
+        if (yr[q])
+          tile[wid * 4 + q0 + q][lane] = ok ? r : sum_as_fp64(I.nslots, [&](int s) { return yr[q][s * stride]; });
+      }
     }
     __syncthreads();
 #pragma unroll
@@ -2741,12 +2751,17 @@ cudaError_t launch_invert_perm(const int64_t* perm, int64_t n, int32_t* iperm, c
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_combine_mr(const BatchInst* inst, int count, int64_t max_n, const float* y, int64_t ld_y,
-                                    float* out, int64_t total_n, int k, int nchunks, cudaStream_t st) {
+cudaError_t launch_batch_combine_mr(const BatchInst* inst, int count, int64_t max_n, int max_slots, const float* y,
+                                    int64_t ld_y, float* out, int64_t total_n, int k, int nchunks, cudaStream_t st) {
   if (count <= 0) return cudaSuccess;
+  const dim3 g(unsigned(std::min<int64_t>((max_n + 31) / 32, 2048)), unsigned(count));
   for (int ch = 0; ch < nchunks; ch++) {
     count_launches(1);
-    batch_combine_mr_kernel<<<dim3(unsigned(std::min<int64_t>((max_n + 31) / 32, 2048)), unsigned(count)), 256, 0, st>>>(inst, y, ld_y, out, total_n, k, ch);
+    // (deep trees: 1D N = 8104, three operators, 206 us with <8, 4>, 200 with <16, 2>)
+    if (max_slots <= 8)
+      batch_combine_mr_kernel<8, 4><<<g, 256, 0, st>>>(inst, y, ld_y, out, total_n, k, ch);
+    else
+      batch_combine_mr_kernel<16, 2><<<g, 256, 0, st>>>(inst, y, ld_y, out, total_n, k, ch);
   }
   return cudaGetLastError();
 }

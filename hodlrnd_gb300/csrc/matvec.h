@@ -255,8 +255,8 @@ cudaError_t launch_panels_mr(const Panel* panels, const Seg* segs, const Item* s
 // x, out: caller order, column major total_n x k (FP32); chunk ch holds columns ch*kMR ..
 cudaError_t launch_batch_gather_mr(const BatchInst* inst, int count, int64_t max_n, const float* x, int64_t total_n,
                                    int k, float* in, int64_t ld_in, int nchunks, cudaStream_t st);
-cudaError_t launch_batch_combine_mr(const BatchInst* inst, int count, int64_t max_n, const float* y, int64_t ld_y,
-                                    float* out, int64_t total_n, int k, int nchunks, cudaStream_t st);
+cudaError_t launch_batch_combine_mr(const BatchInst* inst, int count, int64_t max_n, int max_slots, const float* y,
+                                    int64_t ld_y, float* out, int64_t total_n, int k, int nchunks, cudaStream_t st);
 
 // out[i] = (hi, lo) FP32 pair of x[i] (hi = x rounded to FP32, lo = the rest)
 cudaError_t launch_split(const double* x, void* out, int64_t n, cudaStream_t st);

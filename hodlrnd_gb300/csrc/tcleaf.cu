@@ -20,8 +20,8 @@
 // staged in shared memory once for all of them by bulk copies (two stages), and
 // each warp applies its own segments of the batch, asking for the next one's
 // factors before it multiplies.
-// 4D N = 65536, 64 right-hand sides: 2.2 ms against 5.3 for these blocks through
-// the tcgen05 kernels (the whole product 7.28 -> 3.6 ms).  Of it 0.5 ms waits for
+// 4D N = 65536, 64 right-hand sides: 2.1 ms against 5.3 for these blocks through
+// the tcgen05 kernels (the whole product 7.28 -> 3.5 ms).  Of it 0.5 ms waits for
 // factor loads; the rest is instructions (43% of the issue slots) and the padding
 // of ranks, points and rows to 8.  Measured and not kept: sources read through L1
 // by each warp (3.2 ms), records fetched by each warp (2.8 ms), prefetching the
