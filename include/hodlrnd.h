@@ -326,7 +326,8 @@ int hodlr_aca_block_noalloc(const double* d_points, int64_t ld, int32_t ndim, co
  * BF16 far-field factors (HODLR_PREC_BF16_FACTORS), X and Y device arrays of
  * n x nrhs FP32, column major, caller's point order.  Blocks of 64 columns
  * go through tcgen05 MMAs (BF16 operands, FP32 accumulation in tensor
- * memory), leaf-level blocks through register MMAs: every right-hand side split once into BF16 high and low parts (to
+ * memory) and, where that is faster, the leaf-level blocks through register
+ * MMAs: every right-hand side split once into BF16 high and low parts (to
  * about 2^-17 relative), each BF16 factor entry times its input scale in two
  * BF16 terms, the FP64 near field in three -- the product differs from the
  * stored operator's single-RHS product by about 1e-5 relative, far below the
